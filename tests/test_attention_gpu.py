@@ -204,3 +204,64 @@ def test_config3_full_size_properties(L, api, port):
     assert normwise(got[:, :, :, :256], want_head) < H_TOL
     want_tail = port.sdpa(qf[:, :, :, -128:], kf, vf, causal=True)  # offset kv_len - q_len: the last 128 rows
     assert normwise(got[:, :, :, -128:], want_tail) < H_TOL
+
+
+# ------------------------------------------------------------------ fp32 products from bf16 planes (attn_split.cuh)
+def _exact(q, k, v, scale, seen=None, bias=None):
+    g = q.shape[1] // k.shape[1]
+    s = q.double() @ k.double().repeat_interleave(g, 1).transpose(-1, -2) * scale
+    s = s if bias is None else s + bias.double()
+    s = s if seen is None else s.masked_fill(~seen, float("-inf"))
+    return torch.softmax(s, -1) @ v.double().repeat_interleave(g, 1)
+
+
+@pytest.mark.parametrize("b,kvh,g,lq,lk,d,dt,form", [
+    (1, 1, 1, 64, 256, 128, "f32", "causal"), (1, 2, 2, 129, 257, 128, "f32", "causal"), (2, 2, 4, 33, 65, 64, "f32", "none"),
+    (1, 1, 1, 300, 513, 20, "f32", "causal"), (1, 2, 1, 127, 319, 80, "f32", "bool"), (1, 1, 3, 130, 256, 100, "f32", "bias"),
+    (1, 2, 2, 40, 40, 80, "bf16", "causal"), (1, 1, 2, 200, 129, 96, "f16", "none"), (150, 1, 1, 20, 33, 36, "bf16", "none"),
+    (1, 40, 2, 160, 270, 128, "f32", "causal")])
+def test_planes_against_64_bits(L, api, b, kvh, g, lq, lk, d, dt, form):
+    gen = torch.Generator(device="cuda").manual_seed(lq * 1000 + lk)
+    t = {"f32": torch.float32, "bf16": torch.bfloat16, "f16": torch.float16}[dt]
+    # a fused projection's layout: [batch, position, head, d] seen as [batch, head, position, d]
+    q, k, v = (torch.randn(b, n, h, d, generator=gen, device="cuda").to(t).transpose(1, 2)
+               for n, h in ((lq, kvh * g), (lk, kvh), (lk, kvh)))
+    seen = bias = None
+    if form == "causal":  # (more queries than keys is allowed: the first rows then see none)
+        seen = torch.arange(lk, device="cuda")[None] <= torch.arange(lk - lq, lk, device="cuda")[:, None]
+    elif form == "bool":
+        seen = torch.rand(lq, lk, generator=gen, device="cuda") < 0.6
+        seen[:, 3] = True
+    elif form == "bias":
+        bias = torch.randn(lq, lk, generator=gen, device="cuda")
+    got = api.scaledDotProductAttention(q, k, v, d ** -0.5, seen if form == "bool" else None, bias, causal=form == "causal")
+    want = _exact(q, k, v, d ** -0.5, seen, bias)
+    # fp32: a rounding per product and sum, far below 1e-6. 16 bits: the rounding of the result, in bf16 by the reference's
+    # rule (half a unit is added only to an odd result: up to one unit, 2^-7 of the value), in fp16 half a unit.
+    tol = {"f32": 1e-6, "bf16": 2.0 ** -7, "f16": 2.0 ** -11}[dt]
+    assert (got.double() - want).abs().max() <= tol * want.abs().max()
+    assert L.ytcuda_device_status(None) == 0
+
+
+@pytest.mark.parametrize("name,value", [("q", float("inf")), ("k", float("-inf")), ("v", float("nan")), ("v", 3e38)])
+def test_planes_leave_special_values_to_ffma(L, api, name, value):
+    gen = torch.Generator(device="cuda").manual_seed(5)
+    t = {n: torch.randn(1, 2, 300, 64, generator=gen, device="cuda") for n in "qkv"}
+    t[name][0, 1, 290, 7] = value
+    got = api.scaledDotProductAttention(t["q"], t["k"], t["v"], causal=True)
+    L.ytcuda_attn_set_path(1)
+    want = api.scaledDotProductAttention(t["q"], t["k"], t["v"], causal=True)
+    L.ytcuda_attn_set_path(0)
+    assert torch.equal(torch.nan_to_num(got, 7.0, 8.0, 9.0), torch.nan_to_num(want, 7.0, 8.0, 9.0))
+
+
+def test_planes_step_aside_in_a_capture(api):
+    gen = torch.Generator(device="cuda").manual_seed(6)
+    q, k, v = (torch.randn(1, 4, 320, 128, generator=gen, device="cuda") for _ in range(3))
+    want = api.scaledDotProductAttention(q, k, v, causal=True)
+    graph, out = torch.cuda.CUDAGraph(), torch.empty_like(q)
+    with torch.cuda.graph(graph):
+        out.copy_(api.scaledDotProductAttention(q, k, v, causal=True))
+    out.zero_()
+    graph.replay()
+    assert (out - want).abs().max() <= 2e-6 * want.abs().max()  # (the FFMA kernel: another order of the sums)

@@ -892,7 +892,15 @@ struct AttnSimtParams {
   int window = 0;     // > 0: row r sees only the last `window` keys up to r + causal_off
   int ring = 0;       // > 0: key c lies in row c % ring of K and V
   float softcap = 0;  // > 0: score <- softcap * tanh(score / softcap)
+  const int* gate = nullptr;  // the tiled kernels run only if one of these `n_gate` words is set (null: always)
+  int n_gate = 0;
 };
+__device__ __forceinline__ bool gate_closed(const AttnSimtParams& p) {
+  if (!p.gate) return false;
+  int any = 0;
+  for (int i = threadIdx.x; i < p.n_gate; i += blockDim.x) any |= p.gate[i];
+  return __syncthreads_or(any) == 0;
+}
 
 constexpr int SIMT_MAX_D = 256;
 
@@ -1320,13 +1328,19 @@ __global__ void __launch_bounds__(128) attn_decode_merge_kernel(const AttnDecode
   }
 }
 
+}  // namespace ytk
+
+#include "attn_split.cuh"
+
+namespace ytk {
+
 // ------------------------------------------------------------------ fp32-accumulating tiled kernel (any dtype)
 // 32 query rows x 32 keys per step, 128 threads: thread (i, g) = (row, quarter). S = Q K^T from shared memory with
 // 8 scores per thread in registers, online softmax across the 4 threads of a row by shuffles, then
 // O[i, 32 g .. 32 g + 31] += P[i, :] V with P passed through shared memory. The prefill path of the fp32 decoder.
 constexpr int TL_BM = 32, TL_BN = 32, TL_D = 128, TL_PAD = 4;
 
-__global__ void __launch_bounds__(128) attn_tile_kernel(const AttnSimtParams p) {
+__device__ __forceinline__ void attn_tile_item(const AttnSimtParams& p, int rbk, int h, int b) {
   extern __shared__ __align__(16) float tl_smem[];
   float(*Qs)[TL_D + TL_PAD] = reinterpret_cast<float(*)[TL_D + TL_PAD]>(tl_smem);
   float(*Ks)[TL_D + TL_PAD] = Qs + TL_BM;
@@ -1334,16 +1348,12 @@ __global__ void __launch_bounds__(128) attn_tile_kernel(const AttnSimtParams p) 
   float(*Ps)[TL_BN + 1] = reinterpret_cast<float(*)[TL_BN + 1]>(Vs + TL_BN);
   const int tid = threadIdx.x;
   const int ri = tid >> 2, g = tid & 3;
-  const int heads = p.kv_heads * p.groups;
-  const int row_blocks = (p.q_len + TL_BM - 1) / TL_BM;
-  const int rbk = row_blocks - 1 - static_cast<int>(blockIdx.x);  // long causal rows first
-  const int h = blockIdx.y, b = blockIdx.z;
   const int kvh = h / p.groups;
   const int row0 = rbk * TL_BM;
   const int row = row0 + ri;
   const int64_t qo = b * p.q_sb + h * p.q_sh;
   const int64_t ko = b * p.k_sb + kvh * p.k_sh, vo = b * p.v_sb + kvh * p.v_sh;
-  (void)heads;
+  __syncthreads();  // (the item before has been finished)
   // stage Q (zero-padded to TL_D columns and TL_BM rows)
   // fp32 operands with 16-byte aligned rows are staged with 128-bit loads; anything else element by element
   const bool vec = p.dt == YTC_F32 && p.d % 4 == 0 && p.dv % 4 == 0 && p.q_sr % 4 == 0 && p.k_sr % 4 == 0 &&
@@ -1476,6 +1486,15 @@ __global__ void __launch_bounds__(128) attn_tile_kernel(const AttnSimtParams p) 
     }
   }
 }
+__global__ void __launch_bounds__(128) attn_tile_kernel(const AttnSimtParams p) {
+  dependent_wait();     // (under a programmatic dependent launch: the kernel before this one has finished)
+  dependent_trigger();  // the kernel queued behind this one may be scheduled meanwhile
+  if (gate_closed(p)) return;
+  const int row_blocks = (p.q_len + TL_BM - 1) / TL_BM, heads = p.kv_heads * p.groups;
+  for (int64_t i = blockIdx.x; i < static_cast<int64_t>(row_blocks) * heads * p.batch; i += gridDim.x)  // long causal rows first
+    attn_tile_item(p, row_blocks - 1 - static_cast<int>(i % row_blocks), static_cast<int>(i / row_blocks % heads),
+                   static_cast<int>(i / row_blocks / heads));
+}
 
 // ------------------------------------------------------------------ host side
 
@@ -1489,9 +1508,7 @@ __global__ void __launch_bounds__(128) attn_tile_kernel(const AttnSimtParams p) 
 constexpr int T64_BM = 64, T64_BN = 64, T64_LD = 128 + 4, T64_PLD = 64 + 4;
 constexpr int T64_SMEM = (3 * 64 * T64_LD + T64_BN * T64_PLD) * 4;
 
-__global__ void __launch_bounds__(256, 1) attn_tile64_kernel(const AttnSimtParams p) {
-  dependent_wait();     // (under a programmatic dependent launch: the kernel before this one has finished)
-  dependent_trigger();  // the kernel queued behind this one may be scheduled meanwhile
+__device__ __forceinline__ void attn_tile64_item(const AttnSimtParams& p, int rbk, int h, int b) {
   extern __shared__ __align__(16) float t64_smem[];
   float(*Qs)[T64_LD] = reinterpret_cast<float(*)[T64_LD]>(t64_smem);
   float(*Ks)[T64_LD] = Qs + T64_BM;
@@ -1499,9 +1516,7 @@ __global__ void __launch_bounds__(256, 1) attn_tile64_kernel(const AttnSimtParam
   float(*PsT)[T64_PLD] = reinterpret_cast<float(*)[T64_PLD]>(Vs + T64_BN);  // [key][row]
   const int tid = threadIdx.x;
   const int ry = tid >> 4, kx = tid & 15, cx = kx;
-  const int row_blocks = (p.q_len + T64_BM - 1) / T64_BM;
-  const int rbk = row_blocks - 1 - static_cast<int>(blockIdx.x);  // long causal rows first
-  const int h = blockIdx.y, b = blockIdx.z;
+  __syncthreads();  // (the item before has been finished)
   const int kvh = h / p.groups;
   const int row0 = rbk * T64_BM;
   const float* Qf = static_cast<const float*>(p.Q) + b * p.q_sb + h * p.q_sh;
@@ -1642,6 +1657,27 @@ __global__ void __launch_bounds__(256, 1) attn_tile64_kernel(const AttnSimtParam
       if (64 + cx * 4 + c < p.dv) orow[64 + cx * 4 + c] = acc[i][4 + c] * inv;
     }
   }
+}
+__global__ void __launch_bounds__(256, 1) attn_tile64_kernel(const AttnSimtParams p) {
+  dependent_wait();     // (under a programmatic dependent launch: the kernel before this one has finished)
+  dependent_trigger();  // the kernel queued behind this one may be scheduled meanwhile
+  if (gate_closed(p)) return;
+  const int row_blocks = (p.q_len + T64_BM - 1) / T64_BM, heads = p.kv_heads * p.groups;
+  for (int64_t i = blockIdx.x; i < static_cast<int64_t>(row_blocks) * heads * p.batch; i += gridDim.x)  // long causal rows first
+    attn_tile64_item(p, row_blocks - 1 - static_cast<int>(i % row_blocks), static_cast<int>(i / row_blocks % heads),
+                     static_cast<int>(i / row_blocks / heads));
+}
+
+// Where the tensor-core form is faster than the tiled FFMA kernels, by their steps one after another: a step of 64 keys of
+// attn_tile64_kernel takes about 10 us, one of 32 keys of attn_tile_kernel about 20 (fp32) to 40 (16 bit), the tensor-core
+// form 12 us and two more launches, then 2.8 us per 64 keys. Measured (FFMA / tensor cores): 256 keys, 16 heads 45 / 37 us;
+// 128 keys, 8 heads 30 / 42; 33 keys 45 / 41; 32 sequences of 60 tokens, 16 heads 235 / 58.
+static bool split_attention_pays(const AttnSimtParams& p) {
+  const int heads = p.kv_heads * p.groups;
+  if (heads > 65535 || p.batch > 65535) return false;
+  if (p.dt != YTC_F32 || p.q_len < T64_BM) return p.kv_len > TL_BN;
+  const int64_t items = static_cast<int64_t>((p.q_len + T64_BM - 1) / T64_BM) * heads * p.batch;
+  return (items + sm_count() - 1) / sm_count() * ((p.kv_len + T64_BN - 1) / T64_BN) >= 4;
 }
 
 static std::atomic<int> g_attn_path{0};  // 0 automatic, 1 always the one-warp-per-row kernel, 2 tensor-core kernel or fail
@@ -1924,24 +1960,32 @@ int ytcuda_flash_attn_fwd(int dtype, const void* Q, const void* K, const void* V
     YTC_CUDA(cudaGetLastError());
     return YTC_OK;
   }
+  // Products in fp32 from here on. On the tensor cores (attn_split.cuh) where that pays; the tiled FFMA kernels then run
+  // behind it, and only where a number has no planes.
+  if (g_attn_path != 1 && split_attention_pays(p)) (void)split_attention(p, &p.gate, &p.n_gate, st);
+  auto tile_grid = [&](int bm) {
+    const int64_t items = static_cast<int64_t>((q_len + bm - 1) / bm) * heads * batch;
+    const int64_t most = p.gate ? sm_count() : 0x7fffffff;
+    return dim3(static_cast<unsigned>(items < most ? items : most));
+  };
   if (dtype == YTC_F32 && q_len >= 64 && head_dim <= 128 && value_dim <= 128 && heads <= 65535 && batch <= 65535 &&
       vec_ok && head_dim % 4 == 0 && value_dim % 4 == 0 && q_strides[0] % 4 == 0 && q_strides[1] % 4 == 0 &&
       q_strides[2] % 4 == 0 && (reinterpret_cast<uint64_t>(Q) & 15) == 0) {
-    dim3 grid((q_len + T64_BM - 1) / T64_BM, heads, batch);
     const int sa = ensure_dynamic_smem(reinterpret_cast<const void*>(attn_tile64_kernel), T64_SMEM);
     if (sa != YTC_OK) return sa;
-    YTC_CUDA(launch_overlapped(attn_tile64_kernel, dim3(grid), dim3(256), T64_SMEM, st, p));
+    YTC_CUDA(launch_overlapped(attn_tile64_kernel, tile_grid(T64_BM), dim3(256), T64_SMEM, st, p));
     count_launch();
+    device_workspace_release(st);
     YTC_CUDA(cudaGetLastError());
     return YTC_OK;
   }
   if (head_dim <= TL_D && value_dim <= TL_D && heads <= 65535 && batch <= 65535) {
-    dim3 grid((q_len + TL_BM - 1) / TL_BM, heads, batch);
     constexpr int TL_SMEM = ((TL_BM + 2 * TL_BN) * (TL_D + TL_PAD) + TL_BM * (TL_BN + 1)) * 4;
     const int sa = ensure_dynamic_smem(reinterpret_cast<const void*>(attn_tile_kernel), TL_SMEM);
     if (sa != YTC_OK) return sa;
-    attn_tile_kernel<<<grid, 128, TL_SMEM, st>>>(p);
+    YTC_CUDA(launch_overlapped(attn_tile_kernel, tile_grid(TL_BM), dim3(128), TL_SMEM, st, p));
     count_launch();
+    device_workspace_release(st);
     YTC_CUDA(cudaGetLastError());
     return YTC_OK;
   }
