@@ -30,25 +30,14 @@ __device__ __forceinline__ float bin_apply(int op, float a, float b) {
     default: return a / b;
   }
 }
-// swish(x) = x * sigmoid(x), sigmoid in the reference's two-branch stable form
-// (src/ytensor_function.inl:42-52).
-__device__ __forceinline__ float swish_ref(float v) {
-  float sig;
-  if (v >= 0.f) {
-    const float z = expf(-v);
-    sig = 1.0f / (1.0f + z);
-  } else {
-    const float z = expf(v);
-    sig = z / (1.0f + z);
-  }
-  return v * sig;
-}
-// sigmoid and softplus in the reference's stable forms (src/ytensor_function.inl:42-59)
+// sigmoid and softplus in the reference's stable forms (src/ytensor_function.inl:42-59). The two branches of sigmoid share
+// one exponential and one division here (the same operations on the same numbers): a warp with both signs would run both.
 __device__ __forceinline__ float sigmoid_ref(float v) {
-  if (v >= 0.f) return 1.0f / (1.0f + expf(-v));
-  const float z = expf(v);
-  return z / (1.0f + z);
+  const float z = expf(-fabsf(v));
+  return (v >= 0.f ? 1.0f : z) / (1.0f + z);
 }
+// swish(x) = x * sigmoid(x)
+__device__ __forceinline__ float swish_ref(float v) { return v * sigmoid_ref(v); }
 __device__ __forceinline__ float softplus_ref(float v) { return fmaxf(v, 0.f) + log1pf(expf(-fabsf(v))); }
 
 // First derivatives (the order == 1 branches of src/function/activation.inl)
@@ -160,19 +149,35 @@ __device__ __forceinline__ void st4(void* p, int64_t i, const V4& r, int dt) {
   }
 }
 
-// out[i] = a[i] op b[i % bmod] over contiguous memory, 4 elements per thread per trip.
-__global__ void __launch_bounds__(256) binary_vec_kernel(int op, const void* a, const void* b, void* out, int64_t n4,
+// out[i] = a[i] op b[i % bmod] over contiguous memory, 4 elements per thread per trip; b four at a time where bmod is a
+// multiple of 4 (or b as long as a), else one at a time. The last n % 4 elements go one to a thread.
+// Measured, bf16 3001 x 8191 (a product): 39 us, 209 with the index arithmetic of binary_nd_kernel.
+__global__ void __launch_bounds__(256) binary_vec_kernel(int op, const void* a, const void* b, void* out, int64_t n,
                                                          int64_t bmod, int dt_a, int dt_b, int dt_out) {
-  for (int64_t i = blockIdx.x * static_cast<int64_t>(blockDim.x) + threadIdx.x; i < n4;
-       i += static_cast<int64_t>(gridDim.x) * blockDim.x) {
+  const bool quads = bmod == n || bmod % 4 == 0;
+  const int64_t n4 = n / 4, first = blockIdx.x * static_cast<int64_t>(blockDim.x) + threadIdx.x;
+  for (int64_t i = first; i < n4; i += static_cast<int64_t>(gridDim.x) * blockDim.x) {
     const int64_t e = i * 4;
     const V4 x = ld4(a, e, dt_a);
-    const V4 y = ld4(b, e % bmod, dt_b);
+    // (a 64-bit remainder costs as much as the rest of the trip)
+    int64_t j = bmod == n ? e : n <= 0x7fffffff ? static_cast<uint32_t>(e) % static_cast<uint32_t>(bmod) : e % bmod;
+    V4 y;
+    if (quads) {
+      y = ld4(b, j, dt_b);
+    } else {
+#pragma unroll
+      for (int k = 0; k < 4; ++k) {
+        y.v[k] = load_as_f32(b, j, dt_b);
+        j = j + 1 == bmod ? 0 : j + 1;
+      }
+    }
     V4 r;
 #pragma unroll
     for (int k = 0; k < 4; ++k) r.v[k] = bin_apply(op, x.v[k], y.v[k]);
     st4(out, e, r, dt_out);
   }
+  if (const int64_t e = n4 * 4 + first; e < n)
+    store_from_f32(out, e, bin_apply(op, load_as_f32(a, e, dt_a), load_as_f32(b, e % bmod, dt_b)), dt_out);
 }
 
 struct NdIndex {
@@ -196,10 +201,12 @@ __global__ void __launch_bounds__(256) binary_nd_kernel(int op, const void* a, c
   }
 }
 
-__global__ void __launch_bounds__(256) unary_vec_kernel(int op, const void* x, void* y, int64_t n4, float param,
+// (the last n % 4 elements one to a thread)
+__global__ void __launch_bounds__(256) unary_vec_kernel(int op, const void* x, void* y, int64_t n, float param,
                                                         int dt_in, int dt_out) {
-  for (int64_t i = blockIdx.x * static_cast<int64_t>(blockDim.x) + threadIdx.x; i < n4;
-       i += static_cast<int64_t>(gridDim.x) * blockDim.x) {
+  const int64_t n4 = n / 4, first = blockIdx.x * static_cast<int64_t>(blockDim.x) + threadIdx.x;
+  if (const int64_t e = n4 * 4 + first; e < n) store_from_f32(y, e, un_apply(op, load_as_f32(x, e, dt_in), param), dt_out);
+  for (int64_t i = first; i < n4; i += static_cast<int64_t>(gridDim.x) * blockDim.x) {
     V4 v = ld4(x, i * 4, dt_in);
 #pragma unroll
     for (int k = 0; k < 4; ++k) v.v[k] = un_apply(op, v.v[k], param);
@@ -282,8 +289,8 @@ int ytcuda_binary(int op, int dt_a, int dt_b, int dt_out, const void* a, const v
   if (n == 0) return YTC_OK;
   YTC_REQUIRE(a && b && out, "ytcuda_binary: null tensor");
   cudaStream_t st = static_cast<cudaStream_t>(stream);
-  if (is_contig(ndim, shape, astrides) && is_contig(ndim, shape, ostrides) && n % 4 == 0 && aligned(a, dt_a) &&
-      aligned(b, dt_b) && aligned(out, dt_out)) {
+  if (is_contig(ndim, shape, astrides) && is_contig(ndim, shape, ostrides) && aligned(a, dt_a) && aligned(b, dt_b) &&
+      aligned(out, dt_out)) {
     // b: zero stride on leading dims, contiguous on the trailing ones => index i % bmod
     int split = ndim;
     int64_t exp = 1;
@@ -294,8 +301,8 @@ int ytcuda_binary(int op, int dt_a, int dt_b, int dt_out, const void* a, const v
     bool lead_zero = true;
     for (int d = 0; d < split; ++d)
       if (shape[d] != 1 && bstrides[d] != 0) lead_zero = false;
-    if (lead_zero && exp % 4 == 0) {
-      binary_vec_kernel<<<grid_for(n / 4), 256, 0, st>>>(op, a, b, out, n / 4, exp, dt_a, dt_b, dt_out);
+    if (lead_zero) {
+      binary_vec_kernel<<<grid_for((n + 3) / 4), 256, 0, st>>>(op, a, b, out, n, exp, dt_a, dt_b, dt_out);
       count_launch();
       YTC_CUDA(cudaGetLastError());
       return YTC_OK;
@@ -338,9 +345,8 @@ static int unary_impl(int op, int dt_in, int dt_out, const void* x, void* y, int
   if (n == 0) return YTC_OK;
   YTC_REQUIRE(x && y, "ytcuda_unary: null tensor");
   cudaStream_t st = static_cast<cudaStream_t>(stream);
-  if (is_contig(ndim, shape, xstrides) && is_contig(ndim, shape, ystrides) && n % 4 == 0 && aligned(x, dt_in) &&
-      aligned(y, dt_out)) {
-    unary_vec_kernel<<<grid_for(n / 4), 256, 0, st>>>(op, x, y, n / 4, param, dt_in, dt_out);
+  if (is_contig(ndim, shape, xstrides) && is_contig(ndim, shape, ystrides) && aligned(x, dt_in) && aligned(y, dt_out)) {
+    unary_vec_kernel<<<grid_for((n + 3) / 4), 256, 0, st>>>(op, x, y, n, param, dt_in, dt_out);
   } else {
     NdIndex ix;
     ix.nd = ndim;
