@@ -183,6 +183,13 @@ int ytcuda_layernorm(int dt_in, int dt_out, int dt_w, const void* x, const void*
                      const int64_t* shape, const int64_t* xstrides, const int64_t* ystrides, int ndim, const int* axes,
                      int naxes, float eps, void* stream);
 
+/* The same with gamma and beta at strides of their own: wstrides[ndim] elements per step of each dim, 0 where they do not
+ * depend on it. instanceNorm / batchNorm / groupNorm with their channel-wise gamma and bias in one pass
+ * (src/function/normalization.inl:378-577). Strides that no kernel takes give YTC_UNSUPPORTED. */
+int ytcuda_layernorm_strided(int dt_in, int dt_out, int dt_w, const void* x, const void* gamma, const void* beta, void* y,
+                             const int64_t* shape, const int64_t* xstrides, const int64_t* ystrides, const int64_t* wstrides,
+                             int ndim, const int* axes, int naxes, float eps, void* stream);
+
 /* op 0 = sum, 1 = mean, 2 = max. y is contiguous with size-1 dims on the reduced axes; for max, `index`
  * (may be NULL) receives the position of the FIRST maximum in the odometer walk. Replaces YTensor::sum / mean /
  * max (include/ytensor_math.hpp:105-121, src/ytensor_math.inl:414-692). */

@@ -163,3 +163,78 @@ def test_chain_full_size_properties(api):
     assert torch.equal(out[0], out[31])
     s = out[::7, ::113].float().sum(-1)
     assert torch.all((s - 1).abs() < 2e-2) and torch.all(out[::7, ::113] >= 0)
+
+
+# ------------------------------------------------------------------ lines shared by a cluster of CTAs, odd rows
+def _sixty_four(x, axes, op, w=None, b=None, eps=1e-5):
+    d = x.double()
+    if op == "softmax":
+        m = d.amax(axes, keepdim=True)
+        return (d - m).exp() / (d - m).exp().sum(axes, keepdim=True)
+    if op == "rmsNorm":
+        y = d / (d.pow(2).mean(axes, keepdim=True) + eps).sqrt()
+    else:
+        y = (d - d.mean(axes, keepdim=True)) / (d.var(axes, unbiased=False, keepdim=True) + eps).sqrt()
+    return y if w is None else y * w + (0 if b is None else b)
+
+
+@pytest.mark.parametrize("shape,axes,dtype", [
+    ((3, 5, 7, 7), (0, 2, 3), torch.float32), ((2, 3, 130, 131), (0, 2, 3), torch.float32), ((4, 2, 64, 260), (0, 3), torch.float32),
+    ((1, 2, 300, 1400), (2, 3), torch.float32),   # a share is more than the cache holds
+    ((2, 40001), (1,), torch.float32), ((2, 40000), (1,), torch.bfloat16), ((700, 65), (0,), torch.float32),
+    ((5, 4099, 33), (1,), torch.float16), ((9000, 40), (0,), torch.float32), ((3, 2, 8), (0, 1), torch.float32),
+    ((9, 63), (1,), torch.bfloat16), ((5, 8191), (1,), torch.float32), ((7, 16383), (1,), torch.float16), ((3, 5001), (1,), torch.float32)])
+def test_shared_lines_and_odd_rows(api, shape, axes, dtype):
+    gen = torch.Generator(device="cuda").manual_seed(sum(shape))
+    x = (torch.randn(shape, generator=gen, device="cuda") * 2 + 0.5).to(dtype)
+    sizes = [shape[a] for a in axes]
+    w, b = (torch.rand(sizes, generator=gen, device="cuda").to(dtype) for _ in range(2))
+    spread = [shape[a] if a in axes else 1 for a in range(len(shape))]
+    wv, bv = w.reshape(spread).double(), b.reshape(spread).double()
+    # fp32: sums of R terms in a tree, 1e-6; bf16 is rounded by the reference's rule, up to one unit in the last place
+    tol = {torch.float32: 2e-6, torch.bfloat16: 2.0 ** -7, torch.float16: 2.0 ** -11}[dtype]
+    small = 6e-5 if dtype == torch.float16 else 0.0  # (results below fp16's normal numbers become zero)
+    for got, want in ((api.softmax(x, axes), _sixty_four(x, axes, "softmax")),
+                      (api.rmsNorm(x, w, axes), _sixty_four(x, axes, "rmsNorm", wv)),
+                      (api.layerNorm(x, w, b, axes), _sixty_four(x, axes, "layerNorm", wv, bv)),
+                      (api.layerNorm(x, None, None, axes), _sixty_four(x, axes, "layerNorm"))):
+        assert (got.double() - want).abs().max() <= small + tol * want.abs().max()
+    d = x.double()
+    assert ((api.sum(x, axes).double() - d.sum(axes, keepdim=True)).abs().max()
+            <= max(tol, 1e-5) * d.abs().sum(axes, keepdim=True).max())
+    mv, mi = api.max(x, axes)
+    flat = x.movedim(axes, list(range(-len(axes), 0))).reshape(-1, int(np.prod(sizes)))
+    best = flat.max(1).values
+    assert torch.equal(mv.reshape(-1), best)
+    assert torch.equal(mi.reshape(-1).long(), (flat == best[:, None]).int().argmax(1))  # the first of equal maxima
+
+
+@pytest.mark.parametrize("shape,groups,dtype", [((3, 8, 7, 5), 4, torch.float32), ((2, 24, 56, 56), 8, torch.float32),
+                                                ((1, 8, 9), 2, torch.bfloat16)])
+def test_channel_norms_in_one_pass(api, shape, groups, dtype):
+    gen = torch.Generator(device="cuda").manual_seed(groups)
+    x = torch.randn(shape, generator=gen, device="cuda").to(dtype)
+    w, b = (torch.randn(shape[1], generator=gen, device="cuda").to(dtype) for _ in range(2))
+    wv, bv = (t.double().reshape(1, -1, *[1] * (len(shape) - 2)) for t in (w, b))
+    tail = tuple(range(2, len(shape)))
+    grouped = x.reshape(shape[0], groups, -1)
+    # two roundings more than the plain norm (product, sum); bf16: one unit of the largest result
+    tol = 2e-6 if dtype == torch.float32 else 2.0 ** -7
+    for got, want in ((api.batchNorm(x, w, b), _sixty_four(x, (0, *tail), "layerNorm", wv, bv)),
+                      (api.instanceNorm(x, w, b), _sixty_four(x, tail, "layerNorm", wv, bv)),
+                      (api.groupNorm(x, groups, w, b), _sixty_four(grouped, (2,), "layerNorm").reshape(shape) * wv + bv)):
+        assert (got.double() - want).abs().max() <= tol * want.abs().max()
+    with pytest.raises(ValueError):
+        api.batchNorm(x, w[1:], b)
+
+
+def test_odd_elementwise_sizes(api):
+    gen = torch.Generator(device="cuda").manual_seed(3)
+    for rows, cols in ((1, 1), (3, 5), (7, 1023), (129, 514)):
+        for dt in (torch.float32, torch.float16):
+            x = torch.randn(rows, cols, generator=gen, device="cuda").to(dt)
+            bias, y = torch.randn(cols, generator=gen, device="cuda").to(dt), torch.randn(rows, cols, generator=gen, device="cuda").to(dt)
+            flushed = 0.0 if dt == torch.float32 else 6.2e-5  # (fp16 results below the normal numbers become zero)
+            for got, want in ((api.add(x, bias), x + bias), (api.add(x, y), x + y)):
+                assert (got - want).abs().max() <= flushed
+            assert (api.swish(x).double() - torch.nn.functional.silu(x.double())).abs().max() <= (1e-6 if dt == torch.float32 else 4e-3)

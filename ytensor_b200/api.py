@@ -246,17 +246,21 @@ def layerNorm_(x, gamma=None, bias=None, axes=-1, eps: float = 1e-5):
     return layerNorm(x, gamma, bias, axes, eps, out=x)
 
 
+def _check_affine(y: torch.Tensor, gamma, bias, ax) -> None:
+    if gamma is None or bias is None:
+        raise _lib.YtCudaInvalidArgument(_lib.INVALID_ARG, "gamma and bias come together")
+    want = [y.shape[a] for a in ax]
+    if list(gamma.shape) != want or list(bias.shape) != want:
+        raise _lib.YtCudaInvalidArgument(_lib.INVALID_ARG, "gamma/bias shape must match affine axes")
+
+
 def _affine_(y: torch.Tensor, gamma, bias, axes) -> torch.Tensor:
     """y *= gamma; y += bias with gamma / bias holding one dim per axis (the reference's _applyScale_ / _applyBias_,
     src/function/normalization.inl:88-116, through _makeAffineView)."""
     if gamma is None and bias is None:
         return y
-    if gamma is None or bias is None:
-        raise _lib.YtCudaInvalidArgument(_lib.INVALID_ARG, "gamma and bias come together")
     ax = [a % y.dim() for a in axes]
-    want = [y.shape[a] for a in ax]
-    if list(gamma.shape) != want or list(bias.shape) != want:
-        raise _lib.YtCudaInvalidArgument(_lib.INVALID_ARG, "gamma/bias shape must match affine axes")
+    _check_affine(y, gamma, bias, ax)
     # the reference views the affine tensor's MEMORY with the axis sizes in ascending axis order, whatever order the
     # axes were listed in (src/ytensor_function.inl:137-158): a plain reshape of the contiguous tensor does the same
     view = [1] * y.dim()
@@ -267,6 +271,25 @@ def _affine_(y: torch.Tensor, gamma, bias, axes) -> torch.Tensor:
     _binary("mul", y, g.to(y.dtype), y)
     _binary("add", y, b.to(y.dtype), y)
     return y
+
+
+def _channel_norm(x: torch.Tensor, y: torch.Tensor, axes, eps: float, whole: torch.Tensor, gamma, bias, channel: int,
+                  wstrides) -> torch.Tensor:
+    """layerNorm of x over `axes` into y, then gamma and bias of the channels of `whole` (axis `channel`; x and y may be
+    grouped views, `wstrides` says how far a step of each of their dims moves in gamma). One launch where the strides allow
+    it, else three."""
+    if gamma is not None and bias is not None and gamma.is_cuda and bias.is_cuda:
+        _check_affine(whole, gamma, bias, [channel])
+        _require_cuda(x, y)
+        g, b = gamma.contiguous().to(y.dtype), bias.contiguous().to(y.dtype)
+        rc = lib().ytcuda_layernorm_strided(_dt(x), _dt(y), _dt(y), x.data_ptr(), g.data_ptr(), b.data_ptr(), y.data_ptr(),
+                                            _i64(x.shape), _i64(x.stride()), _i64(y.stride()), _i64(wstrides), x.dim(),
+                                            _i32(axes), len(axes), eps, _stream())
+        if rc != _lib.UNSUPPORTED:
+            check(rc)
+            return whole
+    layerNorm(x, None, None, axes, eps, out=y)
+    return _affine_(whole, gamma, bias, [channel])
 
 
 def normalize(x: torch.Tensor, axes=-1, p: float = 2.0, eps: float = 1e-12, gamma=None, bias=None,
@@ -305,8 +328,8 @@ def instanceNorm(x: torch.Tensor, gamma=None, bias=None, channelAxis: int = 1, e
     axes = [a for a in range(x.dim()) if a not in (0, c)]
     if not axes:
         raise _lib.YtCudaInvalidArgument(_lib.INVALID_ARG, "yt::function::instanceNorm: requires at least one spatial axis")
-    y = layerNorm(x, None, None, axes, eps, out=out)
-    return _affine_(y, gamma, bias, [c])
+    y = torch.empty_like(x, memory_format=torch.contiguous_format) if out is None else out
+    return _channel_norm(x, y, axes, eps, y, gamma, bias, c, [int(a == c) for a in range(x.dim())])
 
 
 def instanceNorm_(x, gamma=None, bias=None, channelAxis: int = 1, eps: float = 1e-5):
@@ -319,8 +342,8 @@ def batchNorm(x: torch.Tensor, gamma=None, bias=None, channelAxis: int = 1, eps:
     src/function/normalization.inl:435-489: statistics of the tensor itself, no running averages)."""
     c = _channel_axis(x, channelAxis, "yt::function::batchNorm_")
     axes = [a for a in range(x.dim()) if a != c]
-    y = layerNorm(x, None, None, axes, eps, out=out)
-    return _affine_(y, gamma, bias, [c])
+    y = torch.empty_like(x, memory_format=torch.contiguous_format) if out is None else out
+    return _channel_norm(x, y, axes, eps, y, gamma, bias, c, [int(a == c) for a in range(x.dim())])
 
 
 def batchNorm_(x, gamma=None, bias=None, channelAxis: int = 1, eps: float = 1e-5):
@@ -345,8 +368,8 @@ def groupNorm(x: torch.Tensor, groups: int, gamma=None, bias=None, channelAxis: 
     y = torch.empty_like(x, memory_format=torch.contiguous_format) if out is None else out
     xg = x.movedim(c, 1).unflatten(1, (groups, ch // groups))
     yg = y.movedim(c, 1).unflatten(1, (groups, ch // groups))
-    layerNorm(xg, None, None, list(range(2, xg.dim())), eps, out=yg)
-    return _affine_(y, gamma, bias, [c])
+    ws = [0, ch // groups, 1] + [0] * (xg.dim() - 3)
+    return _channel_norm(xg, yg, list(range(2, xg.dim())), eps, y, gamma, bias, c, ws)
 
 
 def groupNorm_(x, groups: int, gamma=None, bias=None, channelAxis: int = 1, eps: float = 1e-5):

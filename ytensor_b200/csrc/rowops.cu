@@ -1,11 +1,15 @@
 // Bandwidth-bound reductions over one or several axes: softmax, RMSNorm, LayerNorm, the fused
 // RMSNorm + residual + softmax + cast chain, and sum / mean / max(+argmax).
 //
-// Two kernels:
-//  * row_kernel  : the reduced axes are the trailing, contiguous dims. A group of G threads owns a row,
-//                  keeps it in registers (4 x 128-bit loads per thread), reduces with warp shuffles
-//                  (+ one shared-memory hop above 32 threads) and writes the result once: one read and
-//                  one write of HBM per element.
+// Four kernels:
+//  * row_kernel  : the reduced axes are the trailing, contiguous dims, up to 16384 elements. A group of G
+//                  threads owns a row, keeps it in registers (4 x 128-bit loads per thread, 16 single loads
+//                  where the length or alignment is odd), reduces with warp shuffles (+ one shared-memory
+//                  hop above 32 threads) and writes the result once: one read and one write of HBM per element.
+//  * span_kernel : a line is one or two runs-of-runs whose elements are neighbours in memory (a channel over
+//                  batch and image, a group of channels, a long row). A cluster of CTAs shares the line.
+//  * column_kernel : the reduced axes are one stride apart and the kept elements are neighbours. A cluster of
+//                  CTAs shares the rows of 32 columns.
 //  * line_kernel : any axes, any strides. A "line" is the set of elements reduced together; its
 //                  elements are walked as an odometer over the reduced dims in the order the caller
 //                  listed them (the order the reference's argmax index refers to). Either one CTA
@@ -19,12 +23,14 @@
 #include <atomic>
 #include <mutex>
 
+#include "ptx_sm100.cuh"
 #include "ytc_common.cuh"
 
 namespace ytk {
 
 enum RowOp { OP_SOFTMAX = 0, OP_RMSNORM = 1, OP_LAYERNORM = 2, OP_CHAIN = 3, OP_SUM = 4, OP_MEAN = 5, OP_MAX = 6,
-             OP_LPNORM = 7 };
+             OP_LPNORM = 7,
+             OP_RMSPLANES = 8 };  // rmsNorm of fp32 rows into two bf16 planes (row_kernel only)
 
 struct F4 {
   float v[4];
@@ -133,14 +139,15 @@ struct RowParams {
   const void* b;   // beta (layernorm) or residual r (chain), may be null
   int* idx;        // argmax output (OP_MAX), may be null
   int64_t rows;
-  int L;           // row length (multiple of 4)
+  int L;           // row length
   int64_t x_rs, y_rs;  // row strides in elements
   int64_t r_rows;  // chain: residual row = row % r_rows
   float eps;
   int dt_in, dt_out, dt_w;
 };
 
-template <int OP, int G>
+// VEC: elements per load, 4 (element e of load v of thread t is column (v G + t) 4 + e) or 1 (column (4 v + e) G + t).
+template <int OP, int G, int VEC>
 __global__ void __launch_bounds__(G < 256 ? 256 : G) row_kernel(const RowParams p) {
   dependent_wait();     // (under a programmatic dependent launch: the kernel before this one has finished)
   dependent_trigger();  // the kernel queued behind this one may be scheduled meanwhile
@@ -162,14 +169,21 @@ __global__ void __launch_bounds__(G < 256 ? 256 : G) row_kernel(const RowParams 
     const bool row_ok = row < p.rows;
     if (OP == OP_CHAIN && copies > 1 && row_ok) row = (row % copies) * p.r_rows + row / copies;
     F4 x[VPT];
-    bool act[VPT];
+    auto at = [&](int v, int e) { return VEC == 4 ? (v * G + t) * 4 + e : (4 * v + e) * G + t; };
+    auto on = [&](int v, int e) { return row_ok && at(v, VEC == 4 ? 0 : e) < p.L; };
+    auto load = [&](const void* src, int64_t row0, int v, int dt) {
+      F4 r = {{0.f, 0.f, 0.f, 0.f}};
+      if constexpr (VEC == 4) {
+        if (on(v, 0)) r = load4(src, row0 + at(v, 0), dt);
+      } else {
 #pragma unroll
-    for (int v = 0; v < VPT; ++v) {
-      const int col = (v * G + t) * 4;
-      act[v] = row_ok && col < p.L;
-      if (act[v]) x[v] = load4(p.x, row * p.x_rs + col, p.dt_in);
-      else x[v] = F4{{0.f, 0.f, 0.f, 0.f}};
-    }
+        for (int e = 0; e < 4; ++e)
+          if (on(v, e)) r.v[e] = load_as_f32(src, row0 + at(v, e), dt);
+      }
+      return r;
+    };
+#pragma unroll
+    for (int v = 0; v < VPT; ++v) x[v] = load(p.x, row * p.x_rs, v, p.dt_in);
 
     if constexpr (OP == OP_SUM || OP == OP_MEAN) {
       float s = 0.f;
@@ -183,10 +197,9 @@ __global__ void __launch_bounds__(G < 256 ? 256 : G) row_kernel(const RowParams 
       MaxIdx m = {-CUDART_INF_F, 0x7fffffff};
 #pragma unroll
       for (int v = 0; v < VPT; ++v)
-        if (act[v]) {
 #pragma unroll
-          for (int k = 0; k < 4; ++k) m = max_combine(m, MaxIdx{x[v].v[k], (v * G + t) * 4 + k});
-        }
+        for (int k = 0; k < 4; ++k)
+          if (on(v, k)) m = max_combine(m, MaxIdx{x[v].v[k], at(v, k)});
       m = group_maxidx<G>(m, red, redi, group, t);
       if (row_ok && t == 0) {
         if (m.i == 0x7fffffff) {  // every element failed `>` (all NaN): the reference keeps element 0
@@ -199,7 +212,7 @@ __global__ void __launch_bounds__(G < 256 ? 256 : G) row_kernel(const RowParams 
       continue;
     }
 
-    if constexpr (OP == OP_RMSNORM || OP == OP_CHAIN) {
+    if constexpr (OP == OP_RMSNORM || OP == OP_CHAIN || OP == OP_RMSPLANES) {
       float ss = 0.f;
 #pragma unroll
       for (int v = 0; v < VPT; ++v)
@@ -210,29 +223,26 @@ __global__ void __launch_bounds__(G < 256 ? 256 : G) row_kernel(const RowParams 
       if constexpr (OP == OP_CHAIN) {
         const int64_t r_off = (row_ok ? (p.r_rows == p.rows ? row : row % p.r_rows) : 0) * static_cast<int64_t>(p.L);
 #pragma unroll
-        for (int v = 0; v < VPT; ++v)
-          if (act[v]) {
-            rr[v] = load4(p.b, r_off + (v * G + t) * 4, YTC_F32);
-            ww[v] = load4(p.w, (v * G + t) * 4, YTC_F32);
-          }
+        for (int v = 0; v < VPT; ++v) {
+          rr[v] = load(p.b, r_off, v, YTC_F32);
+          ww[v] = load(p.w, 0, v, YTC_F32);
+        }
       }
       ss = group_sum<G>(ss, red, group, t);
       const float inv = 1.0f / sqrtf(ss * invL + p.eps);
 #pragma unroll
-      for (int v = 0; v < VPT; ++v)
-        if (act[v]) {
-          const int col = (v * G + t) * 4;
+      for (int v = 0; v < VPT; ++v) {
 #pragma unroll
-          for (int k = 0; k < 4; ++k) x[v].v[k] *= inv;
-          if constexpr (OP == OP_CHAIN) {
+        for (int k = 0; k < 4; ++k) x[v].v[k] *= inv;
+        if constexpr (OP == OP_CHAIN) {
 #pragma unroll
-            for (int k = 0; k < 4; ++k) x[v].v[k] = fmaf(x[v].v[k], ww[v].v[k], rr[v].v[k]);
-          } else if (p.w) {
-            const F4 w = load4(p.w, col, p.dt_w);
+          for (int k = 0; k < 4; ++k) x[v].v[k] = fmaf(x[v].v[k], ww[v].v[k], rr[v].v[k]);
+        } else if (p.w) {
+          const F4 w = load(p.w, 0, v, p.dt_w);
 #pragma unroll
-            for (int k = 0; k < 4; ++k) x[v].v[k] *= w.v[k];
-          }
+          for (int k = 0; k < 4; ++k) x[v].v[k] *= w.v[k];
         }
+      }
     }
     if constexpr (OP == OP_LAYERNORM) {
       float s = 0.f;
@@ -242,45 +252,43 @@ __global__ void __launch_bounds__(G < 256 ? 256 : G) row_kernel(const RowParams 
       float ss = 0.f;
 #pragma unroll
       for (int v = 0; v < VPT; ++v)
-        if (act[v]) {
 #pragma unroll
-          for (int k = 0; k < 4; ++k) {
+        for (int k = 0; k < 4; ++k)
+          if (on(v, k)) {
             x[v].v[k] -= mu;
             ss = fmaf(x[v].v[k], x[v].v[k], ss);
           }
-        }
       ss = group_sum<G>(ss, red, group, t);
       const float inv = 1.0f / sqrtf(ss * invL + p.eps);
 #pragma unroll
-      for (int v = 0; v < VPT; ++v)
-        if (act[v]) {
-          const int col = (v * G + t) * 4;
+      for (int v = 0; v < VPT; ++v) {
 #pragma unroll
-          for (int k = 0; k < 4; ++k) x[v].v[k] *= inv;
-          if (p.w) {
-            const F4 w = load4(p.w, col, p.dt_w);
-            const F4 bb = load4(p.b, col, p.dt_w);
+        for (int k = 0; k < 4; ++k) x[v].v[k] *= inv;
+        if (p.w) {
+          const F4 w = load(p.w, 0, v, p.dt_w);
+          const F4 bb = load(p.b, 0, v, p.dt_w);
 #pragma unroll
-            for (int k = 0; k < 4; ++k) x[v].v[k] = x[v].v[k] * w.v[k] + bb.v[k];
-          }
+          for (int k = 0; k < 4; ++k) x[v].v[k] = x[v].v[k] * w.v[k] + bb.v[k];
         }
+      }
     }
     if constexpr (OP == OP_SOFTMAX || OP == OP_CHAIN) {
       float m = -CUDART_INF_F;
 #pragma unroll
       for (int v = 0; v < VPT; ++v)
-        if (act[v]) m = fmaxf(m, fmaxf(fmaxf(x[v].v[0], x[v].v[1]), fmaxf(x[v].v[2], x[v].v[3])));
+#pragma unroll
+        for (int k = 0; k < 4; ++k)
+          if (on(v, k)) m = fmaxf(m, x[v].v[k]);
       m = group_max<G>(m, red, group, t);
       float s = 0.f;
 #pragma unroll
       for (int v = 0; v < VPT; ++v)
-        if (act[v]) {
 #pragma unroll
-          for (int k = 0; k < 4; ++k) {
+        for (int k = 0; k < 4; ++k)
+          if (on(v, k)) {
             x[v].v[k] = __expf(x[v].v[k] - m);
             s += x[v].v[k];
           }
-        }
       s = group_sum<G>(s, red, group, t);
       const float inv = 1.0f / s;
 #pragma unroll
@@ -289,8 +297,32 @@ __global__ void __launch_bounds__(G < 256 ? 256 : G) row_kernel(const RowParams 
         for (int k = 0; k < 4; ++k) x[v].v[k] *= inv;
     }
 #pragma unroll
-    for (int v = 0; v < VPT; ++v)
-      if (act[v]) store4(p.y, row * p.y_rs + (v * G + t) * 4, x[v], p.dt_out);
+    for (int v = 0; v < VPT; ++v) {
+      if constexpr (OP == OP_RMSPLANES) {  // x = hi + lo, both rounded to nearest: 16 mantissa bits
+        if (on(v, 0)) {
+          F4 lo;
+          uint32_t h[2], l[2];
+#pragma unroll
+          for (int e = 0; e < 2; ++e) {
+            const __nv_bfloat162 hb = __floats2bfloat162_rn(x[v].v[2 * e], x[v].v[2 * e + 1]);
+            lo.v[2 * e] = x[v].v[2 * e] - __low2float(hb);
+            lo.v[2 * e + 1] = x[v].v[2 * e + 1] - __high2float(hb);
+            const __nv_bfloat162 lb = __floats2bfloat162_rn(lo.v[2 * e], lo.v[2 * e + 1]);
+            h[e] = *reinterpret_cast<const uint32_t*>(&hb);
+            l[e] = *reinterpret_cast<const uint32_t*>(&lb);
+          }
+          uint16_t* hi = static_cast<uint16_t*>(p.y) + row * p.y_rs + at(v, 0);
+          *reinterpret_cast<uint2*>(hi) = make_uint2(h[0], h[1]);
+          *reinterpret_cast<uint2*>(hi + p.rows * p.y_rs) = make_uint2(l[0], l[1]);
+        }
+      } else if constexpr (VEC == 4) {
+        if (on(v, 0)) store4(p.y, row * p.y_rs + at(v, 0), x[v], p.dt_out);
+      } else {
+#pragma unroll
+        for (int e = 0; e < 4; ++e)
+          if (on(v, e)) store_from_f32(p.y, row * p.y_rs + at(v, e), x[v].v[e], p.dt_out);
+      }
+    }
   }
 }
 
@@ -535,6 +567,317 @@ __global__ void __launch_bounds__(128) line_kernel(const LineParams p) {
   }
 }
 
+// ------------------------------------------------------------------ lines shared by a cluster of CTAs
+// span_kernel: the reduced elements of a line are R1 runs of R2 neighbours. column_kernel: they lie one stride apart and the
+// kept elements next to a line are its neighbours in memory. Both bring a line's elements into shared memory once, as fp32,
+// a share per CTA of a cluster, and pass the partial results through distributed shared memory in the order of the ranks:
+// one read and one write of HBM per element and one launch, where line_kernel walks an odometer with a 64-bit division per
+// element and pass, on one CTA (or thread) per line. Shares above CACHE_FLOATS are read again instead.
+// What bounds them: span_kernel the loads in flight while a share comes in and goes out (16 x 96 x 56 x 56 fp32 over all axes but
+// the channel, gamma and bias included: 965 us with line_kernel and two elementwise passes, 25 here, 6 at the copy rate);
+// column_kernel the latency of its 32-column rows (softmax of fp32 2048 x 4096 along the first axis: 2891 / 60 us).
+constexpr int SHARE_UNROLL = 4, MAX_SHARES = 8;
+constexpr uint32_t CACHE_FLOATS = 50u * 1024;
+
+struct ShareParams {
+  const void* x;
+  void* y;
+  const void* w;
+  const void* b;
+  int* idx;
+  int nk;                                                // kept dims (without the columns of column_kernel)
+  int64_t kshape[MAXD], kxs[MAXD], kys[MAXD], kws[MAXD];  // extent, strides in x, y and gamma / beta
+  uint32_t R, R2;          // elements of a line, of a run (span_kernel)
+  int64_t xs1, ys1, ws1;   // strides of the runs (span_kernel), of the line's elements (column_kernel)
+  int64_t ws2;             // span_kernel: stride of a run's elements in gamma / beta
+  int64_t cols, cws;       // column_kernel: columns, their stride in gamma / beta
+  uint32_t share;          // elements per CTA
+  int shares;
+  int cached;
+  float eps, lp;
+  int dt_in, dt_out, dt_w;
+};
+
+// The sum (or maximum, or first maximum) of `mine` over the CTAs of the cluster, in the order of their ranks; `slot` is a
+// word (pair) of this CTA that nothing else uses until the cluster's last barrier.
+struct ShareSum {
+  __device__ __forceinline__ float operator()(float a, float b) const { return a + b; }
+};
+struct ShareMax {
+  __device__ __forceinline__ float operator()(float a, float b) const { return fmaxf(a, b); }
+};
+__device__ __forceinline__ float ld_cluster_f32(const void* p, uint32_t rank) {
+  float v;
+  asm volatile("ld.shared::cluster.f32 %0, [%1];" : "=f"(v) : "r"(map_to_cta(smem_u32(p), rank)) : "memory");
+  return v;
+}
+template <class F>
+__device__ __forceinline__ float over_shares(float mine, float* slot, bool writes, int shares, F f) {
+  if (shares == 1) return mine;
+  if (writes) *slot = mine;
+  cluster_sync_all();
+  float v = ld_cluster_f32(slot, 0);
+  for (int r = 1; r < shares; ++r) v = f(v, ld_cluster_f32(slot, r));
+  return v;
+}
+__device__ __forceinline__ MaxIdx over_shares(MaxIdx mine, float* slot, int* islot, bool writes, int shares) {
+  if (shares == 1) return mine;
+  if (writes) {
+    *slot = mine.v;
+    *islot = mine.i;
+  }
+  cluster_sync_all();
+  MaxIdx m = {-CUDART_INF_F, 0x7fffffff};
+  for (int r = 0; r < shares; ++r) m = max_combine(m, MaxIdx{ld_cluster_f32(slot, r), __float_as_int(ld_cluster_f32(islot, r))});
+  return m;
+}
+
+// The passes over a line: `sweep(first, f)` calls f(value, index, n) for this thread's elements of the share (n: how many),
+// from global memory the first time and from the cache afterwards; bsum / bmax / bmaxidx reduce over the whole line.
+// `emit(g)` writes y = g(value) * gamma + beta.
+template <int OP, class Sweep, class BSum, class BMax, class BMaxIdx, class Emit, class Result>
+__device__ __forceinline__ void line_passes(const ShareParams& p, Sweep&& sweep, BSum&& bsum, BMax&& bmax, BMaxIdx&& bmaxidx,
+                                            Emit&& emit, Result&& result) {
+  const float invR = 1.0f / static_cast<float>(p.R);
+  if constexpr (OP == OP_MAX) {
+    MaxIdx m = {-CUDART_INF_F, 0x7fffffff};
+    sweep(true, [&](float v, uint32_t r) { m = max_combine(m, MaxIdx{v, static_cast<int>(r)}); });
+    m = bmaxidx(m);
+    result(m.v, m.i);
+  } else if constexpr (OP == OP_SUM || OP == OP_MEAN) {
+    float s = 0.f;
+    sweep(true, [&](float v, uint32_t) { s += v; });
+    s = bsum(s, 0);
+    result(OP == OP_MEAN ? s * invR : s, 0);
+  } else if constexpr (OP == OP_SOFTMAX) {
+    float m = -CUDART_INF_F;
+    sweep(true, [&](float v, uint32_t) { m = fmaxf(m, v); });
+    m = bmax(m, 0);
+    float s = 0.f;
+    sweep(false, [&](float v, uint32_t) { s += __expf(v - m); });
+    const float inv = 1.0f / bsum(s, 1);
+    emit([&](float v) { return __expf(v - m) * inv; });
+  } else if constexpr (OP == OP_RMSNORM) {
+    float ss = 0.f;
+    sweep(true, [&](float v, uint32_t) { ss = fmaf(v, v, ss); });
+    const float inv = 1.0f / sqrtf(bsum(ss, 0) * invR + p.eps);
+    emit([&](float v) { return v * inv; });
+  } else if constexpr (OP == OP_LPNORM) {
+    float s = 0.f;
+    sweep(true, [&](float v, uint32_t) { s += powf(fabsf(v), p.lp); });
+    const float den = powf(bsum(s, 0) + p.eps, 1.0f / p.lp);
+    emit([&](float v) { return v / den; });
+  } else {
+    float s = 0.f;
+    sweep(true, [&](float v, uint32_t) { s += v; });
+    const float mu = bsum(s, 0) * invR;
+    float ss = 0.f;
+    sweep(false, [&](float v, uint32_t) { ss = fmaf(v - mu, v - mu, ss); });
+    const float inv = 1.0f / sqrtf(bsum(ss, 1) * invR + p.eps);
+    emit([&](float v) { return (v - mu) * inv; });
+  }
+}
+
+template <int OP, int VEC, int THREADS>
+__global__ void __launch_bounds__(THREADS) span_kernel(const ShareParams p) {
+  extern __shared__ __align__(16) float cache[];
+  __shared__ float red[32], slot[2];
+  __shared__ int redi[32], islot;
+  const int tid = threadIdx.x;
+  const int rank = blockIdx.x % p.shares;
+  const int64_t line = blockIdx.x / p.shares;
+  int64_t xb = 0, yb = 0, wb = 0, rem = line;
+  for (int d = p.nk - 1; d >= 0; --d) {
+    const int64_t c = rem % p.kshape[d];
+    rem /= p.kshape[d];
+    xb += c * p.kxs[d];
+    yb += c * p.kys[d];
+    wb += c * p.kws[d];
+  }
+  const uint32_t begin = rank * p.share, end = min(begin + p.share, p.R);
+  auto load = [&](uint32_t r) {
+    const uint32_t r1 = p.R2 == p.R ? 0u : r / p.R2;
+    const int64_t o = xb + r1 * p.xs1 + (r - r1 * p.R2);
+    if constexpr (VEC == 4) return load4(p.x, o, p.dt_in);
+    else return F4{{load_as_f32(p.x, o, p.dt_in), 0.f, 0.f, 0.f}};
+  };
+  auto cached = [&](uint32_t r) {
+    if (!p.cached) return load(r);
+    if constexpr (VEC == 4) {
+      const float4 t = *reinterpret_cast<const float4*>(cache + (r - begin));
+      return F4{{t.x, t.y, t.z, t.w}};
+    } else {
+      return F4{{cache[r - begin], 0.f, 0.f, 0.f}};
+    }
+  };
+  auto weights = [&](const void* src, int64_t o) {
+    F4 r;
+    r.v[0] = load_as_f32(src, o, p.dt_w);
+#pragma unroll
+    for (int e = 1; e < VEC; ++e) r.v[e] = p.ws2 == 0 ? r.v[0] : load_as_f32(src, o + e * p.ws2, p.dt_w);
+    return r;
+  };
+  auto sweep = [&](bool first, auto f) {
+    constexpr uint32_t STEP = THREADS * VEC;
+    for (uint32_t r0 = begin + tid * VEC; r0 < end; r0 += STEP * SHARE_UNROLL) {
+      F4 x[SHARE_UNROLL];
+#pragma unroll
+      for (int u = 0; u < SHARE_UNROLL; ++u)
+        if (r0 + u * STEP < end) x[u] = first ? load(r0 + u * STEP) : cached(r0 + u * STEP);
+#pragma unroll
+      for (int u = 0; u < SHARE_UNROLL; ++u) {
+        const uint32_t r = r0 + u * STEP;
+        if (r >= end) break;
+        if (first && p.cached && OP != OP_SUM && OP != OP_MEAN && OP != OP_MAX) {
+          if constexpr (VEC == 4) *reinterpret_cast<float4*>(cache + (r - begin)) = make_float4(x[u].v[0], x[u].v[1], x[u].v[2], x[u].v[3]);
+          else cache[r - begin] = x[u].v[0];
+        }
+#pragma unroll
+        for (int e = 0; e < VEC; ++e) f(x[u].v[e], r + e);
+      }
+    }
+  };
+  line_passes<OP>(
+      p, sweep,
+      [&](float v, int k) { return over_shares(group_sum<THREADS>(v, red, 0, tid), &slot[k], tid == 0, p.shares, ShareSum{}); },
+      [&](float v, int k) { return over_shares(group_max<THREADS>(v, red, 0, tid), &slot[k], tid == 0, p.shares, ShareMax{}); },
+      [&](MaxIdx m) { return over_shares(group_maxidx<THREADS>(m, red, redi, 0, tid), &slot[0], &islot, tid == 0, p.shares); },
+      [&](auto g) {
+        // (gamma and beta of several trips are asked for before the first result is stored: one trip to the L2 for all)
+        constexpr uint32_t STEP = THREADS * VEC;
+        for (uint32_t r0 = begin + tid * VEC; r0 < end; r0 += STEP * SHARE_UNROLL) {
+          F4 v[SHARE_UNROLL], wv[SHARE_UNROLL], bv[SHARE_UNROLL];
+#pragma unroll
+          for (int u = 0; u < SHARE_UNROLL; ++u) {
+            const uint32_t r = r0 + u * STEP;
+            if (r >= end) break;
+            const uint32_t r1 = p.R2 == p.R ? 0u : r / p.R2;
+            const int64_t wo = wb + r1 * p.ws1 + (r - r1 * p.R2) * p.ws2;
+            v[u] = cached(r);
+            if (p.w) wv[u] = weights(p.w, wo);
+            if (p.b) bv[u] = weights(p.b, wo);
+          }
+#pragma unroll
+          for (int u = 0; u < SHARE_UNROLL; ++u) {
+            const uint32_t r = r0 + u * STEP;
+            if (r >= end) break;
+            const uint32_t r1 = p.R2 == p.R ? 0u : r / p.R2;
+#pragma unroll
+            for (int e = 0; e < VEC; ++e) {
+              v[u].v[e] = g(v[u].v[e]);
+              if (p.w) v[u].v[e] *= wv[u].v[e];
+              if (p.b) v[u].v[e] += bv[u].v[e];
+            }
+            const int64_t o = yb + r1 * p.ys1 + (r - r1 * p.R2);
+            if constexpr (VEC == 4) store4(p.y, o, v[u], p.dt_out);
+            else store_from_f32(p.y, o, v[u].v[0], p.dt_out);
+          }
+        }
+      },
+      [&](float v, int i) {
+        if (rank != 0 || tid != 0) return;
+        if (OP == OP_MAX && i == 0x7fffffff) {  // every element failed `>` (all NaN): the reference keeps element 0
+          v = load_as_f32(p.x, xb, p.dt_in);
+          i = 0;
+        }
+        store_from_f32(p.y, yb, v, p.dt_out);
+        if (OP == OP_MAX && p.idx) p.idx[line] = i;
+      });
+  if (p.shares > 1) cluster_sync_all();  // the others may still read this CTA's partial results
+}
+
+template <int OP, int THREADS>
+__global__ void __launch_bounds__(THREADS) column_kernel(const ShareParams p) {
+  constexpr int ROWS = THREADS / 32;
+  extern __shared__ __align__(16) float cache[];  // [share][32]
+  __shared__ float red[ROWS][32], slot[2][32];
+  __shared__ int redi[ROWS][32], islot[32];
+  const int lane = threadIdx.x & 31, q = threadIdx.x >> 5;
+  const int rank = blockIdx.x % p.shares;
+  const int64_t tiles = (p.cols + 31) / 32, item = blockIdx.x / p.shares;
+  const int64_t outer = item / tiles, col = (item - outer * tiles) * 32 + lane;
+  int64_t xb = col, yb = col, wb = col * p.cws, rem = outer;
+  for (int d = p.nk - 1; d >= 0; --d) {
+    const int64_t c = rem % p.kshape[d];
+    rem /= p.kshape[d];
+    xb += c * p.kxs[d];
+    yb += c * p.kys[d];
+    wb += c * p.kws[d];
+  }
+  const bool on = col < p.cols;
+  const uint32_t begin = rank * p.share, end = on ? min(begin + p.share, p.R) : 0u;
+  auto sweep = [&](bool first, auto f) {
+    constexpr int U = 2 * SHARE_UNROLL;
+    for (uint32_t r0 = begin + q; r0 < end; r0 += ROWS * U) {
+      float x[U];
+#pragma unroll
+      for (int u = 0; u < U; ++u) {
+        const uint32_t r = r0 + u * ROWS;
+        if (r < end) x[u] = !first && p.cached ? cache[(r - begin) * 32 + lane] : load_as_f32(p.x, xb + r * p.xs1, p.dt_in);
+      }
+#pragma unroll
+      for (int u = 0; u < U; ++u) {
+        const uint32_t r = r0 + u * ROWS;
+        if (r >= end) break;
+        if (first && p.cached && OP != OP_SUM && OP != OP_MEAN && OP != OP_MAX) cache[(r - begin) * 32 + lane] = x[u];
+        f(x[u], r);
+      }
+    }
+  };
+  auto down = [&](float v, auto f) {  // over the eight threads of a column, in their order
+    red[q][lane] = v;
+    __syncthreads();
+    v = red[0][lane];
+#pragma unroll
+    for (int i = 1; i < ROWS; ++i) v = f(v, red[i][lane]);
+    __syncthreads();
+    return v;
+  };
+  line_passes<OP>(
+      p, sweep, [&](float v, int k) { return over_shares(down(v, ShareSum{}), &slot[k][lane], q == 0, p.shares, ShareSum{}); },
+      [&](float v, int k) { return over_shares(down(v, ShareMax{}), &slot[k][lane], q == 0, p.shares, ShareMax{}); },
+      [&](MaxIdx m) {
+        red[q][lane] = m.v;
+        redi[q][lane] = m.i;
+        __syncthreads();
+#pragma unroll
+        for (int i = 0; i < ROWS; ++i) m = max_combine(m, MaxIdx{red[i][lane], redi[i][lane]});
+        return over_shares(m, &slot[0][lane], &islot[lane], q == 0, p.shares);
+      },
+      [&](auto g) {
+        for (uint32_t r0 = begin + q; r0 < end; r0 += ROWS * SHARE_UNROLL) {
+          float v[SHARE_UNROLL], wv[SHARE_UNROLL], bv[SHARE_UNROLL];
+#pragma unroll
+          for (int u = 0; u < SHARE_UNROLL; ++u) {
+            const uint32_t r = r0 + u * ROWS;
+            if (r >= end) break;
+            v[u] = p.cached ? cache[(r - begin) * 32 + lane] : load_as_f32(p.x, xb + r * p.xs1, p.dt_in);
+            if (p.w) wv[u] = load_as_f32(p.w, wb + r * p.ws1, p.dt_w);
+            if (p.b) bv[u] = load_as_f32(p.b, wb + r * p.ws1, p.dt_w);
+          }
+#pragma unroll
+          for (int u = 0; u < SHARE_UNROLL; ++u) {
+            const uint32_t r = r0 + u * ROWS;
+            if (r >= end) break;
+            v[u] = g(v[u]);
+            if (p.w) v[u] *= wv[u];
+            if (p.b) v[u] += bv[u];
+            store_from_f32(p.y, yb + r * p.ys1, v[u], p.dt_out);
+          }
+        }
+      },
+      [&](float v, int i) {
+        if (rank != 0 || q != 0 || !on) return;
+        if (OP == OP_MAX && i == 0x7fffffff) {
+          v = load_as_f32(p.x, xb, p.dt_in);
+          i = 0;
+        }
+        store_from_f32(p.y, yb, v, p.dt_out);
+        if (OP == OP_MAX && p.idx) p.idx[outer * p.cols + col] = i;
+      });
+  if (p.shares > 1) cluster_sync_all();
+}
+
 // ------------------------------------------------------------------ few lines, long reductions
 // sum / mean / max over very many elements per output (e.g. a whole-tensor sum) would leave all but a
 // few SMs idle with one CTA per line. The reduced range of every line is cut into `chunks` pieces, one
@@ -657,32 +1000,36 @@ static int normalize_axes(const NdArgs& a, int* ax, bool* used, const char* who)
   return YTC_OK;
 }
 
-template <int OP, int G>
+template <int OP, int G, int VEC>
 static void launch_row(const RowParams& p, cudaStream_t st) {
   constexpr int THREADS = G < 256 ? 256 : G;
   constexpr int RPC = THREADS / G;
   const int64_t row_blocks = (p.rows + RPC - 1) / RPC;
   const int64_t cap = static_cast<int64_t>(sm_count()) * (2048 / THREADS) * 2;
   const int grid = static_cast<int>(row_blocks < cap ? row_blocks : cap);
-  (void)launch_overlapped(row_kernel<OP, G>, dim3(grid), dim3(THREADS), 0, st, p);
+  (void)launch_overlapped(row_kernel<OP, G, VEC>, dim3(grid), dim3(THREADS), 0, st, p);
   count_launch();
 }
-template <int OP>
+template <int OP, int VEC>
 static void launch_row_g(const RowParams& p, cudaStream_t st) {
-  if (p.L <= 512) launch_row<OP, 32>(p, st);
-  else if (p.L <= 2048) launch_row<OP, 128>(p, st);
-  else if (p.L <= 4096) launch_row<OP, 256>(p, st);
-  else launch_row<OP, 1024>(p, st);
+  if (p.L <= 512) launch_row<OP, 32, VEC>(p, st);
+  else if (p.L <= 2048) launch_row<OP, 128, VEC>(p, st);
+  else if (p.L <= 4096) launch_row<OP, 256, VEC>(p, st);
+  else if (p.L <= 8192) launch_row<OP, 512, VEC>(p, st);
+  else launch_row<OP, 1024, VEC>(p, st);
 }
+template <int VEC>
 static void launch_row_op(int op, const RowParams& p, cudaStream_t st) {
   switch (op) {
-    case OP_SOFTMAX: launch_row_g<OP_SOFTMAX>(p, st); break;
-    case OP_RMSNORM: launch_row_g<OP_RMSNORM>(p, st); break;
-    case OP_LAYERNORM: launch_row_g<OP_LAYERNORM>(p, st); break;
-    case OP_CHAIN: launch_row_g<OP_CHAIN>(p, st); break;
-    case OP_SUM: launch_row_g<OP_SUM>(p, st); break;
-    case OP_MEAN: launch_row_g<OP_MEAN>(p, st); break;
-    default: launch_row_g<OP_MAX>(p, st); break;
+    case OP_SOFTMAX: launch_row_g<OP_SOFTMAX, VEC>(p, st); break;
+    case OP_RMSNORM: launch_row_g<OP_RMSNORM, VEC>(p, st); break;
+    case OP_LAYERNORM: launch_row_g<OP_LAYERNORM, VEC>(p, st); break;
+    case OP_CHAIN:
+      if constexpr (VEC == 4) launch_row_g<OP_CHAIN, VEC>(p, st);
+      break;
+    case OP_SUM: launch_row_g<OP_SUM, VEC>(p, st); break;
+    case OP_MEAN: launch_row_g<OP_MEAN, VEC>(p, st); break;
+    default: launch_row_g<OP_MAX, VEC>(p, st); break;
   }
 }
 template <int OP>
@@ -709,11 +1056,138 @@ static void launch_line_op(int op, const LineParams& p, bool per_thread, cudaStr
   }
 }
 
+// Launches span_kernel or column_kernel where the dims allow it; YTC_UNSUPPORTED: nothing was launched. `ws`: strides of gamma
+// and beta per dim, null: they are laid out like the reduced dims.
+template <class K>
+static int launch_share(K kernel, const ShareParams& p, int64_t blocks, int threads, size_t smem, cudaStream_t st) {
+  const int s = ensure_dynamic_smem(reinterpret_cast<const void*>(kernel), static_cast<int>(smem));
+  if (s != YTC_OK) return s;
+  cudaLaunchConfig_t cfg{};
+  cfg.gridDim = dim3(static_cast<unsigned>(blocks));
+  cfg.blockDim = dim3(threads);
+  cfg.dynamicSmemBytes = smem;
+  cfg.stream = st;
+  cudaLaunchAttribute attr[1];
+  attr[0].id = cudaLaunchAttributeClusterDimension;
+  attr[0].val.clusterDim.x = p.shares;
+  attr[0].val.clusterDim.y = attr[0].val.clusterDim.z = 1;
+  cfg.attrs = attr;
+  cfg.numAttrs = 1;
+  YTC_CUDA(cudaLaunchKernelEx(&cfg, kernel, p));
+  count_launch();
+  return YTC_OK;
+}
+template <int OP, int THREADS>
+static int launch_share_op(int kind, const ShareParams& p, int64_t blocks, size_t smem, cudaStream_t st) {
+  if (kind == 0) return launch_share(column_kernel<OP, THREADS>, p, blocks, THREADS, smem, st);
+  return kind == 4 ? launch_share(span_kernel<OP, 4, THREADS>, p, blocks, THREADS, smem, st)
+                   : launch_share(span_kernel<OP, 1, THREADS>, p, blocks, THREADS, smem, st);
+}
+template <int OP>
+static int launch_share_threads(int kind, const ShareParams& p, int64_t blocks, size_t smem, bool many, cudaStream_t st) {
+  return many ? launch_share_op<OP, 1024>(kind, p, blocks, smem, st) : launch_share_op<OP, 256>(kind, p, blocks, smem, st);
+}
+static int launch_shared_line(int op, const LineParams& lp, const NdArgs& a, const int64_t* ws, bool reduce_out, cudaStream_t st) {
+  if (lp.R < 2 || lp.R > 0x3fffffff) return YTC_UNSUPPORTED;
+  ShareParams p{};
+  p.x = lp.x; p.y = lp.y; p.w = lp.w; p.b = lp.b; p.idx = lp.idx;
+  p.eps = lp.eps; p.lp = lp.lp; p.dt_in = lp.dt_in; p.dt_out = lp.dt_out; p.dt_w = lp.dt_w;
+  p.R = static_cast<uint32_t>(lp.R);
+  // the reduced dims in listed order, neighbours joined where x, y and the weights allow it
+  int nr = 0;
+  int64_t shape[MAXD], xs[MAXD], ys[MAXD], wst[MAXD];
+  for (int i = 0; i < lp.nr; ++i) {
+    if (lp.rshape[i] == 1) continue;
+    const int ax = ((a.axes[i] % a.ndim) + a.ndim) % a.ndim;
+    const int64_t wd = ws ? ws[ax] : lp.rws[i];
+    if (nr > 0 && xs[nr - 1] == lp.rxs[i] * lp.rshape[i] && (reduce_out || ys[nr - 1] == lp.rys[i] * lp.rshape[i]) &&
+        (!lp.w || wst[nr - 1] == wd * lp.rshape[i])) {
+      shape[nr - 1] *= lp.rshape[i];
+      xs[nr - 1] = lp.rxs[i];
+      ys[nr - 1] = lp.rys[i];
+      wst[nr - 1] = wd;
+      continue;
+    }
+    shape[nr] = lp.rshape[i];
+    xs[nr] = lp.rxs[i];
+    ys[nr] = lp.rys[i];
+    wst[nr++] = wd;
+  }
+  // the kept dims
+  for (int d = 0, k = 0; d < a.ndim; ++d) {
+    bool reduced = false;
+    for (int i = 0; i < a.naxes; ++i) reduced = reduced || ((a.axes[i] % a.ndim) + a.ndim) % a.ndim == d;
+    if (reduced) continue;
+    if (lp.kshape[k] != 1) {
+      p.kshape[p.nk] = lp.kshape[k];
+      p.kxs[p.nk] = lp.kxs[k];
+      p.kys[p.nk] = lp.kys[k];
+      p.kws[p.nk++] = ws ? ws[d] : 0;
+    }
+    ++k;
+  }
+  const int sms = sm_count();
+  int kind;
+  int64_t lines;       // items of one cluster each
+  uint32_t floats = 1;  // of the cache per element of a share
+  if (nr <= 2 && xs[nr - 1] == 1 && (reduce_out || ys[nr - 1] == 1)) {
+    p.R2 = static_cast<uint32_t>(shape[nr - 1]);
+    p.ws2 = wst[nr - 1];
+    if (nr == 2) {
+      p.xs1 = xs[0];
+      p.ys1 = ys[0];
+      p.ws1 = wst[0];
+    }
+    const int ein = dtype_size(lp.dt_in), eout = dtype_size(lp.dt_out);
+    bool quads = p.R2 % 4 == 0 && reinterpret_cast<uint64_t>(lp.x) % (4 * ein) == 0 && p.xs1 % 4 == 0 &&
+                 (reduce_out || (reinterpret_cast<uint64_t>(lp.y) % (4 * eout) == 0 && p.ys1 % 4 == 0));
+    for (int d = 0; d < p.nk; ++d) quads = quads && p.kxs[d] % 4 == 0 && (reduce_out || p.kys[d] % 4 == 0);
+    kind = quads ? 4 : 1;
+    lines = lp.lines;
+  } else if (nr == 1 && p.nk > 0 && p.kxs[p.nk - 1] == 1 && p.kys[p.nk - 1] == 1 && p.kshape[p.nk - 1] >= 8) {
+    --p.nk;
+    p.cols = p.kshape[p.nk];
+    p.cws = p.kws[p.nk];
+    p.xs1 = xs[0];
+    p.ys1 = ys[0];
+    p.ws1 = wst[0];
+    kind = 0;
+    lines = lp.lines / p.cols * ((p.cols + 31) / 32);
+    floats = 32;
+  } else {
+    return YTC_UNSUPPORTED;
+  }
+  // Shares: enough CTAs for two per SM while a share keeps 2048 elements, and shares of half an SM's shared memory.
+  int shares = 1;
+  auto share_of = [&](int n) { return ((p.R + n - 1) / n + 3) / 4 * 4; };
+  while (shares < MAX_SHARES && ((lines * shares < 2 * sms && static_cast<uint64_t>(share_of(shares)) * floats >= 4096) ||
+                                 static_cast<uint64_t>(share_of(shares)) * floats > CACHE_FLOATS / 2))
+    shares *= 2;
+  if (lines * shares > 0x7fffffff) return YTC_UNSUPPORTED;
+  p.shares = shares;
+  p.share = share_of(shares);
+  const bool keeps = op != OP_SUM && op != OP_MEAN && op != OP_MAX;
+  p.cached = keeps && static_cast<uint64_t>(p.share) * floats <= CACHE_FLOATS;
+  const size_t smem = p.cached ? static_cast<size_t>(p.share) * floats * 4 : 0;
+  // A share of which only one fits an SM needs more threads to keep enough loads in flight (batchNorm, bf16, 32 x 256 x 112 x
+  // 112: 1617 us with 256 threads, 605 with 1024); where more fit, 256 are faster (16 x 96 x 56 x 56 fp32: 25 us, 37).
+  const bool many = smem > 110 * 1024;
+  switch (op) {
+    case OP_SOFTMAX: return launch_share_threads<OP_SOFTMAX>(kind, p, lines * shares, smem, many, st);
+    case OP_RMSNORM: return launch_share_threads<OP_RMSNORM>(kind, p, lines * shares, smem, many, st);
+    case OP_LAYERNORM: return launch_share_threads<OP_LAYERNORM>(kind, p, lines * shares, smem, many, st);
+    case OP_LPNORM: return launch_share_threads<OP_LPNORM>(kind, p, lines * shares, smem, many, st);
+    case OP_SUM: return launch_share_threads<OP_SUM>(kind, p, lines * shares, smem, many, st);
+    case OP_MEAN: return launch_share_threads<OP_MEAN>(kind, p, lines * shares, smem, many, st);
+    default: return launch_share_threads<OP_MAX>(kind, p, lines * shares, smem, many, st);
+  }
+}
+
 // Shared driver of all N-d reductions. `reduce_out` = the output keeps size-1 dims on the reduced axes
 // (sum / mean / max) instead of the input's shape (softmax / norms).
 static int run_nd(int op, int dt_in, int dt_out, int dt_w, const void* x, void* y, const void* w, const void* b,
                   int* idx, const NdArgs& a, float eps, bool reduce_out, cudaStream_t st, const char* who,
-                  void* scratch = nullptr, size_t scratch_bytes = 0, float lp = 2.f) {
+                  void* scratch = nullptr, size_t scratch_bytes = 0, float lp = 2.f, const int64_t* ws = nullptr) {
   int ax[MAXD];
   bool used[MAXD];
   int s = normalize_axes(a, ax, used, who);
@@ -728,7 +1202,7 @@ static int run_nd(int op, int dt_in, int dt_out, int dt_w, const void* x, void* 
   const int64_t lines = total / R;
 
   // Fast path: the reduced axes are the trailing dims in ascending listed order, contiguous in x (and in y
-  // for the shape-preserving ops), rows 16-byte aligned.
+  // for the shape-preserving ops).
   bool trailing = true;
   for (int i = 0; i < a.naxes; ++i)
     if (ax[i] != a.ndim - a.naxes + i) trailing = false;
@@ -760,17 +1234,21 @@ static int run_nd(int op, int dt_in, int dt_out, int dt_w, const void* x, void* 
     if (reduce_out && lines > 1 && y_rs != 1) trailing = false;
   }
   const int esz_in = dtype_size(dt_in), esz_out = dtype_size(dt_out);
-  if (op != OP_LPNORM && trailing && R % 4 == 0 && R <= 16384 && x_rs >= 0 && y_rs >= 0 &&
-      (reinterpret_cast<uint64_t>(x) % (4 * esz_in)) == 0 && (x_rs * esz_in) % (4 * esz_in) == 0 &&
-      (reduce_out || ((reinterpret_cast<uint64_t>(y) % (4 * esz_out)) == 0 && (y_rs * esz_out) % (4 * esz_out) == 0)) &&
-      (!w || reinterpret_cast<uint64_t>(w) % (4 * dtype_size(dt_w)) == 0) &&
-      (!b || reinterpret_cast<uint64_t>(b) % (4 * dtype_size(dt_w)) == 0)) {
+  const bool spread = ws != nullptr;  // gamma / beta by strides of their own: the span kernel alone knows them
+  // Rows that can't be read four at a time take single loads: 32 lanes still read neighbours. Measured, rmsNorm bf16
+  // 4096 x 8191: 77 us, 323 with line_kernel; 8192 wide 4 at a time 39.
+  const bool quads = R % 4 == 0 && (reinterpret_cast<uint64_t>(x) % (4 * esz_in)) == 0 && x_rs % 4 == 0 &&
+                     (reduce_out || ((reinterpret_cast<uint64_t>(y) % (4 * esz_out)) == 0 && y_rs % 4 == 0)) &&
+                     (!w || reinterpret_cast<uint64_t>(w) % (4 * dtype_size(dt_w)) == 0) &&
+                     (!b || reinterpret_cast<uint64_t>(b) % (4 * dtype_size(dt_w)) == 0);
+  if (op != OP_LPNORM && trailing && !spread && R <= 16384 && x_rs >= 0 && y_rs >= 0) {
     RowParams p;
     p.x = x; p.y = y; p.w = w; p.b = b; p.idx = idx;
     p.rows = lines; p.L = static_cast<int>(R);
     p.x_rs = x_rs; p.y_rs = y_rs; p.r_rows = 1; p.eps = eps;
     p.dt_in = dt_in; p.dt_out = dt_out; p.dt_w = dt_w;
-    launch_row_op(op, p, st);
+    if (quads) launch_row_op<4>(op, p, st);
+    else launch_row_op<1>(op, p, st);
     YTC_CUDA(cudaGetLastError());
     return YTC_OK;
   }
@@ -805,7 +1283,7 @@ static int run_nd(int op, int dt_in, int dt_out, int dt_w, const void* x, void* 
     p.rws[i] = wstride[ax[i]];
   }
   // few outputs, long reductions: split every line over several CTAs through a scratch buffer
-  if (reduce_out && lines <= 2 * sm_count() && R >= 32768) {
+  if (reduce_out && !spread && lines <= 2 * sm_count() && R >= 32768) {
     SplitParams sp;
     sp.lp = p;
     int64_t chunks = (4ll * sm_count() + lines - 1) / lines;
@@ -850,9 +1328,26 @@ static int run_nd(int op, int dt_in, int dt_out, int dt_w, const void* x, void* 
     YTC_CUDA(cudaGetLastError());
     return YTC_OK;
   }
+  const int shared = launch_shared_line(op, p, a, ws, reduce_out, st);
+  if (shared != YTC_UNSUPPORTED) return shared;
+  if (spread) {
+    set_last_error("%s: these strides are not supported", who);
+    return YTC_UNSUPPORTED;
+  }
   // one thread per line when neighbouring lines sit next to each other in memory
   const bool per_thread = p.nk > 0 && p.kxs[p.nk - 1] == 1 && p.kshape[p.nk - 1] >= 32 && lines >= 4096;
   launch_line_op(op, p, per_thread, st);
+  YTC_CUDA(cudaGetLastError());
+  return YTC_OK;
+}
+
+int rmsnorm_planes(const float* x, const float* w, uint16_t* planes, int64_t rows, int hidden, float eps, cudaStream_t st) {
+  YTC_REQUIRE(hidden % 4 == 0 && hidden <= 16384, "rmsnorm_planes: rows of %d", hidden);
+  RowParams p{};
+  p.x = x; p.y = planes; p.w = w;
+  p.rows = rows; p.L = hidden; p.x_rs = p.y_rs = hidden; p.r_rows = 1; p.eps = eps;
+  p.dt_in = p.dt_w = YTC_F32; p.dt_out = YTC_BF16;
+  launch_row_g<OP_RMSPLANES, 4>(p, st);
   YTC_CUDA(cudaGetLastError());
   return YTC_OK;
 }
@@ -961,6 +1456,16 @@ int ytcuda_layernorm(int dt_in, int dt_out, int dt_w, const void* x, const void*
                 static_cast<cudaStream_t>(stream), "ytcuda_layernorm");
 }
 
+int ytcuda_layernorm_strided(int dt_in, int dt_out, int dt_w, const void* x, const void* gamma, const void* beta, void* y,
+                             const int64_t* shape, const int64_t* xstrides, const int64_t* ystrides, const int64_t* wstrides,
+                             int ndim, const int* axes, int naxes, float eps, void* stream) {
+  YTC_REQUIRE(shape && xstrides && ystrides && wstrides && axes, "ytcuda_layernorm_strided: null shape/strides/axes");
+  YTC_REQUIRE(gamma && beta, "ytcuda_layernorm_strided: null gamma/beta");
+  NdArgs a{shape, xstrides, ystrides, ndim, axes, naxes};
+  return run_nd(OP_LAYERNORM, dt_in, dt_out, dt_w, x, y, gamma, beta, nullptr, a, eps, false,
+                static_cast<cudaStream_t>(stream), "ytcuda_layernorm_strided", nullptr, 0, 2.f, wstrides);
+}
+
 int ytcuda_reduce(int op, int dt_in, int dt_out, const void* x, void* y, int32_t* index, const int64_t* shape,
                   const int64_t* xstrides, int ndim, const int* axes, int naxes, void* stream) {
   YTC_REQUIRE(op >= 0 && op <= 2, "ytcuda_reduce: op must be 0 (sum), 1 (mean) or 2 (max)");
@@ -1013,7 +1518,7 @@ int ytcuda_rmsnorm_add_softmax_cast(int dt_out, const float* x, const float* wei
     YTC_CUDA(cudaGetLastError());
     return YTC_OK;
   }
-  launch_row_op(OP_CHAIN, p, static_cast<cudaStream_t>(stream));
+  launch_row_op<4>(OP_CHAIN, p, static_cast<cudaStream_t>(stream));
   YTC_CUDA(cudaGetLastError());
   return YTC_OK;
 }
