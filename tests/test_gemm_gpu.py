@@ -376,3 +376,36 @@ def test_host_buffer_variant_matches_device(L, api):
                                   1.0, 0.0, 1024, 1, 768, 1, 800, 1, 6, 512 * 1024, 0, 512 * 800))
     assert torch.equal(cv, want)
     assert torch.all(cbig[:, :, 768:] == 7.0)  # the gap between rows is left alone
+
+
+# ------------------------------------------------------------------ rewritten operands, k in pieces
+@pytest.mark.parametrize("dt", [torch.float32, torch.bfloat16, torch.float16])
+@pytest.mark.parametrize("batch,m,n,k,form", [
+    (1, 60, 1001, 1111, "shared"), (1, 257, 513, 1027, "linear"), (3, 129, 255, 777, "batched"), (2, 300, 301, 517, "shared"),
+    (1, 16, 4096, 4096, "shared"), (1, 1, 700, 2048, "linear"), (1, 100, 130, 4104, "columns"), (2, 64, 96, 8191, "batched")])
+def test_odd_sizes_and_k_pieces(api, dt, batch, m, n, k, form):
+    gen = torch.Generator(device="cuda").manual_seed(m * n + k)
+    a = torch.randn(batch, m, k, generator=gen, device="cuda").to(dt)
+    b = (torch.randn(*([batch] if form == "batched" else []), k, n, generator=gen, device="cuda") * k ** -0.5).to(dt)
+    if form == "columns":  # both operands by columns
+        a, b = a.transpose(-1, -2).contiguous().transpose(-1, -2), b.transpose(-1, -2).contiguous().transpose(-1, -2)
+    if form == "linear":
+        got = api.linear(a, b.transpose(-1, -2).contiguous())
+    else:
+        got = api.matmul(a, b)
+    want = a.double() @ b.double()
+    # fp32: a rounding per partial sum; 16 bits: the rounding of the result (bf16 by the reference's rule: up to one unit)
+    tol = {torch.float32: 2e-6, torch.bfloat16: 2.0 ** -7, torch.float16: 2.0 ** -11}[dt]
+    assert (got.double() - want).abs().max() <= tol * want.abs().max()
+
+
+def test_small_fp32_products_keep_infinities(api):
+    gen = torch.Generator(device="cuda").manual_seed(9)
+    a, b = torch.randn(64, 2050, generator=gen, device="cuda"), torch.randn(2050, 1500, generator=gen, device="cuda")
+    a[5, 9] = float("inf")
+    b[:, 77] = 0.0
+    want = a.double() @ b.double()
+    got = api.matmul(a, b)
+    assert torch.equal(got.isnan(), want.isnan()) and torch.equal(got.isinf(), want.isinf())
+    fin = want.isfinite()
+    assert (got.double() - want)[fin].abs().max() <= 1e-5 * want[fin].abs().max()

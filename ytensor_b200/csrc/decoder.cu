@@ -366,6 +366,23 @@ __global__ void __launch_bounds__(256) sum_swiglu_split_kernel(const float* part
   }
 }
 
+// The same from the finished projection [rows][2 * inter].
+__global__ void __launch_bounds__(256) swiglu_split_kernel(const float* gu, uint16_t* hi, uint16_t* lo, int64_t rows, int inter) {
+  dependent_wait();
+  dependent_trigger();
+  const int per_row = inter / 4;
+  const int64_t total = rows * per_row;
+  for (int64_t i = blockIdx.x * static_cast<int64_t>(blockDim.x) + threadIdx.x; i < total;
+       i += static_cast<int64_t>(gridDim.x) * blockDim.x) {
+    const int64_t r = i / per_row;
+    const int c = static_cast<int>(i - r * per_row) * 4;
+    const float4 g = *reinterpret_cast<const float4*>(gu + r * 2 * inter + c);
+    const float4 u = *reinterpret_cast<const float4*>(gu + r * 2 * inter + inter + c);
+    const float f[4] = {ds_swish(g.x) * u.x, ds_swish(g.y) * u.y, ds_swish(g.z) * u.z, ds_swish(g.w) * u.w};
+    split_store4(f, hi + r * inter + c, lo + r * inter + c);
+  }
+}
+
 // ------------------------------------------------------------------ per-head RMSNorm + RoPE + KV append
 // qkv [B, L, (H + 2*KVH) * D] fp32 (the fused projection output). One warp per (b, t, head) vector, D == 128:
 //   q heads: rmsNorm over D with q_norm, rotate-half RoPE at position pos0 + t -> q_out [B, H, L, D]
@@ -552,7 +569,7 @@ static int gemm_pieces(Qwen3Model* m, const uint16_t* W, int64_t M, int N, int K
   out->part = part;
   out->n = splits;
   out->mn = M * N;
-  return ytcuda_gemm(YTC_BF16, YTC_F32, m->hi, W, part, static_cast<int>(2 * M), N, kc, 1.f, 0.f, K, 1, 1, K, N, 1, splits,
+  return gemm_into_workspace(YTC_BF16, YTC_F32, m->hi, W, part, static_cast<int>(2 * M), N, kc, 1.f, 0.f, K, 1, 1, K, N, 1, splits,
                      kc, kc, 2 * out->mn, st);
 }
 
@@ -607,12 +624,10 @@ static int linear_w16(Qwen3Model* m, const float* x, int64_t x_rs, const uint16_
     YTC_CUDA(cudaGetLastError());
     return YTC_OK;
   }
-  // many rows: split the activation into two bf16 planes and run the tensor-core GEMM on each. The lo plane follows
-  // the hi plane: [2 M][K] is then one left operand whose rows M .. 2 M - 1 are the lo plane.
+  // many rows: split the activation into two bf16 planes and multiply both on the tensor cores. The lo plane
+  // follows the hi plane: [2 M][K] is then one left operand whose rows M .. 2 M - 1 are the lo plane.
   int s = split_planes(m, x, x_rs, M, K, st);
   if (s != YTC_OK) return s;
-  uint16_t* hi = m->hi;
-  uint16_t* lo = m->hi + M * K;
   // Few rows (decode with a larger batch): there are only N / 128 output tiles, too few to keep the SMs busy and the
   // weight stream at bandwidth. The k range is cut into pieces that run as "batch" items of one GEMM launch (a k
   // offset is a plain pointer offset for both K-major operands), each writing its own partial result, and a small
@@ -628,11 +643,7 @@ static int linear_w16(Qwen3Model* m, const float* x, int64_t x_rs, const uint16_
     YTC_CUDA(cudaGetLastError());
     return YTC_OK;
   }
-  s = ytcuda_gemm(YTC_BF16, YTC_F32, hi, W, y, static_cast<int>(M), N, K, 1.f, accumulate ? 1.f : 0.f, K, 1, 1,
-                      K, y_rs, 1, 1, 0, 0, 0, st);
-  if (s != YTC_OK) return s;
-  return ytcuda_gemm(YTC_BF16, YTC_F32, lo, W, y, static_cast<int>(M), N, K, 1.f, 1.f, K, 1, 1, K, y_rs, 1, 1, 0, 0,
-                     0, st);
+  return linear_two_planes(m->hi, W, y, y_rs, static_cast<int>(M), N, K, accumulate, st);
 }
 
 static int rmsnorm_rows(const float* x, const float* w, float* y, int64_t rows, int hidden, float eps, cudaStream_t st) {
@@ -1304,12 +1315,20 @@ int ytcuda_qwen3_forward(void* handle, const int32_t* ids, int len, float* logit
       YTC_CUDA(cudaGetLastError());
     }
   }
+  // More rows: the norms and SwiGLU write the planes that the projection behind them reads.
+  const bool planes = rows > 128;
+  const int64_t glue_cap = static_cast<int64_t>(sm_count()) * 16;
   for (int l = fused_glue ? m->layers : 0; l < m->layers; ++l) {
     const LayerW& W = m->lw[l];
     float* kc = m->k_cache + l * cache_layer;
     float* vc = m->v_cache + l * cache_layer;
-    if ((s = rmsnorm_rows(m->x, W.norm1, m->h, rows, Hd, m->eps, st)) != YTC_OK) return s;
-    if ((s = linear_w16(m, m->h, Hd, W.qkv, m->qkv, qkv_w, rows, qkv_w, Hd, false, st)) != YTC_OK) return s;
+    if (planes) {
+      if ((s = rmsnorm_planes(m->x, W.norm1, m->hi, rows, Hd, m->eps, st)) != YTC_OK) return s;
+      if ((s = linear_two_planes(m->hi, W.qkv, m->qkv, qkv_w, static_cast<int>(rows), qkv_w, Hd, false, st)) != YTC_OK) return s;
+    } else {
+      if ((s = rmsnorm_rows(m->x, W.norm1, m->h, rows, Hd, m->eps, st)) != YTC_OK) return s;
+      if ((s = linear_w16(m, m->h, Hd, W.qkv, m->qkv, qkv_w, rows, qkv_w, Hd, false, st)) != YTC_OK) return s;
+    }
     if ((s = ytcuda_qwen3_qkv_post(m->qkv, m->q, kc, vc, W.q_norm, W.k_norm, m->cos_t, m->sin_t, B, len, m->l_heads,
                                    m->l_kv_heads, D, m->max_pos, pos0, slot0, m->eps, st)) != YTC_OK)
       return s;
@@ -1332,16 +1351,27 @@ int ytcuda_qwen3_forward(void* handle, const int32_t* ids, int len, float* logit
       }
       if ((s = add_inplace(m->x, m->proj, rows * Hd, st)) != YTC_OK) return s;
     }
-    if ((s = rmsnorm_rows(m->x, W.norm2, m->h, rows, Hd, m->eps, st)) != YTC_OK) return s;
-    if ((s = linear_w16(m, m->h, Hd, W.gate_up, m->gu, 2 * m->l_inter, rows, 2 * m->l_inter, Hd, false, st)) != YTC_OK)
-      return s;
-    if ((s = ytcuda_swiglu(YTC_F32, YTC_F32, m->gu, m->act, rows, m->l_inter, 2 * m->l_inter, m->l_inter, st)) != YTC_OK)
-      return s;
-    if (m->tp_world == 1) {  // x2 += mlp
-      if ((s = linear_w16(m, m->act, m->l_inter, W.down, m->x, Hd, rows, Hd, m->l_inter, true, st)) != YTC_OK) return s;
-    } else {
-      if ((s = linear_w16(m, m->act, m->l_inter, W.down, m->proj, Hd, rows, Hd, m->l_inter, false, st)) != YTC_OK)
+    float* mlp = m->tp_world == 1 ? m->x : m->proj;  // (x2 += mlp, or this rank's share of it)
+    if (planes) {
+      if ((s = rmsnorm_planes(m->x, W.norm2, m->hi, rows, Hd, m->eps, st)) != YTC_OK) return s;
+      if ((s = linear_two_planes(m->hi, W.gate_up, m->gu, 2 * m->l_inter, static_cast<int>(rows), 2 * m->l_inter, Hd, false, st)) != YTC_OK)
         return s;
+      const int64_t blocks = (rows * (m->l_inter / 4) + 255) / 256;
+      YTC_CUDA(launch_overlapped(swiglu_split_kernel, dim3(static_cast<unsigned>(blocks < glue_cap ? blocks : glue_cap)), dim3(256), 0,
+                                 st, m->gu, m->hi, m->hi + rows * m->l_inter, rows, m->l_inter));
+      count_launch();
+      if ((s = linear_two_planes(m->hi, W.down, mlp, Hd, static_cast<int>(rows), Hd, m->l_inter, m->tp_world == 1, st)) != YTC_OK)
+        return s;
+    } else {
+      if ((s = rmsnorm_rows(m->x, W.norm2, m->h, rows, Hd, m->eps, st)) != YTC_OK) return s;
+      if ((s = linear_w16(m, m->h, Hd, W.gate_up, m->gu, 2 * m->l_inter, rows, 2 * m->l_inter, Hd, false, st)) != YTC_OK)
+        return s;
+      if ((s = ytcuda_swiglu(YTC_F32, YTC_F32, m->gu, m->act, rows, m->l_inter, 2 * m->l_inter, m->l_inter, st)) != YTC_OK)
+        return s;
+      if ((s = linear_w16(m, m->act, m->l_inter, W.down, mlp, Hd, rows, Hd, m->l_inter, m->tp_world == 1, st)) != YTC_OK)
+        return s;
+    }
+    if (m->tp_world > 1) {
       if ((s = m->allreduce(m->proj, rows * Hd, m->allreduce_user)) != 0) {
         set_last_error("ytcuda_qwen3_forward: all-reduce callback failed with %d", s);
         return YTC_CUDA_ERROR;

@@ -37,6 +37,11 @@ struct GemmTcParams {
   int tiles_m, tiles_n, total_tiles, k_blocks;
   int a_prefetch;  // k-blocks by which an L2 prefetch of A runs ahead of the shared-memory loads (0 = off)
   int split_loads; // K-major tiles fetched as 64-row boxes
+  // a product of planes (TcPlanes): `fold` blocks of k of one pair of planes after another; 0 = ordinary
+  int fold, planes_a, planes_b;
+  uint32_t pa, pb;         // plane of A / B per pair, two bits each
+  // k cut into `splits` pieces of split_blocks blocks, one work item each; batch item split * batch + b of C gets a piece
+  int splits, split_blocks;
   int* status;
   // masked product: tile_live[mb * tiles_n + nb] == 0 marks an output tile no element of which is asked for; every
   // role of the kernel passes over it (no loads, no MMAs, no stores). NULL = every tile is computed.
@@ -65,6 +70,28 @@ struct TcSmem {
   static constexpr int OUT_OFFSET = (TOTAL + 127) / 128 * 128;  // staged stores: the epilogue warps' areas
   static constexpr int DYN_STAGED = OUT_OFFSET + 4 * TC_OUT_BYTES + 1024;
 };
+
+// Work item -> batch item of the operands, first and end k block; a product of planes counts its blocks pair by pair from 0
+// and every pair starts at block `first` of k.
+struct TcPiece {
+  int b, kb0, kb1, first;
+};
+__device__ __forceinline__ TcPiece tc_piece(const GemmTcParams& p, int bf) {
+  if (p.splits == 1) return {bf, 0, p.k_blocks, 0};
+  const int split = bf / p.batch, b = bf - split * p.batch;
+  if (p.fold > 0) return {b, 0, p.split_blocks, split * p.fold};
+  return {b, split * p.split_blocks, min(p.k_blocks, (split + 1) * p.split_blocks), 0};
+}
+// Where k block kb lies: block kk of plane (or batch item) za of A and zb of B.
+struct TcBlock {
+  int kk, za, zb;
+};
+__device__ __forceinline__ TcBlock tc_block(const GemmTcParams& p, int first, int kb, int ba, int bb) {
+  if (p.fold == 0) return {kb, ba, bb};
+  const int pair = kb / p.fold;
+  return {first + kb - pair * p.fold, ba * p.planes_a + static_cast<int>((p.pa >> (2 * pair)) & 3),
+          bb * p.planes_b + static_cast<int>((p.pb >> (2 * pair)) & 3)};
+}
 
 template <int BN, int OUT_DT>
 __device__ __forceinline__ void tc_store_chunk(const GemmTcParams& p, const uint32_t (&r)[32], int64_t row_off,
@@ -325,17 +352,18 @@ __global__ void __launch_bounds__(TC_THREADS, 1)
         }
       }
       for (int tile = blockIdx.x; ok && tile < p.total_tiles; tile += gridDim.x) {
-        const int b = tile / tiles_per_batch;
-        const int rem = tile - b * tiles_per_batch;
+        const int bf = tile / tiles_per_batch;
+        const int rem = tile - bf * tiles_per_batch;
+        const TcPiece piece = tc_piece(p, bf);
         if (p.tile_live && !p.tile_live[rem]) continue;
         const int mb = rem / p.tiles_n;
         const int nb = rem - mb * p.tiles_n;
         const int group = p.tile_group ? p.tile_group[mb] : 0;
         if (group < 0) continue;
         const int n_row0 = group * p.group_rows + nb * BN;
-        const int ba = p.a_bcast ? 0 : b;
-        const int bb = p.b_bcast ? 0 : b;
-        for (int kb = 0; kb < p.k_blocks; ++kb) {
+        const int ba = p.a_bcast ? 0 : piece.b;
+        const int bb = p.b_bcast ? 0 : piece.b;
+        for (int kb = piece.kb0; kb < piece.kb1; ++kb) {
           if (!mbar_wait(&empty_bar[stage], phase ^ 1u, abort_word)) {
             ok = false;
             break;
@@ -347,6 +375,7 @@ __global__ void __launch_bounds__(TC_THREADS, 1)
               pf_tile += gridDim.x;
             }
           }
+          const TcBlock at = tc_block(p, piece.first, kb, ba, bb);
           mbar_expect_tx(&full_bar[stage], S::STAGE_BYTES);
           uint8_t* sa = smem + stage * S::STAGE_BYTES;
           uint8_t* sb = sa + S::A_BYTES;
@@ -354,27 +383,27 @@ __global__ void __launch_bounds__(TC_THREADS, 1)
             if (p.split_loads) {
 #pragma unroll
               for (int c = 0; c < TC_BM / 64; ++c)
-                tma_load_3d(sa + c * 8192, &tmA, &full_bar[stage], kb * TC_BK, mb * TC_BM + c * 64, ba);
+                tma_load_3d(sa + c * 8192, &tmA, &full_bar[stage], at.kk * TC_BK, mb * TC_BM + c * 64, at.za);
             } else {
-              tma_load_3d(sa, &tmA, &full_bar[stage], kb * TC_BK, mb * TC_BM, ba);
+              tma_load_3d(sa, &tmA, &full_bar[stage], at.kk * TC_BK, mb * TC_BM, at.za);
             }
           } else {
 #pragma unroll
             for (int c = 0; c < TC_BM / 64; ++c)
-              tma_load_3d(sa + c * 8192, &tmA, &full_bar[stage], mb * TC_BM + c * 64, kb * TC_BK, ba);
+              tma_load_3d(sa + c * 8192, &tmA, &full_bar[stage], mb * TC_BM + c * 64, at.kk * TC_BK, at.za);
           }
           if (!p.b_mn) {
             if (p.split_loads) {
 #pragma unroll
               for (int c = 0; c < BN / 64; ++c)
-                tma_load_3d(sb + c * 8192, &tmB, &full_bar[stage], kb * TC_BK, n_row0 + c * 64, bb);
+                tma_load_3d(sb + c * 8192, &tmB, &full_bar[stage], at.kk * TC_BK, n_row0 + c * 64, at.zb);
             } else {
-              tma_load_3d(sb, &tmB, &full_bar[stage], kb * TC_BK, n_row0, bb);
+              tma_load_3d(sb, &tmB, &full_bar[stage], at.kk * TC_BK, n_row0, at.zb);
             }
           } else {
 #pragma unroll
             for (int c = 0; c < BN / 64; ++c)
-              tma_load_3d(sb + c * 8192, &tmB, &full_bar[stage], n_row0 + c * 64, kb * TC_BK, bb);
+              tma_load_3d(sb + c * 8192, &tmB, &full_bar[stage], n_row0 + c * 64, at.kk * TC_BK, at.zb);
           }
           ++issued;
           if (++stage == TC_STAGES) {
@@ -413,7 +442,8 @@ __global__ void __launch_bounds__(TC_THREADS, 1)
         if (!mbar_wait(&tempty_bar[acc], acc_phase ^ 1u, abort_word)) break;
         tc_fence_after();
         const uint32_t d_tmem = tmem_base + static_cast<uint32_t>(acc * BN);
-        for (int kb = 0; kb < p.k_blocks; ++kb) {
+        const TcPiece piece = tc_piece(p, tile / tiles_per_batch);
+        for (int kb = piece.kb0; kb < piece.kb1; ++kb) {
           if (!mbar_wait(&full_bar[stage], phase, abort_word)) {
             ok = false;
             break;
@@ -427,7 +457,7 @@ __global__ void __launch_bounds__(TC_THREADS, 1)
                                           : umma_smem_desc_sw128(a_base + k * 32, 16, 1024);
             const uint64_t bdesc = p.b_mn ? umma_smem_desc_sw128(b_base + k * 2048, 8192, 1024)
                                           : umma_smem_desc_sw128(b_base + k * 32, 16, 1024);
-            tc_mma_f16(d_tmem, adesc, bdesc, p.idesc, (kb | k) != 0 ? 1u : 0u);
+            tc_mma_f16(d_tmem, adesc, bdesc, p.idesc, kb != piece.kb0 || k != 0 ? 1u : 0u);
           }
           tc_commit(&empty_bar[stage]);  // frees the stage once these MMAs have read it
           if (++stage == TC_STAGES) {
@@ -585,6 +615,7 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(TC_THREADS, 1)
         const int m0 = mb * 256 + static_cast<int>(cta) * TC_BM;
         const int n0 = nb * TC2_BN + static_cast<int>(cta) * (TC2_BN / 2);
         for (int kb = 0; kb < p.k_blocks; ++kb) {
+          const TcBlock at = tc_block(p, 0, kb, ba, bb);
           if (!mbar_wait(&empty_bar[stage], phase ^ 1u, abort_word)) {
             ok = false;
             break;
@@ -594,16 +625,16 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(TC_THREADS, 1)
           uint8_t* sa = smem + stage * S::STAGE_BYTES;
           uint8_t* sb = sa + S::A_BYTES;
           if (!p.a_mn) {
-            tma_load_3d_pair(sa, &tmA, full_leader, kb * TC_BK, m0, ba);
+            tma_load_3d_pair(sa, &tmA, full_leader, at.kk * TC_BK, m0, at.za);
           } else {
 #pragma unroll
-            for (int c = 0; c < TC_BM / 64; ++c) tma_load_3d_pair(sa + c * 8192, &tmA, full_leader, m0 + c * 64, kb * TC_BK, ba);
+            for (int c = 0; c < TC_BM / 64; ++c) tma_load_3d_pair(sa + c * 8192, &tmA, full_leader, m0 + c * 64, at.kk * TC_BK, at.za);
           }
           if (!p.b_mn) {
-            tma_load_3d_pair(sb, &tmB, full_leader, kb * TC_BK, n0, bb);
+            tma_load_3d_pair(sb, &tmB, full_leader, at.kk * TC_BK, n0, at.zb);
           } else {
 #pragma unroll
-            for (int c = 0; c < TC2_BN / 128; ++c) tma_load_3d_pair(sb + c * 8192, &tmB, full_leader, n0 + c * 64, kb * TC_BK, bb);
+            for (int c = 0; c < TC2_BN / 128; ++c) tma_load_3d_pair(sb + c * 8192, &tmB, full_leader, n0 + c * 64, at.kk * TC_BK, at.zb);
           }
           if (++stage == TC2_STAGES) {
             stage = 0;
@@ -723,6 +754,8 @@ struct GemmSimtParams {
   int in_dtype, out_dtype;
   int tiles_m, tiles_n;
   const uint8_t* tile_live;  // masked product: 0 marks a 128 x 128 output tile nobody asks for (NULL: all computed)
+  const int* gate;  // the kernel runs only if one of these `n_gate` words is set (NULL: always)
+  int n_gate;
 };
 
 template <int IN_DT>
@@ -732,6 +765,11 @@ __global__ void __launch_bounds__(SM_THREADS) gemm_simt_kernel(const GemmSimtPar
 
   const int tid = threadIdx.x;
   const int tile = blockIdx.x;
+  if (p.gate) {
+    int any = 0;
+    for (int i = tid; i < p.n_gate; i += SM_THREADS) any |= p.gate[i];
+    if (!__syncthreads_or(any)) return;
+  }
   if (p.tile_live && !p.tile_live[tile]) return;
   const int b = blockIdx.y;
   const int mb = tile / p.tiles_n, nb = tile - mb * p.tiles_n;
@@ -919,32 +957,62 @@ static int make_tile_live(int m, int n, int bm, int bn, cudaStream_t st, uint8_t
   return YTC_OK;
 }
 
+// A product of planes: operand A is [batch][planes_a][rows][cols] with plane_a elements a plane (its batch stride is
+// planes_a * plane_a), B likewise; the accumulator takes `pairs` plane products in the order of pa / pb (two bits a pair).
+struct TcPlanes {
+  int planes_a, planes_b, pairs;
+  uint32_t pa, pb;
+  int64_t plane_a, plane_b;
+};
+
+// Whether CTA pairs take this product (large problems; small ones keep one CTA per tile: more tiles to spread over the SMs).
+static bool tc_takes_pairs(int m, int n, int64_t k, int64_t batch) {
+  return g_mask.kind == 0 && g_tc_pair != 2 &&
+         (g_tc_pair == 1 || (m >= 512 && n >= 256 && k >= 256 &&
+                             static_cast<int64_t>((m + 255) / 256) * ((n + 255) / 256) * batch >= 74));
+}
+static int tc_tile_n(int m, int n, int64_t batch) {
+  return (n <= 128 || static_cast<int64_t>((m + 127) / 128) * ((n + 255) / 256) * batch < sm_count() / 2) ? 128 : 256;
+}
+// Pieces of k that fill the SMs when the tiles alone leave more than half of them idle; a piece keeps 512 / pairs of k.
+// Measured, bf16 16 x 4096 x 4096: one piece 24.5 us, four and their sum 13.7.
+static int tc_splits(int m, int n, int k, int pairs, int64_t batch) {
+  const int k_blocks = (k + TC_BK - 1) / TC_BK;
+  if (g_mask.kind != 0 || g_tc_pair != 0 || tc_takes_pairs(m, n, static_cast<int64_t>(k) * pairs, batch)) return 1;
+  const int bn = tc_tile_n(m, n, batch);
+  const int64_t tiles = static_cast<int64_t>((m + 127) / 128) * ((n + bn - 1) / bn) * batch;
+  if (tiles * 2 > sm_count()) return 1;
+  const int64_t most = static_cast<int64_t>(k_blocks) * pairs / 8;
+  int64_t want = sm_count() / tiles < most ? sm_count() / tiles : most;
+  if (want > k_blocks) want = k_blocks;
+  if (want < 2) return 1;
+  const int64_t per = (k_blocks + want - 1) / want;
+  return static_cast<int>((k_blocks + per - 1) / per);
+}
+
 static int launch_tc(int dtype_in, int dtype_out, const void* A, const void* B, void* C, int m, int n, int k,
                      float alpha, float beta, int a_mn, int64_t lda, int b_mn, int64_t ldb, int64_t rsc, int64_t csc,
                      int64_t batch, int64_t bsa, int64_t bsb, int64_t bsc, cudaStream_t st,
-                     const LinearEpilogue* ex = nullptr) {
+                     const LinearEpilogue* ex = nullptr, const TcPlanes* pl = nullptr, int splits = 1) {
   // A: unit axis = K (a_mn 0, dims {K, M}) or M (a_mn 1, dims {M, K}). B likewise with N.
   CUtensorMap tmA, tmB;
   const int a_bcast = (batch > 1 && bsa == 0) ? 1 : 0;
   const int b_bcast = (batch > 1 && bsb == 0) ? 1 : 0;
   // 256-wide tiles unless the problem is narrow or would leave most SMs without a tile
-  const int BN = (n <= 128 || static_cast<int64_t>((m + 127) / 128) * ((n + 255) / 256) * batch < sm_count() / 2) ? 128 : 256;
-  // CTA pairs pay off on large problems; small ones keep one CTA per tile (more tiles to spread over the SMs)
+  const int BN = tc_tile_n(m, n, batch);
   // (a masked product keeps one CTA per tile: the tile-skipping form of the kernel)
   const bool grouped = ex && ex->tile_group;
-  const bool pair = g_mask.kind == 0 && g_tc_pair != 2 && !grouped &&
-                    (g_tc_pair == 1 || (m >= 512 && n >= 256 && k >= 256 &&
-                                        static_cast<int64_t>((m + 255) / 256) * ((n + 255) / 256) * batch >= 74));
+  const bool pair = !grouped && tc_takes_pairs(m, n, pl ? static_cast<int64_t>(k) * pl->pairs : k, batch);
   {
     const uint64_t nb = (a_bcast || batch == 1) ? 1 : static_cast<uint64_t>(batch);
     uint64_t dims[3], strides[2];
     uint32_t box[3];
     if (!a_mn) { dims[0] = k; dims[1] = m; box[0] = TC_BK; box[1] = g_tc_split_loads ? 64 : TC_BM; }
     else       { dims[0] = m; dims[1] = k; box[0] = 64;    box[1] = TC_BK; }
-    dims[2] = nb;
+    dims[2] = nb * (pl ? pl->planes_a : 1);
     box[2] = 1;
     strides[0] = static_cast<uint64_t>(lda) * 2;
-    strides[1] = (nb > 1) ? static_cast<uint64_t>(bsa) * 2 : strides[0] * dims[1];
+    strides[1] = pl ? static_cast<uint64_t>(pl->plane_a) * 2 : (nb > 1) ? static_cast<uint64_t>(bsa) * 2 : strides[0] * dims[1];
     int s = encode_tensor_map(&tmA, CU_TENSOR_MAP_DATA_TYPE_UINT16, 3, A, dims, strides, box,
                               CU_TENSOR_MAP_SWIZZLE_128B);
     if (s != YTC_OK) return s;
@@ -956,10 +1024,10 @@ static int launch_tc(int dtype_in, int dtype_out, const void* A, const void* B, 
     const uint64_t b_rows = grouped ? static_cast<uint64_t>(n) * ex->groups : static_cast<uint64_t>(n);
     if (!b_mn) { dims[0] = k; dims[1] = b_rows; box[0] = TC_BK; box[1] = pair ? 128u : (g_tc_split_loads ? 64u : static_cast<uint32_t>(BN)); }
     else       { dims[0] = n; dims[1] = k; box[0] = 64;    box[1] = TC_BK; }
-    dims[2] = nb;
+    dims[2] = nb * (pl ? pl->planes_b : 1);
     box[2] = 1;
     strides[0] = static_cast<uint64_t>(ldb) * 2;
-    strides[1] = (nb > 1) ? static_cast<uint64_t>(bsb) * 2 : strides[0] * dims[1];
+    strides[1] = pl ? static_cast<uint64_t>(pl->plane_b) * 2 : (nb > 1) ? static_cast<uint64_t>(bsb) * 2 : strides[0] * dims[1];
     int s = encode_tensor_map(&tmB, CU_TENSOR_MAP_DATA_TYPE_UINT16, 3, B, dims, strides, box,
                               CU_TENSOR_MAP_SWIZZLE_128B);
     if (s != YTC_OK) return s;
@@ -975,14 +1043,23 @@ static int launch_tc(int dtype_in, int dtype_out, const void* A, const void* B, 
   p.out_dtype = dtype_out;
   p.tiles_m = (m + TC_BM - 1) / TC_BM;
   p.tiles_n = (n + BN - 1) / BN;
-  const int64_t total = static_cast<int64_t>(p.tiles_m) * p.tiles_n * batch;
+  const int64_t total = static_cast<int64_t>(p.tiles_m) * p.tiles_n * batch * splits;
   if (total > 0x7FFFFFFFll) {
     set_last_error("ytcuda_gemm: too many tiles (%lld)", (long long)total);
     return YTC_UNSUPPORTED;
   }
   p.total_tiles = static_cast<int>(total);
   p.k_blocks = (k + TC_BK - 1) / TC_BK;
-  p.a_prefetch = g_tc_a_prefetch;
+  p.fold = 0;
+  p.splits = splits;
+  p.split_blocks = (p.k_blocks + splits - 1) / splits;
+  if (pl) {  // (every piece holds its share of k of all pairs)
+    p.fold = p.split_blocks;
+    p.split_blocks *= pl->pairs;
+    p.k_blocks = p.split_blocks;
+    p.planes_a = pl->planes_a; p.planes_b = pl->planes_b; p.pa = pl->pa; p.pb = pl->pb;
+  }
+  p.a_prefetch = pl || splits > 1 ? 0 : g_tc_a_prefetch.load();
   p.split_loads = g_tc_split_loads;
   p.tile_live = nullptr;
   const LinearEpilogue none, *e = ex ? ex : &none;
@@ -1054,8 +1131,10 @@ int linear_tc(const void* x, int64_t ldx, const void* w, int64_t ldw, void* y, i
 
 static int launch_simt(int dtype_in, int dtype_out, const void* A, const void* B, void* C, int m, int n, int k,
                        float alpha, float beta, int64_t rsa, int64_t csa, int64_t rsb, int64_t csb, int64_t rsc,
-                       int64_t csc, int64_t batch, int64_t bsa, int64_t bsb, int64_t bsc, cudaStream_t st) {
+                       int64_t csc, int64_t batch, int64_t bsa, int64_t bsb, int64_t bsc, cudaStream_t st,
+                       const int* gate = nullptr, int n_gate = 0) {
   GemmSimtParams p;
+  p.gate = gate; p.n_gate = n_gate;
   p.A = A; p.B = B; p.C = C;
   p.M = m; p.N = n; p.K = k;
   p.rsa = rsa; p.csa = csa; p.rsb = rsb; p.csb = csb; p.rsc = rsc; p.csc = csc;
@@ -1095,77 +1174,106 @@ static int launch_simt(int dtype_in, int dtype_out, const void* A, const void* B
   return YTC_OK;
 }
 
-// x (fp32) = h + m + l with h = bf16(x), m = bf16(x - h), l = bf16(x - h - m): three 16-bit values that together
-// carry the 24 mantissa bits of x (the differences are exact in fp32). The six partial products of an fp32 GEMM
-// that matter, (l,h) (m,m) (h,l) (m,h) (h,m) (h,h) smallest first, are laid side by side along k so that ONE
-// bf16 GEMM with k' = 6 k forms their sum in its fp32 accumulator:
-//   left operand  (is_b == 0, x is [rows = m][cols = k]): out[b][i][c k + j] = plane_a(c) of x[b][i][j]
-//   right operand (is_b == 1, x is [rows = k][cols = n]): out[b][c k + i][j] = plane_b(c) of x[b][i][j]
-// with plane_a = l m h m h h and plane_b = h m l h m h. Non-finite values keep m = l = 0 (an infinite operand then
-// meets zero planes of the other operand and the sum becomes NaN where the FFMA kernel gives the infinity).
-// One operand of the split; `blocks` CTAs of the launch work on it.
-struct SplitOp {
-  const float* x;
+// Operands that the TMA cannot take as they lie, rewritten: fp32 as three bf16 planes, x = h + m + l with h = bf16(x),
+// m = bf16(x - h), l = bf16(x - h - m), which together carry the 24 mantissa bits of x (the differences are exact in fp32);
+// 16-bit operands of odd strides as they are. Rows of `cols` elements become rows of a multiple of 8, zeros behind the end.
+// Of the nine plane products of an fp32 GEMM the six that matter, (l,h) (m,m) (h,l) (m,h) (h,m) (h,h), smallest first, form
+// in one accumulator (TcPlanes). Non-finite values keep m = l = 0 (an infinite operand then meets zero planes of the other
+// operand and the sum becomes NaN where the FFMA kernel gives the infinity); `unfit`, a word per block, says whether there
+// were any. fp16 numbers below the normal ones are doubled, which is how the reference's type and the FFMA kernel read them.
+struct PlaneOp {
+  const void* x;
   int64_t rs, cs, bs;
-  int rows, cols;
-  int64_t batch;
-  int is_b;
-  __nv_bfloat16* out;
+  int rows, cols, cols8;   // cols8: groups of 8 columns of an output row
+  int64_t n8;              // groups over all rows and batch items
+  uint16_t* out;
+  int64_t plane;           // elements of a plane of one batch item
   int blocks;
+  int wide;                // fp32: groups of 8 can be read 16 bytes at a time
 };
-// One launch splits both operands (or one: b.blocks == 0): CTAs [0, a.blocks) take a, the rest b.
-__global__ void __launch_bounds__(256) gemm_split3_kernel(const SplitOp oa, const SplitOp ob) {
+// One launch for both operands: CTAs [0, a.blocks) take a, the rest b. Bound by memory: 4 bytes read, 6 written a value.
+template <int DT>
+__global__ void __launch_bounds__(256) gemm_planes_kernel(const PlaneOp oa, const PlaneOp ob, int* unfit) {
   dependent_wait();     // (under a programmatic dependent launch: the kernel before this one has finished)
   dependent_trigger();  // the kernel queued behind this one may be scheduled and set itself up meanwhile
+  constexpr int PLANES = DT == YTC_F32 ? 3 : 1;
   const bool second = static_cast<int>(blockIdx.x) >= oa.blocks;
-  const SplitOp& op = second ? ob : oa;
-  const float* x = op.x;
-  const int64_t rs = op.rs, cs = op.cs, bs = op.bs, batch = op.batch;
-  const int rows = op.rows, cols = op.cols, is_b = op.is_b;
-  __nv_bfloat16* out = op.out;
+  const PlaneOp& op = second ? ob : oa;
   const int64_t block = static_cast<int64_t>(blockIdx.x) - (second ? oa.blocks : 0);
-  const int64_t per = static_cast<int64_t>(rows) * cols;
-  const int64_t total = per * batch;
-  for (int64_t t = block * static_cast<int64_t>(blockDim.x) + threadIdx.x; t < total;
-       t += static_cast<int64_t>(op.blocks) * blockDim.x) {
-    const int64_t b = t / per, r = t - b * per;
-    const int i = static_cast<int>(r / cols), j = static_cast<int>(r - static_cast<int64_t>(i) * cols);
-    const float v = x[b * bs + i * rs + j * cs];
-    __nv_bfloat16 p[3];  // h, m, l
-    p[0] = __float2bfloat16_rn(v);
-    p[1] = p[2] = __float2bfloat16_rn(0.f);
-    float fh = __bfloat162float(p[0]);
-    if (!isfinite(fh) && isfinite(v)) {
-      // a finite value so close to the largest float that rounding its top plane overflows: truncate instead, the
-      // two lower planes still hold the remaining 16 mantissa bits exactly
-      fh = __uint_as_float(__float_as_uint(v) & 0xffff0000u);
-      p[0] = __float2bfloat16_rn(fh);
-    }
-    if (isfinite(fh)) {
-      const float r1 = v - fh;
-      p[1] = __float2bfloat16_rn(r1);
-      p[2] = __float2bfloat16_rn(r1 - __bfloat162float(p[1]));
-    }
-    __nv_bfloat16* o = out + b * per * 6;
-    if (is_b) {
-      // chunks h m l h m h
-      const int64_t at = static_cast<int64_t>(i) * cols + j;
-      o[at] = p[0];
-      o[per + at] = p[1];
-      o[2 * per + at] = p[2];
-      o[3 * per + at] = p[0];
-      o[4 * per + at] = p[1];
-      o[5 * per + at] = p[0];
+  bool bad = false;
+  for (int64_t t = block * 256 + threadIdx.x; t < op.n8; t += op.blocks * 256ll) {
+    const int64_t row = t / op.cols8;  // (of all batch items)
+    const int c = static_cast<int>(t - row * op.cols8) * 8;
+    const int64_t b = row / op.rows, i = row - b * op.rows;
+    const int64_t from = b * op.bs + i * op.rs + c * op.cs;
+    uint16_t p[PLANES][8];
+    if constexpr (DT == YTC_F32) {
+      float v[8];
+      if (op.wide && c + 8 <= op.cols) {
+        const float4 v0 = *reinterpret_cast<const float4*>(static_cast<const float*>(op.x) + from);
+        const float4 v1 = *reinterpret_cast<const float4*>(static_cast<const float*>(op.x) + from + 4);
+        v[0] = v0.x; v[1] = v0.y; v[2] = v0.z; v[3] = v0.w; v[4] = v1.x; v[5] = v1.y; v[6] = v1.z; v[7] = v1.w;
+      } else {
+#pragma unroll
+        for (int e = 0; e < 8; ++e) v[e] = c + e < op.cols ? static_cast<const float*>(op.x)[from + e * op.cs] : 0.f;
+      }
+#pragma unroll
+      for (int e = 0; e < 8; ++e) {
+        __nv_bfloat16 q = __float2bfloat16_rn(v[e]);
+        float fh = __bfloat162float(q);
+        if (!isfinite(fh) && isfinite(v[e])) {
+          // a finite value so close to the largest float that rounding its top plane overflows: truncate instead, the
+          // two lower planes still hold the remaining 16 mantissa bits exactly
+          fh = __uint_as_float(__float_as_uint(v[e]) & 0xffff0000u);
+          q = __float2bfloat16_rn(fh);
+        }
+        p[0][e] = *reinterpret_cast<const uint16_t*>(&q);
+        p[1][e] = p[2][e] = 0;
+        if (isfinite(fh)) {
+          const float r1 = v[e] - fh;
+          q = __float2bfloat16_rn(r1);
+          p[1][e] = *reinterpret_cast<const uint16_t*>(&q);
+          q = __float2bfloat16_rn(r1 - __bfloat162float(q));
+          p[2][e] = *reinterpret_cast<const uint16_t*>(&q);
+        } else {
+          bad = true;
+        }
+      }
     } else {
-      // chunks l m h m h h
-      __nv_bfloat16* row = o + static_cast<int64_t>(i) * cols * 6 + j;
-      row[0] = p[2];
-      row[cols] = p[1];
-      row[2 * cols] = p[0];
-      row[3 * cols] = p[1];
-      row[4 * cols] = p[0];
-      row[5 * cols] = p[0];
+#pragma unroll
+      for (int e = 0; e < 8; ++e) {
+        uint16_t h = c + e < op.cols ? static_cast<const uint16_t*>(op.x)[from + e * op.cs] : 0;
+        if (DT == YTC_F16 && (h & 0x7C00u) == 0) h = static_cast<uint16_t>((h & 0x8000u) | ((h & 0x3FFu) << 1));
+        p[0][e] = h;
+      }
     }
+    uint16_t* o = op.out + b * op.plane * PLANES + (i * op.cols8 * 8 + c);
+#pragma unroll
+    for (int i3 = 0; i3 < PLANES; ++i3) {
+      uint32_t w[4];
+#pragma unroll
+      for (int e = 0; e < 4; ++e) w[e] = p[i3][2 * e] | (static_cast<uint32_t>(p[i3][2 * e + 1]) << 16);
+      *reinterpret_cast<uint4*>(o + i3 * op.plane) = make_uint4(w[0], w[1], w[2], w[3]);
+    }
+  }
+  const int any = __syncthreads_or(bad);
+  if (unfit && threadIdx.x == 0) unfit[blockIdx.x] = any;
+}
+
+// C = alpha * (the sum of the k pieces, in their order) + beta * C; part is [splits][batch][m][n].
+__global__ void __launch_bounds__(256) gemm_sum_kernel(const float* part, int splits, int64_t total, int m, int n, void* C,
+                                                       int dt, int64_t rsc, int64_t csc, int64_t bsc, float alpha, float beta) {
+  dependent_wait();
+  dependent_trigger();
+  for (int64_t t = blockIdx.x * 256ll + threadIdx.x; t < total; t += gridDim.x * 256ll) {
+    float v = 0.f;
+#pragma unroll 8
+    for (int s = 0; s < splits; ++s) v += part[s * total + t];
+    const int64_t row = t / n;
+    const int64_t b = row / m, at = b * bsc + (row - b * m) * rsc + (t - row * n) * csc;
+    v *= alpha;
+    if (beta != 0.f) v += beta * load_as_f32(C, at, dt);
+    store_from_f32(C, at, v, dt);
   }
 }
 
@@ -1194,62 +1302,168 @@ static std::atomic<int> g_gemm_path{0};
 // 2 = whenever the shapes allow.
 static std::atomic<int> g_f32_split{0};
 
-static bool f32_split_ok(int m, int n, int k, int64_t rsc, int64_t csc, int64_t bsc) {
-  if (g_f32_split == 1) return false;
-  if (k % 8 || n % 8 || rsc < 0 || csc < 0 || bsc < 0) return false;
-  if (g_f32_split == 2) return m >= 1 && n >= 8 && k >= 8;
-  return m >= 256 && n >= 256 && k >= 256;
+// The FFMA kernel takes about 0.17 us (fp32; 16 bit 0.3) per element of k and wave of 128 x 128 tiles, whatever m is. The planes
+// cost about 8 us of launches and 10 bytes of traffic a value, six products a sixth of the tensor rate. Measured (FFMA / planes):
+// fp32 16 x 4096 x 4096 705 / 88 us, 60 x 1001 x 1111 205 / 56, 130 x 8192 x 8192 1548 / 453, 77 x 130 x 300 70 / 45; bf16
+// 777 x 1001 x 1111 340 / 30.
+static double simt_us(int m, int n, int k, int64_t batch, bool wide) {
+  const int64_t tiles = static_cast<int64_t>((m + SM_BM - 1) / SM_BM) * ((n + SM_BN - 1) / SM_BN) * batch;
+  return (wide ? 0.17 : 0.3) * k * static_cast<double>((tiles + sm_count() - 1) / sm_count());
+}
+static double planes_us(int m, int n, int k, int64_t batch, bool b_shared, bool wide) {
+  const double values = static_cast<double>(m) * k * batch + static_cast<double>(k) * n * (b_shared ? 1 : batch);
+  return 12.0 + values * (wide ? 10 : 4) / 3e6 + 2.0 * m * n * k * batch * (wide ? 6 : 1) / 5e8;
 }
 
-static int launch_f32_split(const float* A, const float* B, float* C, int m, int n, int k, float alpha, float beta,
-                            int64_t rsa, int64_t csa, int64_t rsb, int64_t csb, int64_t rsc, int64_t csc, int64_t batch,
-                            int64_t bsa, int64_t bsb, int64_t bsc, cudaStream_t st) {
-  // the split launches and the product are one chain of dependent kernels: each is scheduled while the one before it
-  // still runs (programmatic dependent launches)
+// 0: FFMA, 1: planes, as for every large problem, 2: planes where FFMA is slower, with FFMA behind them for what has none
+static int f32_planes_form(int m, int n, int k, float beta, int64_t rsc, int64_t csc, int64_t bsc, int64_t batch, int64_t bsb) {
+  if (g_f32_split == 1) return 0;
+  if (rsc < 0 || csc < 0 || bsc < 0) return 0;
+  if (k % 8 == 0 && n % 8 == 0 && (g_f32_split == 2 ? n >= 8 && k >= 8 : m >= 256 && n >= 256 && k >= 256)) return 1;
+  return g_mask.kind == 0 && beta == 0.f && simt_us(m, n, k, batch, true) > 1.5 * planes_us(m, n, k, batch, bsb == 0, true) ? 2 : 0;
+}
+
+static bool stream_captures(cudaStream_t st) {  // (scratch that grows inside a capture would belong to the graph)
+  cudaStreamCaptureStatus cap = cudaStreamCaptureStatusNone;
+  return cudaStreamIsCapturing(st, &cap) != cudaSuccess || cap != cudaStreamCaptureStatusNone;
+}
+
+// The product through rewritten operands (gemm_planes_kernel), k cut into pieces where the tiles are few. `check`: FFMA runs
+// behind it if an operand held a number without planes (beta must be 0).
+template <int DT>
+static int launch_planes(const void* A, const void* B, void* C, int dtype_out, int m, int n, int k, float alpha, float beta,
+                         int64_t rsa, int64_t csa, int64_t rsb, int64_t csb, int64_t rsc, int64_t csc, int64_t batch,
+                         int64_t bsa, int64_t bsb, int64_t bsc, bool check, cudaStream_t st) {
+  // the launches are one chain of dependent kernels: each is scheduled while the one before it still runs
   struct Scope {
     bool was = overlap_scope();
     Scope() { overlap_scope() = true; }
     ~Scope() { overlap_scope() = was; }
   } scope;
-  const bool b_shared = batch > 1 && bsb == 0;
-  const int64_t a_per = static_cast<int64_t>(m) * k * 6, b_per = static_cast<int64_t>(k) * n * 6;  // bf16 elements
-  // batch items per pass so that the expanded operands stay below about 2 GiB
+  constexpr int PLANES = DT == YTC_F32 ? 3 : 1;
+  const int esz = dtype_size(DT);
+  const bool a_shared = batch > 1 && bsa == 0, b_shared = batch > 1 && bsb == 0;
+  // rows along the operand's unit stride: A as [m][k] or [k][m], B as [k][n] or [n][k]
+  const bool a_mn = csa != 1 && rsa == 1, b_kn = csb == 1 || rsb != 1;
+  auto op_of = [&](const void* x, int64_t rs, int64_t cs, int64_t bs, int rows, int cols, int64_t items) {
+    PlaneOp o{};
+    o.x = x; o.rs = rs; o.cs = cs; o.bs = bs; o.rows = rows; o.cols = cols;
+    o.cols8 = (cols + 7) / 8;
+    o.n8 = items * rows * o.cols8;
+    o.plane = static_cast<int64_t>(rows) * o.cols8 * 8;
+    const int64_t want = (o.n8 + 511) / 512, most = static_cast<int64_t>(sm_count()) * 8;
+    o.blocks = static_cast<int>(want < most ? want : most);
+    o.wide = DT == YTC_F32 && cs == 1 && rs % 4 == 0 && bs % 4 == 0 && (reinterpret_cast<uint64_t>(x) & 15) == 0;
+    return o;
+  };
+  auto a_op = [&](int64_t b0, int64_t items) {
+    const char* x = static_cast<const char*>(A) + b0 * bsa * esz;
+    return a_mn ? op_of(x, csa, rsa, bsa, k, m, items) : op_of(x, rsa, csa, bsa, m, k, items);
+  };
+  auto b_op = [&](int64_t b0, int64_t items) {
+    const char* x = static_cast<const char*>(B) + b0 * bsb * esz;
+    return b_kn ? op_of(x, rsb, csb, bsb, k, n, items) : op_of(x, csb, rsb, bsb, n, k, items);
+  };
+  PlaneOp oa = a_op(0, 1), ob = b_op(0, 1);
+  // batch items per pass so that the planes stay below about 2 GiB
+  const int64_t a_item = oa.plane * PLANES * 2, b_item = ob.plane * PLANES * 2;
   int64_t chunk = batch;
-  const int64_t per_item = 2 * (a_per + (b_shared ? 0 : b_per));
-  const int64_t budget = (int64_t{2} << 30) - (b_shared ? 2 * b_per : 0);
-  if (per_item * chunk > budget) chunk = budget / per_item > 0 ? budget / per_item : 1;
-  const size_t a_bytes = (static_cast<size_t>(2) * a_per * chunk + 255) / 256 * 256;
-  const size_t b_bytes = static_cast<size_t>(2) * b_per * (b_shared ? 1 : chunk);
-  char* ws = static_cast<char*>(device_workspace(a_bytes + b_bytes, st));
+  const int64_t fixed = (a_shared ? a_item : 0) + (b_shared ? b_item : 0), per_item = (a_shared ? 0 : a_item) + (b_shared ? 0 : b_item);
+  if (per_item > 0 && per_item * chunk > (int64_t{2} << 30) - fixed) {
+    chunk = ((int64_t{2} << 30) - fixed) / per_item;
+    if (chunk < 1) chunk = 1;
+  }
+  TcPlanes pl{PLANES, PLANES, 1, 0, 0, oa.plane, ob.plane};
+  if (PLANES == 3) {  // (l,h) (m,m) (h,l) (m,h) (h,m) (h,h)
+    pl.pairs = 6;
+    pl.pa = 2u | (1u << 2) | (0u << 4) | (1u << 6) | (0u << 8) | (0u << 10);
+    pl.pb = 0u | (1u << 2) | (2u << 4) | (0u << 6) | (1u << 8) | (0u << 10);
+  }
+  int splits = DT == YTC_F32 && g_f32_split != 0 ? 1 : tc_splits(m, n, k, pl.pairs, chunk);
+  // An accumulator of the tensor cores drops a fraction of a unit at every step of 16; FFMA rounds. Products that FFMA took
+  // before keep 256 of k per accumulator and add the pieces in fp32. Error against 64 bits (2-norm), 16 x 4096 x 4096: FFMA 1.2e-6,
+  // here 2.5e-7; one accumulator would be above 3e-6.
+  if (check && splits < (k + 255) / 256) splits = (k + 255) / 256;
+  auto up = [](int64_t v) { return static_cast<size_t>((v + 255) / 256 * 256); };
+  const int most_blocks = 2 * sm_count() * 8;  // (of both operands)
+  const size_t gate_bytes = up(most_blocks * 4), a_bytes = up(a_item * (a_shared ? 1 : chunk)), b_bytes = up(b_item * (b_shared ? 1 : chunk));
+  const size_t part_bytes = splits > 1 ? up(static_cast<int64_t>(splits) * chunk * m * n * 4) : 0;
+  char* ws = static_cast<char*>(device_workspace(gate_bytes + a_bytes + b_bytes + part_bytes, st));
   if (!ws) {
-    set_last_error("ytcuda_gemm: could not allocate %zu bytes for the bf16 form of an fp32 product", a_bytes + b_bytes);
+    set_last_error("ytcuda_gemm: could not allocate %zu bytes for rewritten operands", gate_bytes + a_bytes + b_bytes + part_bytes);
     return YTC_CUDA_ERROR;
   }
-  __nv_bfloat16* a6 = reinterpret_cast<__nv_bfloat16*>(ws);
-  __nv_bfloat16* b6 = reinterpret_cast<__nv_bfloat16*>(ws + a_bytes);
-  const int64_t cap = static_cast<int64_t>(sm_count()) * 16;
-  auto op_of = [&](const float* x, int64_t rs, int64_t cs, int64_t bs, int rows, int cols, int64_t nb, int is_b,
-                   __nv_bfloat16* out) {
-    const int64_t blocks = (static_cast<int64_t>(rows) * cols * nb + 255) / 256;
-    return SplitOp{x, rs, cs, bs, rows, cols, nb, is_b, out, static_cast<int>(blocks < cap ? blocks : cap)};
-  };
-  auto split = [&](const SplitOp& a, const SplitOp& b) {  // b.blocks == 0: one operand only
-    (void)launch_overlapped(gemm_split3_kernel, dim3(static_cast<unsigned>(a.blocks + b.blocks)), dim3(256), 0, st, a, b);
+  int* gate = check ? reinterpret_cast<int*>(ws) : nullptr;
+  uint16_t* a_out = reinterpret_cast<uint16_t*>(ws + gate_bytes);
+  uint16_t* b_out = reinterpret_cast<uint16_t*>(ws + gate_bytes + a_bytes);
+  float* part = reinterpret_cast<float*>(ws + gate_bytes + a_bytes + b_bytes);
+  auto planes = [&](const PlaneOp& a, const PlaneOp& b, int* words) {  // (no blocks: nothing to do for that operand)
+    const cudaError_t e = launch_overlapped(gemm_planes_kernel<DT>, dim3(static_cast<unsigned>(a.blocks + b.blocks)), dim3(256), 0, st, a, b, words);
     count_launch();
+    return e;
   };
-  const SplitOp none{nullptr, 0, 0, 0, 0, 0, 0, 0, nullptr, 0};
-  if (b_shared) split(op_of(B, rsb, csb, 0, k, n, 1, 1, b6), none);
+  const int64_t ldb_all = ob.cols8 * 8;
+  const PlaneOp none{};
+  int shared_blocks = 0;  // an operand that all batch items share is rewritten once
+  if (b_shared) {
+    ob.out = b_out;
+    YTC_CUDA(planes(none, ob, gate));
+    shared_blocks = ob.blocks;
+  }
   for (int64_t b0 = 0; b0 < batch; b0 += chunk) {
     const int64_t nb = batch - b0 < chunk ? batch - b0 : chunk;
-    split(op_of(A + b0 * bsa, rsa, csa, bsa, m, k, nb, 0, a6),
-          b_shared ? none : op_of(B + b0 * bsb, rsb, csb, bsb, k, n, nb, 1, b6));
-    YTC_CUDA(cudaGetLastError());
-    const int s = launch_tc(YTC_BF16, YTC_F32, a6, b6, C + b0 * bsc, m, n, 6 * k, alpha, beta, /*a_mn=*/0, 6 * k,
-                            /*b_mn=*/1, n, rsc, csc, nb, a_per, b_shared ? 0 : b_per, bsc, st);
+    oa = a_op(a_shared ? 0 : b0, a_shared ? 1 : nb);
+    ob = b_shared ? none : b_op(b0, nb);
+    oa.out = a_out;
+    ob.out = b_out;
+    YTC_CUDA(planes(oa, ob, gate ? gate + shared_blocks : nullptr));
+    char* c = static_cast<char*>(C) + b0 * bsc * dtype_size(dtype_out);
+    const int64_t lda = oa.cols8 * 8, ldb = ldb_all, mn = static_cast<int64_t>(m) * n;
+    const int tc_dt = DT == YTC_F32 ? YTC_BF16 : DT;
+    int s = splits > 1 ? launch_tc(tc_dt, YTC_F32, a_out, b_out, part, m, n, k, 1.f, 0.f, a_mn, lda, b_kn, ldb, n, 1, nb,
+                                   a_shared ? 0 : a_item / 2, b_shared ? 0 : b_item / 2, mn, st, nullptr, &pl, splits)
+                       : launch_tc(tc_dt, dtype_out, a_out, b_out, c, m, n, k, alpha, beta, a_mn, lda, b_kn, ldb, rsc, csc, nb,
+                                   a_shared ? 0 : a_item / 2, b_shared ? 0 : b_item / 2, bsc, st, nullptr, &pl);
     if (s != YTC_OK) return s;
+    if (splits > 1) {
+      const int64_t total = nb * mn, blocks = (total + 255) / 256, cap = static_cast<int64_t>(sm_count()) * 8;
+      YTC_CUDA(launch_overlapped(gemm_sum_kernel, dim3(static_cast<unsigned>(blocks < cap ? blocks : cap)), dim3(256), 0, st, part,
+                                 splits, total, m, n, c, dtype_out, rsc, csc, bsc, alpha, beta));
+      count_launch();
+    }
+    if (check && (s = launch_simt(DT, dtype_out, static_cast<const char*>(A) + b0 * bsa * esz, static_cast<const char*>(B) + b0 * bsb * esz,
+                                  c, m, n, k, alpha, beta, rsa, csa, rsb, csb, rsc, csc, nb, bsa, bsb, bsc, st, gate,
+                                  shared_blocks + oa.blocks + ob.blocks)) != YTC_OK)
+      return s;
   }
-  device_workspace_release(st);  // large expanded operands do not stay resident
+  device_workspace_release(st);  // large operands do not stay resident
   return YTC_OK;
+}
+
+// The product with k in pieces, operands as they lie.
+static int launch_tc_split(int dtype_in, int dtype_out, const void* A, const void* B, void* C, int m, int n, int k, float alpha,
+                           float beta, int a_mn, int64_t lda, int b_mn, int64_t ldb, int64_t rsc, int64_t csc, int64_t batch,
+                           int64_t bsa, int64_t bsb, int64_t bsc, int splits, float* part, cudaStream_t st) {
+  struct Scope {
+    bool was = overlap_scope();
+    Scope() { overlap_scope() = true; }
+    ~Scope() { overlap_scope() = was; }
+  } scope;
+  const int64_t mn = static_cast<int64_t>(m) * n, total = batch * mn;
+  const int s = launch_tc(dtype_in, YTC_F32, A, B, part, m, n, k, 1.f, 0.f, a_mn, lda, b_mn, ldb, n, 1, batch, bsa, bsb, mn, st,
+                          nullptr, nullptr, splits);
+  if (s != YTC_OK) return s;
+  const int64_t blocks = (total + 255) / 256, cap = static_cast<int64_t>(sm_count()) * 8;
+  YTC_CUDA(launch_overlapped(gemm_sum_kernel, dim3(static_cast<unsigned>(blocks < cap ? blocks : cap)), dim3(256), 0, st, part, splits,
+                             total, m, n, C, dtype_out, rsc, csc, bsc, alpha, beta));
+  count_launch();
+  return YTC_OK;
+}
+
+// y[m, n] (+)= (hi + lo)[m, k] . W[n, k]^T: both bf16 planes ([2][m][k]) of the activations in one accumulator, lo first.
+int linear_two_planes(const void* planes, const void* w, float* y, int64_t ldy, int m, int n, int k, bool accumulate, cudaStream_t st) {
+  const TcPlanes pl{2, 1, 2, 1u, 0u, static_cast<int64_t>(m) * k, static_cast<int64_t>(n) * k};
+  return launch_tc(YTC_BF16, YTC_F32, planes, w, y, m, n, k, 1.f, accumulate ? 1.f : 0.f, 0, k, 0, k, ldy, 1, 1, 0, 0, 0, st, nullptr, &pl);
 }
 
 }  // namespace ytk
@@ -1283,9 +1497,14 @@ int ytcuda_gemm_set_path(int path) {
   return YTC_OK;
 }
 
-int ytcuda_gemm(int dtype_in, int dtype_out, const void* A, const void* B, void* C, int m, int n, int k, float alpha,
-                float beta, int64_t rsa, int64_t csa, int64_t rsb, int64_t csb, int64_t rsc, int64_t csc,
-                int64_t batch, int64_t bsa, int64_t bsb, int64_t bsc, void* stream) {
+}  // extern "C"
+
+namespace ytk {
+
+// scratch: whether the call may use this stream's workspace (a caller that writes into the workspace itself says no)
+static int gemm_any(int dtype_in, int dtype_out, const void* A, const void* B, void* C, int m, int n, int k, float alpha,
+                    float beta, int64_t rsa, int64_t csa, int64_t rsb, int64_t csb, int64_t rsc, int64_t csc,
+                    int64_t batch, int64_t bsa, int64_t bsb, int64_t bsc, bool scratch, void* stream) {
   YTC_REQUIRE(dtype_in >= YTC_F32 && dtype_in <= YTC_F16, "ytcuda_gemm: bad dtype_in %d", dtype_in);
   YTC_REQUIRE(dtype_out >= YTC_F32 && dtype_out <= YTC_F16, "ytcuda_gemm: bad dtype_out %d", dtype_out);
   YTC_REQUIRE(m >= 0 && n >= 0 && k >= 0 && batch >= 0, "ytcuda_gemm: negative extent (m=%d n=%d k=%d batch=%lld)", m,
@@ -1306,9 +1525,12 @@ int ytcuda_gemm(int dtype_in, int dtype_out, const void* A, const void* B, void*
     YTC_CUDA(cudaGetLastError());
     return YTC_OK;
   }
-  if (dtype_in == YTC_F32 && dtype_out == YTC_F32 && g_gemm_path != 1 && f32_split_ok(m, n, k, rsc, csc, bsc))
-    return launch_f32_split(static_cast<const float*>(A), static_cast<const float*>(B), static_cast<float*>(C), m, n, k,
-                            alpha, beta, rsa, csa, rsb, csb, rsc, csc, batch, bsa, bsb, bsc, st);
+  if (dtype_in == YTC_F32 && dtype_out == YTC_F32 && g_gemm_path != 1) {
+    const int form = f32_planes_form(m, n, k, beta, rsc, csc, bsc, batch, bsb);
+    if (form == 1 || (form == 2 && scratch && !stream_captures(st)))
+      return launch_planes<YTC_F32>(A, B, C, dtype_out, m, n, k, alpha, beta, rsa, csa, rsb, csb, rsc, csc, batch, bsa, bsb, bsc,
+                                    form == 2, st);
+  }
   int a_mn = 0, b_mn = 0;
   bool tc = (dtype_in != YTC_F32) && g_gemm_path != 1;
   if (tc) {
@@ -1330,11 +1552,46 @@ int ytcuda_gemm(int dtype_in, int dtype_out, const void* A, const void* B, void*
     const int64_t lda = a_mn ? csa : rsa;
     const int64_t ldb = b_mn ? rsb : csb;
     // A single k extent of 1 makes both strides of an axis "unit"; the leading stride must still be sane.
+    const int splits = scratch ? tc_splits(m, n, k, 1, batch) : 1;
+    if (splits > 1 && !stream_captures(st)) {
+      float* part = static_cast<float*>(device_workspace(static_cast<size_t>(splits) * batch * m * n * 4, st));
+      if (part) {
+        const int s = launch_tc_split(dtype_in, dtype_out, A, B, C, m, n, k, alpha, beta, a_mn, lda, b_mn, ldb, rsc, csc, batch,
+                                      bsa, bsb, bsc, splits, part, st);
+        device_workspace_release(st);
+        return s;
+      }
+    }
     return launch_tc(dtype_in, dtype_out, A, B, C, m, n, k, alpha, beta, a_mn, lda, b_mn, ldb, rsc, csc, batch, bsa,
                      bsb, bsc, st);
   }
+  // 16-bit operands that the TMA cannot take (odd sizes and strides): rewritten where that pays
+  if (dtype_in != YTC_F32 && g_gemm_path != 1 && scratch && g_mask.kind == 0 && rsc >= 0 && csc >= 0 && bsc >= 0 &&
+      dtype_out != YTC_F32 &&  // (an fp32 result would show the tensor cores' accumulation)
+      simt_us(m, n, k, batch, false) > 1.5 * planes_us(m, n, k, batch, bsb == 0, false) && !stream_captures(st)) {
+    return dtype_in == YTC_BF16
+               ? launch_planes<YTC_BF16>(A, B, C, dtype_out, m, n, k, alpha, beta, rsa, csa, rsb, csb, rsc, csc, batch, bsa, bsb, bsc, false, st)
+               : launch_planes<YTC_F16>(A, B, C, dtype_out, m, n, k, alpha, beta, rsa, csa, rsb, csb, rsc, csc, batch, bsa, bsb, bsc, false, st);
+  }
   return launch_simt(dtype_in, dtype_out, A, B, C, m, n, k, alpha, beta, rsa, csa, rsb, csb, rsc, csc, batch, bsa,
                      bsb, bsc, st);
+}
+
+// ytcuda_gemm for callers whose C lies in this stream's workspace.
+int gemm_into_workspace(int dtype_in, int dtype_out, const void* A, const void* B, void* C, int m, int n, int k, float alpha,
+                        float beta, int64_t rsa, int64_t csa, int64_t rsb, int64_t csb, int64_t rsc, int64_t csc, int64_t batch,
+                        int64_t bsa, int64_t bsb, int64_t bsc, cudaStream_t st) {
+  return gemm_any(dtype_in, dtype_out, A, B, C, m, n, k, alpha, beta, rsa, csa, rsb, csb, rsc, csc, batch, bsa, bsb, bsc, false, st);
+}
+
+}  // namespace ytk
+
+extern "C" {
+
+int ytcuda_gemm(int dtype_in, int dtype_out, const void* A, const void* B, void* C, int m, int n, int k, float alpha,
+                float beta, int64_t rsa, int64_t csa, int64_t rsb, int64_t csb, int64_t rsc, int64_t csc,
+                int64_t batch, int64_t bsa, int64_t bsb, int64_t bsc, void* stream) {
+  return gemm_any(dtype_in, dtype_out, A, B, C, m, n, k, alpha, beta, rsa, csa, rsb, csb, rsc, csc, batch, bsa, bsb, bsc, true, stream);
 }
 
 }  // extern "C"
