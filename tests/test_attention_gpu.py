@@ -215,6 +215,14 @@ def _exact(q, k, v, scale, seen=None, bias=None):
     return torch.softmax(s, -1) @ v.double().repeat_interleave(g, 1)
 
 
+def _f32_bound(q, k, v, d, bias=None):
+    """Rows of few visible keys average nothing out: a weight is off by the exponential's 2^-22 and by the roundings of its
+    score, 2^-24 of the score (log2 units) in the product, the scale and the bias each."""
+    s = (q.double() @ k.double().repeat_interleave(q.shape[1] // k.shape[1], 1).transpose(-1, -2)).abs().max() * d ** -0.5
+    s = s + (0 if bias is None else bias.abs().max())
+    return 2.0 ** -22 * (1 + 1.4427 * s) * v.abs().max()
+
+
 @pytest.mark.parametrize("b,kvh,g,lq,lk,d,dt,form", [
     (1, 1, 1, 64, 256, 128, "f32", "causal"), (1, 2, 2, 129, 257, 128, "f32", "causal"), (2, 2, 4, 33, 65, 64, "f32", "none"),
     (1, 1, 1, 300, 513, 20, "f32", "causal"), (1, 2, 1, 127, 319, 80, "f32", "bool"), (1, 1, 3, 130, 256, 100, "f32", "bias"),
@@ -236,10 +244,10 @@ def test_planes_against_64_bits(L, api, b, kvh, g, lq, lk, d, dt, form):
         bias = torch.randn(lq, lk, generator=gen, device="cuda")
     got = api.scaledDotProductAttention(q, k, v, d ** -0.5, seen if form == "bool" else None, bias, causal=form == "causal")
     want = _exact(q, k, v, d ** -0.5, seen, bias)
-    # fp32: a rounding per product and sum, far below 1e-6. 16 bits: the rounding of the result, in bf16 by the reference's
-    # rule (half a unit is added only to an odd result: up to one unit, 2^-7 of the value), in fp16 half a unit.
-    tol = {"f32": 1e-6, "bf16": 2.0 ** -7, "f16": 2.0 ** -11}[dt]
-    assert (got.double() - want).abs().max() <= tol * want.abs().max()
+    # 16 bits: the rounding of the result, in bf16 by the reference's rule (half a unit is added only to an odd result: up to
+    # one unit, 2^-7 of the value), in fp16 half a unit.
+    bound = _f32_bound(q, k, v, d, bias) if dt == "f32" else {"bf16": 2.0 ** -7, "f16": 2.0 ** -11}[dt] * want.abs().max()
+    assert (got.double() - want).abs().max() <= bound
     assert L.ytcuda_device_status(None) == 0
 
 
@@ -265,3 +273,28 @@ def test_planes_step_aside_in_a_capture(api):
     out.zero_()
     graph.replay()
     assert (out - want).abs().max() <= 2e-6 * want.abs().max()  # (the FFMA kernel: another order of the sums)
+
+
+@pytest.mark.parametrize("lq,lk,d,dt", [(300, 336, 128, "bf16"), (257, 333, 64, "f16"), (129, 131, 128, "bf16"), (256, 301, 128, "f32"),
+                                        (200, 288, 80, "f32")])
+@pytest.mark.parametrize("form", ["bool", "bias", "both", "slices"])
+def test_masks_and_biases_of_any_alignment(L, api, lq, lk, d, dt, form):
+    gen = torch.Generator(device="cuda").manual_seed(lq + lk)
+    t = {"f32": torch.float32, "bf16": torch.bfloat16, "f16": torch.float16}[dt]
+    q, k, v = (torch.randn(1, h, n, d, generator=gen, device="cuda").to(t) for h, n in ((4, lq), (2, lk), (2, lk)))
+    seen = torch.rand(lq, lk + 5, generator=gen, device="cuda") < 0.5
+    bias = torch.randn(lq, lk + 7, generator=gen, device="cuda")
+    seen[7] = False  # a row that sees no key
+    seen[lq - 1] = False
+    seen[lq - 1, lk - 1] = True
+    off = 3 if form == "slices" else 0  # rows that start at odd addresses, strides of the wider tensor
+    seen, bias = seen[:, off:off + lk], bias[:, off:off + lk]
+    if form != "slices":
+        seen, bias = seen.contiguous(), bias.contiguous()
+    m, b = (None if form == "bias" else seen), (None if form == "bool" else bias)
+    got = api.scaledDotProductAttention(q, k, v, d ** -0.5, m, b)
+    want = torch.nan_to_num(_exact(q, k, v, d ** -0.5, m, b))
+    # 16 bits: P and the result are rounded to 16 bits
+    bound = _f32_bound(q, k, v, d, bias) if dt == "f32" else {"bf16": H_TOL, "f16": 2e-3}[dt] * want.abs().max()
+    assert (got.double() - want).abs().max() <= bound
+    assert m is None or not got[0, :, 7].any()

@@ -425,14 +425,9 @@ __global__ void __launch_bounds__(SA_THREADS, 1)
             for (int e = 0; e < 32; ++e)
               r[e] = __float_as_uint(c0 + e <= cl ? __uint_as_float(r[e]) * p.scale_log2 : -CUDART_INF_F);
           } else {
-#pragma unroll
-            for (int e = 0; e < 32; ++e) {
-              bool vis = c0 + e <= cl;
-              if (vis && p.a.mask) vis = p.a.mask[qi * p.a.mask_rs + key0 + c0 + e] != 0;
-              float v = __uint_as_float(r[e]) * p.scale_log2;
-              if (vis && p.a.bias) v += p.a.bias[qi * p.a.bias_rs + (key0 + c0 + e) * p.a.bias_cs] * FA_LOG2E;
-              r[e] = __float_as_uint(vis ? v : -CUDART_INF_F);
-            }
+            masked_scores(r, p.a.mask ? p.a.mask + qi * p.a.mask_rs + key0 + c0 : nullptr,
+                          p.a.bias ? p.a.bias + qi * p.a.bias_rs + (key0 + c0) * p.a.bias_cs : nullptr, p.a.bias_cs, cl - c0 + 1,
+                          p.scale_log2);
           }
 #pragma unroll
           for (int e = 0; e < 32; e += 2) mx = fmax3(mx, __uint_as_float(r[e]), __uint_as_float(r[e + 1]));

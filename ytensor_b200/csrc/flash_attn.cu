@@ -162,6 +162,56 @@ __device__ __forceinline__ float fast_rcp(float x) {
   return y;
 }
 
+// Scores of 32 keys of one row under a bool mask and / or a bias, in log2 units over the raw products in r; -inf where hidden:
+// beyond the first `n` keys (n may be anything) or masked out. mask / bias point at the row's first of these keys. All loads
+// are asked for before the first is used, 16 bytes at a time where the rows allow it: one element after the other, behind its
+// own branch and in both passes of the softmax, they were nine tenths of a tile's time (8 heads of 128, 1024 x 1024, bf16
+// with a bias: 327 us, 65 here; a bool mask, 2048 x 2048: 622, 90).
+__device__ __forceinline__ void masked_scores(uint32_t (&r)[32], const uint8_t* mask, const float* bias, int64_t bias_cs, int n,
+                                              float scale_log2) {
+  if (n > 32) n = 32;
+  uint32_t seen = n <= 0 ? 0u : 0xFFFFFFFFu >> (32 - n);
+  if (mask && n > 0) {
+    uint32_t w[9];
+    const uint32_t skew = static_cast<uint32_t>(reinterpret_cast<uint64_t>(mask)) & 3u;
+    if (n == 32 && (reinterpret_cast<uint64_t>(mask) & 15u) == 0) {
+      const uint4 a = *reinterpret_cast<const uint4*>(mask), b = *reinterpret_cast<const uint4*>(mask + 16);
+      w[0] = a.x; w[1] = a.y; w[2] = a.z; w[3] = a.w; w[4] = b.x; w[5] = b.y; w[6] = b.z; w[7] = b.w; w[8] = 0u;
+    } else {  // (whole words that hold at least one byte of the row)
+      const uint32_t* p = reinterpret_cast<const uint32_t*>(mask - skew);
+      const int words = (static_cast<int>(skew) + n + 3) >> 2;
+#pragma unroll
+      for (int i = 0; i < 9; ++i) w[i] = i < words ? p[i] : 0u;
+    }
+    uint32_t bits = 0;
+#pragma unroll
+    for (int i = 0; i < 8; ++i) {
+      const uint32_t t = __vsetne4(__funnelshift_r(w[i], w[i + 1], skew * 8u), 0u);
+      bits |= ((t | (t >> 7) | (t >> 14) | (t >> 21)) & 15u) << (4 * i);
+    }
+    seen &= bits;
+  }
+  if (bias) {
+    float b[32];
+    if (n == 32 && bias_cs == 1 && (reinterpret_cast<uint64_t>(bias) & 15u) == 0) {
+#pragma unroll
+      for (int i = 0; i < 8; ++i) {
+        const float4 t = reinterpret_cast<const float4*>(bias)[i];
+        b[4 * i] = t.x; b[4 * i + 1] = t.y; b[4 * i + 2] = t.z; b[4 * i + 3] = t.w;
+      }
+    } else {
+#pragma unroll
+      for (int e = 0; e < 32; ++e) b[e] = e < n ? bias[e * bias_cs] : 0.f;
+    }
+#pragma unroll
+    for (int e = 0; e < 32; ++e)
+      r[e] = __float_as_uint((seen >> e) & 1u ? __uint_as_float(r[e]) * scale_log2 + b[e] * FA_LOG2E : -CUDART_INF_F);
+  } else {
+#pragma unroll
+    for (int e = 0; e < 32; ++e) r[e] = __float_as_uint((seen >> e) & 1u ? __uint_as_float(r[e]) * scale_log2 : -CUDART_INF_F);
+  }
+}
+
 template <int D>
 struct FaSmem {
   static constexpr int TILE_BYTES = FA_BM * D * 2;  // one Q / K / V tile
@@ -605,14 +655,6 @@ __global__ void __launch_bounds__(FA_THREADS, 1)
           if (lane == 0) mbar_arrive(&p_full[t]);
           continue;
         }
-        auto score = [&](uint32_t raw, int c) -> float {  // general tiles only
-          float v = __uint_as_float(raw) * p.scale_log2;
-          const int key = key0 + c;
-          bool vis = c <= cl;
-          if (vis && p.mask) vis = p.mask[static_cast<int64_t>(row) * p.mask_rs + key] != 0;
-          if (vis && p.bias) v += p.bias[static_cast<int64_t>(row) * p.bias_rs + key * p.bias_cs] * FA_LOG2E;
-          return vis ? v : -CUDART_INF_F;
-        };
         // pass 1: row maximum. Without mask / bias the maximum is taken over the raw scores (one instruction per
         // element, two with the per-row limit) and scaled afterwards; a negative scale flips max into min.
         float mx = -CUDART_INF_F;
@@ -662,14 +704,20 @@ __global__ void __launch_bounds__(FA_THREADS, 1)
           const float ext = pos ? fmaxf(fmaxf(a0, a1), fmaxf(a2, a3)) : fminf(fminf(a0, a1), fminf(a2, a3));
           mx = (ext == ident) ? -CUDART_INF_F : ext * p.scale_log2;
         } else {
+          // the scores go back over S: pass 2 reads them as they are
 #pragma unroll 1
           for (int c0 = 0; c0 < FA_BN; c0 += 32) {
             uint32_t r[32];
             tmem_ld_32x32b_x32(ts + c0, r);
             tmem_ld_wait();
+            masked_scores(r, p.mask ? p.mask + static_cast<int64_t>(row) * p.mask_rs + key0 + c0 : nullptr,
+                          p.bias ? p.bias + static_cast<int64_t>(row) * p.bias_rs + (key0 + c0) * p.bias_cs : nullptr, p.bias_cs,
+                          cl - c0 + 1, p.scale_log2);
 #pragma unroll
-            for (int e = 0; e < 32; ++e) mx = fmaxf(mx, score(r[e], c0 + e));
+            for (int e = 0; e < 32; e += 2) mx = fmax3(mx, __uint_as_float(r[e]), __uint_as_float(r[e + 1]));
+            tmem_st_32x32b_x32(ts + c0, r);
           }
+          tmem_st_wait();
         }
         const float m_new = fmaxf(m_run, mx);
         if (j == 0) {
@@ -788,8 +836,8 @@ __global__ void __launch_bounds__(FA_THREADS, 1)
             uint32_t pk[16];
 #pragma unroll
             for (int e = 0; e < 32; e += 2) {
-              const float p0 = fast_exp2(score(r[e], c0 + e) + neg_m);
-              const float p1 = fast_exp2(score(r[e + 1], c0 + e + 1) + neg_m);
+              const float p0 = fast_exp2(__uint_as_float(r[e]) + neg_m);
+              const float p1 = fast_exp2(__uint_as_float(r[e + 1]) + neg_m);
               l0 += p0;
               l1 += p1;
               pk[e >> 1] = pack2(p0, p1);
@@ -1288,6 +1336,13 @@ __global__ void __launch_bounds__(DF_WARPS * 32) attn_decode_fast_kernel(const A
       o4.z = fmaf(ow.z, f, o4.z);
       o4.w = fmaf(ow.w, f, o4.w);
     }
+    if (dp.splits == 1) {  // nothing to merge
+      float* out = static_cast<float*>(dp.a.O) + b * dp.a.o_sb + (kvh * G + g) * dp.a.o_sh + lane * 4;
+      const float o[4] = {o4.x, o4.y, o4.z, o4.w};
+#pragma unroll
+      for (int e = 0; e < 4; ++e) out[e] = lsum > 0.f ? o[e] / lsum : 0.f;
+      return;
+    }
     // the layout attn_decode_merge_kernel reads: [m, l, o[dv]] per (kv head, split, row); row = g (q_len == 1)
     float* dst = dp.part + ((static_cast<int64_t>(bk) * dp.splits + split) * G + g) * (2 + D);
     if (lane == 0) {
@@ -1670,7 +1725,7 @@ __global__ void __launch_bounds__(256, 1) attn_tile64_kernel(const AttnSimtParam
 
 // Where the tensor-core form is faster than the tiled FFMA kernels, by their steps one after another: a step of 64 keys of
 // attn_tile64_kernel takes about 10 us, one of 32 keys of attn_tile_kernel about 20 (fp32) to 40 (16 bit), the tensor-core
-// form 12 us and two more launches, then 2.8 us per 64 keys. Measured (FFMA / tensor cores): 256 keys, 16 heads 45 / 37 us;
+// form 12 us and two more launches, then 2.4 us per 64 keys. Measured (FFMA / tensor cores): 256 keys, 16 heads 45 / 37 us;
 // 128 keys, 8 heads 30 / 42; 33 keys 45 / 41; 32 sequences of 60 tokens, 16 heads 235 / 58.
 static bool split_attention_pays(const AttnSimtParams& p) {
   const int heads = p.kv_heads * p.groups;
@@ -1937,17 +1992,20 @@ int ytcuda_flash_attn_fwd(int dtype, const void* Q, const void* K, const void* V
     const int max_splits = (kv_len + 31) / 32;
     if (splits > max_splits) splits = max_splits;
     if (splits < 1) splits = 1;
-    dp.keys_per_split = (kv_len + splits - 1) / splits;
-    dp.splits = (kv_len + dp.keys_per_split - 1) / dp.keys_per_split;
-    const size_t need = static_cast<size_t>(bk) * dp.splits * groups * q_len * (2 + value_dim) * sizeof(float);
-    dp.part = static_cast<float*>(device_workspace(need, st));
-    if (!dp.part) {
-      set_last_error("ytcuda_flash_attn_fwd: cannot allocate %zu bytes of scratch", need);
-      return YTC_CUDA_ERROR;
-    }
     const bool fast = dtype == YTC_F32 && q_len == 1 && head_dim == 128 && value_dim == 128 && !mptr && !bias &&
                       (groups == 1 || groups == 2 || groups == 4) && q_strides[1] % 4 == 0 && q_strides[0] % 4 == 0 &&
                       (reinterpret_cast<uint64_t>(Q) & 15) == 0 && g_attn_path != 1;
+    // One piece where that saves the merge and costs no second trip over the keys (eight warps of 16), or where every SM has
+    // a CTA anyhow. Measured, a decode step of 32 sequences of 60 to 80 keys (28 layers): 2.0 -> 1.85 ms.
+    if (fast && (kv_len <= DF_WARPS * DF_KB || (bk >= sm_count() && kv_len <= 512))) splits = 1;
+    dp.keys_per_split = (kv_len + splits - 1) / splits;
+    dp.splits = (kv_len + dp.keys_per_split - 1) / dp.keys_per_split;
+    const size_t need = fast && dp.splits == 1 ? 0 : static_cast<size_t>(bk) * dp.splits * groups * q_len * (2 + value_dim) * sizeof(float);
+    dp.part = need ? static_cast<float*>(device_workspace(need, st)) : nullptr;
+    if (need && !dp.part) {
+      set_last_error("ytcuda_flash_attn_fwd: cannot allocate %zu bytes of scratch", need);
+      return YTC_CUDA_ERROR;
+    }
     if (fast) {
       if (groups == 1) YTC_CUDA(launch_overlapped(attn_decode_fast_kernel<1>, dim3(dp.splits, bk), dim3(DF_WARPS * 32), 0, st, dp));
       else if (groups == 2) YTC_CUDA(launch_overlapped(attn_decode_fast_kernel<2>, dim3(dp.splits, bk), dim3(DF_WARPS * 32), 0, st, dp));
@@ -1955,8 +2013,9 @@ int ytcuda_flash_attn_fwd(int dtype, const void* Q, const void* K, const void* V
     } else {
       attn_decode_kernel<<<dim3(dp.splits, bk), DEC_WARPS * 32, 0, st>>>(dp);
     }
-    YTC_CUDA(launch_overlapped(attn_decode_merge_kernel, dim3(bk), dim3(128), 0, st, dp));
-    count_launch(2);
+    const bool whole = fast && dp.splits == 1;  // (the fast kernel stores the result itself)
+    if (!whole) YTC_CUDA(launch_overlapped(attn_decode_merge_kernel, dim3(bk), dim3(128), 0, st, dp));
+    count_launch(whole ? 1 : 2);
     YTC_CUDA(cudaGetLastError());
     return YTC_OK;
   }
