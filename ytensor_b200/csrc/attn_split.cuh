@@ -5,31 +5,32 @@
 //  * attn_planes_kernel: K and V (any type, any strides of whole groups of four) -> planes
 //    [plane][batch * kv head][key][64 or 128] in scratch memory, and a word per block that says whether it met a number
 //    that has no planes (infinity, NaN, 2^127 and above).
-//  * attn_split_kernel: 128 query rows x 64 keys per step, one persistent CTA per SM. The planes of Q sit in tensor memory
-//    (operand A of Q K^T: from shared memory A and B together would need 192 bytes a clock), K and V tiles come by TMA
-//    through two stages each. Two softmax warpgroups take the key tiles in turn, each with a running maximum, sum and O of
-//    its own in registers, so that the chain S -> maximum -> P of one tile runs under the MMAs of the other; P V of a tile
-//    starts from zero in tensor memory and is added to the registers in fp32 (a sum over thousands of keys inside the
-//    accumulator would collect a truncation per step). At the end the warpgroups merge through tensor memory.
+//  * attn_split_kernel: 128 query rows x 128 keys per step, one persistent CTA per SM. The planes of Q sit in shared memory;
+//    K and V come plane by plane, 32 KB each, by TMA through a ring of four, in the order in which the MMAs take them. Two
+//    softmax warpgroups take the key tiles in turn, each with a running maximum, sum and O of its own in registers, so that
+//    the chain S -> maximum -> P of one tile runs under the MMAs of the other; P V of a tile starts from zero in tensor
+//    memory and is added to the registers in fp32 (a sum over thousands of keys inside the accumulator would collect a
+//    truncation per step). At the end the warpgroups merge through tensor memory.
 //
-// What bounds it: the tensor pipe, 72 MMAs of at least 64 clocks a tile (one with A in tensor memory takes 64 clocks for 64
-// columns as for 128): 5200 clocks measured, 4600 of them MMAs. Measured on a B200, causal, fp32, 16 query and 8 key heads
-// of 128, planes and check included, FFMA kernel / here: 1000 queries and keys 256 / 78 us, 2000: 761 / 185; bf16, 8 heads of
-// 80, 1024: 1345 / 59. Error against 64 bits (2-norm) at 1000 keys: 3.8e-7 / 1.8e-7.
+// What bounds it: the tensor pipe and the shared memory that feeds it (Q K^T reads 8 KB per MMA of 64 clocks, the copies add a
+// quarter): 6 products of 128 x 128 x 128 for S and for P V, 96 MMAs a tile. Measured on a B200, causal, fp32, 16 query and 8
+// key heads of 128, planes and check included, FFMA kernel / here: 1000 queries and keys 256 / 70 us, 2000: 761 / 159; bf16,
+// 8 heads of 80, 1024: 1345 / 58. (Q in tensor memory and tiles of 64 keys: 78, 185 and 59 us; an MMA of 64 columns takes as
+// long there as one of 128.) Error against 64 bits (2-norm) at 1000 keys: 3.9e-7 / 2.1e-7.
 #pragma once
 
 namespace ytk {
 
-constexpr int SA_BM = 128, SA_BN = 64, SA_THREADS = 384;  // a service warpgroup, two softmax warpgroups
-constexpr int SA_BLOCK = SA_BN * 128;               // bytes of 64 keys x 64 columns of one plane
-constexpr int SA_TILE = 3 * 2 * SA_BLOCK;           // three planes of two column blocks
-constexpr int SA_K_OFF = 0, SA_V_OFF = 2 * SA_TILE;
-constexpr int SA_ML_OFF = 4 * SA_TILE;              // [2][128] running maximum, [2][128] sum
-constexpr int SA_BAR_OFF = SA_ML_OFF + 4 * 128 * 4;
-constexpr int SA_NBAR = 8 + 4 + 6;
+constexpr int SA_BM = 128, SA_BN = 128, SA_THREADS = 384;  // a service warpgroup, two softmax warpgroups
+constexpr int SA_BLOCK = SA_BN * 128;               // bytes of 128 rows x 64 columns of one plane
+constexpr int SA_PLANE = 2 * SA_BLOCK;
+constexpr int SA_SLOTS = 4;
+constexpr int SA_Q_OFF = 0, SA_RING_OFF = 3 * SA_PLANE;
+constexpr int SA_BAR_OFF = SA_RING_OFF + SA_SLOTS * SA_PLANE;
+constexpr int SA_NBAR = 2 * SA_SLOTS + 6 + 4;
 constexpr int SA_DYN_BYTES = SA_BAR_OFF + SA_NBAR * 8 + 32 + 1024;
-// tensor-memory columns: planes of Q [3][64], two S / P buffers of 96, one O
-constexpr uint32_t SA_T_S = 192, SA_T_SP = 96, SA_T_O = 384;
+// tensor-memory columns: two S / P buffers of 192 (S 128, three planes of P 64 each), one O
+constexpr uint32_t SA_T_SP = 192, SA_T_O = 384;
 
 struct SplitAttnParams {
   AttnSimtParams a;
@@ -39,7 +40,7 @@ struct SplitAttnParams {
   int n_units, n_items;
   int flat;         // a unit is a K/V head
   int o_vec;        // O is stored four values at a time
-  uint32_t idesc_s, idesc_pv;
+  uint32_t idesc_s, idesc_s_half, idesc_pv;  // (half: a last tile of at most 64 keys)
   float scale_log2;
   int* unfit;       // [CTAs] set where Q holds a number without planes
   int* status;
@@ -113,6 +114,7 @@ __global__ void __launch_bounds__(256) attn_planes_kernel(const PlanesParams p) 
 
 struct SplitItem {
   int r0, unit, n;  // first query row within the unit, unit, key tiles
+  bool half;        // no row sees more than 64 keys of the last tile
 };
 __device__ __forceinline__ SplitItem split_item(const SplitAttnParams& p, int w) {
   SplitItem it;
@@ -125,6 +127,7 @@ __device__ __forceinline__ SplitItem split_item(const SplitAttnParams& p, int w)
     last = min(last, (q0 == q1 ? r1 - q1 * p.a.q_len : p.a.q_len - 1) + p.a.causal_off);
   }
   it.n = last < 0 ? 0 : last / SA_BN + 1;
+  it.half = last % SA_BN < 64;
   return it;
 }
 
@@ -132,10 +135,9 @@ __global__ void __launch_bounds__(SA_THREADS, 1)
     attn_split_kernel(const __grid_constant__ CUtensorMap tmK, const __grid_constant__ CUtensorMap tmV, const SplitAttnParams p) {
   extern __shared__ uint8_t smem_raw[];
   uint8_t* smem = smem_raw + ((1024u - (smem_u32(smem_raw) & 1023u)) & 1023u);
-  float* ml = reinterpret_cast<float*>(smem + SA_ML_OFF);
   uint64_t* bars = reinterpret_cast<uint64_t*>(smem + SA_BAR_OFF);
-  uint64_t *k_full = bars, *k_empty = bars + 2, *v_full = bars + 4, *v_empty = bars + 6, *s_full = bars + 8, *p_full = bars + 10;
-  uint64_t *o_full = bars + 12, *o_free = bars + 14, *q_ready = bars + 15, *merge_in = bars + 16, *merge_out = bars + 17;
+  uint64_t *full = bars, *empty = bars + SA_SLOTS, *s_full = empty + SA_SLOTS, *p_full = s_full + 2, *o_full = p_full + 2;
+  uint64_t *o_free = o_full + 2, *q_ready = o_free + 1, *merge_in = o_free + 2, *merge_out = o_free + 3;
   uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(bars + SA_NBAR);
   volatile int* abort_word = reinterpret_cast<volatile int*>(tmem_slot + 1);
   int* unfit_word = reinterpret_cast<int*>(tmem_slot + 2);
@@ -143,11 +145,11 @@ __global__ void __launch_bounds__(SA_THREADS, 1)
   const int bkv = p.a.batch * p.a.kv_heads;
 
   if (threadIdx.x == 0) {
+    for (int s = 0; s < SA_SLOTS; ++s) {
+      mbar_init(&full[s], 1);
+      mbar_init(&empty[s], 1);
+    }
     for (int s = 0; s < 2; ++s) {
-      mbar_init(&k_full[s], 1);
-      mbar_init(&k_empty[s], 1);
-      mbar_init(&v_full[s], 1);
-      mbar_init(&v_empty[s], 1);
       mbar_init(&s_full[s], 1);
       mbar_init(&o_full[s], 1);
       mbar_init(&p_full[s], 4);  // one arrival per warp of a warpgroup
@@ -174,148 +176,152 @@ __global__ void __launch_bounds__(SA_THREADS, 1)
   dependent_wait();
   dependent_trigger();
 
-  // `g` counts the key tiles of all items so far: stage, buffer and warpgroup g & 1, phase (g >> 1) & 1. Items without a
-  // visible key touch no barrier.
+  // `g` counts the key tiles of all items so far: S / P buffer and warpgroup g & 1, phase (g >> 1) & 1. `n_pl` counts the
+  // planes of K and V, loaded and multiplied in one order: K of tiles 0 and 1, then V of tile j and K of tile j + 2; of a tile
+  // the last plane first. Items without a visible key touch no barrier.
   if (warp < 4) {
-    // (168 registers a thread at launch, 56 + 2 * 224 afterwards, the same sum: the softmax keeps 128 columns of O)
-    asm volatile("setmaxnreg.dec.sync.aligned.u32 56;");
+    // (168 registers a thread at launch, 72 + 2 * 216 afterwards, the same sum: the softmax keeps 128 columns of O)
+    asm volatile("setmaxnreg.dec.sync.aligned.u32 72;");
     if (warp == 0) {
       // ------------------------------------------------------------ TMA producer
       if (lane == 0) {
         const int kblocks = (p.a.d + 63) / 64, vblocks = (p.a.dv + 63) / 64;
-        int g = 0;
-        bool ok = true;
-        auto load = [&](const CUtensorMap* tm, uint64_t* bar, uint8_t* dst, int blocks, int key, int bh) {
-          mbar_expect_tx(bar, static_cast<uint32_t>(p.planes * blocks * SA_BLOCK));
+        int n_pl = 0;
+        auto load = [&](const CUtensorMap* tm, int blocks, int tile, int bh) {
 #pragma unroll 1
-          for (int i = 0; i < p.planes; ++i)
+          for (int i = p.planes - 1; i >= 0; --i, ++n_pl) {
+            const int s = n_pl % SA_SLOTS;
+            if (!mbar_wait(&empty[s], ((n_pl / SA_SLOTS) & 1) ^ 1, abort_word)) return false;
+            mbar_expect_tx(&full[s], static_cast<uint32_t>(blocks * SA_BLOCK));
 #pragma unroll 1
-            for (int c = 0; c < blocks; ++c) tma_load_3d(dst + (i * 2 + c) * SA_BLOCK, tm, bar, c * 64, key, i * bkv + bh);
+            for (int c = 0; c < blocks; ++c)
+              tma_load_3d(smem + SA_RING_OFF + s * SA_PLANE + c * SA_BLOCK, tm, &full[s], c * 64, tile * SA_BN, i * bkv + bh);
+          }
+          return true;
         };
+        bool ok = true;
         for (int w = blockIdx.x; ok && w < p.n_items; w += gridDim.x) {
           const SplitItem it = split_item(p, w);
           const int bh = p.flat ? it.unit : it.unit / p.a.groups;
-          for (int j = 0; ok && j < it.n; ++j, ++g) {
-            const int s = g & 1;
-            const uint32_t ph = ((g >> 1) & 1) ^ 1;
-            ok = mbar_wait(&k_empty[s], ph, abort_word);
-            if (!ok) break;
-            load(&tmK, &k_full[s], smem + SA_K_OFF + s * SA_TILE, kblocks, j * SA_BN, bh);
-            ok = mbar_wait(&v_empty[s], ph, abort_word);
-            if (!ok) {  // (the K copies above must land before the CTA may end)
-              const long long t0 = clock64();
-              while (!mbar_try_wait(&k_full[s], ph ^ 1) && clock64() - t0 < 20000000ll) {
-              }
-              break;
-            }
-            load(&tmV, &v_full[s], smem + SA_V_OFF + s * SA_TILE, vblocks, j * SA_BN, bh);
+          for (int j = 0; ok && j < 2 && j < it.n; ++j) ok = load(&tmK, kblocks, j, bh);
+          for (int j = 0; ok && j < it.n; ++j) {
+            ok = load(&tmV, vblocks, j, bh);
+            if (ok && j + 2 < it.n) ok = load(&tmK, kblocks, j + 2, bh);
           }
         }
-        // a give-up elsewhere: bounded drain of the last copies of both stages
+        // a give-up elsewhere: bounded drain of the last copies
         const long long t0 = clock64();
-        for (int k = 1; k <= 2 && g - k >= 0; ++k) {
-          const int s = (g - k) & 1;
-          const uint32_t ph = ((g - k) >> 1) & 1;
-          while ((!mbar_try_wait(&k_full[s], ph) || !mbar_try_wait(&v_full[s], ph)) && clock64() - t0 < 20000000ll) {
+        for (int k = n_pl - SA_SLOTS > 0 ? n_pl - SA_SLOTS : 0; k < n_pl; ++k)
+          while (!mbar_try_wait(&full[k % SA_SLOTS], (k / SA_SLOTS) & 1) && clock64() - t0 < 20000000ll) {
           }
-        }
       }
     } else if (warp == 1) {
       // ------------------------------------------------------------ MMA issuer
-      // The whole warp runs this code and lane 0 issues: straight code, constant offsets, operands in uniform registers.
-      // Measured per MMA: 190 clocks for a loop that forms descriptors in a one-lane branch; 64, the pipe's own time, here.
+      // The whole warp runs this code and lane 0 issues: straight code, constant offsets, operands in uniform registers
+      // (a loop that forms descriptors in a one-lane branch costs 190 clocks per MMA, the tensor pipe needs 64).
       const uint32_t lead = lane == 0;
-      const uint64_t kd = umma_smem_desc_sw128(smem_u32(smem + SA_K_OFF), 16, 1024);
-      const uint64_t vd = umma_smem_desc_sw128(smem_u32(smem + SA_V_OFF), SA_BLOCK, 1024);
-      constexpr uint32_t PLANE = 2 * SA_BLOCK / 16, BLOCK = SA_BLOCK / 16;  // (descriptors count 16 bytes)
+      const uint64_t qd = umma_smem_desc_sw128(smem_u32(smem + SA_Q_OFF), 16, 1024);
+      const uint64_t kd = umma_smem_desc_sw128(smem_u32(smem + SA_RING_OFF), 16, 1024);
+      const uint64_t vd = umma_smem_desc_sw128(smem_u32(smem + SA_RING_OFF), SA_BLOCK, 1024);
+      constexpr uint32_t PLANE = SA_PLANE / 16, BLOCK = SA_BLOCK / 16;  // (descriptors count 16 bytes)
       const int ksteps = (p.a.d + 15) / 16;
+      // (every lane waits: a give-up is agreed on before the next step)
+      auto wait = [&](uint64_t* bar, uint32_t ph) { return __all_sync(0xffffffffu, mbar_wait(bar, ph, abort_word)) != 0; };
       auto commit = [&](uint64_t* bar) {
         if (lead) tc_commit(bar);
         __syncwarp();
       };
-      auto issue_s = [&](int s) {  // S = Q K^T, planes (i, j) with i + j <= 2, smallest products first
-        const uint64_t kb = kd + s * (SA_TILE / 16);
-        const uint32_t ds = SA_T_S + s * SA_T_SP;
-        auto steps = [&](int k0, int k1, int i, int j, bool add) {
+      int n_pl = 0;
+      // The products of plane J of K (or V) with planes I of Q (or P), I + J <= 2, the smallest first
+      auto k_plane = [&](auto plane, uint32_t ds, uint32_t idesc) {
+        constexpr int J = decltype(plane)::value;
+        if (J >= p.planes) return true;
+        const int s = n_pl % SA_SLOTS;
+        if (!wait(&full[s], (n_pl / SA_SLOTS) & 1)) return false;
+        tc_fence_after();
+        const uint64_t kb = kd + s * PLANE;
+        auto steps = [&](int k0, int k1, int i, bool add) {
 #pragma unroll
           for (int k = k0; k < k1; ++k)
-            tc_mma_f16_ts_lead(ds, i * 64 + k * 8, kb + (j * PLANE + (k >> 2) * BLOCK + (k & 3) * 2), p.idesc_s, add || k > 0,
-                               lead);
+            tc_mma_f16_lead(ds, qd + (i * PLANE + (k >> 2) * BLOCK + (k & 3) * 2), kb + ((k >> 2) * BLOCK + (k & 3) * 2), idesc,
+                            add || k > 0, lead);
         };
-        auto product = [&](int i, int j, bool add) {  // (zeros behind column d, to 64, 96 or 128)
-          steps(0, 4, i, j, add);
-          if (ksteps > 4) steps(4, 6, i, j, true);
-          if (ksteps > 6) steps(6, 8, i, j, true);
-        };
-        if (p.planes == 3) {
-          product(0, 2, false);
-          product(2, 0, true);
-        }
-        if (p.planes >= 2) {
-          product(1, 1, p.planes == 3);
-          product(0, 1, true);
-          product(1, 0, true);
-        }
-        product(0, 0, p.planes >= 2);
-        commit(&s_full[s]);
-        commit(&k_empty[s]);
-      };
-      auto issue_pv = [&](int s) {  // O = P V: P has three planes, laid out around the columns of S (see the softmax)
-        const uint64_t vb = vd + s * (SA_TILE / 16);
-        const uint32_t as = SA_T_S + s * SA_T_SP;
-        auto product = [&](int i, int j, bool add) {
 #pragma unroll
-          for (int k = 0; k < SA_BN / 16; ++k)
-            tc_mma_f16_ts_lead(SA_T_O, as + (i == 0 ? 64 + k * 8 : (k >> 1) * 32 + (i - 1) * 16 + (k & 1) * 8),
-                               vb + (j * PLANE + k * 128), p.idesc_pv, add || k > 0, lead);
-        };
-        product(2, 0, false);
-        if (p.planes >= 2) product(1, 1, true);
-        if (p.planes == 3) product(0, 2, true);
-        product(1, 0, true);
-        if (p.planes >= 2) product(0, 1, true);
-        product(0, 0, true);
-        commit(&o_full[s]);
-        commit(&v_empty[s]);
+        for (int i = 2 - J; i >= 0; --i) {
+          if (i >= p.planes) continue;
+          const bool add = !(J == p.planes - 1 && i == (2 - J < p.planes - 1 ? 2 - J : p.planes - 1));
+          steps(0, 4, i, add);  // (zeros behind column d, to 64, 96 or 128)
+          if (ksteps > 4) steps(4, 6, i, true);
+          if (ksteps > 6) steps(6, 8, i, true);
+        }
+        commit(&empty[s]);
+        ++n_pl;
+        return true;
       };
-      // (every lane waits: a give-up is agreed on before the next step)
-      auto wait = [&](uint64_t* bar, uint32_t ph) { return __all_sync(0xffffffffu, mbar_wait(bar, ph, abort_word)) != 0; };
+      auto v_plane = [&](auto plane, uint32_t as, bool half) {  // P: see the softmax for where its planes lie
+        constexpr int J = decltype(plane)::value;
+        if (J >= p.planes) return true;
+        const int s = n_pl % SA_SLOTS;
+        if (!wait(&full[s], (n_pl / SA_SLOTS) & 1)) return false;
+        tc_fence_after();
+        const uint64_t vb = vd + s * PLANE;
+        auto steps = [&](int k0, int k1, int i, bool add) {
+#pragma unroll
+          for (int k = k0; k < k1; ++k)
+            tc_mma_f16_ts_lead(SA_T_O, as + (i == 0 ? 128 + k * 8 : (k >> 1) * 32 + (i - 1) * 16 + (k & 1) * 8), vb + k * 128,
+                               p.idesc_pv, add || k > 0, lead);
+        };
+#pragma unroll
+        for (int i = 2 - J; i >= 0; --i) {
+          steps(0, 4, i, !(J == p.planes - 1 && i == 2 - J));
+          if (!half) steps(4, 8, i, true);
+        }
+        commit(&empty[s]);
+        ++n_pl;
+        return true;
+      };
+      using P0 = std::integral_constant<int, 0>;
+      using P1 = std::integral_constant<int, 1>;
+      using P2 = std::integral_constant<int, 2>;
+      auto issue_s = [&](int b, bool half) {
+        const uint32_t ds = b * SA_T_SP, idesc = half ? p.idesc_s_half : p.idesc_s;
+        if (!k_plane(P2{}, ds, idesc) || !k_plane(P1{}, ds, idesc) || !k_plane(P0{}, ds, idesc)) return false;
+        commit(&s_full[b]);
+        return true;
+      };
+      auto issue_pv = [&](int b, bool half) {
+        const uint32_t as = b * SA_T_SP;
+        if (!v_plane(P2{}, as, half) || !v_plane(P1{}, as, half) || !v_plane(P0{}, as, half)) return false;
+        commit(&o_full[b]);
+        return true;
+      };
       int g = 0, n_item = 0;
       bool ok = true;
       for (int w = blockIdx.x; ok && w < p.n_items; w += gridDim.x) {
         const SplitItem it = split_item(p, w);
         if (it.n == 0) continue;
         if (!wait(q_ready, n_item & 1)) break;
-        for (int j = 0; ok && j < 2 && j < it.n; ++j) {
-          ok = wait(&k_full[(g + j) & 1], ((g + j) >> 1) & 1);
-          if (!ok) break;
-          tc_fence_after();
-          issue_s((g + j) & 1);
-        }
+        tc_fence_after();
+        for (int j = 0; ok && j < 2 && j < it.n; ++j) ok = issue_s((g + j) & 1, it.half && j == it.n - 1);
         for (int j = 0; ok && j < it.n; ++j, ++g) {
-          const int s = g & 1;
-          const uint32_t ph = (g >> 1) & 1;
-          ok = wait(&v_full[s], ph) && wait(&p_full[s], ph) && (g == 0 || wait(o_free, (g - 1) & 1));
+          const int b = g & 1;
+          ok = wait(&p_full[b], (g >> 1) & 1) && (g == 0 || wait(o_free, (g - 1) & 1));
           if (!ok) break;
           tc_fence_after();
-          issue_pv(s);
-          if (j + 2 < it.n) {
-            ok = wait(&k_full[s], ph ^ 1);
-            if (!ok) break;
-            tc_fence_after();
-            issue_s(s);  // (runs behind the P V that reads this buffer: MMAs of one thread keep their order)
-          }
+          ok = issue_pv(b, it.half && j == it.n - 1);
+          // (S of tile j + 2 runs behind the P V that reads this buffer: MMAs of one thread keep their order)
+          if (ok && j + 2 < it.n) ok = issue_s(b, it.half && j + 2 == it.n - 1);
         }
         ++n_item;
       }
     }
   } else {
     // ------------------------------------------------------------ softmax warpgroups
-    asm volatile("setmaxnreg.inc.sync.aligned.u32 224;");
+    asm volatile("setmaxnreg.inc.sync.aligned.u32 216;");
     const int wg = (warp - 4) >> 2, quad = warp & 3;
     const int row = quad * 32 + lane;
     const uint32_t tl = tmem + (static_cast<uint32_t>(quad * 32) << 16);
-    const uint32_t ts = tl + SA_T_S + wg * SA_T_SP, to = tl + SA_T_O;
+    const uint32_t ts = tl + wg * SA_T_SP, to = tl + SA_T_O;
     const bool general = p.a.mask != nullptr || p.a.bias != nullptr;
     const int esz = p.a.dt == YTC_F32 ? 4 : 2;
     int g = 0, n_item = 0;
@@ -352,43 +358,48 @@ __global__ void __launch_bounds__(SA_THREADS, 1)
           for (int c = wg * 64; c < min(p.a.dv, wg * 64 + 64); c += 4) store4(c, 0.f, 0.f, 0.f, 0.f);
         continue;
       }
-      {  // columns 64 wg .. 64 wg + 63 of this thread's query row into tensor memory
+      {  // columns 64 wg .. 64 wg + 63 of this thread's query row, three planes, swizzled as the TMA would
         if (n_item > 0 && !mbar_wait(merge_out, (n_item - 1) & 1, abort_word)) break;
-        tc_fence_after();
         const char* qrow = static_cast<const char*>(p.a.Q) + (b * p.a.q_sb + h * p.a.q_sh + qi * p.a.q_sr) * esz;
+        uint8_t* qs = smem + SA_Q_OFF + wg * SA_BLOCK + row * 128;
 #pragma unroll 1
-        for (int c0 = wg * 64; c0 < (wg == 0 ? 64 : p.a.d); c0 += 32) {  // (zeros behind the last column)
-          uint32_t pk[3][16];
+        for (int c0 = wg * 64; c0 < (wg == 0 ? 64 : p.a.d); c0 += 8) {  // (zeros behind the last column)
+          float x[8];
 #pragma unroll
-          for (int c = 0; c < 32; c += 4) {
-            float x[4] = {0.f, 0.f, 0.f, 0.f};
+          for (int e = 0; e < 8; ++e) x[e] = 0.f;
+#pragma unroll
+          for (int c = 0; c < 8; c += 4)
             if (valid && c0 + c < p.a.d) {
               if (p.a.dt == YTC_F32) {
                 const float4 v = *reinterpret_cast<const float4*>(qrow + (c0 + c) * 4);
-                x[0] = v.x; x[1] = v.y; x[2] = v.z; x[3] = v.w;
+                x[c] = v.x; x[c + 1] = v.y; x[c + 2] = v.z; x[c + 3] = v.w;
               } else {
 #pragma unroll
-                for (int k = 0; k < 4; ++k) x[k] = load_as_f32(qrow, c0 + c + k, p.a.dt);
+                for (int k = 0; k < 4; ++k) x[c + k] = load_as_f32(qrow, c0 + c + k, p.a.dt);
               }
             }
-            uint16_t pl[4][3];
+          uint16_t pl[8][3];
 #pragma unroll
-            for (int k = 0; k < 4; ++k) {
-              unfit |= has_no_planes(x[k]);
-              split_planes(x[k], pl[k]);
-            }
-#pragma unroll
-            for (int i = 0; i < 3; ++i) {
-              pk[i][c / 2] = pl[0][i] | (static_cast<uint32_t>(pl[1][i]) << 16);
-              pk[i][c / 2 + 1] = pl[2][i] | (static_cast<uint32_t>(pl[3][i]) << 16);
-            }
+          for (int e = 0; e < 8; ++e) {
+            unfit |= has_no_planes(x[e]);
+            split_planes(x[e], pl[e]);
           }
+          uint8_t* dst = qs + ((((c0 & 63) >> 3) ^ (row & 7)) << 4);
 #pragma unroll
           for (int i = 0; i < 3; ++i)
-            if (i < p.planes) tmem_st_32x32b_x16(tl + i * 64 + c0 / 2, pk[i]);
+            if (i < p.planes) {
+              uint32_t u[4];
+#pragma unroll
+              for (int e = 0; e < 4; ++e) u[e] = pl[2 * e][i] | (static_cast<uint32_t>(pl[2 * e + 1][i]) << 16);
+              *reinterpret_cast<uint4*>(dst + i * SA_PLANE) = make_uint4(u[0], u[1], u[2], u[3]);
+            }
         }
-        tmem_st_wait();
-        tc_fence_before();
+        // columns of the 16-column steps that the products of a d above 64 take with the last ones
+        if (wg == 1 && p.a.d > 64)
+          for (int c0 = (p.a.d + 7) / 8 * 8; c0 < (p.a.d + 31) / 32 * 32; c0 += 8)
+            for (int i = 0; i < p.planes; ++i)
+              *reinterpret_cast<uint4*>(qs + i * SA_PLANE + ((((c0 & 63) >> 3) ^ (row & 7)) << 4)) = make_uint4(0u, 0u, 0u, 0u);
+        fence_proxy_async_smem();
         __syncwarp();
         if (lane == 0) mbar_arrive(q_ready);
       }
@@ -402,12 +413,13 @@ __global__ void __launch_bounds__(SA_THREADS, 1)
         if (!ok) break;
         tc_fence_after();
         const int key0 = j * SA_BN, cl = limit - key0;  // columns 0 .. cl are visible to this row
-        const bool full = !general && __all_sync(0xffffffffu, cl >= SA_BN - 1);
+        const int cols = it.half && j == it.n - 1 ? 64 : SA_BN;
+        const bool full = !general && __all_sync(0xffffffffu, cl >= cols - 1);
         // Pass 1: the maximum. Tiles with hidden keys, a mask or a bias get their scores (log2 units, -inf where hidden)
         // written back over S, so that pass 2 is one piece of code: the instructions a softmax warp cycles through stay few.
         float mx = -CUDART_INF_F;
 #pragma unroll 1
-        for (int c0 = 0; c0 < SA_BN; c0 += 32) {
+        for (int c0 = 0; c0 < cols; c0 += 32) {
           uint32_t r[32];
           tmem_ld_32x32b_x32(ts + c0, r);
           tmem_ld_wait();
@@ -438,12 +450,12 @@ __global__ void __launch_bounds__(SA_THREADS, 1)
         const float m_use = m_new == -CUDART_INF_F ? 0.f : m_new;
         const float alpha = m_run == -CUDART_INF_F ? 0.f : fast_exp2(m_run - m_use);
         m_run = m_new;
-        // Pass 2: P of 32 keys at a time over columns of S that have been read: the second and third plane of keys 0..31 on
-        // columns 0..31, of keys 32..63 on columns 32..63, the first plane behind S.
+        // Pass 2: P of 32 keys at a time, the second and third plane over the 32 columns of S that have been read, the first
+        // plane behind S.
         const float sl = full ? p.scale_log2 : 1.f;
         uint64_t ps = f2_pack(0.f, 0.f);
 #pragma unroll 1
-        for (int c0 = 0; c0 < SA_BN; c0 += 32) {
+        for (int c0 = 0; c0 < cols; c0 += 32) {
           uint32_t r[32], pk[16];
           tmem_ld_32x32b_x32(ts + c0, r);
           tmem_ld_wait();
@@ -467,7 +479,7 @@ __global__ void __launch_bounds__(SA_THREADS, 1)
                 r[e + 1] = __float_as_uint(__uint_as_float(r[e + 1]) - __uint_as_float(r[e + 1] & 0xFFFF0000u));
               }
             }
-            tmem_st_32x32b_x16(ts + (i == 0 ? 64 + c0 / 2 : c0 + (i - 1) * 16), pk);
+            tmem_st_32x32b_x16(ts + (i == 0 ? 128 + c0 / 2 : c0 + (i - 1) * 16), pk);
           }
         }
         tmem_st_wait();
@@ -496,26 +508,31 @@ __global__ void __launch_bounds__(SA_THREADS, 1)
       }
       if (!ok) break;
       g += it.n;
-      // Merge: each warpgroup hands the other 64 columns of its O over through the columns of Q, which no MMA reads any
-      // more once the S of the last tile is there.
-      if (!mbar_wait(&s_full[(g - 1) & 1], ((g - 1) >> 1) & 1, abort_word)) break;
-      tc_fence_after();
+      // Merge: each warpgroup hands the other 64 columns of its O, its maximum and its sum over in its own S / P buffer, whose
+      // last P V it has waited for.
 #pragma unroll
       for (int c = 0; c < 64; c += 32) {
         uint32_t r[32];
 #pragma unroll
         for (int e = 0; e < 32; ++e) r[e] = __float_as_uint(wg == 0 ? acc[64 + c + e] : acc[c + e]);
-        tmem_st_32x32b_x32(tl + (wg == 0 ? 64 + c : c), r);
+        tmem_st_32x32b_x32(ts + c, r);
       }
-      ml[wg * 128 + row] = m_run;
-      ml[(2 + wg) * 128 + row] = l_run;
+      uint32_t ml[16];
+#pragma unroll
+      for (int e = 2; e < 16; ++e) ml[e] = 0u;
+      ml[0] = __float_as_uint(m_run);
+      ml[1] = __float_as_uint(l_run);
+      tmem_st_32x32b_x16(ts + 64, ml);
       tmem_st_wait();
       tc_fence_before();
       __syncwarp();
       if (lane == 0) mbar_arrive(merge_in);
       if (!mbar_wait(merge_in, n_item & 1, abort_word)) break;
       tc_fence_after();
-      const float m_o = ml[(1 - wg) * 128 + row], l_o = ml[(3 - wg) * 128 + row];
+      const uint32_t tx = tl + (1 - wg) * SA_T_SP;
+      tmem_ld_32x32b_x16(tx + 64, ml);
+      tmem_ld_wait();
+      const float m_o = __uint_as_float(ml[0]), l_o = __uint_as_float(ml[1]);
       const float m = fmaxf(m_run, m_o);
       const float f = m_run == -CUDART_INF_F ? 0.f : fast_exp2(m_run - m), f_o = m_o == -CUDART_INF_F ? 0.f : fast_exp2(m_o - m);
       const float l = l_run * f + l_o * f_o;
@@ -523,7 +540,7 @@ __global__ void __launch_bounds__(SA_THREADS, 1)
 #pragma unroll
       for (int c = 0; c < 64; c += 32) {
         uint32_t r[32];
-        tmem_ld_32x32b_x32(tl + wg * 64 + c, r);
+        tmem_ld_32x32b_x32(tx + c, r);
         tmem_ld_wait();
         float x[32];
 #pragma unroll
@@ -585,6 +602,7 @@ static bool split_attention(const AttnSimtParams& a, const int** gate, int* n_ga
   p.n_items = static_cast<int>(units * p.row_tiles);
   p.o_vec = (reinterpret_cast<uint64_t>(a.O) % (4 * esz)) == 0 && a.o_sb % 4 == 0 && a.o_sh % 4 == 0 && a.o_sr % 4 == 0;
   p.idesc_s = umma_idesc(1u, 0, 0, SA_BM, SA_BN);
+  p.idesc_s_half = umma_idesc(1u, 0, 0, SA_BM, 64);
   p.idesc_pv = umma_idesc(1u, 0, 1, SA_BM, static_cast<uint32_t>((a.dv + 15) / 16 * 16));
   p.scale_log2 = a.scale * FA_LOG2E;
   p.status = device_status_word();

@@ -200,8 +200,18 @@ __device__ __forceinline__ void tc_mma_f16_ts(uint32_t tmem_d, uint32_t tmem_a, 
       "r"(tmem_a), "l"(bdesc), "r"(idesc), "r"(accumulate)
       : "memory");
 }
-// The same for a whole warp that runs the issuing code converged, one lane with `lead` set: the operands' arithmetic then
-// stays in uniform registers, where the instruction wants them (in a branch of one lane every operand is moved there).
+// Both for a whole warp that runs the issuing code converged, one lane with `lead` set: the operands' arithmetic then stays
+// in uniform registers, where the instruction wants them (in a branch of one lane every operand is moved there).
+__device__ __forceinline__ void tc_mma_f16_lead(uint32_t tmem_d, uint64_t adesc, uint64_t bdesc, uint32_t idesc,
+                                                uint32_t accumulate, uint32_t lead) {
+  asm volatile(
+      "{\n\t.reg .pred p, q;\n\t"
+      "setp.ne.b32 p, %4, 0;\n\t"
+      "setp.ne.b32 q, %5, 0;\n\t"
+      "@q tcgen05.mma.cta_group::1.kind::f16 [%0], %1, %2, %3, p;\n\t}" ::"r"(tmem_d),
+      "l"(adesc), "l"(bdesc), "r"(idesc), "r"(accumulate), "r"(lead)
+      : "memory");
+}
 __device__ __forceinline__ void tc_mma_f16_ts_lead(uint32_t tmem_d, uint32_t tmem_a, uint64_t bdesc, uint32_t idesc,
                                                    uint32_t accumulate, uint32_t lead) {
   asm volatile(
