@@ -82,16 +82,27 @@ __device__ __forceinline__ TcPiece tc_piece(const GemmTcParams& p, int bf) {
   if (p.fold > 0) return {b, 0, p.split_blocks, split * p.fold};
   return {b, split * p.split_blocks, min(p.k_blocks, (split + 1) * p.split_blocks), 0};
 }
-// Where k block kb lies: block kk of plane (or batch item) za of A and zb of B.
+// Where a k block lies: block kk of plane (or batch item) za of A and zb of B; next() steps to the block behind it.
+template <bool PIECES>
 struct TcBlock {
-  int kk, za, zb;
+  int kk, za, zb, end, pair;
+  __device__ __forceinline__ void plane(const GemmTcParams& p, int ba, int bb, int first) {
+    kk = first;
+    end = first + p.fold;
+    za = ba * p.planes_a + static_cast<int>((p.pa >> (2 * pair)) & 3);
+    zb = bb * p.planes_b + static_cast<int>((p.pb >> (2 * pair)) & 3);
+  }
+  __device__ __forceinline__ TcBlock(const GemmTcParams& p, const TcPiece& w, int ba, int bb)
+      : kk(w.kb0), za(ba), zb(bb), end(0x7fffffff), pair(0) {
+    if (PIECES && p.fold > 0) plane(p, ba, bb, w.first);
+  }
+  __device__ __forceinline__ void next(const GemmTcParams& p, const TcPiece& w, int ba, int bb) {
+    if (++kk == end && PIECES) {
+      ++pair;
+      plane(p, ba, bb, w.first);
+    }
+  }
 };
-__device__ __forceinline__ TcBlock tc_block(const GemmTcParams& p, int first, int kb, int ba, int bb) {
-  if (p.fold == 0) return {kb, ba, bb};
-  const int pair = kb / p.fold;
-  return {first + kb - pair * p.fold, ba * p.planes_a + static_cast<int>((p.pa >> (2 * pair)) & 3),
-          bb * p.planes_b + static_cast<int>((p.pb >> (2 * pair)) & 3)};
-}
 
 template <int BN, int OUT_DT>
 __device__ __forceinline__ void tc_store_chunk(const GemmTcParams& p, const uint32_t (&r)[32], int64_t row_off,
@@ -269,7 +280,8 @@ __device__ __forceinline__ void tc_store_staged(const GemmTcParams& p, const uin
   __syncwarp();
 }
 
-template <int BN>
+// PIECES: a product of planes, or k in pieces (the few instructions more cost an ordinary short product 0.2 us).
+template <int BN, bool PIECES>
 __global__ void __launch_bounds__(TC_THREADS, 1)
     gemm_tc_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ CUtensorMap tmB,
                    const GemmTcParams p) {
@@ -354,7 +366,8 @@ __global__ void __launch_bounds__(TC_THREADS, 1)
       for (int tile = blockIdx.x; ok && tile < p.total_tiles; tile += gridDim.x) {
         const int bf = tile / tiles_per_batch;
         const int rem = tile - bf * tiles_per_batch;
-        const TcPiece piece = tc_piece(p, bf);
+        TcPiece piece{bf, 0, p.k_blocks, 0};
+        if (PIECES) piece = tc_piece(p, bf);
         if (p.tile_live && !p.tile_live[rem]) continue;
         const int mb = rem / p.tiles_n;
         const int nb = rem - mb * p.tiles_n;
@@ -363,7 +376,8 @@ __global__ void __launch_bounds__(TC_THREADS, 1)
         const int n_row0 = group * p.group_rows + nb * BN;
         const int ba = p.a_bcast ? 0 : piece.b;
         const int bb = p.b_bcast ? 0 : piece.b;
-        for (int kb = piece.kb0; kb < piece.kb1; ++kb) {
+        TcBlock<PIECES> at(p, piece, ba, bb);
+        for (int kb = piece.kb0; kb < piece.kb1; ++kb, at.next(p, piece, ba, bb)) {
           if (!mbar_wait(&empty_bar[stage], phase ^ 1u, abort_word)) {
             ok = false;
             break;
@@ -375,7 +389,6 @@ __global__ void __launch_bounds__(TC_THREADS, 1)
               pf_tile += gridDim.x;
             }
           }
-          const TcBlock at = tc_block(p, piece.first, kb, ba, bb);
           mbar_expect_tx(&full_bar[stage], S::STAGE_BYTES);
           uint8_t* sa = smem + stage * S::STAGE_BYTES;
           uint8_t* sb = sa + S::A_BYTES;
@@ -442,7 +455,8 @@ __global__ void __launch_bounds__(TC_THREADS, 1)
         if (!mbar_wait(&tempty_bar[acc], acc_phase ^ 1u, abort_word)) break;
         tc_fence_after();
         const uint32_t d_tmem = tmem_base + static_cast<uint32_t>(acc * BN);
-        const TcPiece piece = tc_piece(p, tile / tiles_per_batch);
+        TcPiece piece{0, 0, p.k_blocks, 0};
+        if (PIECES) piece = tc_piece(p, tile / tiles_per_batch);
         for (int kb = piece.kb0; kb < piece.kb1; ++kb) {
           if (!mbar_wait(&full_bar[stage], phase, abort_word)) {
             ok = false;
@@ -549,6 +563,7 @@ struct Tc2Smem {
   static constexpr int DYN_STAGED = OUT_OFFSET + 4 * TC_OUT_BYTES + 1024;
 };
 
+template <bool PIECES>
 __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(TC_THREADS, 1)
     gemm_tc2_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ CUtensorMap tmB,
                     const GemmTcParams p) {
@@ -614,8 +629,9 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(TC_THREADS, 1)
         const int bb = p.b_bcast ? 0 : b;
         const int m0 = mb * 256 + static_cast<int>(cta) * TC_BM;
         const int n0 = nb * TC2_BN + static_cast<int>(cta) * (TC2_BN / 2);
-        for (int kb = 0; kb < p.k_blocks; ++kb) {
-          const TcBlock at = tc_block(p, 0, kb, ba, bb);
+        const TcPiece piece{b, 0, p.k_blocks, 0};
+        TcBlock<PIECES> at(p, piece, ba, bb);
+        for (int kb = 0; kb < p.k_blocks; ++kb, at.next(p, piece, ba, bb)) {
           if (!mbar_wait(&empty_bar[stage], phase ^ 1u, abort_word)) {
             ok = false;
             break;
@@ -1059,7 +1075,8 @@ static int launch_tc(int dtype_in, int dtype_out, const void* A, const void* B, 
     p.k_blocks = p.split_blocks;
     p.planes_a = pl->planes_a; p.planes_b = pl->planes_b; p.pa = pl->pa; p.pb = pl->pb;
   }
-  p.a_prefetch = pl || splits > 1 ? 0 : g_tc_a_prefetch.load();
+  const bool pieces = pl || splits > 1;
+  p.a_prefetch = pieces ? 0 : g_tc_a_prefetch.load();
   p.split_loads = g_tc_split_loads;
   p.tile_live = nullptr;
   const LinearEpilogue none, *e = ex ? ex : &none;
@@ -1084,10 +1101,10 @@ static int launch_tc(int dtype_in, int dtype_out, const void* A, const void* B, 
     int clusters = sm_count() / 2;
     if (clusters > p.total_tiles) clusters = p.total_tiles;
     {
-      const int s = ensure_dynamic_smem(reinterpret_cast<const void*>(gemm_tc2_kernel), smem);
+      const int s = ensure_dynamic_smem(reinterpret_cast<const void*>(pieces ? gemm_tc2_kernel<true> : gemm_tc2_kernel<false>), smem);
       if (s != YTC_OK) return s;
     }
-    YTC_CUDA(launch_overlapped(gemm_tc2_kernel, dim3(clusters * 2), dim3(TC_THREADS), smem, st, tmA, tmB, p));
+    YTC_CUDA(launch_overlapped(pieces ? gemm_tc2_kernel<true> : gemm_tc2_kernel<false>, dim3(clusters * 2), dim3(TC_THREADS), smem, st, tmA, tmB, p));
     count_launch();
     YTC_CUDA(cudaGetLastError());
     return YTC_OK;
@@ -1101,14 +1118,16 @@ static int launch_tc(int dtype_in, int dtype_out, const void* A, const void* B, 
   }
   if (BN == 256) {
     const int smem = p.staged ? TcSmem<256>::DYN_STAGED : TcSmem<256>::DYN_BYTES;
-    const int s = ensure_dynamic_smem(reinterpret_cast<const void*>(gemm_tc_kernel<256>), smem);
+    auto* fn = pieces ? gemm_tc_kernel<256, true> : gemm_tc_kernel<256, false>;
+    const int s = ensure_dynamic_smem(reinterpret_cast<const void*>(fn), smem);
     if (s != YTC_OK) return s;
-    YTC_CUDA(launch_overlapped(gemm_tc_kernel<256>, dim3(grid), dim3(TC_THREADS), smem, st, tmA, tmB, p));
+    YTC_CUDA(launch_overlapped(fn, dim3(grid), dim3(TC_THREADS), smem, st, tmA, tmB, p));
   } else {
     const int smem = p.staged ? TcSmem<128>::DYN_STAGED : TcSmem<128>::DYN_BYTES;
-    const int s = ensure_dynamic_smem(reinterpret_cast<const void*>(gemm_tc_kernel<128>), smem);
+    auto* fn = pieces ? gemm_tc_kernel<128, true> : gemm_tc_kernel<128, false>;
+    const int s = ensure_dynamic_smem(reinterpret_cast<const void*>(fn), smem);
     if (s != YTC_OK) return s;
-    YTC_CUDA(launch_overlapped(gemm_tc_kernel<128>, dim3(grid), dim3(TC_THREADS), smem, st, tmA, tmB, p));
+    YTC_CUDA(launch_overlapped(fn, dim3(grid), dim3(TC_THREADS), smem, st, tmA, tmB, p));
   }
   count_launch();
   if (live) cudaFreeAsync(live, st);

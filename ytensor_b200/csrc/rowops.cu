@@ -1060,6 +1060,12 @@ static void launch_line_op(int op, const LineParams& p, bool per_thread, cudaStr
 // and beta per dim, null: they are laid out like the reduced dims.
 template <class K>
 static int launch_share(K kernel, const ShareParams& p, int64_t blocks, int threads, size_t smem, cudaStream_t st) {
+  if (p.shares == 1 && smem <= 32 * 1024) {  // the smallest calls: nothing to look up, an ordinary launch
+    kernel<<<static_cast<unsigned>(blocks), threads, smem, st>>>(p);
+    count_launch();
+    YTC_CUDA(cudaGetLastError());
+    return YTC_OK;
+  }
   const int s = ensure_dynamic_smem(reinterpret_cast<const void*>(kernel), static_cast<int>(smem));
   if (s != YTC_OK) return s;
   cudaLaunchConfig_t cfg{};
