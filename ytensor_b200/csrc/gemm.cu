@@ -1317,7 +1317,7 @@ __global__ void __launch_bounds__(256) gemm_apply_mask_kernel(void* C, int dt, i
 // Which kernel ytcuda_gemm picks: 0 = automatic, 1 = force FFMA, 2 = require tcgen05.
 static std::atomic<int> g_gemm_path{0};
 
-// fp32 GEMM on the tensor cores (see gemm_split3_kernel): 0 = automatic (large problems), 1 = never,
+// fp32 GEMM on the tensor cores (see gemm_planes_kernel): 0 = automatic (where it is faster), 1 = never,
 // 2 = whenever the shapes allow.
 static std::atomic<int> g_f32_split{0};
 
