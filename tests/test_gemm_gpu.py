@@ -409,3 +409,31 @@ def test_small_fp32_products_keep_infinities(api):
     assert torch.equal(got.isnan(), want.isnan()) and torch.equal(got.isinf(), want.isinf())
     fin = want.isfinite()
     assert (got.double() - want)[fin].abs().max() <= 1e-5 * want[fin].abs().max()
+
+
+# More than 74 tiles of 256 x 256: the size from which whole products go to the CTA-pair kernel.
+@pytest.mark.parametrize("dt", [torch.float32, torch.bfloat16, torch.float16])
+@pytest.mark.parametrize("batch,m,n,k,form", [
+    (1, 2048, 2500, 1024, "shared"), (1, 600, 20001, 777, "linear"), (8, 1000, 1001, 1001, "batched"), (1, 2500, 2500, 1300, "columns"),
+    (1, 513, 19000, 513, "shared")])
+@pytest.mark.parametrize("pair_mode", [0, 1, 2])
+def test_large_odd_products(L, api, dt, batch, m, n, k, form, pair_mode):
+    gen = torch.Generator(device="cuda").manual_seed(m + n + k)
+    # the scratch of this stream holds NaN before: a part of it that is read without having been written shows
+    api.matmul(torch.full((300, 8191), float("nan"), device="cuda"), torch.zeros(8191, 1001, device="cuda"))
+    a = torch.randn(batch, m, k, generator=gen, device="cuda").to(dt)
+    b = (torch.randn(*([batch] if form == "batched" else []), k, n, generator=gen, device="cuda") * k ** -0.5).to(dt)
+    if form == "columns":  # both operands by columns
+        a, b = a.transpose(-1, -2).contiguous().transpose(-1, -2), b.transpose(-1, -2).contiguous().transpose(-1, -2)
+    w = b.transpose(-1, -2).contiguous()
+    L.ytcuda_gemm_set_pair_mode(pair_mode)
+    try:
+        got = api.linear(a, w) if form == "linear" else api.matmul(a, b)
+    finally:
+        L.ytcuda_gemm_set_pair_mode(0)
+    # fp32: a rounding per partial sum; 16 bits: the rounding of the result (bf16 by the reference's rule: up to one unit)
+    tol = {torch.float32: 2e-6, torch.bfloat16: 2.0 ** -7, torch.float16: 2.0 ** -11}[dt]
+    for i in range(batch):
+        want = a[i].double() @ (b[i] if form == "batched" else b).double()
+        assert (got[i].double() - want).abs().max() <= tol * want.abs().max()
+    assert L.ytcuda_device_status(None) == 0

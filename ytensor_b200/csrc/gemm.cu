@@ -1018,7 +1018,12 @@ static int launch_tc(int dtype_in, int dtype_out, const void* A, const void* B, 
   const int BN = tc_tile_n(m, n, batch);
   // (a masked product keeps one CTA per tile: the tile-skipping form of the kernel)
   const bool grouped = ex && ex->tile_group;
-  const bool pair = !grouped && tc_takes_pairs(m, n, pl ? static_cast<int64_t>(k) * pl->pairs : k, batch);
+  // (k pieces are work items of the one-CTA kernel; gemm_tc2_kernel knows whole products only)
+  const bool pair = !grouped && splits == 1 && tc_takes_pairs(m, n, pl ? static_cast<int64_t>(k) * pl->pairs : k, batch);
+  if (splits > 1 && (ex || g_mask.kind != 0 || splits > (k + TC_BK - 1) / TC_BK)) {
+    set_last_error("ytcuda_gemm: %d pieces of k = %d do not go with an epilogue or a mask", splits, k);
+    return YTC_UNSUPPORTED;
+  }
   {
     const uint64_t nb = (a_bcast || batch == 1) ? 1 : static_cast<uint64_t>(batch);
     uint64_t dims[3], strides[2];
