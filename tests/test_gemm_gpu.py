@@ -437,3 +437,36 @@ def test_large_odd_products(L, api, dt, batch, m, n, k, form, pair_mode):
         want = a[i].double() @ (b[i] if form == "batched" else b).double()
         assert (got[i].double() - want).abs().max() <= tol * want.abs().max()
     assert L.ytcuda_device_status(None) == 0
+
+
+def _scratch_high():
+    """Most bytes that were in use at once in the device's default memory pool (the library's scratch) since the last call."""
+    rt, driver = pytest.importorskip("cuda.bindings.runtime"), pytest.importorskip("cuda.bindings.driver")
+    pool, attr = rt.cudaDeviceGetDefaultMemPool(0)[1], rt.cudaMemPoolAttr.cudaMemPoolAttrUsedMemHigh
+    torch.cuda.synchronize()
+    high = int(rt.cudaMemPoolGetAttribute(pool, attr)[1])
+    rt.cudaMemPoolSetAttribute(pool, attr, driver.cuuint64_t(0))  # (back to what is in use now)
+    return high
+
+
+@pytest.mark.parametrize("batch,m,n,k", [(1, 300, 1001, 30001), (1, 130, 8191, 9000), (1, 2001, 2002, 4099), (40, 150, 701, 3001),
+                                         (1, 5001, 6000, 1025)])
+def test_odd_products_in_bounded_scratch(api, batch, m, n, k):
+    """Small odd fp32 products use no more scratch than a stream keeps, and no more of it when k doubles."""
+    gen = torch.Generator(device="cuda").manual_seed(k)
+    used = []
+    for kk in (k, 2 * k):
+        a = torch.randn(batch, m, kk, generator=gen, device="cuda")
+        b = torch.randn(kk, n, generator=gen, device="cuda") * kk ** -0.5
+        stream = torch.cuda.Stream()
+        stream.wait_stream(torch.cuda.current_stream())
+        _scratch_high()
+        before = _scratch_high()
+        with torch.cuda.stream(stream):
+            got = api.matmul(a, b)
+        used.append(_scratch_high() - before)
+        for i in range(0, batch, 13):
+            want = a[i].double() @ b.double()
+            assert (got[i].double() - want).abs().max() <= 2e-6 * want.abs().max()
+    assert max(used) <= 256 << 20
+    assert used[1] <= max(used[0], 250 << 20)

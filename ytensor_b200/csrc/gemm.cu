@@ -1216,8 +1216,9 @@ struct PlaneOp {
   int wide;                // fp32: groups of 8 can be read 16 bytes at a time
 };
 // One launch for both operands: CTAs [0, a.blocks) take a, the rest b. Bound by memory: 4 bytes read, 6 written a value.
+// `keep`: the words in `unfit` hold what an earlier launch saw of the same operands, and stay set.
 template <int DT>
-__global__ void __launch_bounds__(256) gemm_planes_kernel(const PlaneOp oa, const PlaneOp ob, int* unfit) {
+__global__ void __launch_bounds__(256) gemm_planes_kernel(const PlaneOp oa, const PlaneOp ob, int* unfit, int keep) {
   dependent_wait();     // (under a programmatic dependent launch: the kernel before this one has finished)
   dependent_trigger();  // the kernel queued behind this one may be scheduled and set itself up meanwhile
   constexpr int PLANES = DT == YTC_F32 ? 3 : 1;
@@ -1281,20 +1282,22 @@ __global__ void __launch_bounds__(256) gemm_planes_kernel(const PlaneOp oa, cons
     }
   }
   const int any = __syncthreads_or(bad);
-  if (unfit && threadIdx.x == 0) unfit[blockIdx.x] = any;
+  if (unfit && threadIdx.x == 0) unfit[blockIdx.x] = any | (keep ? unfit[blockIdx.x] : 0);
 }
 
-// C = alpha * (the sum of the k pieces, in their order) + beta * C; part is [splits][batch][m][n].
-__global__ void __launch_bounds__(256) gemm_sum_kernel(const float* part, int splits, int64_t total, int m, int n, void* C,
-                                                       int dt, int64_t rsc, int64_t csc, int64_t bsc, float alpha, float beta) {
+// C = alpha * (the sum of the partial sums, in their order) + beta * C; part is [splits][batch][m][ldp], `stride` elements each.
+__global__ void __launch_bounds__(256) gemm_sum_kernel(const float* part, int splits, int64_t stride, int64_t total, int m, int n,
+                                                       int64_t ldp, void* C, int dt, int64_t rsc, int64_t csc, int64_t bsc,
+                                                       float alpha, float beta) {
   dependent_wait();
   dependent_trigger();
   for (int64_t t = blockIdx.x * 256ll + threadIdx.x; t < total; t += gridDim.x * 256ll) {
+    const int64_t row = t / n, col = t - row * n;
+    const float* from = part + row * ldp + col;
     float v = 0.f;
 #pragma unroll 8
-    for (int s = 0; s < splits; ++s) v += part[s * total + t];
-    const int64_t row = t / n;
-    const int64_t b = row / m, at = b * bsc + (row - b * m) * rsc + (t - row * n) * csc;
+    for (int s = 0; s < splits; ++s) v += from[s * stride];
+    const int64_t b = row / m, at = b * bsc + (row - b * m) * rsc + col * csc;
     v *= alpha;
     if (beta != 0.f) v += beta * load_as_f32(C, at, dt);
     store_from_f32(C, at, v, dt);
@@ -1380,38 +1383,58 @@ static int launch_planes(const void* A, const void* B, void* C, int dtype_out, i
     o.wide = DT == YTC_F32 && cs == 1 && rs % 4 == 0 && bs % 4 == 0 && (reinterpret_cast<uint64_t>(x) & 15) == 0;
     return o;
   };
-  auto a_op = [&](int64_t b0, int64_t items) {
-    const char* x = static_cast<const char*>(A) + b0 * bsa * esz;
-    return a_mn ? op_of(x, csa, rsa, bsa, k, m, items) : op_of(x, rsa, csa, bsa, m, k, items);
+  auto a_op = [&](int64_t b0, int64_t items, int k0, int kc) {
+    const char* x = static_cast<const char*>(A) + (b0 * bsa + k0 * csa) * esz;
+    return a_mn ? op_of(x, csa, rsa, bsa, kc, m, items) : op_of(x, rsa, csa, bsa, m, kc, items);
   };
-  auto b_op = [&](int64_t b0, int64_t items) {
-    const char* x = static_cast<const char*>(B) + b0 * bsb * esz;
-    return b_kn ? op_of(x, rsb, csb, bsb, k, n, items) : op_of(x, csb, rsb, bsb, n, k, items);
+  auto b_op = [&](int64_t b0, int64_t items, int k0, int kc) {
+    const char* x = static_cast<const char*>(B) + (b0 * bsb + k0 * rsb) * esz;
+    return b_kn ? op_of(x, rsb, csb, bsb, kc, n, items) : op_of(x, csb, rsb, bsb, n, kc, items);
   };
-  PlaneOp oa = a_op(0, 1), ob = b_op(0, 1);
-  // batch items per pass so that the planes stay below about 2 GiB
-  const int64_t a_item = oa.plane * PLANES * 2, b_item = ob.plane * PLANES * 2;
-  int64_t chunk = batch;
-  const int64_t fixed = (a_shared ? a_item : 0) + (b_shared ? b_item : 0), per_item = (a_shared ? 0 : a_item) + (b_shared ? 0 : b_item);
-  if (per_item > 0 && per_item * chunk > (int64_t{2} << 30) - fixed) {
-    chunk = ((int64_t{2} << 30) - fixed) / per_item;
-    if (chunk < 1) chunk = 1;
-  }
-  TcPlanes pl{PLANES, PLANES, 1, 0, 0, oa.plane, ob.plane};
+  TcPlanes pl{PLANES, PLANES, 1, 0, 0, 0, 0};
   if (PLANES == 3) {  // (l,h) (m,m) (h,l) (m,h) (h,m) (h,h)
     pl.pairs = 6;
     pl.pa = 2u | (1u << 2) | (0u << 4) | (1u << 6) | (0u << 8) | (0u << 10);
     pl.pb = 0u | (1u << 2) | (2u << 4) | (0u << 6) | (1u << 8) | (0u << 10);
   }
-  int splits = DT == YTC_F32 && g_f32_split != 0 ? 1 : tc_splits(m, n, k, pl.pairs, chunk);
   // An accumulator of the tensor cores drops a fraction of a unit at every step of 16; FFMA rounds. Products that FFMA took
-  // before keep 256 of k per accumulator and add the pieces in fp32. Error against 64 bits (2-norm), 16 x 4096 x 4096: FFMA 1.2e-6,
-  // here 2.5e-7; one accumulator would be above 3e-6.
-  if (check && splits < (k + 255) / 256) splits = (k + 255) / 256;
+  // before (`check`) keep 256 of k per accumulator and add the pieces in fp32. Error against 64 bits (2-norm), 16 x 4096 x 4096:
+  // FFMA 1.2e-6, here 2.5e-7; one accumulator would be above 3e-6. Their scratch stays below the size that a stream keeps (256 MB;
+  // larger buffers come and go with every call, which took from 0.6 to 6 ms at 130 x 8192 x 8192), however long k is: k goes by in
+  // windows of some pieces, each rewritten and multiplied by a launch of its own, whose partial sums stay and are added to. Only
+  // C itself may need more (partial sums of a C that is larger, or whose rows do not start at 16 bytes).
+  // The other products take whole k, and as many batch items per pass as keep the planes below 2 GiB.
+  constexpr int PIECE = 256;
+  constexpr int64_t PLANE_ROOM = int64_t{112} << 20, PART_ROOM = int64_t{128} << 20;
+  const int64_t ldp = check ? (n + 3) / 4 * 4 : n, mn = m * ldp;  // (rows of partial sums that are added to start at 16 bytes)
+  const int64_t a_item = a_op(0, 1, 0, check && k > PIECE ? PIECE : k).plane * PLANES * 2;
+  const int64_t b_item = b_op(0, 1, 0, check && k > PIECE ? PIECE : k).plane * PLANES * 2;
+  const int64_t fixed = (a_shared ? a_item : 0) + (b_shared ? b_item : 0);
+  const int64_t per_item = (a_shared ? 0 : a_item) + (b_shared ? 0 : b_item);
+  int64_t chunk = batch;
+  auto at_most = [&](int64_t room, int64_t each) {
+    if (each > 0 && each * chunk > room) chunk = room / each > 1 ? room / each : 1;
+  };
+  at_most((check ? PLANE_ROOM : int64_t{2} << 30) - fixed, per_item);
+  if (check) at_most(PART_ROOM, mn * 4);
+  int splits = DT == YTC_F32 && g_f32_split != 0 ? 1 : tc_splits(m, n, k, pl.pairs, chunk), window = k;
+  if (check) {
+    const int64_t pieces = (k + PIECE - 1) / PIECE, room = PART_ROOM / (chunk * mn * 4), wide = PLANE_ROOM / (fixed + chunk * per_item);
+    int64_t side = g_tc_pair == 1 ? 1 : pieces;  // pieces side by side
+    if (side > room) side = room;
+    if (side > wide) side = wide;
+    splits = side < 1 ? 1 : static_cast<int>(side);
+    if (splits < pieces) window = splits * PIECE;
+  }
+  const bool direct = splits == 1 && (window == k || (csc == 1 && rsc % 4 == 0 && (batch == 1 || bsc % 4 == 0) &&
+                                                      (reinterpret_cast<uint64_t>(C) & 15) == 0));  // (C itself takes the sums)
   auto up = [](int64_t v) { return static_cast<size_t>((v + 255) / 256 * 256); };
-  const int most_blocks = 2 * sm_count() * 8;  // (of both operands)
-  const size_t gate_bytes = up(most_blocks * 4), a_bytes = up(a_item * (a_shared ? 1 : chunk)), b_bytes = up(b_item * (b_shared ? 1 : chunk));
-  const size_t part_bytes = splits > 1 ? up(static_cast<int64_t>(splits) * chunk * m * n * 4) : 0;
+  // CTAs (and words of the gate) of either operand: those of the first, largest rewriting
+  const PlaneOp largest_a = a_op(0, a_shared ? 1 : chunk, 0, window), largest_b = b_op(0, b_shared ? 1 : chunk, 0, window);
+  const int n_gate = largest_a.blocks + largest_b.blocks;
+  const size_t gate_bytes = up(n_gate * 4), a_bytes = up(largest_a.plane * PLANES * 2 * (a_shared ? 1 : chunk));
+  const size_t b_bytes = up(largest_b.plane * PLANES * 2 * (b_shared ? 1 : chunk));
+  const size_t part_bytes = direct ? 0 : up(static_cast<int64_t>(splits) * chunk * mn * 4);
   char* ws = static_cast<char*>(device_workspace(gate_bytes + a_bytes + b_bytes + part_bytes, st));
   if (!ws) {
     set_last_error("ytcuda_gemm: could not allocate %zu bytes for rewritten operands", gate_bytes + a_bytes + b_bytes + part_bytes);
@@ -1421,43 +1444,51 @@ static int launch_planes(const void* A, const void* B, void* C, int dtype_out, i
   uint16_t* a_out = reinterpret_cast<uint16_t*>(ws + gate_bytes);
   uint16_t* b_out = reinterpret_cast<uint16_t*>(ws + gate_bytes + a_bytes);
   float* part = reinterpret_cast<float*>(ws + gate_bytes + a_bytes + b_bytes);
-  auto planes = [&](const PlaneOp& a, const PlaneOp& b, int* words) {  // (no blocks: nothing to do for that operand)
-    const cudaError_t e = launch_overlapped(gemm_planes_kernel<DT>, dim3(static_cast<unsigned>(a.blocks + b.blocks)), dim3(256), 0, st, a, b, words);
-    count_launch();
-    return e;
-  };
-  const int64_t ldb_all = ob.cols8 * 8;
-  const PlaneOp none{};
-  int shared_blocks = 0;  // an operand that all batch items share is rewritten once
-  if (b_shared) {
-    ob.out = b_out;
-    YTC_CUDA(planes(none, ob, gate));
-    shared_blocks = ob.blocks;
-  }
+  const int tc_dt = DT == YTC_F32 ? YTC_BF16 : DT;
   for (int64_t b0 = 0; b0 < batch; b0 += chunk) {
     const int64_t nb = batch - b0 < chunk ? batch - b0 : chunk;
-    oa = a_op(a_shared ? 0 : b0, a_shared ? 1 : nb);
-    ob = b_shared ? none : b_op(b0, nb);
-    oa.out = a_out;
-    ob.out = b_out;
-    YTC_CUDA(planes(oa, ob, gate ? gate + shared_blocks : nullptr));
     char* c = static_cast<char*>(C) + b0 * bsc * dtype_size(dtype_out);
-    const int64_t lda = oa.cols8 * 8, ldb = ldb_all, mn = static_cast<int64_t>(m) * n;
-    const int tc_dt = DT == YTC_F32 ? YTC_BF16 : DT;
-    int s = splits > 1 ? launch_tc(tc_dt, YTC_F32, a_out, b_out, part, m, n, k, 1.f, 0.f, a_mn, lda, b_kn, ldb, n, 1, nb,
-                                   a_shared ? 0 : a_item / 2, b_shared ? 0 : b_item / 2, mn, st, nullptr, &pl, splits)
-                       : launch_tc(tc_dt, dtype_out, a_out, b_out, c, m, n, k, alpha, beta, a_mn, lda, b_kn, ldb, rsc, csc, nb,
-                                   a_shared ? 0 : a_item / 2, b_shared ? 0 : b_item / 2, bsc, st, nullptr, &pl);
-    if (s != YTC_OK) return s;
-    if (splits > 1) {
-      const int64_t total = nb * mn, blocks = (total + 255) / 256, cap = static_cast<int64_t>(sm_count()) * 8;
+    int s;
+    for (int k0 = 0; k0 < k; k0 += window) {
+      const int kc = k - k0 < window ? k - k0 : window;
+      PlaneOp oa = a_op(a_shared ? 0 : b0, a_shared ? 1 : nb, k0, kc), ob = b_op(b_shared ? 0 : b0, b_shared ? 1 : nb, k0, kc);
+      oa.out = a_out;
+      ob.out = b_out;
+      oa.blocks = largest_a.blocks;
+      ob.blocks = largest_b.blocks;
+      const int64_t lda = oa.cols8 * 8, ldb = ob.cols8 * 8;
+      pl.plane_a = oa.plane;
+      pl.plane_b = ob.plane;
+      // an operand that all batch items share is rewritten once, if it is rewritten whole
+      const bool again = b0 > 0 && window == k, do_a = !(a_shared && again), do_b = !(b_shared && again);
+      const PlaneOp none{};
+      auto planes = [&](const PlaneOp& x, const PlaneOp& y, int word) {  // (no blocks: nothing to do for that operand)
+        const cudaError_t e = launch_overlapped(gemm_planes_kernel<DT>, dim3(static_cast<unsigned>(x.blocks + y.blocks)), dim3(256), 0,
+                                                st, x, y, gate ? gate + word : nullptr, k0 > 0 ? 1 : 0);
+        count_launch();
+        return e;
+      };
+      if (do_a && do_b && (check || !b_shared)) {
+        YTC_CUDA(planes(oa, ob, 0));
+      } else {
+        if (do_b) YTC_CUDA(planes(none, ob, oa.blocks));
+        if (do_a) YTC_CUDA(planes(oa, none, 0));
+      }
+      const int64_t bsa_p = a_shared ? 0 : oa.plane * PLANES, bsb_p = b_shared ? 0 : ob.plane * PLANES;
+      s = direct ? launch_tc(tc_dt, dtype_out, a_out, b_out, c, m, n, kc, alpha, k0 > 0 ? 1.f : beta, a_mn, lda, b_kn, ldb, rsc, csc,
+                             nb, bsa_p, bsb_p, bsc, st, nullptr, &pl)
+                 : launch_tc(tc_dt, YTC_F32, a_out, b_out, part, m, n, kc, 1.f, k0 > 0 ? 1.f : 0.f, a_mn, lda, b_kn, ldb, ldp, 1, nb,
+                             bsa_p, bsb_p, mn, st, nullptr, &pl, check ? (kc + PIECE - 1) / PIECE : splits);
+      if (s != YTC_OK) return s;
+    }
+    if (!direct) {
+      const int64_t total = nb * m * n, blocks = (total + 255) / 256, cap = static_cast<int64_t>(sm_count()) * 8;
       YTC_CUDA(launch_overlapped(gemm_sum_kernel, dim3(static_cast<unsigned>(blocks < cap ? blocks : cap)), dim3(256), 0, st, part,
-                                 splits, total, m, n, c, dtype_out, rsc, csc, bsc, alpha, beta));
+                                 splits, nb * mn, total, m, n, ldp, c, dtype_out, rsc, csc, bsc, alpha, beta));
       count_launch();
     }
     if (check && (s = launch_simt(DT, dtype_out, static_cast<const char*>(A) + b0 * bsa * esz, static_cast<const char*>(B) + b0 * bsb * esz,
-                                  c, m, n, k, alpha, beta, rsa, csa, rsb, csb, rsc, csc, nb, bsa, bsb, bsc, st, gate,
-                                  shared_blocks + oa.blocks + ob.blocks)) != YTC_OK)
+                                  c, m, n, k, alpha, beta, rsa, csa, rsb, csb, rsc, csc, nb, bsa, bsb, bsc, st, gate, n_gate)) != YTC_OK)
       return s;
   }
   device_workspace_release(st);  // large operands do not stay resident
@@ -1479,7 +1510,7 @@ static int launch_tc_split(int dtype_in, int dtype_out, const void* A, const voi
   if (s != YTC_OK) return s;
   const int64_t blocks = (total + 255) / 256, cap = static_cast<int64_t>(sm_count()) * 8;
   YTC_CUDA(launch_overlapped(gemm_sum_kernel, dim3(static_cast<unsigned>(blocks < cap ? blocks : cap)), dim3(256), 0, st, part, splits,
-                             total, m, n, C, dtype_out, rsc, csc, bsc, alpha, beta));
+                             total, total, m, n, n, C, dtype_out, rsc, csc, bsc, alpha, beta));
   count_launch();
   return YTC_OK;
 }
