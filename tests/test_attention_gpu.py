@@ -298,3 +298,23 @@ def test_masks_and_biases_of_any_alignment(L, api, lq, lk, d, dt, form):
     bound = _f32_bound(q, k, v, d, bias) if dt == "f32" else {"bf16": H_TOL, "f16": 2e-3}[dt] * want.abs().max()
     assert (got.double() - want).abs().max() <= bound
     assert m is None or not got[0, :, 7].any()
+
+
+@pytest.mark.parametrize("lq,lk,d,dt", [(300, 336, 128, "f32"), (129, 131, 20, "f32"), (40, 70, 80, "bf16")])
+def test_bias_of_the_lowest_float(L, api, lq, lk, d, dt):
+    """Masks are often written as the lowest float: such a key weighs nothing beside others, and a row that has no other keys
+    weighs all of them alike (the score is lost in the rounding of the sum)."""
+    gen = torch.Generator(device="cuda").manual_seed(lk)
+    t = {"f32": torch.float32, "bf16": torch.bfloat16}[dt]
+    q, k, v = (torch.randn(1, h, n, d, generator=gen, device="cuda").to(t) for h, n in ((2, lq), (2, lk), (2, lk)))
+    low = torch.finfo(torch.float32).min
+    bias = torch.where(torch.rand(lq, lk, generator=gen, device="cuda") < 0.5, low, 0.0)
+    bias[5], bias[lq - 1], bias[11, 3:], bias[12] = low, low, float("-inf"), float("-inf")
+    bias[11, :3] = low
+    bias[17] = torch.where(torch.arange(lk, device="cuda") == 9, -2.6e38, -3.3e38)  # (finite, one far above the others)
+    got = api.scaledDotProductAttention(q, k, v, d ** -0.5, None, bias).double()
+    s = (q.double() @ k.double().transpose(-1, -2) * d ** -0.5).float() + bias  # the sum in 32 bits
+    want = torch.nan_to_num(torch.softmax(s.double(), -1) @ v.double())
+    bound = _f32_bound(q, k, v, d) if dt == "f32" else 2.0 ** -7 * want.abs().max()
+    assert (got - want).abs().max() <= bound
+    assert not got[0, :, 12].any()  # no key at all

@@ -323,6 +323,10 @@ __global__ void __launch_bounds__(SA_THREADS, 1)
     const uint32_t tl = tmem + (static_cast<uint32_t>(quad * 32) << 16);
     const uint32_t ts = tl + wg * SA_T_SP, to = tl + SA_T_O;
     const bool general = p.a.mask != nullptr || p.a.bias != nullptr;
+    // Scores are kept in log2 units, under a bias in its own: the lowest float, the usual mask, would become -infinity, and a
+    // row that holds nothing else would weigh none of its keys instead of all alike. `unit`: one score in log2 units.
+    const bool biased = p.a.bias != nullptr;
+    const float unit = biased ? FA_LOG2E : 1.f;
     const int esz = p.a.dt == YTC_F32 ? 4 : 2;
     int g = 0, n_item = 0;
     bool ok = true, unfit = false;
@@ -415,7 +419,7 @@ __global__ void __launch_bounds__(SA_THREADS, 1)
         const int key0 = j * SA_BN, cl = limit - key0;  // columns 0 .. cl are visible to this row
         const int cols = it.half && j == it.n - 1 ? 64 : SA_BN;
         const bool full = !general && __all_sync(0xffffffffu, cl >= cols - 1);
-        // Pass 1: the maximum. Tiles with hidden keys, a mask or a bias get their scores (log2 units, -inf where hidden)
+        // Pass 1: the maximum. Tiles with hidden keys, a mask or a bias get their scores (-inf where hidden)
         // written back over S, so that pass 2 is one piece of code: the instructions a softmax warp cycles through stay few.
         float mx = -CUDART_INF_F;
 #pragma unroll 1
@@ -439,7 +443,7 @@ __global__ void __launch_bounds__(SA_THREADS, 1)
           } else {
             masked_scores(r, p.a.mask ? p.a.mask + qi * p.a.mask_rs + key0 + c0 : nullptr,
                           p.a.bias ? p.a.bias + qi * p.a.bias_rs + (key0 + c0) * p.a.bias_cs : nullptr, p.a.bias_cs, cl - c0 + 1,
-                          p.scale_log2);
+                          biased ? p.a.scale : p.scale_log2, 1.f);
           }
 #pragma unroll
           for (int e = 0; e < 32; e += 2) mx = fmax3(mx, __uint_as_float(r[e]), __uint_as_float(r[e + 1]));
@@ -448,21 +452,25 @@ __global__ void __launch_bounds__(SA_THREADS, 1)
         if (!full) tmem_st_wait();
         const float m_new = fmaxf(m_run, mx);
         const float m_use = m_new == -CUDART_INF_F ? 0.f : m_new;
-        const float alpha = m_run == -CUDART_INF_F ? 0.f : fast_exp2(m_run - m_use);
+        const float alpha = m_run == -CUDART_INF_F ? 0.f : fast_exp2((m_run - m_use) * unit);
         m_run = m_new;
         // Pass 2: P of 32 keys at a time, the second and third plane over the 32 columns of S that have been read, the first
         // plane behind S.
-        const float sl = full ? p.scale_log2 : 1.f;
+        const float sl = full ? p.scale_log2 : 1.f, sub = biased ? 0.f : -m_use;
         uint64_t ps = f2_pack(0.f, 0.f);
 #pragma unroll 1
         for (int c0 = 0; c0 < cols; c0 += 32) {
           uint32_t r[32], pk[16];
           tmem_ld_32x32b_x32(ts + c0, r);
           tmem_ld_wait();
+          if (biased) {  // (the difference first: score and maximum may both be the lowest float)
+#pragma unroll
+            for (int e = 0; e < 32; ++e) r[e] = __float_as_uint((__uint_as_float(r[e]) - m_use) * FA_LOG2E);
+          }
 #pragma unroll
           for (int e = 0; e < 32; e += 2) {
             float t0, t1;
-            f2_unpack(f2_fma(f2_pack(__uint_as_float(r[e]), __uint_as_float(r[e + 1])), f2_pack(sl, sl), f2_pack(-m_use, -m_use)), t0, t1);
+            f2_unpack(f2_fma(f2_pack(__uint_as_float(r[e]), __uint_as_float(r[e + 1])), f2_pack(sl, sl), f2_pack(sub, sub)), t0, t1);
             t0 = fast_exp2(t0);
             t1 = fast_exp2(t1);
             ps = f2_add(ps, f2_pack(t0, t1));
@@ -534,7 +542,7 @@ __global__ void __launch_bounds__(SA_THREADS, 1)
       tmem_ld_wait();
       const float m_o = __uint_as_float(ml[0]), l_o = __uint_as_float(ml[1]);
       const float m = fmaxf(m_run, m_o);
-      const float f = m_run == -CUDART_INF_F ? 0.f : fast_exp2(m_run - m), f_o = m_o == -CUDART_INF_F ? 0.f : fast_exp2(m_o - m);
+      const float f = m_run == -CUDART_INF_F ? 0.f : fast_exp2((m_run - m) * unit), f_o = m_o == -CUDART_INF_F ? 0.f : fast_exp2((m_o - m) * unit);
       const float l = l_run * f + l_o * f_o;
       const float inv = l > 0.f ? 1.0f / l : 0.f;
 #pragma unroll

@@ -162,13 +162,13 @@ __device__ __forceinline__ float fast_rcp(float x) {
   return y;
 }
 
-// Scores of 32 keys of one row under a bool mask and / or a bias, in log2 units over the raw products in r; -inf where hidden:
-// beyond the first `n` keys (n may be anything) or masked out. mask / bias point at the row's first of these keys. All loads
+// Scores of 32 keys of one row under a bool mask and / or a bias, r * scale + bias * unit over the raw products in r; -inf where
+// hidden: beyond the first `n` keys (n may be anything) or masked out. mask / bias point at the row's first of these keys. All loads
 // are asked for before the first is used, 16 bytes at a time where the rows allow it: one element after the other, behind its
 // own branch and in both passes of the softmax, they were nine tenths of a tile's time (8 heads of 128, 1024 x 1024, bf16
 // with a bias: 327 us, 65 here; a bool mask, 2048 x 2048: 622, 90).
 __device__ __forceinline__ void masked_scores(uint32_t (&r)[32], const uint8_t* mask, const float* bias, int64_t bias_cs, int n,
-                                              float scale_log2) {
+                                              float scale, float unit) {
   if (n > 32) n = 32;
   uint32_t seen = n <= 0 ? 0u : 0xFFFFFFFFu >> (32 - n);
   if (mask && n > 0) {
@@ -205,10 +205,10 @@ __device__ __forceinline__ void masked_scores(uint32_t (&r)[32], const uint8_t* 
     }
 #pragma unroll
     for (int e = 0; e < 32; ++e)
-      r[e] = __float_as_uint((seen >> e) & 1u ? __uint_as_float(r[e]) * scale_log2 + b[e] * FA_LOG2E : -CUDART_INF_F);
+      r[e] = __float_as_uint((seen >> e) & 1u ? __uint_as_float(r[e]) * scale + b[e] * unit : -CUDART_INF_F);
   } else {
 #pragma unroll
-    for (int e = 0; e < 32; ++e) r[e] = __float_as_uint((seen >> e) & 1u ? __uint_as_float(r[e]) * scale_log2 : -CUDART_INF_F);
+    for (int e = 0; e < 32; ++e) r[e] = __float_as_uint((seen >> e) & 1u ? __uint_as_float(r[e]) * scale : -CUDART_INF_F);
   }
 }
 
@@ -712,7 +712,7 @@ __global__ void __launch_bounds__(FA_THREADS, 1)
             tmem_ld_wait();
             masked_scores(r, p.mask ? p.mask + static_cast<int64_t>(row) * p.mask_rs + key0 + c0 : nullptr,
                           p.bias ? p.bias + static_cast<int64_t>(row) * p.bias_rs + (key0 + c0) * p.bias_cs : nullptr, p.bias_cs,
-                          cl - c0 + 1, p.scale_log2);
+                          cl - c0 + 1, p.scale_log2, FA_LOG2E);
 #pragma unroll
             for (int e = 0; e < 32; e += 2) mx = fmax3(mx, __uint_as_float(r[e]), __uint_as_float(r[e + 1]));
             tmem_st_32x32b_x32(ts + c0, r);
