@@ -470,3 +470,33 @@ def test_odd_products_in_bounded_scratch(api, batch, m, n, k):
             assert (got[i].double() - want).abs().max() <= 2e-6 * want.abs().max()
     assert max(used) <= 256 << 20
     assert used[1] <= max(used[0], 250 << 20)
+
+
+@pytest.mark.parametrize("dt,m,n,k", [(torch.float32, 700, 2501, 1030), (torch.float32, 1024, 2048, 1024), (torch.bfloat16, 1300, 2501, 1111),
+                                      (torch.float16, 1300, 2501, 1111), (torch.bfloat16, 128, 8192, 8192)])
+def test_products_without_scratch(api, dt, m, n, k):
+    """Where the device has no room for scratch the kernels that need none take the product."""
+    rt = pytest.importorskip("cuda.bindings.runtime")
+    gen = torch.Generator(device="cuda").manual_seed(k)
+    a = torch.randn(m, k, generator=gen, device="cuda").to(dt)
+    b = (torch.randn(k, n, generator=gen, device="cuda") * k ** -0.5).to(dt)
+    out = torch.empty(m, n, dtype=dt, device="cuda")
+    torch.cuda.synchronize()
+    props = rt.cudaMemPoolProps()
+    props.allocType, props.location.type, props.location.id = rt.cudaMemAllocationType.cudaMemAllocationTypePinned, \
+        rt.cudaMemLocationType.cudaMemLocationTypeDevice, 0
+    props.maxSize = 4 << 20
+    err, pool = rt.cudaMemPoolCreate(props)
+    assert int(err) == 0
+    old = rt.cudaDeviceGetMemPool(0)[1]
+    err, handle = rt.cudaStreamCreateWithFlags(1)  # (a stream that has no scratch yet; kept, so that its name is not given again)
+    try:
+        assert int(rt.cudaDeviceSetMemPool(0, pool)[0]) == 0
+        with torch.cuda.stream(torch.cuda.ExternalStream(int(handle))):
+            api.matmul(a, b, out)
+        torch.cuda.synchronize()
+    finally:
+        rt.cudaDeviceSetMemPool(0, old)
+    want = a.double() @ b.double()
+    tol = {torch.float32: 1e-5, torch.bfloat16: 2.0 ** -7, torch.float16: 2.0 ** -11}[dt]
+    assert (out.double() - want).abs().max() <= tol * want.abs().max()

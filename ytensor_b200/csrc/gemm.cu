@@ -1356,7 +1356,8 @@ static bool stream_captures(cudaStream_t st) {  // (scratch that grows inside a 
 }
 
 // The product through rewritten operands (gemm_planes_kernel), k cut into pieces where the tiles are few. `check`: FFMA runs
-// behind it if an operand held a number without planes (beta must be 0).
+// behind it if an operand held a number without planes (beta must be 0). NO_SCRATCH: nothing was queued.
+constexpr int NO_SCRATCH = -1;
 template <int DT>
 static int launch_planes(const void* A, const void* B, void* C, int dtype_out, int m, int n, int k, float alpha, float beta,
                          int64_t rsa, int64_t csa, int64_t rsb, int64_t csb, int64_t rsc, int64_t csc, int64_t batch,
@@ -1436,10 +1437,7 @@ static int launch_planes(const void* A, const void* B, void* C, int dtype_out, i
   const size_t b_bytes = up(largest_b.plane * PLANES * 2 * (b_shared ? 1 : chunk));
   const size_t part_bytes = direct ? 0 : up(static_cast<int64_t>(splits) * chunk * mn * 4);
   char* ws = static_cast<char*>(device_workspace(gate_bytes + a_bytes + b_bytes + part_bytes, st));
-  if (!ws) {
-    set_last_error("ytcuda_gemm: could not allocate %zu bytes for rewritten operands", gate_bytes + a_bytes + b_bytes + part_bytes);
-    return YTC_CUDA_ERROR;
-  }
+  if (!ws) return NO_SCRATCH;
   int* gate = check ? reinterpret_cast<int*>(ws) : nullptr;
   uint16_t* a_out = reinterpret_cast<uint16_t*>(ws + gate_bytes);
   uint16_t* b_out = reinterpret_cast<uint16_t*>(ws + gate_bytes + a_bytes);
@@ -1582,9 +1580,11 @@ static int gemm_any(int dtype_in, int dtype_out, const void* A, const void* B, v
   }
   if (dtype_in == YTC_F32 && dtype_out == YTC_F32 && g_gemm_path != 1) {
     const int form = f32_planes_form(m, n, k, beta, rsc, csc, bsc, batch, bsb);
-    if (form == 1 || (form == 2 && scratch && !stream_captures(st)))
-      return launch_planes<YTC_F32>(A, B, C, dtype_out, m, n, k, alpha, beta, rsa, csa, rsb, csb, rsc, csc, batch, bsa, bsb, bsc,
-                                    form == 2, st);
+    if (form == 1 || (form == 2 && scratch && !stream_captures(st))) {
+      const int s = launch_planes<YTC_F32>(A, B, C, dtype_out, m, n, k, alpha, beta, rsa, csa, rsb, csb, rsc, csc, batch, bsa, bsb,
+                                           bsc, form == 2, st);
+      if (s != NO_SCRATCH) return s;  // (FFMA needs none)
+    }
   }
   int a_mn = 0, b_mn = 0;
   bool tc = (dtype_in != YTC_F32) && g_gemm_path != 1;
@@ -1624,9 +1624,10 @@ static int gemm_any(int dtype_in, int dtype_out, const void* A, const void* B, v
   if (dtype_in != YTC_F32 && g_gemm_path != 1 && scratch && g_mask.kind == 0 && rsc >= 0 && csc >= 0 && bsc >= 0 &&
       dtype_out != YTC_F32 &&  // (an fp32 result would show the tensor cores' accumulation)
       simt_us(m, n, k, batch, false) > 1.5 * planes_us(m, n, k, batch, bsb == 0, false) && !stream_captures(st)) {
-    return dtype_in == YTC_BF16
-               ? launch_planes<YTC_BF16>(A, B, C, dtype_out, m, n, k, alpha, beta, rsa, csa, rsb, csb, rsc, csc, batch, bsa, bsb, bsc, false, st)
-               : launch_planes<YTC_F16>(A, B, C, dtype_out, m, n, k, alpha, beta, rsa, csa, rsb, csb, rsc, csc, batch, bsa, bsb, bsc, false, st);
+    const int s = dtype_in == YTC_BF16
+                      ? launch_planes<YTC_BF16>(A, B, C, dtype_out, m, n, k, alpha, beta, rsa, csa, rsb, csb, rsc, csc, batch, bsa, bsb, bsc, false, st)
+                      : launch_planes<YTC_F16>(A, B, C, dtype_out, m, n, k, alpha, beta, rsa, csa, rsb, csb, rsc, csc, batch, bsa, bsb, bsc, false, st);
+    if (s != NO_SCRATCH) return s;
   }
   return launch_simt(dtype_in, dtype_out, A, B, C, m, n, k, alpha, beta, rsa, csa, rsb, csb, rsc, csc, batch, bsa,
                      bsb, bsc, st);
