@@ -500,3 +500,30 @@ def test_products_without_scratch(api, dt, m, n, k):
     want = a.double() @ b.double()
     tol = {torch.float32: 1e-5, torch.bfloat16: 2.0 ** -7, torch.float16: 2.0 ** -11}[dt]
     assert (out.double() - want).abs().max() <= tol * want.abs().max()
+
+
+@pytest.mark.parametrize("sa,sb", [(2.0 ** 70, 2.0 ** 70), (2.0 ** 64, 2.0 ** 61), (2.0 ** -118, 2.0 ** 20), (2.0 ** -60, 2.0 ** -55)])
+@pytest.mark.parametrize("m,n,k", [(70, 1001, 1300), (600, 9001, 515)])
+def test_small_and_odd_products_at_the_ends_of_the_range(L, api, sa, sb, m, n, k):
+    """Results beyond the largest float are what FFMA says, operands near the smallest lose nothing."""
+    gen = torch.Generator(device="cuda").manual_seed(m)
+    a, b = torch.randn(m, k, generator=gen, device="cuda"), torch.randn(k, n, generator=gen, device="cuda")
+    a[:, 5::3], b[:, 9::2] = a[:, 5::3] * sa, b[:, 9::2] * sb  # (ordinary numbers beside them)
+    if sa < 1:
+        a[:, 0:5] = 0
+        a[:, 6::3] = a[:, 7::3] = 0
+    got = api.matmul(a, b)
+    L.ytcuda_gemm_set_path(1)
+    try:
+        ffma = api.matmul(a, b)
+    finally:
+        L.ytcuda_gemm_set_path(0)
+    want, fin = a.double() @ b.double(), ffma.isfinite()
+    # (a partial sum may overflow in one order and not in another: where the result is beyond any doubt)
+    size = a.double().abs() @ b.double().abs()
+    sure = (want.abs() > 2.0 ** 130) | (size < 2.0 ** 126)
+    assert torch.equal(got.isnan() & sure, ffma.isnan() & sure) and torch.equal(got.isinf() & sure, ffma.isinf() & sure)
+    inf = sure & ffma.isinf()
+    assert torch.equal(got[inf], ffma[inf])
+    fin = sure & fin
+    assert fin.any() and ((got.double() - want)[fin].abs() <= 2e-6 * size[fin]).all()

@@ -770,8 +770,8 @@ struct GemmSimtParams {
   int in_dtype, out_dtype;
   int tiles_m, tiles_n;
   const uint8_t* tile_live;  // masked product: 0 marks a 128 x 128 output tile nobody asks for (NULL: all computed)
-  const int* gate;  // the kernel runs only if one of these `n_gate` words is set (NULL: always)
-  int n_gate;
+  const int* gate;  // the kernel runs only if one of these `n_gate` words is set (NULL: always), and for tiles of C (fp32) that
+  int n_gate;       // hold a number that isn't finite
 };
 
 template <int IN_DT>
@@ -781,15 +781,24 @@ __global__ void __launch_bounds__(SM_THREADS) gemm_simt_kernel(const GemmSimtPar
 
   const int tid = threadIdx.x;
   const int tile = blockIdx.x;
+  const int mb = tile / p.tiles_n, nb = tile - mb * p.tiles_n;
+  const int m0 = mb * SM_BM, n0 = nb * SM_BN;
   if (p.gate) {
     int any = 0;
     for (int i = tid; i < p.n_gate; i += SM_THREADS) any |= p.gate[i];
-    if (!__syncthreads_or(any)) return;
+    if (!__syncthreads_or(any)) {
+      // A product that overflows has plane products of either sign that overflow: NaN where the sum is an infinity.
+      const float* c = static_cast<const float*>(p.C) + blockIdx.y * p.bsc;
+      for (int i = tid; i < SM_BM * SM_BN; i += SM_THREADS) {
+        const int fast = i % SM_BN, slow = i / SM_BN;
+        const int r = m0 + (p.csc == 1 ? slow : fast), col = n0 + (p.csc == 1 ? fast : slow);
+        if (r < p.M && col < p.N) any |= !isfinite(c[r * p.rsc + col * p.csc]);
+      }
+      if (!__syncthreads_or(any)) return;
+    }
   }
   if (p.tile_live && !p.tile_live[tile]) return;
   const int b = blockIdx.y;
-  const int mb = tile / p.tiles_n, nb = tile - mb * p.tiles_n;
-  const int m0 = mb * SM_BM, n0 = nb * SM_BN;
   const int64_t a_off = static_cast<int64_t>(b) * p.bsa;
   const int64_t b_off = static_cast<int64_t>(b) * p.bsb;
 
@@ -1203,8 +1212,8 @@ static int launch_simt(int dtype_in, int dtype_out, const void* A, const void* B
 // 16-bit operands of odd strides as they are. Rows of `cols` elements become rows of a multiple of 8, zeros behind the end.
 // Of the nine plane products of an fp32 GEMM the six that matter, (l,h) (m,m) (h,l) (m,h) (h,m) (h,h), smallest first, form
 // in one accumulator (TcPlanes). Non-finite values keep m = l = 0 (an infinite operand then meets zero planes of the other
-// operand and the sum becomes NaN where the FFMA kernel gives the infinity); `unfit`, a word per block, says whether there
-// were any. fp16 numbers below the normal ones are doubled, which is how the reference's type and the FFMA kernel read them.
+// operand and the sum becomes NaN where the FFMA kernel gives the infinity), and below 2^-110 the last plane would lie under
+// bf16's smallest number; `unfit`, a word per block, says whether there were any of either. fp16 numbers below the normal ones are doubled, which is how the reference's type and the FFMA kernel read them.
 struct PlaneOp {
   const void* x;
   int64_t rs, cs, bs;
@@ -1260,6 +1269,7 @@ __global__ void __launch_bounds__(256) gemm_planes_kernel(const PlaneOp oa, cons
           p[1][e] = *reinterpret_cast<const uint16_t*>(&q);
           q = __float2bfloat16_rn(r1 - __bfloat162float(q));
           p[2][e] = *reinterpret_cast<const uint16_t*>(&q);
+          bad |= v[e] != 0.f && fabsf(v[e]) < 0x1p-110f;
         } else {
           bad = true;
         }
