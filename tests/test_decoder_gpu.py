@@ -271,3 +271,44 @@ def test_full_model_32_sequences_match_reference(Q):
     assert (margins > 2e-3).mean() > 0.97  # the check above covered nearly every token
     assert free_running_equal or (margins <= 2e-3).any()
     m.close()
+
+
+def test_long_prompts_of_wide_models(Q):
+    """A hidden size above what the norm that writes planes takes: one prompt of 130 tokens, and the same in two parts."""
+    cfg = Q.Qwen3Config(**{**SMALL, "hidden_size": 16392, "num_hidden_layers": 1, "vocab_size": 64, "num_attention_heads": 1,
+                           "num_key_value_heads": 1, "max_position_embeddings": 256})
+    m = Q.Qwen3ForCausalLM(cfg)
+    m.load_weights(Q.random_weights(cfg, seed=3, std=0.01))
+    ids = np.random.default_rng(1).integers(0, 64, (1, 130))
+    m.forward(dev_ids(ids[:, :100]))
+    want = m.forward(dev_ids(ids[:, 100:])).cpu().numpy()
+    m.reset_kv_cache()
+    assert normwise(m.forward(dev_ids(ids)).cpu().numpy(), want) < 1e-4
+    m.close()
+
+
+def test_long_prompts_of_an_odd_share_of_the_ffn(Q):
+    """A rank whose share of the FFN has rows that do not start at 16 bytes (40 / 2 columns) computes what one GPU does with
+    the same weights and columns of zeros behind them. The sums over the ranks are left out."""
+    cfg = Q.Qwen3Config(**{**SMALL, "num_attention_heads": 2, "intermediate_size": 40, "max_position_embeddings": 256})
+    w = Q.random_weights(cfg, seed=3, std=0.05)
+    m = Q.Qwen3ForCausalLM(cfg, tp_rank=0, tp_world=2, connect_peers=False)
+    m._cb = Q._ALLREDUCE_T(lambda buf, count, user: 0)
+    assert m.L.ytcuda_qwen3_set_allreduce(m.h, Q.C.cast(m._cb, Q.C.c_void_p), None) == 0
+    m.load_weights(w)
+    one = Q.Qwen3Config(**{**SMALL, "num_attention_heads": 1, "num_key_value_heads": 1, "intermediate_size": 24,
+                           "max_position_embeddings": 256})
+    part = {}
+    for key, x in w.items():
+        name = key if isinstance(key, str) else key[0]
+        x = Q.shard_weight(cfg, name, x, 0, 2)
+        if name == "gate_up":
+            x = np.concatenate([np.pad(x[:20], ((0, 4), (0, 0))), np.pad(x[20:], ((0, 4), (0, 0)))])
+        part[key] = np.pad(x, ((0, 0), (0, 4))) if name == "down" else x
+    n = Q.Qwen3ForCausalLM(one)
+    n.load_weights(part)
+    ids = np.random.default_rng(1).integers(0, 512, (1, 150))
+    got, want = m.forward(dev_ids(ids)).cpu().numpy(), n.forward(dev_ids(ids)).cpu().numpy()
+    assert normwise(got, want[:, :256]) < 1e-4
+    m.close()
+    n.close()

@@ -1315,8 +1315,8 @@ int ytcuda_qwen3_forward(void* handle, const int32_t* ids, int len, float* logit
       YTC_CUDA(cudaGetLastError());
     }
   }
-  // More rows: the norms and SwiGLU write the planes that the projection behind them reads.
-  const bool planes = rows > 128;
+  // More rows: the norms and SwiGLU write the planes that the projection behind them reads (as far as their kernels go).
+  const bool planes = rows > 128 && Hd <= RMS_PLANES_MAX && m->l_inter % 4 == 0;
   const int64_t glue_cap = static_cast<int64_t>(sm_count()) * 16;
   for (int l = fused_glue ? m->layers : 0; l < m->layers; ++l) {
     const LayerW& W = m->lw[l];

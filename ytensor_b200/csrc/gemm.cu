@@ -1523,8 +1523,15 @@ static int launch_tc_split(int dtype_in, int dtype_out, const void* A, const voi
   return YTC_OK;
 }
 
-// y[m, n] (+)= (hi + lo)[m, k] . W[n, k]^T: both bf16 planes ([2][m][k]) of the activations in one accumulator, lo first.
+// y[m, n] (+)= (hi + lo)[m, k] . W[n, k]^T: both bf16 planes ([2][m][k]) of the activations in one accumulator, lo first; rows
+// that do not start at 16 bytes (of a rank's share of the FFN width, say) as two products.
 int linear_two_planes(const void* planes, const void* w, float* y, int64_t ldy, int m, int n, int k, bool accumulate, cudaStream_t st) {
+  int unused;
+  if (!tc_operand_ok(planes, k, 1, 0, 1, m, k, &unused) || !tc_operand_ok(w, k, 1, 0, 1, n, k, &unused)) {
+    const char* lo = static_cast<const char*>(planes) + static_cast<int64_t>(m) * k * 2;
+    const int s = ytcuda_gemm(YTC_BF16, YTC_F32, planes, w, y, m, n, k, 1.f, accumulate ? 1.f : 0.f, k, 1, 1, k, ldy, 1, 1, 0, 0, 0, st);
+    return s != YTC_OK ? s : ytcuda_gemm(YTC_BF16, YTC_F32, lo, w, y, m, n, k, 1.f, 1.f, k, 1, 1, k, ldy, 1, 1, 0, 0, 0, st);
+  }
   const TcPlanes pl{2, 1, 2, 1u, 0u, static_cast<int64_t>(m) * k, static_cast<int64_t>(n) * k};
   return launch_tc(YTC_BF16, YTC_F32, planes, w, y, m, n, k, 1.f, accumulate ? 1.f : 0.f, 0, k, 0, k, ldy, 1, 1, 0, 0, 0, st, nullptr, &pl);
 }

@@ -1348,7 +1348,7 @@ static int run_nd(int op, int dt_in, int dt_out, int dt_w, const void* x, void* 
 }
 
 int rmsnorm_planes(const float* x, const float* w, uint16_t* planes, int64_t rows, int hidden, float eps, cudaStream_t st) {
-  YTC_REQUIRE(hidden % 4 == 0 && hidden <= 16384, "rmsnorm_planes: rows of %d", hidden);
+  YTC_REQUIRE(hidden % 4 == 0 && hidden <= RMS_PLANES_MAX, "rmsnorm_planes: rows of %d", hidden);
   RowParams p{};
   p.x = x; p.y = planes; p.w = w;
   p.rows = rows; p.L = hidden; p.x_rs = p.y_rs = hidden; p.r_rows = 1; p.eps = eps;

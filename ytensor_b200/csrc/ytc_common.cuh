@@ -265,9 +265,10 @@ void device_workspace_release(cudaStream_t st);
 int gemm_into_workspace(int dtype_in, int dtype_out, const void* A, const void* B, void* C, int m, int n, int k, float alpha,
                         float beta, int64_t rsa, int64_t csa, int64_t rsb, int64_t csb, int64_t rsc, int64_t csc, int64_t batch,
                         int64_t bsa, int64_t bsb, int64_t bsc, cudaStream_t st);
-// y[m, n] (+)= (hi + lo)[m, k] . W[n, k]^T, planes = hi [m][k], then lo, bf16, rows of whole 16 bytes (gemm.cu).
+// y[m, n] (+)= (hi + lo)[m, k] . W[n, k]^T, planes = hi [m][k], then lo, bf16 (gemm.cu).
 int linear_two_planes(const void* planes, const void* w, float* y, int64_t ldy, int m, int n, int k, bool accumulate, cudaStream_t st);
-// rmsNorm of contiguous fp32 rows into two bf16 planes, hi [rows][hidden], then lo (rowops.cu); hidden % 4 == 0, <= 16384.
+// rmsNorm of contiguous fp32 rows into two bf16 planes, hi [rows][hidden], then lo (rowops.cu); hidden % 4 == 0, at most:
+constexpr int RMS_PLANES_MAX = 16384;
 int rmsnorm_planes(const float* x, const float* w, uint16_t* planes, int64_t rows, int hidden, float eps, cudaStream_t st);
 // Raises the dynamic shared-memory limit of `fn` on the current device to at least `bytes` (once per device).
 int ensure_dynamic_smem(const void* fn, int bytes);
