@@ -318,3 +318,36 @@ def test_bias_of_the_lowest_float(L, api, lq, lk, d, dt):
     bound = _f32_bound(q, k, v, d) if dt == "f32" else 2.0 ** -7 * want.abs().max()
     assert (got - want).abs().max() <= bound
     assert not got[0, :, 12].any()  # no key at all
+
+
+@pytest.mark.parametrize("dt", ["f32", "f16"])
+@pytest.mark.parametrize("case", ["scores", "sums", "tiny"])
+def test_planes_leave_the_ends_of_the_range_to_ffma(L, api, case, dt):
+    """Scores and sums beyond the largest float, operands near the smallest: what FFMA makes of them."""
+    gen = torch.Generator(device="cuda").manual_seed(8)
+    t = {n: torch.randn(1, 2, 300, 96, generator=gen, device="cuda") for n in "qkv"}
+    if dt == "f16":
+        if case != "scores":
+            pytest.skip("fp16 numbers do not reach there")
+        t = {n: x.half() for n, x in t.items()}
+        scale = 1e37
+    else:
+        scale = None
+        if case == "scores":  # one key whose scores overflow to either infinity: a negative one weighs nothing
+            t["q"][0, 1, :, 3:9] *= 2.0 ** 70
+            t["k"][0, 1, 290, 3:9] *= 2.0 ** 66
+        elif case == "sums":
+            t["v"] = t["v"].abs() * 2.0 ** 124
+        else:
+            t["q"] *= 2.0 ** 60
+            t["k"] *= 2.0 ** -60
+            t["v"] *= 2.0 ** -119
+    run = lambda: api.scaledDotProductAttention(t["q"], t["k"], t["v"], *([scale] if scale else []), causal=True)  # noqa: E731
+    got = run()
+    L.ytcuda_attn_set_path(1)
+    try:
+        want = run()
+    finally:
+        L.ytcuda_attn_set_path(0)
+    assert torch.equal(torch.nan_to_num(got, 7.0, 8.0, 9.0), torch.nan_to_num(want, 7.0, 8.0, 9.0))
+    assert case == "tiny" or not want.isfinite().all()

@@ -57,7 +57,12 @@ struct PlanesParams {
   int* unfit;               // [blocks]
 };
 
-__device__ __forceinline__ bool has_no_planes(float x) { return (__float_as_uint(x) & 0x7F800000u) >= 0x7F000000u; }
+// Infinities, NaN and 2^127 and above; and where a number takes more than one plane, those under 2^-110 (the last plane would
+// lie below bf16's smallest number) but zero.
+__device__ __forceinline__ bool has_no_planes(float x, int planes) {
+  const uint32_t e = __float_as_uint(x) & 0x7FFFFFFFu;
+  return e >= 0x7F000000u || (planes > 1 && e != 0u && e < 0x08800000u);
+}
 
 __device__ __forceinline__ void split_planes(float x, uint16_t (&pl)[3]) {
 #pragma unroll
@@ -98,7 +103,7 @@ __global__ void __launch_bounds__(256) attn_planes_kernel(const PlanesParams p) 
     uint16_t pl[4][3];
 #pragma unroll
     for (int k = 0; k < 4; ++k) {
-      unfit |= has_no_planes(x[k]);
+      unfit |= has_no_planes(x[k], p.planes);
       split_planes(x[k], pl[k]);
     }
     uint16_t* d = p.dst[s] + static_cast<int64_t>(e) * 4;
@@ -385,7 +390,7 @@ __global__ void __launch_bounds__(SA_THREADS, 1)
           uint16_t pl[8][3];
 #pragma unroll
           for (int e = 0; e < 8; ++e) {
-            unfit |= has_no_planes(x[e]);
+            unfit |= has_no_planes(x[e], p.planes);
             split_planes(x[e], pl[e]);
           }
           uint8_t* dst = qs + ((((c0 & 63) >> 3) ^ (row & 7)) << 4);
@@ -545,6 +550,10 @@ __global__ void __launch_bounds__(SA_THREADS, 1)
       const float f = m_run == -CUDART_INF_F ? 0.f : fast_exp2((m_run - m) * unit), f_o = m_o == -CUDART_INF_F ? 0.f : fast_exp2((m_o - m) * unit);
       const float l = l_run * f + l_o * f_o;
       const float inv = l > 0.f ? 1.0f / l : 0.f;
+      // A score or a sum that overflows has plane products of either sign that overflow: NaN where FFMA has an infinity, of which
+      // a negative one weighs nothing. Rows that are not finite, or weigh no key though they see some, are left to FFMA.
+      if (valid && !general && limit >= 0) unfit |= !(l > 0.f);
+      float zero = 0.f;
 #pragma unroll
       for (int c = 0; c < 64; c += 32) {
         uint32_t r[32];
@@ -557,9 +566,13 @@ __global__ void __launch_bounds__(SA_THREADS, 1)
         if (valid) {
 #pragma unroll
           for (int e = 0; e < 32; e += 4)
-            if (wg * 64 + c + e < p.a.dv) store4(wg * 64 + c + e, x[e], x[e + 1], x[e + 2], x[e + 3]);
+            if (wg * 64 + c + e < p.a.dv) {
+              store4(wg * 64 + c + e, x[e], x[e + 1], x[e + 2], x[e + 3]);
+              zero = fmaf(x[e], 0.f, fmaf(x[e + 1], 0.f, fmaf(x[e + 2], 0.f, fmaf(x[e + 3], 0.f, zero))));
+            }
         }
       }
+      unfit |= !(zero == 0.f);
       tc_fence_before();
       __syncwarp();
       if (lane == 0) mbar_arrive(merge_out);
