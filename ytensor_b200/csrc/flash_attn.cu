@@ -1395,6 +1395,7 @@ namespace ytk {
 // O[i, 32 g .. 32 g + 31] += P[i, :] V with P passed through shared memory. The prefill path of the fp32 decoder.
 constexpr int TL_BM = 32, TL_BN = 32, TL_D = 128, TL_PAD = 4;
 
+template <bool GATED>
 __device__ __forceinline__ void attn_tile_item(const AttnSimtParams& p, int rbk, int h, int b) {
   extern __shared__ __align__(16) float tl_smem[];
   float(*Qs)[TL_D + TL_PAD] = reinterpret_cast<float(*)[TL_D + TL_PAD]>(tl_smem);
@@ -1408,7 +1409,7 @@ __device__ __forceinline__ void attn_tile_item(const AttnSimtParams& p, int rbk,
   const int row = row0 + ri;
   const int64_t qo = b * p.q_sb + h * p.q_sh;
   const int64_t ko = b * p.k_sb + kvh * p.k_sh, vo = b * p.v_sb + kvh * p.v_sh;
-  __syncthreads();  // (the item before has been finished)
+  if (GATED) __syncthreads();  // (the item before has been finished)
   // stage Q (zero-padded to TL_D columns and TL_BM rows)
   // fp32 operands with 16-byte aligned rows are staged with 128-bit loads; anything else element by element
   const bool vec = p.dt == YTC_F32 && p.d % 4 == 0 && p.dv % 4 == 0 && p.q_sr % 4 == 0 && p.k_sr % 4 == 0 &&
@@ -1541,14 +1542,21 @@ __device__ __forceinline__ void attn_tile_item(const AttnSimtParams& p, int rbk,
     }
   }
 }
+// GATED: behind the tensor-core form, a CTA takes the items in turn if the gate is open. Else a CTA per row block, head and batch
+// item (the loop over items costs 20 registers and spills: 32 heads, 30 queries and keys of 128, 28.7 us with it, 26.7 without).
+template <bool GATED>
 __global__ void __launch_bounds__(128) attn_tile_kernel(const AttnSimtParams p) {
   dependent_wait();     // (under a programmatic dependent launch: the kernel before this one has finished)
   dependent_trigger();  // the kernel queued behind this one may be scheduled meanwhile
-  if (gate_closed(p)) return;
-  const int row_blocks = (p.q_len + TL_BM - 1) / TL_BM, heads = p.kv_heads * p.groups;
-  for (int64_t i = blockIdx.x; i < static_cast<int64_t>(row_blocks) * heads * p.batch; i += gridDim.x)  // long causal rows first
-    attn_tile_item(p, row_blocks - 1 - static_cast<int>(i % row_blocks), static_cast<int>(i / row_blocks % heads),
-                   static_cast<int>(i / row_blocks / heads));
+  const int row_blocks = (p.q_len + TL_BM - 1) / TL_BM, heads = p.kv_heads * p.groups;  // (long causal rows first)
+  if constexpr (!GATED) {
+    attn_tile_item<false>(p, row_blocks - 1 - static_cast<int>(blockIdx.x), blockIdx.y, blockIdx.z);
+  } else {
+    if (gate_closed(p)) return;
+    for (int64_t i = blockIdx.x; i < static_cast<int64_t>(row_blocks) * heads * p.batch; i += gridDim.x)
+      attn_tile_item<true>(p, row_blocks - 1 - static_cast<int>(i % row_blocks), static_cast<int>(i / row_blocks % heads),
+               static_cast<int>(i / row_blocks / heads));
+  }
 }
 
 // ------------------------------------------------------------------ host side
@@ -1563,6 +1571,7 @@ __global__ void __launch_bounds__(128) attn_tile_kernel(const AttnSimtParams p) 
 constexpr int T64_BM = 64, T64_BN = 64, T64_LD = 128 + 4, T64_PLD = 64 + 4;
 constexpr int T64_SMEM = (3 * 64 * T64_LD + T64_BN * T64_PLD) * 4;
 
+template <bool GATED>
 __device__ __forceinline__ void attn_tile64_item(const AttnSimtParams& p, int rbk, int h, int b) {
   extern __shared__ __align__(16) float t64_smem[];
   float(*Qs)[T64_LD] = reinterpret_cast<float(*)[T64_LD]>(t64_smem);
@@ -1571,7 +1580,7 @@ __device__ __forceinline__ void attn_tile64_item(const AttnSimtParams& p, int rb
   float(*PsT)[T64_PLD] = reinterpret_cast<float(*)[T64_PLD]>(Vs + T64_BN);  // [key][row]
   const int tid = threadIdx.x;
   const int ry = tid >> 4, kx = tid & 15, cx = kx;
-  __syncthreads();  // (the item before has been finished)
+  if (GATED) __syncthreads();  // (the item before has been finished)
   const int kvh = h / p.groups;
   const int row0 = rbk * T64_BM;
   const float* Qf = static_cast<const float*>(p.Q) + b * p.q_sb + h * p.q_sh;
@@ -1713,14 +1722,20 @@ __device__ __forceinline__ void attn_tile64_item(const AttnSimtParams& p, int rb
     }
   }
 }
+// GATED: as attn_tile_kernel.
+template <bool GATED>
 __global__ void __launch_bounds__(256, 1) attn_tile64_kernel(const AttnSimtParams p) {
   dependent_wait();     // (under a programmatic dependent launch: the kernel before this one has finished)
   dependent_trigger();  // the kernel queued behind this one may be scheduled meanwhile
-  if (gate_closed(p)) return;
-  const int row_blocks = (p.q_len + T64_BM - 1) / T64_BM, heads = p.kv_heads * p.groups;
-  for (int64_t i = blockIdx.x; i < static_cast<int64_t>(row_blocks) * heads * p.batch; i += gridDim.x)  // long causal rows first
-    attn_tile64_item(p, row_blocks - 1 - static_cast<int>(i % row_blocks), static_cast<int>(i / row_blocks % heads),
-                     static_cast<int>(i / row_blocks / heads));
+  const int row_blocks = (p.q_len + T64_BM - 1) / T64_BM, heads = p.kv_heads * p.groups;  // (long causal rows first)
+  if constexpr (!GATED) {
+    attn_tile64_item<false>(p, row_blocks - 1 - static_cast<int>(blockIdx.x), blockIdx.y, blockIdx.z);
+  } else {
+    if (gate_closed(p)) return;
+    for (int64_t i = blockIdx.x; i < static_cast<int64_t>(row_blocks) * heads * p.batch; i += gridDim.x)
+      attn_tile64_item<true>(p, row_blocks - 1 - static_cast<int>(i % row_blocks), static_cast<int>(i / row_blocks % heads),
+               static_cast<int>(i / row_blocks / heads));
+  }
 }
 
 // Where the tensor-core form is faster than the tiled FFMA kernels, by their steps one after another: a step of 64 keys of
@@ -2022,31 +2037,28 @@ int ytcuda_flash_attn_fwd(int dtype, const void* Q, const void* K, const void* V
   // Products in fp32 from here on. On the tensor cores (attn_split.cuh) where that pays; the tiled FFMA kernels then run
   // behind it, and only where a number has no planes.
   if (g_attn_path != 1 && split_attention_pays(p)) (void)split_attention(p, &p.gate, &p.n_gate, st);
-  auto tile_grid = [&](int bm) {
-    const int64_t items = static_cast<int64_t>((q_len + bm - 1) / bm) * heads * batch;
-    const int64_t most = p.gate ? sm_count() : 0x7fffffff;
-    return dim3(static_cast<unsigned>(items < most ? items : most));
+  auto launch_tiles = [&](auto* plain, auto* gated, int bm, int threads, int smem) {
+    const int sa = ensure_dynamic_smem(reinterpret_cast<const void*>(p.gate ? gated : plain), smem);
+    if (sa != YTC_OK) return sa;
+    const int row_blocks = (q_len + bm - 1) / bm;
+    if (p.gate) {
+      const int64_t items = static_cast<int64_t>(row_blocks) * heads * batch;
+      YTC_CUDA(launch_overlapped(gated, dim3(static_cast<unsigned>(items < sm_count() ? items : sm_count())), dim3(threads), smem, st, p));
+    } else {
+      YTC_CUDA(launch_overlapped(plain, dim3(row_blocks, heads, batch), dim3(threads), smem, st, p));
+    }
+    count_launch();
+    device_workspace_release(st);
+    YTC_CUDA(cudaGetLastError());
+    return static_cast<int>(YTC_OK);
   };
   if (dtype == YTC_F32 && q_len >= 64 && head_dim <= 128 && value_dim <= 128 && heads <= 65535 && batch <= 65535 &&
       vec_ok && head_dim % 4 == 0 && value_dim % 4 == 0 && q_strides[0] % 4 == 0 && q_strides[1] % 4 == 0 &&
-      q_strides[2] % 4 == 0 && (reinterpret_cast<uint64_t>(Q) & 15) == 0) {
-    const int sa = ensure_dynamic_smem(reinterpret_cast<const void*>(attn_tile64_kernel), T64_SMEM);
-    if (sa != YTC_OK) return sa;
-    YTC_CUDA(launch_overlapped(attn_tile64_kernel, tile_grid(T64_BM), dim3(256), T64_SMEM, st, p));
-    count_launch();
-    device_workspace_release(st);
-    YTC_CUDA(cudaGetLastError());
-    return YTC_OK;
-  }
+      q_strides[2] % 4 == 0 && (reinterpret_cast<uint64_t>(Q) & 15) == 0)
+    return launch_tiles(attn_tile64_kernel<false>, attn_tile64_kernel<true>, T64_BM, 256, T64_SMEM);
   if (head_dim <= TL_D && value_dim <= TL_D && heads <= 65535 && batch <= 65535) {
     constexpr int TL_SMEM = ((TL_BM + 2 * TL_BN) * (TL_D + TL_PAD) + TL_BM * (TL_BN + 1)) * 4;
-    const int sa = ensure_dynamic_smem(reinterpret_cast<const void*>(attn_tile_kernel), TL_SMEM);
-    if (sa != YTC_OK) return sa;
-    YTC_CUDA(launch_overlapped(attn_tile_kernel, tile_grid(TL_BM), dim3(128), TL_SMEM, st, p));
-    count_launch();
-    device_workspace_release(st);
-    YTC_CUDA(cudaGetLastError());
-    return YTC_OK;
+    return launch_tiles(attn_tile_kernel<false>, attn_tile_kernel<true>, TL_BM, 128, TL_SMEM);
   }
   const int64_t rows = static_cast<int64_t>(batch) * heads * q_len;
   const int64_t blocks = (rows + 3) / 4;
