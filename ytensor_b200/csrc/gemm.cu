@@ -999,14 +999,18 @@ static bool tc_takes_pairs(int m, int n, int64_t k, int64_t batch) {
 static int tc_tile_n(int m, int n, int64_t batch) {
   return (n <= 128 || static_cast<int64_t>((m + 127) / 128) * ((n + 255) / 256) * batch < sm_count() / 2) ? 128 : 256;
 }
-// Pieces of k that fill the SMs when the tiles alone leave more than half of them idle; a piece keeps 512 / pairs of k.
-// Measured, bf16 16 x 4096 x 4096: one piece 24.5 us, four and their sum 13.7.
+// Pieces of k that fill the SMs when the tiles alone leave more than half of them idle; a piece keeps 512 / pairs of k. Not for
+// products of less than 6144 / pairs of k: their time is the caller's (30 us for a call of api.matmul, 0.35 us per block of 64 here),
+// and the launch that adds the pieces 2 to 4 us of it. Measured, bf16 16 x 4096 x k, one piece / pieces, calls one after the other:
+// k = 2048 30.5 / 32.7 us, 4096 30.5 / 32.9, 6144 34.8 / 33.0, 8192 45.1 / 33.4.
+constexpr int SPLIT_MIN_BLOCKS = 96;
 static int tc_splits(int m, int n, int k, int pairs, int64_t batch) {
   const int k_blocks = (k + TC_BK - 1) / TC_BK;
   if (g_mask.kind != 0 || g_tc_pair != 0 || tc_takes_pairs(m, n, static_cast<int64_t>(k) * pairs, batch)) return 1;
   const int bn = tc_tile_n(m, n, batch);
   const int64_t tiles = static_cast<int64_t>((m + 127) / 128) * ((n + bn - 1) / bn) * batch;
   if (tiles * 2 > sm_count()) return 1;
+  if (static_cast<int64_t>(k_blocks) * pairs < SPLIT_MIN_BLOCKS) return 1;
   const int64_t most = static_cast<int64_t>(k_blocks) * pairs / 8;
   int64_t want = sm_count() / tiles < most ? sm_count() / tiles : most;
   if (want > k_blocks) want = k_blocks;
