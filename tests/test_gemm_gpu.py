@@ -527,3 +527,37 @@ def test_small_and_odd_products_at_the_ends_of_the_range(L, api, sa, sb, m, n, k
     assert torch.equal(got[inf], ffma[inf])
     fin = sure & fin
     assert fin.any() and ((got.double() - want)[fin].abs() <= 2e-6 * size[fin]).all()
+
+
+def test_threads_share_a_stream(api):
+    """Two threads that queue products and attention on one stream: each call's launches hand scratch to one another, and none of
+    the other thread's may come between them."""
+    import threading
+    gen = torch.Generator(device="cuda").manual_seed(2)
+
+    def work(i):
+        a = torch.randn(30 + 200 * i, 2050, generator=gen, device="cuda")
+        b = torch.randn(2050, 601 + 100 * i, generator=gen, device="cuda")
+        q, k, v = (torch.randn(1, 2, 200 + 300 * i, 64, generator=gen, device="cuda") for _ in range(3))
+        h = torch.randn(16, 8192, generator=gen, device="cuda").bfloat16()
+        w = torch.randn(300 + 100 * i, 8192, generator=gen, device="cuda").bfloat16()
+        long = torch.randn(2, 3, 40000 + i, generator=gen, device="cuda")
+        return [lambda: api.matmul(a, b), lambda: api.scaledDotProductAttention(q, k, v, causal=True), lambda: api.linear(h, w),
+                lambda: api.scaledDotProductAttention(q[:, :, -1:], k, v), lambda: api.sum(long, -1)]
+
+    calls = [work(0), work(1)]
+    want = [[f() for f in c] for c in calls]
+    bad, stream = [], torch.cuda.current_stream()
+
+    def loop(i):
+        with torch.cuda.stream(stream):
+            for _ in range(60):
+                for f, x in zip(calls[i], want[i]):
+                    bad.append((f() != x).any())
+
+    threads = [threading.Thread(target=loop, args=(i,)) for i in range(2)]
+    for t in threads:
+        t.start()
+    for t in threads:
+        t.join()
+    assert not torch.stack(bad).any()

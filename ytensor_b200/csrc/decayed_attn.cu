@@ -513,6 +513,7 @@ static int decayed_chunks(const DecayedAttn& all, cudaStream_t st) {
   int s = ensure_dynamic_smem(reinterpret_cast<const void*>(decayed_chunk_state_kernel), DS_SMEM);
   if (s == YTC_OK) s = ensure_dynamic_smem(reinterpret_cast<const void*>(decayed_chunk_out_kernel), DO_SMEM);
   if (s != YTC_OK) return s;
+  const WorkspaceScope workspace(st);
   auto* ws = static_cast<char*>(device_workspace(static_cast<size_t>(group * per_seq * unit_bytes), st));
   if (!ws) {
     set_last_error("decayed_attention: no scratch memory");

@@ -633,6 +633,7 @@ static int linear_w16(Qwen3Model* m, const float* x, int64_t x_rs, const uint16_
   // offset is a plain pointer offset for both K-major operands), each writing its own partial result, and a small
   // kernel adds the partials of both planes in a fixed order.
   if (split_k_ok(M, K)) {
+    const WorkspaceScope workspace(st);
     Pieces pc;
     if ((s = gemm_pieces(m, W, M, N, K, &pc, st)) != YTC_OK) return s;
     const int64_t cap = static_cast<int64_t>(sm_count()) * 16;
@@ -1273,6 +1274,7 @@ int ytcuda_qwen3_forward(void* handle, const int32_t* ids, int len, float* logit
                           rows > SK_MAX_ROWS && split_k_ok(rows, Hd) && split_k_ok(rows, m->l_heads * D) &&
                           split_k_ok(rows, m->l_inter) && Hd <= 3072;
   if (fused_glue) {
+    const WorkspaceScope workspace(st);
     Pieces pc;  // the projection whose pieces still have to be added to the residual stream
     const int64_t cap = static_cast<int64_t>(sm_count()) * 16;
     for (int l = 0; l < m->layers; ++l) {

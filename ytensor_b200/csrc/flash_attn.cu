@@ -1993,6 +1993,7 @@ int ytcuda_flash_attn_fwd(int dtype, const void* Q, const void* K, const void* V
   p.d = head_dim; p.dv = value_dim;
   p.causal = causal; p.causal_off = causal_offset;
   p.scale = scale; p.dt = dtype;
+  const WorkspaceScope workspace(st);
   // few query rows per K/V head (decode): split the keys over CTAs, merge through a scratch buffer
   const bool vec_ok = dtype != YTC_F32 ||
                       (k_strides[2] % 4 == 0 && k_strides[1] % 4 == 0 && k_strides[0] % 4 == 0 && v_strides[2] % 4 == 0 &&

@@ -1382,6 +1382,7 @@ static int launch_planes(const void* A, const void* B, void* C, int dtype_out, i
     Scope() { overlap_scope() = true; }
     ~Scope() { overlap_scope() = was; }
   } scope;
+  const WorkspaceScope workspace(st);
   constexpr int PLANES = DT == YTC_F32 ? 3 : 1;
   const int esz = dtype_size(DT);
   const bool a_shared = batch > 1 && bsa == 0, b_shared = batch > 1 && bsb == 0;
@@ -1630,6 +1631,7 @@ static int gemm_any(int dtype_in, int dtype_out, const void* A, const void* B, v
     // A single k extent of 1 makes both strides of an axis "unit"; the leading stride must still be sane.
     const int splits = scratch ? tc_splits(m, n, k, 1, batch) : 1;
     if (splits > 1 && !stream_captures(st)) {
+      const WorkspaceScope workspace(st);
       float* part = static_cast<float*>(device_workspace(static_cast<size_t>(splits) * batch * m * n * 4, st));
       if (part) {
         const int s = launch_tc_split(dtype_in, dtype_out, A, B, C, m, n, k, alpha, beta, a_mn, lda, b_mn, ldb, rsc, csc, batch,

@@ -727,6 +727,7 @@ extern "C" int ytcuda_latent_attn_fwd(int dtype, const void* q, const void* uk_b
   d.batch = batch; d.len = len; d.pos0 = pos0; d.max_keys = pos0 + len; d.scale = scale;
   d.out = out; d.ld_out = static_cast<int64_t>(heads) * vdim;
   const int64_t rows = static_cast<int64_t>(batch) * len, qa = (rows * heads * (rank + rot) + 3) / 4 * 4;
+  const WorkspaceScope workspace(st);
   auto* ws = static_cast<float*>(device_workspace((qa + latent_part_floats(d.s, rows, d.max_keys)) * sizeof(float), st));
   if (!ws) return YTC_CUDA_ERROR;
   d.qa = ws;

@@ -1308,6 +1308,7 @@ static int run_nd(int op, int dt_in, int dt_out, int dt_w, const void* x, void* 
     }
     sp.contiguous = contig ? 1 : 0;
     const size_t need = static_cast<size_t>(lines) * chunks;
+    const WorkspaceScope workspace(st);
     void* ws = scratch ? scratch : device_workspace(need * 8, st);
     if (!ws) {
       set_last_error("%s: cannot allocate %zu bytes of scratch", who, need * 8);

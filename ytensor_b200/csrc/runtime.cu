@@ -102,6 +102,14 @@ static std::unordered_map<WsKey, WsBuf, WsKeyHash> g_ws;
 // Buffers above this size are handed back after the call that asked for them (device_workspace_release).
 static constexpr size_t kWsKeep = 256u << 20;
 
+std::recursive_mutex& workspace_mutex(cudaStream_t st) {
+  static std::unordered_map<WsKey, std::recursive_mutex, WsKeyHash> mutexes;  // (never erased: a reference stays good)
+  int dev = 0;
+  (void)cudaGetDevice(&dev);
+  std::lock_guard<std::mutex> lk(g_mu);
+  return mutexes[WsKey{dev, st}];
+}
+
 void* device_workspace(size_t bytes, cudaStream_t st) {
   int dev = 0;
   if (cudaGetDevice(&dev) != cudaSuccess) return nullptr;

@@ -8,6 +8,8 @@
 #include <stdint.h>
 #include <string.h>
 
+#include <mutex>
+
 #include "../../include/ytcuda.h"
 
 namespace ytk {
@@ -257,8 +259,19 @@ int* device_status_word();
 int read_device_status(cudaStream_t st);
 
 // Scratch buffer owned by the library, one per (device, stream), grown on demand with stream-ordered allocation:
-// calls on different streams never share scratch, calls on one stream are ordered by the stream itself.
+// calls on different streams never share scratch, calls on one stream are ordered by the stream itself. Whoever asks for it
+// holds a WorkspaceScope of that stream until the last kernel that uses it has been queued.
 void* device_workspace(size_t bytes, cudaStream_t st);
+std::recursive_mutex& workspace_mutex(cudaStream_t st);
+// The launches of one call that hand scratch to one another are queued as one piece: another thread on the same stream would
+// put kernels between them that write the same buffer, or free it to grow it.
+class WorkspaceScope {
+ public:
+  explicit WorkspaceScope(cudaStream_t st) : lock_(workspace_mutex(st)) {}
+
+ private:
+  std::lock_guard<std::recursive_mutex> lock_;
+};
 // Hands a buffer above 256 MiB back (stream-ordered) once the kernels using it have been queued; smaller ones stay.
 void device_workspace_release(cudaStream_t st);
 // ytcuda_gemm for callers whose C lies in this stream's workspace (gemm.cu).
