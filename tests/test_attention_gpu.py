@@ -351,3 +351,16 @@ def test_planes_leave_the_ends_of_the_range_to_ffma(L, api, case, dt):
         L.ytcuda_attn_set_path(0)
     assert torch.equal(torch.nan_to_num(got, 7.0, 8.0, 9.0), torch.nan_to_num(want, 7.0, 8.0, 9.0))
     assert case == "tiny" or not want.isfinite().all()
+
+
+def test_attention_over_its_queries(L, api):
+    """O may lie over Q: an infinity sends the call to the FFMA kernel, which has to find Q as it was."""
+    gen = torch.Generator(device="cuda").manual_seed(4)
+    q, k, v = (torch.randn(1, 2, 300, 64, generator=gen, device="cuda") for _ in range(3))
+    k[0, 1, 299, 5] = float("inf")
+    want, out = api.scaledDotProductAttention(q, k, v, causal=True), q.clone()
+    import ctypes
+    strides = (ctypes.c_int64 * 3)(*q.stride()[:3])
+    rc = L.ytcuda_flash_attn_fwd(0, out.data_ptr(), k.data_ptr(), v.data_ptr(), out.data_ptr(), 1, 2, 1, 300, 300, 64, 64, 0.125, strides,
+                                 strides, strides, strides, 1, 0, None, 0, None, 0, 0, torch.cuda.current_stream().cuda_stream)
+    assert rc == 0 and torch.equal(torch.nan_to_num(out, 7.0, 8.0, 9.0), torch.nan_to_num(want, 7.0, 8.0, 9.0))

@@ -2037,7 +2037,10 @@ int ytcuda_flash_attn_fwd(int dtype, const void* Q, const void* K, const void* V
   }
   // Products in fp32 from here on. On the tensor cores (attn_split.cuh) where that pays; the tiled FFMA kernels then run
   // behind it, and only where a number has no planes.
-  if (g_attn_path != 1 && split_attention_pays(p)) (void)split_attention(p, &p.gate, &p.n_gate, st);
+  // (O over Q: the kernel behind it could not read Q again.)
+  if (g_attn_path != 1 && O != Q && split_attention_pays(p)) {
+    (void)split_attention(p, &p.gate, &p.n_gate, st);
+  }
   auto launch_tiles = [&](auto* plain, auto* gated, int bm, int threads, int smem) {
     const int sa = ensure_dynamic_smem(reinterpret_cast<const void*>(p.gate ? gated : plain), smem);
     if (sa != YTC_OK) return sa;
