@@ -353,6 +353,24 @@ def test_planes_leave_the_ends_of_the_range_to_ffma(L, api, case, dt):
     assert case == "tiny" or not want.isfinite().all()
 
 
+@pytest.mark.parametrize("b,kvh,g,lq,lk,d,dt", [(5, 3, 2, 70, 24000, 64, "f32"), (1, 7, 1, 40, 50001, 36, "f32"), (3, 2, 1, 33, 130000, 80, "bf16")])
+def test_planes_in_bounded_scratch(L, api, b, kvh, g, lq, lk, d, dt):
+    """Keys and values whose planes are more than a stream keeps as scratch go by in groups of heads and batch items."""
+    gen = torch.Generator(device="cuda").manual_seed(lk)
+    t = {"f32": torch.float32, "bf16": torch.bfloat16}[dt]
+    q, k, v = (torch.randn(b, n, h, d, generator=gen, device="cuda").to(t).transpose(1, 2)
+               for n, h in ((lq, kvh * g), (lk, kvh), (lk, kvh)))
+    got = api.scaledDotProductAttention(q, k, v, causal=True)
+    seen = torch.arange(lk, device="cuda")[None] <= torch.arange(lk - lq, lk, device="cuda")[:, None]
+    for i in range(b):
+        want = _exact(q[i:i + 1], k[i:i + 1], v[i:i + 1], d ** -0.5, seen)
+        bound = _f32_bound(q[i:i + 1], k[i:i + 1], v, d) if dt == "f32" else 2.0 ** -7 * want.abs().max()
+        assert (got[i:i + 1].double() - want).abs().max() <= bound
+    before = L.ytcuda_launch_count()
+    api.scaledDotProductAttention(q, k, v, causal=True)
+    assert L.ytcuda_launch_count() - before > 3  # (planes, product, check: more than one group)
+
+
 def test_attention_over_its_queries(L, api):
     """O may lie over Q: an infinity sends the call to the FFMA kernel, which has to find Q as it was."""
     gen = torch.Generator(device="cuda").manual_seed(4)

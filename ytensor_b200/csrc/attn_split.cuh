@@ -593,6 +593,12 @@ __global__ void __launch_bounds__(SA_THREADS, 1)
   }
 }
 
+constexpr int64_t SA_SCRATCH = int64_t{240} << 20;
+static int64_t split_attention_bytes(const AttnSimtParams& a) {  // (of the planes)
+  const int planes = a.dt == YTC_F32 ? 3 : a.dt == YTC_F16 ? 2 : 1;
+  return static_cast<int64_t>(a.batch) * a.kv_heads * a.kv_len * ((a.d + 63) / 64 + (a.dv + 63) / 64) * 64 * 2 * planes;
+}
+
 // Queues the planes and the attention; false: nothing was queued (a size, alignment or capture the path does not take, no
 // scratch). On true the caller queues the fp32 kernel behind it with `gate`, which runs only where a number had no planes.
 static bool split_attention(const AttnSimtParams& a, const int** gate, int* n_gate, cudaStream_t st) {

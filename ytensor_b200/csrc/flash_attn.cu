@@ -2039,6 +2039,27 @@ int ytcuda_flash_attn_fwd(int dtype, const void* Q, const void* K, const void* V
   // behind it, and only where a number has no planes.
   // (O over Q: the kernel behind it could not read Q again.)
   if (g_attn_path != 1 && O != Q && split_attention_pays(p)) {
+    // As many batch items and K/V heads at a time as keep the planes within the scratch that a stream keeps: larger buffers come
+    // and go with every call.
+    const int64_t bytes = split_attention_bytes(p), items = static_cast<int64_t>(batch) * kv_heads;
+    if (bytes > SA_SCRATCH && items > 1) {
+      const int64_t fit = items * SA_SCRATCH / bytes, per = fit > 1 ? fit : 1;
+      const int nb = per >= kv_heads ? static_cast<int>(per / kv_heads) : 1, nh = per >= kv_heads ? kv_heads : static_cast<int>(per);
+      const int64_t esz = dtype_size(dtype);
+      for (int b0 = 0; b0 < batch; b0 += nb)
+        for (int h0 = 0; h0 < kv_heads; h0 += nh) {
+          auto at = [&](const void* x, const int64_t* strides, int64_t g) {
+            return static_cast<const char*>(x) + (b0 * strides[0] + h0 * g * strides[1]) * esz;
+          };
+          const int s = ytcuda_flash_attn_fwd(dtype, at(Q, q_strides, groups), at(K, k_strides, 1), at(V, v_strides, 1),
+                                              const_cast<char*>(at(O, o_strides, groups)), batch - b0 < nb ? batch - b0 : nb,
+                                              kv_heads - h0 < nh ? kv_heads - h0 : nh, groups, q_len, kv_len, head_dim, value_dim, scale,
+                                              q_strides, k_strides, v_strides, o_strides, mask_kind, causal_offset, mask, mask_row_stride,
+                                              bias, bias_row_stride, bias_col_stride, stream);
+          if (s != YTC_OK) return s;
+        }
+      return YTC_OK;
+    }
     (void)split_attention(p, &p.gate, &p.n_gate, st);
   }
   auto launch_tiles = [&](auto* plain, auto* gated, int bm, int threads, int smem) {
