@@ -170,6 +170,8 @@ __global__ void __launch_bounds__(G < 256 ? 256 : G) row_kernel(const RowParams 
     if (OP == OP_CHAIN && copies > 1 && row_ok) row = (row % copies) * p.r_rows + row / copies;
     F4 x[VPT];
     auto at = [&](int v, int e) { return VEC == 4 ? (v * G + t) * 4 + e : (4 * v + e) * G + t; };
+    // (a load that is off for its first element is off for all: its arithmetic is jumped over. Softmax of fp32 100000 x 100: 24 us,
+    // 43 with a test per element alone)
     auto on = [&](int v, int e) { return row_ok && at(v, VEC == 4 ? 0 : e) < p.L; };
     auto load = [&](const void* src, int64_t row0, int v, int dt) {
       F4 r = {{0.f, 0.f, 0.f, 0.f}};
@@ -197,9 +199,11 @@ __global__ void __launch_bounds__(G < 256 ? 256 : G) row_kernel(const RowParams 
       MaxIdx m = {-CUDART_INF_F, 0x7fffffff};
 #pragma unroll
       for (int v = 0; v < VPT; ++v)
+        if (on(v, 0)) {
 #pragma unroll
-        for (int k = 0; k < 4; ++k)
-          if (on(v, k)) m = max_combine(m, MaxIdx{x[v].v[k], at(v, k)});
+          for (int k = 0; k < 4; ++k)
+            if (VEC == 4 || on(v, k)) m = max_combine(m, MaxIdx{x[v].v[k], at(v, k)});
+        }
       m = group_maxidx<G>(m, red, redi, group, t);
       if (row_ok && t == 0) {
         if (m.i == 0x7fffffff) {  // every element failed `>` (all NaN): the reference keeps element 0
@@ -232,6 +236,7 @@ __global__ void __launch_bounds__(G < 256 ? 256 : G) row_kernel(const RowParams 
       const float inv = 1.0f / sqrtf(ss * invL + p.eps);
 #pragma unroll
       for (int v = 0; v < VPT; ++v) {
+        if (!on(v, 0)) continue;
 #pragma unroll
         for (int k = 0; k < 4; ++k) x[v].v[k] *= inv;
         if constexpr (OP == OP_CHAIN) {
@@ -252,16 +257,19 @@ __global__ void __launch_bounds__(G < 256 ? 256 : G) row_kernel(const RowParams 
       float ss = 0.f;
 #pragma unroll
       for (int v = 0; v < VPT; ++v)
+        if (on(v, 0)) {
 #pragma unroll
-        for (int k = 0; k < 4; ++k)
-          if (on(v, k)) {
-            x[v].v[k] -= mu;
-            ss = fmaf(x[v].v[k], x[v].v[k], ss);
-          }
+          for (int k = 0; k < 4; ++k)
+            if (VEC == 4 || on(v, k)) {
+              x[v].v[k] -= mu;
+              ss = fmaf(x[v].v[k], x[v].v[k], ss);
+            }
+        }
       ss = group_sum<G>(ss, red, group, t);
       const float inv = 1.0f / sqrtf(ss * invL + p.eps);
 #pragma unroll
       for (int v = 0; v < VPT; ++v) {
+        if (!on(v, 0)) continue;
 #pragma unroll
         for (int k = 0; k < 4; ++k) x[v].v[k] *= inv;
         if (p.w) {
@@ -276,19 +284,23 @@ __global__ void __launch_bounds__(G < 256 ? 256 : G) row_kernel(const RowParams 
       float m = -CUDART_INF_F;
 #pragma unroll
       for (int v = 0; v < VPT; ++v)
+        if (on(v, 0)) {
 #pragma unroll
-        for (int k = 0; k < 4; ++k)
-          if (on(v, k)) m = fmaxf(m, x[v].v[k]);
+          for (int k = 0; k < 4; ++k)
+            if (VEC == 4 || on(v, k)) m = fmaxf(m, x[v].v[k]);
+        }
       m = group_max<G>(m, red, group, t);
       float s = 0.f;
 #pragma unroll
       for (int v = 0; v < VPT; ++v)
+        if (on(v, 0)) {
 #pragma unroll
-        for (int k = 0; k < 4; ++k)
-          if (on(v, k)) {
-            x[v].v[k] = __expf(x[v].v[k] - m);
-            s += x[v].v[k];
-          }
+          for (int k = 0; k < 4; ++k)
+            if (VEC == 4 || on(v, k)) {
+              x[v].v[k] = __expf(x[v].v[k] - m);
+              s += x[v].v[k];
+            }
+        }
       s = group_sum<G>(s, red, group, t);
       const float inv = 1.0f / s;
 #pragma unroll
