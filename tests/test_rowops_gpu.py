@@ -238,3 +238,21 @@ def test_odd_elementwise_sizes(api):
             for got, want in ((api.add(x, bias), x + bias), (api.add(x, y), x + y)):
                 assert (got - want).abs().max() <= flushed
             assert (api.swish(x).double() - torch.nn.functional.silu(x.double())).abs().max() <= (1e-6 if dt == torch.float32 else 4e-3)
+
+
+# either side of where short lines go to line_kernel: columns of 14 (softmax, norms) and 32 (reductions), spans of 256, one element
+@pytest.mark.parametrize("shape,axes,dtype", [
+    ((13, 4160), (0,), torch.float32), ((14, 4160), (0,), torch.bfloat16), ((31, 4099), (0,), torch.float32), ((32, 4099), (0,), torch.float16),
+    ((3, 6, 85), (0, 2), torch.float32), ((4, 6, 64), (0, 2), torch.bfloat16), ((5, 5000, 3), (0, 2), torch.float32),
+    ((130, 33, 1), (2,), torch.float32), ((9000, 2), (1,), torch.bfloat16), ((2, 9, 2048), (1,), torch.float32)])
+def test_short_lines(api, shape, axes, dtype):
+    test_shared_lines_and_odd_rows(api, shape, axes, dtype)
+
+
+def test_channel_norms_of_many_short_lines(api):
+    gen = torch.Generator(device="cuda").manual_seed(1)
+    x = torch.randn(4, 12000, 3, generator=gen, device="cuda")
+    w, b = (torch.randn(12000, generator=gen, device="cuda") for _ in range(2))
+    for got, axes in ((api.instanceNorm(x, w, b), (2,)), (api.batchNorm(x, w, b), (0, 2))):
+        want = _sixty_four(x, axes, "layerNorm", w.double()[:, None], b.double()[:, None])
+        assert (got.double() - want).abs().max() <= 1e-5 * want.abs().max()  # (variances near zero: eps of 1e-5 under the root)

@@ -1068,6 +1068,15 @@ static void launch_line_op(int op, const LineParams& p, bool per_thread, cudaStr
   }
 }
 
+// one thread per line when neighbouring lines sit next to each other in memory
+static bool line_per_thread(const LineParams& p) {
+  return p.nk > 0 && p.kxs[p.nk - 1] == 1 && p.kshape[p.nk - 1] >= 32 && p.lines >= 4096;
+}
+// Lines shorter than these stay with line_kernel. Measured, fp32, line_kernel / here: softmax over the first axis of 12 x 600000 81 /
+// 84 us, 16 x 600000 108 / 92, 5 x 300000 22 / 35, 2 x 4000000 100 / 354; sum of 24 x 600000 48.6 / 47.7, 32 x 600000 65 / 43, 3 x
+// 1000000 21 / 47; over the outer axes of 4 x 30000 x w, softmax: w = 48 127 / 160, 72 178 / 166, 512 1036 / 261.
+constexpr int SHORT_COLUMNS = 14, SHORT_COLUMNS_REDUCED = 32, SHORT_SPANS = 256;
+
 // Launches span_kernel or column_kernel where the dims allow it; YTC_UNSUPPORTED: nothing was launched. `ws`: strides of gamma
 // and beta per dim, null: they are laid out like the reduced dims.
 template <class K>
@@ -1175,6 +1184,12 @@ static int launch_shared_line(int op, const LineParams& lp, const NdArgs& a, con
   } else {
     return YTC_UNSUPPORTED;
   }
+  // Short lines stay with line_kernel, whose CTAs are smaller and which takes a thread per line where lines lie side by side.
+  // With gamma and beta (one launch here, three there) only where the lines are so many that the launches don't matter.
+  const bool keeps = op != OP_SUM && op != OP_MEAN && op != OP_MAX;
+  if (kind == 0 ? lp.R < (keeps ? SHORT_COLUMNS : SHORT_COLUMNS_REDUCED) && line_per_thread(lp) && (!ws || lp.lines > (1 << 20))
+                : lp.R < SHORT_SPANS && (!ws || lp.lines > (1 << 15)))
+    return YTC_UNSUPPORTED;
   // Shares: enough CTAs for two per SM while a share keeps 2048 elements, and shares of half an SM's shared memory.
   int shares = 1;
   auto share_of = [&](int n) { return ((p.R + n - 1) / n + 3) / 4 * 4; };
@@ -1184,7 +1199,6 @@ static int launch_shared_line(int op, const LineParams& lp, const NdArgs& a, con
   if (lines * shares > 0x7fffffff) return YTC_UNSUPPORTED;
   p.shares = shares;
   p.share = share_of(shares);
-  const bool keeps = op != OP_SUM && op != OP_MEAN && op != OP_MAX;
   p.cached = keeps && static_cast<uint64_t>(p.share) * floats <= CACHE_FLOATS;
   const size_t smem = p.cached ? static_cast<size_t>(p.share) * floats * 4 : 0;
   // A share of which only one fits an SM needs more threads to keep enough loads in flight (batchNorm, bf16, 32 x 256 x 112 x
@@ -1259,7 +1273,10 @@ static int run_nd(int op, int dt_in, int dt_out, int dt_w, const void* x, void* 
                      (reduce_out || ((reinterpret_cast<uint64_t>(y) % (4 * esz_out)) == 0 && y_rs % 4 == 0)) &&
                      (!w || reinterpret_cast<uint64_t>(w) % (4 * dtype_size(dt_w)) == 0) &&
                      (!b || reinterpret_cast<uint64_t>(b) % (4 * dtype_size(dt_w)) == 0);
-  if (op != OP_LPNORM && trailing && !spread && R <= 16384 && x_rs >= 0 && y_rs >= 0) {
+  // (lines of one element side by side: a thread each, line_kernel)
+  const int last_kept = a.ndim - a.naxes - 1;
+  const bool single = R == 1 && x_rs == 1 && lines >= 4096 && last_kept >= 0 && a.shape[last_kept] >= 32;
+  if (op != OP_LPNORM && trailing && !spread && !single && R <= 16384 && x_rs >= 0 && y_rs >= 0) {
     RowParams p;
     p.x = x; p.y = y; p.w = w; p.b = b; p.idx = idx;
     p.rows = lines; p.L = static_cast<int>(R);
@@ -1353,9 +1370,7 @@ static int run_nd(int op, int dt_in, int dt_out, int dt_w, const void* x, void* 
     set_last_error("%s: these strides are not supported", who);
     return YTC_UNSUPPORTED;
   }
-  // one thread per line when neighbouring lines sit next to each other in memory
-  const bool per_thread = p.nk > 0 && p.kxs[p.nk - 1] == 1 && p.kshape[p.nk - 1] >= 32 && lines >= 4096;
-  launch_line_op(op, p, per_thread, st);
+  launch_line_op(op, p, line_per_thread(p), st);
   YTC_CUDA(cudaGetLastError());
   return YTC_OK;
 }
