@@ -22,6 +22,7 @@
 #include <math_constants.h>
 
 #include <atomic>
+#include <optional>
 #include <type_traits>
 
 #include "lm_ops.cuh"
@@ -1993,7 +1994,6 @@ int ytcuda_flash_attn_fwd(int dtype, const void* Q, const void* K, const void* V
   p.d = head_dim; p.dv = value_dim;
   p.causal = causal; p.causal_off = causal_offset;
   p.scale = scale; p.dt = dtype;
-  const WorkspaceScope workspace(st);
   // few query rows per K/V head (decode): split the keys over CTAs, merge through a scratch buffer
   const bool vec_ok = dtype != YTC_F32 ||
                       (k_strides[2] % 4 == 0 && k_strides[1] % 4 == 0 && k_strides[0] % 4 == 0 && v_strides[2] % 4 == 0 &&
@@ -2001,6 +2001,7 @@ int ytcuda_flash_attn_fwd(int dtype, const void* Q, const void* K, const void* V
                        (reinterpret_cast<uint64_t>(V) & 15) == 0);
   if (groups * q_len <= DEC_MAX_ROWS && head_dim % 4 == 0 && value_dim % 4 == 0 && head_dim <= 128 * DEC_MAX_VEC &&
       value_dim <= 128 * DEC_MAX_VEC && kv_len > 0 && vec_ok && static_cast<int64_t>(batch) * kv_heads <= 65535) {
+    const WorkspaceScope workspace(st);
     AttnDecodeParams dp;
     dp.a = p;
     const int bk = batch * kv_heads;
@@ -2038,7 +2039,9 @@ int ytcuda_flash_attn_fwd(int dtype, const void* Q, const void* K, const void* V
   // Products in fp32 from here on. On the tensor cores (attn_split.cuh) where that pays; the tiled FFMA kernels then run
   // behind it, and only where a number has no planes.
   // (O over Q: the kernel behind it could not read Q again.)
+  std::optional<WorkspaceScope> workspace;
   if (g_attn_path != 1 && O != Q && split_attention_pays(p)) {
+    workspace.emplace(st);
     // As many batch items and K/V heads at a time as keep the planes within the scratch that a stream keeps: larger buffers come
     // and go with every call.
     const int64_t bytes = split_attention_bytes(p), items = static_cast<int64_t>(batch) * kv_heads;
@@ -2073,7 +2076,7 @@ int ytcuda_flash_attn_fwd(int dtype, const void* Q, const void* K, const void* V
       YTC_CUDA(launch_overlapped(plain, dim3(row_blocks, heads, batch), dim3(threads), smem, st, p));
     }
     count_launch();
-    device_workspace_release(st);
+    if (workspace) device_workspace_release(st);
     YTC_CUDA(cudaGetLastError());
     return static_cast<int>(YTC_OK);
   };
