@@ -770,12 +770,15 @@ struct GemmSimtParams {
   int in_dtype, out_dtype;
   int tiles_m, tiles_n;
   const uint8_t* tile_live;  // masked product: 0 marks a 128 x 128 output tile nobody asks for (NULL: all computed)
-  const int* gate;  // the kernel runs only if one of these `n_gate` words is set (NULL: always), and for tiles of C (fp32) that
-  int n_gate;       // hold a number that isn't finite
+  const int* gate;  // GATED: the kernel runs only if one of these `n_gate` words is set
+  int n_gate;
+  int scan;         // ... and for tiles of C (fp32) that hold a number that isn't finite
 };
 
-template <int IN_DT>
-__global__ void __launch_bounds__(SM_THREADS) gemm_simt_kernel(const GemmSimtParams p) {
+// GATED: behind a product of planes, for what that cannot form. (An instance of its own: one for both took 167 registers, and
+// an SM one CTA. 8 x 500 x 700 x 100: 63 us, 84 with that.)
+template <int IN_DT, bool GATED>
+__global__ void __launch_bounds__(SM_THREADS, 2) gemm_simt_kernel(const GemmSimtParams p) {
   __shared__ __align__(16) float As[2][SM_BK][SM_BM + SM_PAD];
   __shared__ __align__(16) float Bs[2][SM_BK][SM_BN + SM_PAD];
 
@@ -783,16 +786,25 @@ __global__ void __launch_bounds__(SM_THREADS) gemm_simt_kernel(const GemmSimtPar
   const int tile = blockIdx.x;
   const int mb = tile / p.tiles_n, nb = tile - mb * p.tiles_n;
   const int m0 = mb * SM_BM, n0 = nb * SM_BN;
-  if (p.gate) {
+  if constexpr (GATED) {
     int any = 0;
     for (int i = tid; i < p.n_gate; i += SM_THREADS) any |= p.gate[i];
     if (!__syncthreads_or(any)) {
+      if (!p.scan) return;
       // A product that overflows has plane products of either sign that overflow: NaN where the sum is an infinity.
       const float* c = static_cast<const float*>(p.C) + blockIdx.y * p.bsc;
-      for (int i = tid; i < SM_BM * SM_BN; i += SM_THREADS) {
-        const int fast = i % SM_BN, slow = i / SM_BN;
-        const int r = m0 + (p.csc == 1 ? slow : fast), col = n0 + (p.csc == 1 ? fast : slow);
-        if (r < p.M && col < p.N) any |= !isfinite(c[r * p.rsc + col * p.csc]);
+      const int fast = tid % SM_BN, slow0 = tid / SM_BN;
+      constexpr int AT_ONCE = 16, ROWS = SM_THREADS / SM_BN;
+#pragma unroll 1
+      for (int s0 = slow0; s0 < SM_BM; s0 += AT_ONCE * ROWS) {
+        float v[AT_ONCE];
+#pragma unroll
+        for (int u = 0; u < AT_ONCE; ++u) {
+          const int slow = s0 + u * ROWS, r = m0 + (p.csc == 1 ? slow : fast), col = n0 + (p.csc == 1 ? fast : slow);
+          v[u] = r < p.M && col < p.N ? c[r * p.rsc + col * p.csc] : 0.f;
+        }
+#pragma unroll
+        for (int u = 0; u < AT_ONCE; ++u) any |= !isfinite(v[u]);
       }
       if (!__syncthreads_or(any)) return;
     }
@@ -1169,9 +1181,9 @@ int linear_tc(const void* x, int64_t ldx, const void* w, int64_t ldw, void* y, i
 static int launch_simt(int dtype_in, int dtype_out, const void* A, const void* B, void* C, int m, int n, int k,
                        float alpha, float beta, int64_t rsa, int64_t csa, int64_t rsb, int64_t csb, int64_t rsc,
                        int64_t csc, int64_t batch, int64_t bsa, int64_t bsb, int64_t bsc, cudaStream_t st,
-                       const int* gate = nullptr, int n_gate = 0) {
+                       const int* gate = nullptr, int n_gate = 0, bool scan = false) {
   GemmSimtParams p;
-  p.gate = gate; p.n_gate = n_gate;
+  p.gate = gate; p.n_gate = n_gate; p.scan = scan;
   p.A = A; p.B = B; p.C = C;
   p.M = m; p.N = n; p.K = k;
   p.rsa = rsa; p.csa = csa; p.rsb = rsb; p.csb = csb; p.rsc = rsc; p.csc = csc;
@@ -1201,9 +1213,10 @@ static int launch_simt(int dtype_in, int dtype_out, const void* A, const void* B
     q.B = static_cast<const char*>(B) + b0 * bsb * dtype_size(dtype_in);
     q.C = static_cast<char*>(C) + b0 * bsc * dtype_size(dtype_out);
     dim3 grid(static_cast<unsigned>(tiles), static_cast<unsigned>(nb));
-    if (dtype_in == YTC_F32) gemm_simt_kernel<YTC_F32><<<grid, SM_THREADS, 0, st>>>(q);
-    else if (dtype_in == YTC_BF16) gemm_simt_kernel<YTC_BF16><<<grid, SM_THREADS, 0, st>>>(q);
-    else gemm_simt_kernel<YTC_F16><<<grid, SM_THREADS, 0, st>>>(q);
+    if (gate) gemm_simt_kernel<YTC_F32, true><<<grid, SM_THREADS, 0, st>>>(q);
+    else if (dtype_in == YTC_F32) gemm_simt_kernel<YTC_F32, false><<<grid, SM_THREADS, 0, st>>>(q);
+    else if (dtype_in == YTC_BF16) gemm_simt_kernel<YTC_BF16, false><<<grid, SM_THREADS, 0, st>>>(q);
+    else gemm_simt_kernel<YTC_F16, false><<<grid, SM_THREADS, 0, st>>>(q);
     count_launch();
   }
   if (live) cudaFreeAsync(live, st);
@@ -1267,13 +1280,13 @@ __global__ void __launch_bounds__(256) gemm_planes_kernel(const PlaneOp oa, cons
         }
         p[0][e] = *reinterpret_cast<const uint16_t*>(&q);
         p[1][e] = p[2][e] = 0;
+        bad |= (__float_as_uint(v[e]) & 0x7FFFFFFFu) - 1u < 0x08800000u - 1u;  // (below 2^-110, but not zero)
         if (isfinite(fh)) {
           const float r1 = v[e] - fh;
           q = __float2bfloat16_rn(r1);
           p[1][e] = *reinterpret_cast<const uint16_t*>(&q);
           q = __float2bfloat16_rn(r1 - __bfloat162float(q));
           p[2][e] = *reinterpret_cast<const uint16_t*>(&q);
-          bad |= v[e] != 0.f && fabsf(v[e]) < 0x1p-110f;
         } else {
           bad = true;
         }
@@ -1300,11 +1313,13 @@ __global__ void __launch_bounds__(256) gemm_planes_kernel(const PlaneOp oa, cons
 }
 
 // C = alpha * (the sum of the partial sums, in their order) + beta * C; part is [splits][batch][m][ldp], `stride` elements each.
+// `unfit` (may be null) is set where a sum isn't finite.
 __global__ void __launch_bounds__(256) gemm_sum_kernel(const float* part, int splits, int64_t stride, int64_t total, int m, int n,
                                                        int64_t ldp, void* C, int dt, int64_t rsc, int64_t csc, int64_t bsc,
-                                                       float alpha, float beta) {
+                                                       float alpha, float beta, int* unfit) {
   dependent_wait();
   dependent_trigger();
+  bool bad = false;
   for (int64_t t = blockIdx.x * 256ll + threadIdx.x; t < total; t += gridDim.x * 256ll) {
     const int64_t row = t / n, col = t - row * n;
     const float* from = part + row * ldp + col;
@@ -1315,7 +1330,9 @@ __global__ void __launch_bounds__(256) gemm_sum_kernel(const float* part, int sp
     v *= alpha;
     if (beta != 0.f) v += beta * load_as_f32(C, at, dt);
     store_from_f32(C, at, v, dt);
+    bad |= !isfinite(v);
   }
+  if (unfit && bad) *unfit = 1;
 }
 
 // C[b][i][j] = masked_value wherever mask[i][j] == 0 (the mask is shared by every batch item); the second half of
@@ -1442,8 +1459,9 @@ static int launch_planes(const void* A, const void* B, void* C, int dtype_out, i
     splits = side < 1 ? 1 : static_cast<int>(side);
     if (splits < pieces) window = splits * PIECE;
   }
-  const bool direct = splits == 1 && (window == k || (csc == 1 && rsc % 4 == 0 && (batch == 1 || bsc % 4 == 0) &&
-                                                      (reinterpret_cast<uint64_t>(C) & 15) == 0));  // (C itself takes the sums)
+  // C itself takes the sums: of one window, and of several where its rows start at 16 bytes
+  const bool rows16 = csc == 1 && rsc % 4 == 0 && (batch == 1 || bsc % 4 == 0) && (reinterpret_cast<uint64_t>(C) & 15) == 0;
+  const bool direct = splits == 1 && (rows16 || window == k);
   auto up = [](int64_t v) { return static_cast<size_t>((v + 255) / 256 * 256); };
   // CTAs (and words of the gate) of either operand: those of the first, largest rewriting
   const PlaneOp largest_a = a_op(0, a_shared ? 1 : chunk, 0, window), largest_b = b_op(0, b_shared ? 1 : chunk, 0, window);
@@ -1497,11 +1515,12 @@ static int launch_planes(const void* A, const void* B, void* C, int dtype_out, i
     if (!direct) {
       const int64_t total = nb * m * n, blocks = (total + 255) / 256, cap = static_cast<int64_t>(sm_count()) * 8;
       YTC_CUDA(launch_overlapped(gemm_sum_kernel, dim3(static_cast<unsigned>(blocks < cap ? blocks : cap)), dim3(256), 0, st, part,
-                                 splits, nb * mn, total, m, n, ldp, c, dtype_out, rsc, csc, bsc, alpha, beta));
+                                 splits, nb * mn, total, m, n, ldp, c, dtype_out, rsc, csc, bsc, alpha, beta, gate));
       count_launch();
     }
     if (check && (s = launch_simt(DT, dtype_out, static_cast<const char*>(A) + b0 * bsa * esz, static_cast<const char*>(B) + b0 * bsb * esz,
-                                  c, m, n, k, alpha, beta, rsa, csa, rsb, csb, rsc, csc, nb, bsa, bsb, bsc, st, gate, n_gate)) != YTC_OK)
+                                  c, m, n, k, alpha, beta, rsa, csa, rsb, csb, rsc, csc, nb, bsa, bsb, bsc, st, gate, n_gate, direct)) !=
+                     YTC_OK)
       return s;
   }
   device_workspace_release(st);  // large operands do not stay resident
@@ -1523,7 +1542,7 @@ static int launch_tc_split(int dtype_in, int dtype_out, const void* A, const voi
   if (s != YTC_OK) return s;
   const int64_t blocks = (total + 255) / 256, cap = static_cast<int64_t>(sm_count()) * 8;
   YTC_CUDA(launch_overlapped(gemm_sum_kernel, dim3(static_cast<unsigned>(blocks < cap ? blocks : cap)), dim3(256), 0, st, part, splits,
-                             total, total, m, n, n, C, dtype_out, rsc, csc, bsc, alpha, beta));
+                             total, total, m, n, n, C, dtype_out, rsc, csc, bsc, alpha, beta, static_cast<int*>(nullptr)));
   count_launch();
   return YTC_OK;
 }
