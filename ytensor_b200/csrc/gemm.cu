@@ -1360,17 +1360,20 @@ static std::atomic<int> g_gemm_path{0};
 // 2 = whenever the shapes allow.
 static std::atomic<int> g_f32_split{0};
 
-// The FFMA kernel takes about 0.17 us (fp32; 16 bit 0.3) per element of k and wave of 128 x 128 tiles, whatever m is. The planes
-// cost about 8 us of launches and 10 bytes of traffic a value, six products a sixth of the tensor rate. Measured (FFMA / planes):
-// fp32 16 x 4096 x 4096 705 / 88 us, 60 x 1001 x 1111 205 / 56, 130 x 8192 x 8192 1548 / 453, 77 x 130 x 300 70 / 45; bf16
-// 777 x 1001 x 1111 340 / 30.
+// The FFMA kernel takes 0.17 to 0.22 us (fp32; 16 bit 0.25 to 0.36) per element of k and wave of 128 x 128 tiles, the less where the
+// left operand has few rows to load. The planes cost 19 us of launches, 10 bytes of traffic a value, six products a sixth of the
+// tensor rate, and 8 bytes per result and 256 of k for its partial sums. Measured (FFMA / planes, us): fp32 1 x 512 x 120 27.8 / 32.4,
+// x 180 34.9 / 32.9, 60 x 1001 x 120 34.9 / 32.5, 16 x 4096 x 4096 709 / 82, 777 x 1001 x 1111 227 / 47, 2000 x 4001 x 64 82 / 142, 2000 x
+// 2001 x 257 107 / 74; bf16 1 x 513 x 101 27.1 / 30.3, x 131 32.8 / 30.1, 60 x 1002 x 75 32.8 / 30.0, 777 x 1001 x 1111 340 / 30.
 static double simt_us(int m, int n, int k, int64_t batch, bool wide) {
   const int64_t tiles = static_cast<int64_t>((m + SM_BM - 1) / SM_BM) * ((n + SM_BN - 1) / SM_BN) * batch;
-  return (wide ? 0.17 : 0.3) * k * static_cast<double>((tiles + sm_count() - 1) / sm_count());
+  const double each = wide ? (m < 16 ? 0.17 : 0.22) : (m < 16 ? 0.25 : 0.36);
+  return each * k * static_cast<double>((tiles + sm_count() - 1) / sm_count());
 }
 static double planes_us(int m, int n, int k, int64_t batch, bool b_shared, bool wide) {
   const double values = static_cast<double>(m) * k * batch + static_cast<double>(k) * n * (b_shared ? 1 : batch);
-  return 12.0 + values * (wide ? 10 : 4) / 3e6 + 2.0 * m * n * k * batch * (wide ? 6 : 1) / 5e8;
+  const double sums = wide ? static_cast<double>(m) * n * batch * ((k + 255) / 256) * 8 : 0.0;
+  return 19.0 + (values * (wide ? 10 : 4) + sums) / 3e6 + 2.0 * m * n * k * batch * (wide ? 6 : 1) / 5e8;
 }
 
 // 0: FFMA, 1: planes, as for every large problem, 2: planes where FFMA is slower, with FFMA behind them for what has none
