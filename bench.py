@@ -585,8 +585,8 @@ def attention_arm(args) -> dict | None:
 # ======================================================================================= fp32 GEMM
 def gemm32_arm(args) -> dict | None:
     """fp32 GEMM 1024 x 1024 x 1024 (the reference's own CPU-runnable case). The device forms the product
-    on the tensor cores from three bf16 planes per operand (six partial products side by side along k, one GEMM
-    launch). The L2 is flushed between steps because the 12.6 MB of operands would otherwise stay cached."""
+    on the tensor cores from three bf16 planes per operand (six products of planes in one accumulator; k in two
+    pieces and a launch that adds them). The L2 is flushed between steps because the 12.6 MB of operands would otherwise stay cached."""
     D = Dist()
     torch = D.torch
     from ytensor_b200 import _lib, api
@@ -639,7 +639,7 @@ def gemm32_arm(args) -> dict | None:
         "vs_baseline": None, "dtype": "f32 (three bf16 planes per operand, fp32 accumulate)", "data": "synthetic",
         "config": {"workload": "configs[0]: fp32 GEMM 1024 x 1024 x 1024", "l2": "flushed between steps (192 MB write)"},
         "roofline": {"bound": "tensor", "achieved": val, "peak": peak, "unit": "TFLOP/s", "frac": val / peak,
-                     "traffic": None, "kernel": "gemm_split3_kernel (one launch for both operands) + gemm_tc kernel over k' = 6 k, queued as dependent launches",
+                     "traffic": None, "kernel": "gemm_planes_kernel (one launch for both operands) + gemm_tc_kernel over six pairs of planes, k in pieces + gemm_sum_kernel, queued as dependent launches",
                      "peak_source": f"{peaks['source']} (burst cuBLAS bf16 / 6 partial products)",
                      "algorithmic_flops_per_launch": flops},
         "ffma_kernel": {"ms_per_step": res["ffma"][0], "tflops": flops / (res["ffma"][0] * 1e-3) / 1e12},

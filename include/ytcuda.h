@@ -78,11 +78,17 @@ int64_t ytcuda_get_wait_limit(void);
  * NULL) receives the cycles spent. No counterpart in the reference. */
 int ytcuda_wait_probe(int64_t* waited_cycles_dev, void* stream);
 
-/* Scratch memory. The entry points that need scratch beyond their inputs and outputs (fp32 GEMM on the tensor cores,
- * long reductions, attention over a KV cache split over keys, the decoder's split-k linears) take it from a buffer the
- * library keeps per (device, stream), grown with stream-ordered allocation on the caller's stream: calls on different
- * streams never share scratch, and growing does not synchronise the device. Such a call may therefore allocate; make
- * the first call of each kind outside any stream capture. ytcuda_reduce_noalloc is the form that never allocates. */
+/* Scratch memory. The entry points that need scratch beyond their inputs and outputs (GEMM of rewritten operands or with
+ * k in pieces, long reductions, fp32 attention, attention over a KV cache split over keys, the decoder's split-k linears)
+ * take it from a buffer the library keeps per (device, stream), grown with stream-ordered allocation on the caller's
+ * stream: calls on different streams never share scratch, threads that use one stream queue such calls one after the
+ * other, and growing does not synchronise the device. A buffer above 256 MB is handed back when its call has been queued.
+ * Such a call may therefore allocate; make the first call of each kind outside any stream capture. Products and attention
+ * that can do without scratch do so where none is to be had, and
+ * under a stream capture: fp32 attention, fp32 products that are small or odd (below: ytcuda_gemm_set_f32_mode) and 16-bit
+ * products of odd sizes or strides run on the FFMA kernels there, 16-bit products take k in one piece. A replayed graph
+ * then has the FFMA kernels' speed, and its sums are in another order than the eager call's.
+ * ytcuda_reduce_noalloc is the form that never allocates. */
 
 /* ---------------------------------------------------------------- GEMM
  * C[b] = alpha * A[b] . B[b] + beta * C[b],  A [m,k], B [k,n], C [m,n], b in [0,batch).
@@ -93,7 +99,9 @@ int ytcuda_wait_probe(int64_t* waited_cycles_dev, void* stream);
  * dtype_in in {F32, BF16, F16}; accumulation is fp32; C is rounded to dtype_out with the
  * reference's own conversion (yt::bfloat16 / yt::float16 constructors).
  * BF16/F16 inputs run on tcgen05 when each operand has a unit stride along one of its two
- * axes and 16-byte aligned rows; every other layout, and F32, runs on the FFMA kernel. */
+ * axes and 16-byte aligned rows; other layouts are rewritten for it where that is faster and
+ * the result has 16 bits, F32 runs there as bf16 planes (ytcuda_gemm_set_f32_mode); what is
+ * left runs on the FFMA kernel. */
 int ytcuda_gemm(int dtype_in, int dtype_out, const void* A, const void* B, void* C, int m, int n, int k,
                 float alpha, float beta, int64_t rsa, int64_t csa, int64_t rsb, int64_t csb, int64_t rsc,
                 int64_t csc, int64_t batch, int64_t bsa, int64_t bsb, int64_t bsc, void* stream);
@@ -104,13 +112,16 @@ int ytcuda_gemm(int dtype_in, int dtype_out, const void* A, const void* B, void*
 int ytcuda_gemm_set_path(int path);
 /* fp32 products (sgemm, include/kernel/avx2/sgemm.hpp:51-63) on the tensor cores: each operand is split into three
  * bfloat16 planes (24 mantissa bits) and the six partial products that matter at fp32 precision are accumulated in fp32
- * by one bf16 GEMM. Every finite input is represented exactly (values next to
- * the largest float included). One deviation from sgemm: an INFINITE operand gives NaN in the outputs it reaches
- * (its top plane meets zero or opposite-signed lower planes of the other operand) where sgemm gives the infinity;
- * NaN inputs give NaN in both. Callers that rely on infinities select mode 1. (Products that are smaller or odd, but large
- * enough for the planes to be faster, are checked on the device: an infinity or NaN leaves them to the FFMA kernel.)
- * 0 = automatic (m, n, k >= 256 with n and k multiples of 8; otherwise where FFMA is slower), 1 = never (FFMA kernel), 2 = whenever n and k
- * are multiples of 8. Process-wide, meant for tests; no counterpart in the reference. */
+ * by one bf16 GEMM. Every finite input of 2^-110 and above is represented exactly (values next to the largest float
+ * included); below that the last planes lie under bf16's smallest number and bits are lost. Two deviations from sgemm: an
+ * INFINITE operand gives NaN in the outputs it reaches (its top plane meets zero or opposite-signed lower planes of the
+ * other operand) where sgemm gives the infinity, and so may a finite product that overflows; NaN inputs give NaN in both.
+ * Callers that rely on infinities, or multiply numbers below 2^-110, select mode 1.
+ * Products that are smaller or odd, but large enough for the planes to be faster, are checked on the device: an infinity,
+ * NaN or number below 2^-110 (other than zero) in an operand leaves them to the FFMA kernel, a result that is not finite
+ * leaves its 128 x 128 tile to it.
+ * 0 = automatic (m, n, k >= 256 with n and k multiples of 8; otherwise where FFMA is slower), 1 = never (FFMA kernel),
+ * 2 = whenever n and k are multiples of 8. Process-wide, meant for tests; no counterpart in the reference. */
 int ytcuda_gemm_set_f32_mode(int mode);
 
 /* Tuning knobs of the tcgen05 kernel. a_prefetch_kblocks: how many 64-wide k-blocks an L2 prefetch of the
@@ -264,8 +275,12 @@ int ytcuda_swiglu(int dt_in, int dt_out, const void* gate_up, void* out, int64_t
  * make_causal_mask uses causal_offset = kv_len - q_len, qwen3.cpp:46-55); 2: bool mask bytes [q_len, kv_len] with
  * row stride mask_row_stride. bias: optional fp32 [q_len, kv_len] added to the scaled scores. A query row that sees
  * no key yields zeros (src/kernel/avx2/flash_attention.inl:241-244,327-331).
- * BF16 / F16 with head_dim == value_dim in {64, 128} and 16-byte aligned rows run on the tcgen05 kernel; every other
- * case (F32 included) runs on the one-warp-per-row kernel.
+ * BF16 / F16 with head_dim == value_dim in {64, 128} and 16-byte aligned rows run on the tcgen05 kernel. F32, and 16 bits
+ * with other head sizes up to 128, keep fp32 products: few query rows per K/V head on the decode kernels, more on tcgen05 from
+ * bf16 planes (rows of whole 16-byte groups of four, enough keys to pay), else on the tiled FFMA kernels, heads above 128 on
+ * the one-warp-per-row kernel. The planes leave a call to the tiled FFMA kernels if Q, K or V holds an infinity, NaN, 2^127
+ * or more, or (F32) a number below 2^-110 other than zero, or if a row comes out not finite; of scores that overflow
+ * to -infinity under a mask or bias a row that has no other key comes out as zeros.
  * Replaces yt::function::scaledDotProductAttention (include/function/ops.hpp:26-70, src/function/ops.inl:109-234,
  * 368-503) and yt::kernel::avx2::flash_attention (include/kernel/avx2/flash_attention.hpp:21-69). */
 int ytcuda_flash_attn_fwd(int dtype, const void* Q, const void* K, const void* V, void* O, int batch, int kv_heads,
@@ -275,8 +290,8 @@ int ytcuda_flash_attn_fwd(int dtype, const void* Q, const void* K, const void* V
                           int64_t mask_row_stride, const float* bias, int64_t bias_row_stride, int64_t bias_col_stride,
                           void* stream);
 
-/* Kernel choice of ytcuda_flash_attn_fwd: 0 = automatic, 1 = always the one-warp-per-row kernel, 2 = tcgen05 or
- * YTC_UNSUPPORTED. The counterpart of the per-call sdpaBackend argument (include/function/ops.hpp:21-24). */
+/* Kernel choice of ytcuda_flash_attn_fwd: 0 = automatic, 1 = always the FFMA kernels, 2 = the 16-bit tcgen05 kernel
+ * or YTC_UNSUPPORTED. The counterpart of the per-call sdpaBackend argument (include/function/ops.hpp:21-24). */
 int ytcuda_attn_set_path(int path);
 
 /* ---------------------------------------------------------------- decoder (Qwen3 block structure)
