@@ -1321,12 +1321,14 @@ __global__ void __launch_bounds__(256) gemm_sum_kernel(const float* part, int sp
   dependent_trigger();
   bool bad = false;
   for (int64_t t = blockIdx.x * 256ll + threadIdx.x; t < total; t += gridDim.x * 256ll) {
-    const int64_t row = t / n, col = t - row * n;
+    // (64-bit divisions took most of the kernel: 2048 x 2500, four pieces, 81 us under the profiler)
+    const int64_t row = total <= 0xffffffffll ? static_cast<uint32_t>(t) / static_cast<uint32_t>(n) : t / n, col = t - row * n;
     const float* from = part + row * ldp + col;
     float v = 0.f;
 #pragma unroll 8
     for (int s = 0; s < splits; ++s) v += from[s * stride];
-    const int64_t b = row / m, at = b * bsc + (row - b * m) * rsc + col * csc;
+    const int64_t b = row < m ? 0 : total <= 0xffffffffll ? static_cast<uint32_t>(row) / static_cast<uint32_t>(m) : row / m;
+    const int64_t at = b * bsc + (row - b * m) * rsc + col * csc;
     v *= alpha;
     if (beta != 0.f) v += beta * load_as_f32(C, at, dt);
     store_from_f32(C, at, v, dt);
