@@ -114,6 +114,41 @@ def test_single_kernel_decode_step_matches_operator_path(Q, B):
         m.close()
 
 
+@pytest.mark.parametrize("B,heads,kv_heads,inter,prompt,steps", [
+    (5, 4, 2, 2816, 30, 4), (8, 4, 4, 256, 1, 2), (9, 8, 2, 768, 62, 4), (16, 4, 2, 2048, 95, 3), (17, 16, 8, 512, 31, 3),
+    (32, 16, 8, 3072, 63, 3), (31, 8, 8, 1536, 128, 2)])
+def test_layers_in_one_kernel_match_operator_path(Q, B, heads, kv_heads, inter, prompt, steps):
+    """decode_wide_kernel (5 .. 32 sequences) against one launch per operator: group sizes 1, 2 and 4; one attention unit per
+    CTA, one per half of it, and several in a row; caches that end inside, at and behind a chunk of 32 keys, and an empty one;
+    feed-forwards whose tiles have 24, 44, 48 and 64 gate rows. Both carry activations as two bf16 planes and sum in fp32:
+    they differ by the order of the sums."""
+    cfg = Q.Qwen3Config(hidden_size=256 if heads < 16 else 1024, num_hidden_layers=3, vocab_size=500, intermediate_size=inter,
+                        num_attention_heads=heads, num_key_value_heads=kv_heads, head_dim=128, max_position_embeddings=160)
+    w = Q.random_weights(cfg, seed=21, std=0.05)
+    ids = dev_ids(np.random.default_rng(B).integers(0, cfg.vocab_size, (B, prompt + steps)))
+    a, b = Q.Qwen3ForCausalLM(cfg, batch=B), Q.Qwen3ForCausalLM(cfg, batch=B)
+    count = Q._lib.lib().ytcuda_launch_count
+    for m in (a, b):
+        m.load_weights(w)
+    a.set_decode_path(1)
+    for first in (0, prompt):  # from an empty cache, then behind the prompt
+        for m in (a, b):
+            m.reset_kv_cache()
+            if first:
+                m.forward(ids[:, :first].contiguous())
+        for t in range(first, first + steps):
+            tok = ids[:, t:t + 1].contiguous()
+            n0 = count()
+            want = a.forward(tok).cpu().numpy()
+            n1 = count()
+            got = b.forward(tok).cpu().numpy()
+            assert count() - n1 < 8 < n1 - n0
+            assert normwise(got, want) < 2e-5, (first, t)
+    assert Q._lib.lib().ytcuda_device_status(None) == 0
+    a.close()
+    b.close()
+
+
 def test_long_prefill_uses_tensor_cores_and_matches_oracle(Q, port):
     """More than 32 rows: activations are split into two bf16 planes and multiplied on tcgen05."""
     cfg = Q.Qwen3Config(**SMALL)
