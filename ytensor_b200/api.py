@@ -8,7 +8,7 @@ function calls the C ABI of libytensor_cuda.so; nothing here computes with torch
 from __future__ import annotations
 
 import builtins
-import ctypes as C
+import struct
 
 import torch
 
@@ -16,6 +16,13 @@ from . import _lib
 from ._lib import BF16, F16, F32, check, lib
 
 _DT = {torch.float32: F32, torch.bfloat16: BF16, torch.float16: F16}
+
+
+# What a call costs on the host is most of what a small operator costs (the kernels take 2 us): shapes and strides go to the
+# library as packed bytes, results are allocated once, broadcasting is arithmetic on the strides instead of views, and the
+# stream is asked for as a number. bias [1024] added to [7, 1024]: 33 us a call before, see the table of cases.
+_PACK64 = [struct.Struct(f"{n}q").pack for n in range(65)]
+_PACK32 = [struct.Struct(f"{n}i").pack for n in range(65)]
 
 
 def _dt(t: torch.Tensor) -> int:
@@ -26,7 +33,7 @@ def _dt(t: torch.Tensor) -> int:
 
 
 def _stream() -> int:
-    return torch.cuda.current_stream().cuda_stream
+    return torch._C._cuda_getCurrentRawStream(torch._C._cuda_getDevice())
 
 
 def _require_cuda(*ts: torch.Tensor) -> None:
@@ -35,10 +42,32 @@ def _require_cuda(*ts: torch.Tensor) -> None:
             raise _lib.YtCudaInvalidArgument(_lib.INVALID_ARG, "device backend: tensor is not on a CUDA device")
 
 
-def _batch_view(t: torch.Tensor):
-    """Splits a [..., r, c] view into (batch_count, batch_stride) if the leading dims collapse
-    into one stride; returns None otherwise."""
-    lead_shape, lead_stride = t.shape[:-2], t.stride()[:-2]
+def _broadcast(a: torch.Tensor, b: torch.Tensor):
+    """Common shape of a and b, and the strides with which each of them is read in it (torch's expand)."""
+    sa, sb, ta, tb = tuple(a.shape), tuple(b.shape), a.stride(), b.stride()
+    if sa == sb:
+        return sa, ta, tb
+    na, nb = len(sa), len(sb)
+    if nb <= na and sa[na - nb:] == sb:
+        return sa, ta, (0,) * (na - nb) + tb
+    n = na if na > nb else nb
+    shape, xa, xb = [0] * n, [0] * n, [0] * n
+    for i in range(1, n + 1):
+        x = sa[na - i] if i <= na else 1
+        y = sb[nb - i] if i <= nb else 1
+        if x != y and x != 1 and y != 1:
+            torch.broadcast_shapes(sa, sb)  # (raises, with the sizes)
+        size = y if x == 1 else x
+        shape[n - i] = size
+        if i <= na and x == size:
+            xa[n - i] = ta[na - i]
+        if i <= nb and y == size:
+            xb[n - i] = tb[nb - i]
+    return tuple(shape), tuple(xa), tuple(xb)
+
+
+def _batch_view(lead_shape, lead_stride):
+    """(batch count, batch stride) if the leading dims collapse into one stride; None otherwise."""
     dims = [(n, s) for n, s in zip(lead_shape, lead_stride) if n != 1]
     if not dims:
         return 1, 0
@@ -58,37 +87,55 @@ def matmul(a: torch.Tensor, b: torch.Tensor, out: torch.Tensor | None = None, *,
     `a` must equal the second-to-last of `b` or std::invalid_argument (here ValueError) is raised.
     One batched launch replaces the reference's per-matrix loop (:1035-1049).
     """
+    return _product(a, b, False, out, alpha, beta, out_dtype)
+
+
+def _product(a: torch.Tensor, b: torch.Tensor, turned: bool, out=None, alpha: float = 1.0, beta: float = 0.0,
+             out_dtype=None) -> torch.Tensor:
+    """matmul; turned: b holds [..., n, k]."""
     _require_cuda(a, b, out)
-    if a.dim() < 1 or b.dim() < 1:
+    sa, sb, ta, tb = tuple(a.shape), tuple(b.shape), a.stride(), b.stride()
+    if not sa or not sb:
         raise _lib.YtCudaInvalidArgument(_lib.INVALID_ARG, "matmul: operands must have at least 1 dim")
-    a2 = a if a.dim() >= 2 else a.unsqueeze(0)
-    b2 = b if b.dim() >= 2 else b.unsqueeze(-1)
-    if a2.shape[-1] != b2.shape[-2]:
-        raise _lib.YtCudaInvalidArgument(
-            _lib.INVALID_ARG, f"matmul: inner dims differ ({a2.shape[-1]} vs {b2.shape[-2]})")
-    if a2.dtype != b2.dtype:
+    if len(sa) == 1:
+        sa, ta = (1, *sa), (sa[0] * ta[0], *ta)
+    if len(sb) == 1:
+        sb, tb = (*sb, 1), (*tb, 1)
+    m, k = sa[-2:]
+    ra, ca = ta[-2:]
+    if turned:
+        n, kb = sb[-2:]
+        cb, rb = tb[-2:]
+    else:
+        kb, n = sb[-2:]
+        rb, cb = tb[-2:]
+    if k != kb:
+        raise _lib.YtCudaInvalidArgument(_lib.INVALID_ARG, f"matmul: inner dims differ ({k} vs {kb})")
+    dt = a.dtype
+    if dt != b.dtype:
         raise _lib.YtCudaInvalidArgument(_lib.INVALID_ARG, "matmul: operand dtypes differ")
-    m, k = a2.shape[-2:]
-    n = b2.shape[-1]
-    bshape = torch.broadcast_shapes(a2.shape[:-2], b2.shape[:-2])
-    ae = a2.expand(*bshape, m, k)
-    be = b2.expand(*bshape, k, n)
-    odt = out_dtype or a2.dtype
+    la, lb = sa[:-2], sb[:-2]
+    if la == lb or not lb:
+        lead, xa, xb = la, ta[:-2], tb[:-2] if lb else (0,) * len(la)
+    elif not la:
+        lead, xa, xb = lb, (0,) * len(lb), tb[:-2]
+    else:
+        lead = torch.broadcast_shapes(la, lb)
+        xa, xb = a.reshape(sa).expand(*lead, m, k).stride()[:-2], b.reshape(sb).expand(*lead, *sb[-2:]).stride()[:-2]
     if out is None:
-        out = torch.empty(*bshape, m, n, dtype=odt, device=a.device)
-    elif tuple(out.shape) != (*bshape, m, n):
+        out = torch.empty(*lead, m, n, dtype=out_dtype or dt, device=a.device)
+    elif tuple(out.shape) != (*lead, m, n):
         raise _lib.YtCudaInvalidArgument(_lib.INVALID_ARG, "matmul: out has the wrong shape")
-    av, bv, ov = _batch_view(ae), _batch_view(be), _batch_view(out)
-    L = lib()
+    to = out.stride()
+    av, bv, ov = (_batch_view(lead, x) for x in (xa, xb, to[:-2])) if lead else ((1, 0),) * 3
     if av is not None and bv is not None and ov is not None:
-        batch = builtins.max(av[0], bv[0], ov[0])
-        check(L.ytcuda_gemm(_dt(ae), _dt(out), ae.data_ptr(), be.data_ptr(), out.data_ptr(), m, n, k, alpha, beta,
-                            ae.stride(-2), ae.stride(-1), be.stride(-2), be.stride(-1), out.stride(-2),
-                            out.stride(-1), batch, av[1], bv[1], ov[1], _stream()))
+        check(lib().ytcuda_gemm(_dt(a), _dt(out), a.data_ptr(), b.data_ptr(), out.data_ptr(), m, n, k, alpha, beta, ra, ca,
+                                rb, cb, to[-2], to[-1], builtins.max(av[0], bv[0], ov[0]), av[1], bv[1], ov[1], _stream()))
     else:
         # Leading dims that do not collapse into one stride: one call per outermost slice.
-        for idx in range(bshape[0]):
-            matmul(ae[idx], be[idx], out[idx], alpha=alpha, beta=beta)
+        ae, be = a.reshape(sa).expand(*lead, m, k), b.reshape(sb).expand(*lead, *sb[-2:])
+        for idx in range(lead[0]):
+            _product(ae[idx], be[idx], turned, out[idx], alpha, beta)
     return out
 
 
@@ -134,7 +181,7 @@ def masked_matmul(a: torch.Tensor, b: torch.Tensor, mask, masked_value: float = 
     bshape = torch.broadcast_shapes(a.shape[:-2], b.shape[:-2])
     ae, be = a.expand(*bshape, m, k), b.expand(*bshape, k, n)
     out = torch.empty(*bshape, m, n, dtype=out_dtype or a.dtype, device=a.device)
-    av, bv, ov = _batch_view(ae), _batch_view(be), _batch_view(out)
+    av, bv, ov = (_batch_view(t.shape[:-2], t.stride()[:-2]) for t in (ae, be, out))
     if av is None or bv is None or ov is None:
         for idx in range(bshape[0]):
             out[idx] = masked_matmul(ae[idx], be[idx], mask, masked_value, out_dtype=out_dtype)
@@ -155,40 +202,44 @@ def masked_matmul(a: torch.Tensor, b: torch.Tensor, mask, masked_value: float = 
 
 def linear(x: torch.Tensor, weight: torch.Tensor, bias: torch.Tensor | None = None) -> torch.Tensor:
     """x . weight^T (+ bias), weight [out_features, in_features] (reference src/function/ops.inl:84-105)."""
-    y = matmul(x, weight.transpose(-1, -2))
+    y = _product(x, weight, True) if weight.dim() >= 2 else matmul(x, weight.transpose(-1, -2))
     if bias is not None:
         add_(y, bias)
     return y
 
 
 # ------------------------------------------------------------------ N-d helpers
-def _i64(vals):
-    return (C.c_int64 * len(vals))(*[int(v) for v in vals])
+def _i64(vals) -> bytes:
+    return _PACK64[len(vals)](*vals)
 
 
-def _i32(vals):
-    return (C.c_int * len(vals))(*[int(v) for v in vals])
+def _i32(vals) -> bytes:
+    return _PACK32[len(vals)](*vals)
 
 
 def _axes(axes) -> list[int]:
-    return [int(axes)] if isinstance(axes, int) else [int(a) for a in axes]
+    return [axes] if type(axes) is int else [int(axes)] if isinstance(axes, int) else [int(a) for a in axes]
 
 
 def _nd(t: torch.Tensor):
-    if t.dim() == 0:
-        t = t.reshape(1)
-    return t, _i64(t.shape), _i64(t.stride())
+    """(dims, shape, strides) as the library takes them; a scalar counts as one element."""
+    n = t.dim()
+    return (n, _i64(t.shape), _i64(t.stride())) if n else (1, _i64((1,)), _i64((1,)))
+
+
+def _like(x: torch.Tensor, dtype: torch.dtype | None = None) -> torch.Tensor:
+    return torch.empty_like(x, dtype=dtype, memory_format=torch.contiguous_format)
 
 
 # ------------------------------------------------------------------ softmax / norms
 def softmax(x: torch.Tensor, axes=-1, out: torch.Tensor | None = None) -> torch.Tensor:
     """Softmax jointly over `axes` (reference yt::function::softmax, src/function/activation.inl:336-375)."""
     _require_cuda(x, out)
-    y = torch.empty_like(x, memory_format=torch.contiguous_format) if out is None else out
+    y = _like(x) if out is None else out
     ax = _axes(axes)
-    xx, shape, xs = _nd(x)
+    nd, shape, xs = _nd(x)
     check(lib().ytcuda_softmax(_dt(x), _dt(y), x.data_ptr(), y.data_ptr(), shape, xs, _i64(y.stride() or (1,)),
-                               xx.dim(), _i32(ax), len(ax), _stream()))
+                               nd, _i32(ax), len(ax), _stream()))
     return y
 
 
@@ -208,11 +259,11 @@ def rmsNorm(x: torch.Tensor, weight: torch.Tensor | None, axes=-1, eps: float = 
         if list(weight.shape) != want:
             raise _lib.YtCudaInvalidArgument(_lib.INVALID_ARG, "rmsNorm: weight shape must match affine axes")
         weight = weight.contiguous()
-    y = torch.empty_like(x, memory_format=torch.contiguous_format) if out is None else out
-    xx, shape, xs = _nd(x)
+    y = _like(x) if out is None else out
+    nd, shape, xs = _nd(x)
     check(lib().ytcuda_rmsnorm(_dt(x), _dt(y), _dt(weight) if weight is not None else F32, x.data_ptr(),
                                weight.data_ptr() if weight is not None else None, y.data_ptr(), shape, xs,
-                               _i64(y.stride() or (1,)), xx.dim(), _i32(ax), len(ax), eps, _stream()))
+                               _i64(y.stride() or (1,)), nd, _i32(ax), len(ax), eps, _stream()))
     return y
 
 
@@ -233,12 +284,12 @@ def layerNorm(x: torch.Tensor, gamma: torch.Tensor | None = None, bias: torch.Te
         if list(gamma.shape) != want or list(bias.shape) != want:
             raise _lib.YtCudaInvalidArgument(_lib.INVALID_ARG, "layerNorm: gamma/bias shape must match affine axes")
         gamma, bias = gamma.contiguous(), bias.contiguous().to(gamma.dtype)
-    y = torch.empty_like(x, memory_format=torch.contiguous_format) if out is None else out
-    xx, shape, xs = _nd(x)
+    y = _like(x) if out is None else out
+    nd, shape, xs = _nd(x)
     check(lib().ytcuda_layernorm(_dt(x), _dt(y), _dt(gamma) if gamma is not None else F32, x.data_ptr(),
                                  gamma.data_ptr() if gamma is not None else None,
                                  bias.data_ptr() if bias is not None else None, y.data_ptr(), shape, xs,
-                                 _i64(y.stride() or (1,)), xx.dim(), _i32(ax), len(ax), eps, _stream()))
+                                 _i64(y.stride() or (1,)), nd, _i32(ax), len(ax), eps, _stream()))
     return y
 
 
@@ -273,23 +324,23 @@ def _affine_(y: torch.Tensor, gamma, bias, axes) -> torch.Tensor:
     return y
 
 
-def _channel_norm(x: torch.Tensor, y: torch.Tensor, axes, eps: float, whole: torch.Tensor, gamma, bias, channel: int,
+def _channel_norm(x: torch.Tensor, y: torch.Tensor, shape, xt, yt, axes, eps: float, gamma, bias, channel: int,
                   wstrides) -> torch.Tensor:
-    """layerNorm of x over `axes` into y, then gamma and bias of the channels of `whole` (axis `channel`; x and y may be
-    grouped views, `wstrides` says how far a step of each of their dims moves in gamma). One launch where the strides allow
-    it, else three."""
+    """layerNorm of x over `axes` into y, then gamma and bias of the channels (axis `channel`). x and y are read as
+    shape / xt and shape / yt, which may group the channels; `wstrides` says how far a step of each of those dims moves in
+    gamma. One launch where the strides allow it, else three."""
     if gamma is not None and bias is not None and gamma.is_cuda and bias.is_cuda:
-        _check_affine(whole, gamma, bias, [channel])
+        _check_affine(y, gamma, bias, [channel])
         _require_cuda(x, y)
         g, b = gamma.contiguous().to(y.dtype), bias.contiguous().to(y.dtype)
         rc = lib().ytcuda_layernorm_strided(_dt(x), _dt(y), _dt(y), x.data_ptr(), g.data_ptr(), b.data_ptr(), y.data_ptr(),
-                                            _i64(x.shape), _i64(x.stride()), _i64(y.stride()), _i64(wstrides), x.dim(),
-                                            _i32(axes), len(axes), eps, _stream())
+                                            _i64(shape), _i64(xt), _i64(yt), _i64(wstrides), len(shape), _i32(axes),
+                                            len(axes), eps, _stream())
         if rc != _lib.UNSUPPORTED:
             check(rc)
-            return whole
-    layerNorm(x, None, None, axes, eps, out=y)
-    return _affine_(whole, gamma, bias, [channel])
+            return y
+    layerNorm(x.as_strided(shape, xt), None, None, axes, eps, out=y.as_strided(shape, yt))
+    return _affine_(y, gamma, bias, [channel])
 
 
 def normalize(x: torch.Tensor, axes=-1, p: float = 2.0, eps: float = 1e-12, gamma=None, bias=None,
@@ -300,10 +351,10 @@ def normalize(x: torch.Tensor, axes=-1, p: float = 2.0, eps: float = 1e-12, gamm
     if p <= 0:
         raise _lib.YtCudaInvalidArgument(_lib.INVALID_ARG, "yt::function::normalize: p must be positive")
     ax = _axes(axes)
-    y = torch.empty_like(x, memory_format=torch.contiguous_format) if out is None else out
-    xx, shape, xs = _nd(x)
+    y = _like(x) if out is None else out
+    nd, shape, xs = _nd(x)
     check(lib().ytcuda_normalize(_dt(x), _dt(y), x.data_ptr(), y.data_ptr(), shape, xs, _i64(y.stride() or (1,)),
-                                 xx.dim(), _i32(ax), len(ax), float(p), float(eps), _stream()))
+                                 nd, _i32(ax), len(ax), float(p), float(eps), _stream()))
     return _affine_(y, gamma, bias, ax)
 
 
@@ -328,8 +379,8 @@ def instanceNorm(x: torch.Tensor, gamma=None, bias=None, channelAxis: int = 1, e
     axes = [a for a in range(x.dim()) if a not in (0, c)]
     if not axes:
         raise _lib.YtCudaInvalidArgument(_lib.INVALID_ARG, "yt::function::instanceNorm: requires at least one spatial axis")
-    y = torch.empty_like(x, memory_format=torch.contiguous_format) if out is None else out
-    return _channel_norm(x, y, axes, eps, y, gamma, bias, c, [int(a == c) for a in range(x.dim())])
+    y = _like(x) if out is None else out
+    return _channel_norm(x, y, x.shape, x.stride(), y.stride(), axes, eps, gamma, bias, c, [int(a == c) for a in range(x.dim())])
 
 
 def instanceNorm_(x, gamma=None, bias=None, channelAxis: int = 1, eps: float = 1e-5):
@@ -342,8 +393,8 @@ def batchNorm(x: torch.Tensor, gamma=None, bias=None, channelAxis: int = 1, eps:
     src/function/normalization.inl:435-489: statistics of the tensor itself, no running averages)."""
     c = _channel_axis(x, channelAxis, "yt::function::batchNorm_")
     axes = [a for a in range(x.dim()) if a != c]
-    y = torch.empty_like(x, memory_format=torch.contiguous_format) if out is None else out
-    return _channel_norm(x, y, axes, eps, y, gamma, bias, c, [int(a == c) for a in range(x.dim())])
+    y = _like(x) if out is None else out
+    return _channel_norm(x, y, x.shape, x.stride(), y.stride(), axes, eps, gamma, bias, c, [int(a == c) for a in range(x.dim())])
 
 
 def batchNorm_(x, gamma=None, bias=None, channelAxis: int = 1, eps: float = 1e-5):
@@ -365,11 +416,16 @@ def groupNorm(x: torch.Tensor, groups: int, gamma=None, bias=None, channelAxis: 
                                          "yt::function::groupNorm: channel count must be divisible by groups")
     if x.dim() + 1 > 8:
         raise _lib.YtCudaInvalidArgument(_lib.UNSUPPORTED, "groupNorm: at most 7 dims")
-    y = torch.empty_like(x, memory_format=torch.contiguous_format) if out is None else out
-    xg = x.movedim(c, 1).unflatten(1, (groups, ch // groups))
-    yg = y.movedim(c, 1).unflatten(1, (groups, ch // groups))
-    ws = [0, ch // groups, 1] + [0] * (xg.dim() - 3)
-    return _channel_norm(xg, yg, list(range(2, xg.dim())), eps, y, gamma, bias, c, ws)
+    y = _like(x) if out is None else out
+    per = ch // groups  # the channel axis in two: [n, groups, per, the other axes in their order]
+
+    def grouped(v, split):
+        return [v[0], *split(v[c]), *(v[a] for a in range(1, len(v)) if a != c)]
+
+    shape = grouped(x.shape, lambda _: (groups, per))
+    xt, yt = (grouped(t.stride(), lambda st: (st * per, st)) for t in (x, y))
+    ws = [0, per, 1] + [0] * (len(shape) - 3)
+    return _channel_norm(x, y, shape, xt, yt, list(range(2, len(shape))), eps, gamma, bias, c, ws)
 
 
 def groupNorm_(x, groups: int, gamma=None, bias=None, channelAxis: int = 1, eps: float = 1e-5):
@@ -397,14 +453,14 @@ def rmsnorm_add_softmax_cast(x: torch.Tensor, weight: torch.Tensor, residual: to
 def _reduce(op: int, x: torch.Tensor, axes, want_index: bool):
     _require_cuda(x)
     ax = _axes(axes)
-    xx, shape, xs = _nd(x)
-    ks = list(xx.shape)
+    nd, shape, xs = _nd(x)
+    ks = list(x.shape) or [1]
     for a in ax:
-        ks[a % xx.dim()] = 1
-    y = torch.empty(ks, dtype=x.dtype, device=x.device)
-    idx = torch.empty(ks, dtype=torch.int32, device=x.device) if want_index else None
+        ks[a % nd] = 1
+    y = torch.empty(*ks, dtype=x.dtype, device=x.device)
+    idx = torch.empty(*ks, dtype=torch.int32, device=x.device) if want_index else None
     check(lib().ytcuda_reduce(op, _dt(x), _dt(y), x.data_ptr(), y.data_ptr(), idx.data_ptr() if want_index else None,
-                              shape, xs, xx.dim(), _i32(ax), len(ax), _stream()))
+                              shape, xs, nd, _i32(ax), len(ax), _stream()))
     return (y, idx) if want_index else y
 
 
@@ -434,20 +490,16 @@ def _binary(op: str, a: torch.Tensor, b, out: torch.Tensor | None) -> torch.Tens
                       {"add": float(b), "sub": -float(b), "mul": float(b), "div": 1.0 / float(b)}[op])
     _require_cuda(a, b, out)
     try:
-        shape = torch.broadcast_shapes(a.shape, b.shape)
+        shape, xa, xb = _broadcast(a, b)
     except RuntimeError as e:  # std::runtime_error in the reference (src/kernel/broadcast.inl:133)
         raise _lib.YtCudaError(_lib.INVALID_ARG, f"broadcast mismatch: {e}")
     if out is None:
-        out = torch.empty(shape, dtype=a.dtype, device=a.device)
-    elif tuple(out.shape) != tuple(shape):
+        out = _like(a) if shape == a.shape else torch.empty(shape, dtype=a.dtype, device=a.device)
+    elif tuple(out.shape) != shape:
         raise _lib.YtCudaError(_lib.INVALID_ARG, "in-place operand cannot be broadcast to the result shape")
-    ae, be = a.expand(shape), b.expand(shape)
-    if len(shape) == 0:
-        ae, be, o = ae.reshape(1), be.reshape(1), out.reshape(1)
-    else:
-        o = out
-    check(lib().ytcuda_binary(_BIN[op], _dt(a), _dt(b), _dt(out), ae.data_ptr(), be.data_ptr(), o.data_ptr(), o.dim(),
-                              _i64(o.shape), _i64(ae.stride()), _i64(be.stride()), _i64(o.stride()), _stream()))
+    nd, osh, ost = _nd(out)
+    check(lib().ytcuda_binary(_BIN[op], _dt(a), _dt(b), _dt(out), a.data_ptr(), b.data_ptr(), out.data_ptr(), nd, osh,
+                              _i64(xa or (1,)), _i64(xb or (1,)), ost, _stream()))
     return out
 
 
@@ -465,12 +517,12 @@ def _unary(op: int, x: torch.Tensor, out: torch.Tensor | None, param: float = 0.
            out_dtype: torch.dtype | None = None) -> torch.Tensor:
     _require_cuda(x, out)
     if out is None:
-        out = torch.empty(x.shape, dtype=out_dtype or x.dtype, device=x.device)
-    elif tuple(out.shape) != tuple(x.shape):
+        out = _like(x, out_dtype)
+    elif out is not x and out.shape != x.shape:
         raise _lib.YtCudaInvalidArgument(_lib.INVALID_ARG, "unary: shape mismatch")
-    xx, oo = (x.reshape(1), out.reshape(1)) if x.dim() == 0 else (x, out)
-    check(lib().ytcuda_unary(op, _dt(x), _dt(out), xx.data_ptr(), oo.data_ptr(), xx.dim(), _i64(xx.shape),
-                             _i64(xx.stride()), _i64(oo.stride()), param, _stream()))
+    nd, shape, xs = _nd(x)
+    check(lib().ytcuda_unary(op, _dt(x), _dt(out), x.data_ptr(), out.data_ptr(), nd, shape, xs, _i64(out.stride() or (1,)),
+                             param, _stream()))
     return out
 
 
@@ -524,8 +576,7 @@ for _n, _op in _ACTIVATIONS.items():
 def cast(x: torch.Tensor, dtype: torch.dtype) -> torch.Tensor:
     """dtype conversion with the reference's rounding (YTensorBase::cast, include/ytensor_base.hpp:399-404)."""
     _require_cuda(x)
-    out = torch.empty(x.shape, dtype=dtype, device=x.device)
-    return copy_(out, x)
+    return copy_(_like(x, dtype), x)
 
 
 FP8_KINDS = {"float8_e5m2": _lib.F8_E5M2, "float8_e4m3": _lib.F8_E4M3, "float8_e8m0": _lib.F8_E8M0}
@@ -560,11 +611,11 @@ def cast_from_fp8(bits: torch.Tensor, kind: str, dtype: torch.dtype = torch.floa
 def copy_(dst: torch.Tensor, src: torch.Tensor) -> torch.Tensor:
     """Strided copy with conversion (YTensorBase::copy_, src/ytensor_base.inl:257-430)."""
     _require_cuda(dst, src)
-    if tuple(dst.shape) != tuple(src.shape):
+    if dst.shape != src.shape:
         raise _lib.YtCudaInvalidArgument(_lib.INVALID_ARG, "copy_: shape mismatch")
-    d, s_ = (dst.reshape(1), src.reshape(1)) if dst.dim() == 0 else (dst, src)
-    check(lib().ytcuda_cast(_dt(src), _dt(dst), s_.data_ptr(), d.data_ptr(), d.dim(), _i64(d.shape), _i64(s_.stride()),
-                            _i64(d.stride()), _stream()))
+    nd, shape, ds = _nd(dst)
+    check(lib().ytcuda_cast(_dt(src), _dt(dst), src.data_ptr(), dst.data_ptr(), nd, shape, _i64(src.stride() or (1,)), ds,
+                            _stream()))
     return dst
 
 
@@ -597,7 +648,7 @@ def swiglu(gate_up: torch.Tensor, out_dtype: torch.dtype | None = None) -> torch
     if gate_up.stride(-1) != 1 or gate_up.shape[-1] % 2:
         raise _lib.YtCudaInvalidArgument(_lib.INVALID_ARG, "swiglu: last dim must be contiguous and even")
     inter = gate_up.shape[-1] // 2
-    g2 = gate_up.reshape(-1, 2 * inter)
+    g2 = gate_up if gate_up.dim() == 2 else gate_up.reshape(-1, 2 * inter)
     out = torch.empty(*gate_up.shape[:-1], inter, dtype=out_dtype or gate_up.dtype, device=gate_up.device)
     check(lib().ytcuda_swiglu(_dt(g2), _dt(out), g2.data_ptr(), out.data_ptr(), g2.shape[0], inter, g2.stride(0), inter,
                               _stream()))
@@ -661,7 +712,8 @@ def scaledDotProductAttention(query: torch.Tensor, key: torch.Tensor, value: tor
         if tuple(mask.shape) != (lq, lk):
             raise _lib.YtCudaInvalidArgument(
                 _lib.INVALID_ARG, "Mask shape must match the last two dimensions of the score tensor.")
-        m8 = mask.to(torch.uint8) if mask.dtype != torch.uint8 else mask
+        # (a bool is a byte of 0 or 1: read as it lies)
+        m8 = mask if mask.dtype == torch.uint8 else mask.view(torch.uint8) if mask.dtype == torch.bool else mask.to(torch.uint8)
         m8 = m8.contiguous()
         mask_kind, mptr, mrs = 2, m8.data_ptr(), m8.stride(0)
     elif causal:
@@ -673,9 +725,9 @@ def scaledDotProductAttention(query: torch.Tensor, key: torch.Tensor, value: tor
                 _lib.INVALID_ARG, "Bias shape must match the last two dimensions of the score tensor.")
         bias = bias.float()
         bptr, brs, bcs = bias.data_ptr(), bias.stride(0), bias.stride(1)
-    out = torch.empty(b, kvh * g, lq, dv, dtype=query.dtype, device=query.device)
+    out = torch.empty(*out_shape, dtype=query.dtype, device=query.device)  # ([b, heads, q_len, dv], whatever the leading dims)
     check(lib().ytcuda_flash_attn_fwd(_dt(q), q.data_ptr(), k.data_ptr(), v.data_ptr(), out.data_ptr(), b, kvh, g, lq,
                                       lk, d, dv, float(scale), _i64(q.stride()[:3]), _i64(k.stride()[:3]),
-                                      _i64(v.stride()[:3]), _i64(out.stride()[:3]), mask_kind, off, mptr, mrs, bptr,
-                                      brs, bcs, _stream()))
-    return out.reshape(out_shape)
+                                      _i64(v.stride()[:3]), _i64((kvh * g * lq * dv, lq * dv, dv)), mask_kind, off, mptr, mrs,
+                                      bptr, brs, bcs, _stream()))
+    return out
