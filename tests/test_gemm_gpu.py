@@ -561,3 +561,24 @@ def test_threads_share_a_stream(api):
     for t in threads:
         t.join()
     assert not torch.stack(bad).any()
+
+
+@pytest.mark.parametrize("out_dtype", [torch.float32, torch.bfloat16, torch.float16])
+@pytest.mark.parametrize("b,m,n,k", [(1, 1, 8, 72), (1, 33, 24, 64), (3, 127, 136, 200), (1, 129, 264, 72), (2, 160, 520, 136),
+                                     (1, 4097, 1032, 264), (2, 2304, 1288, 256)])
+def test_results_through_tma_stores(L, api, out_dtype, b, m, n, k):
+    """C whose rows start at 16 bytes leaves through TMA stores, other C through stores of the lanes: the same bits, and nothing
+    outside C, at the edges of tiles of both kernels."""
+    dt = torch.float16 if out_dtype == torch.float16 else torch.bfloat16
+    g = torch.Generator(device="cuda").manual_seed(m + n)
+    a, w = (torch.randn(s, generator=g, device="cuda").to(dt) for s in ((b, m, k), (k, n)))
+    got = []
+    for first in (8, 1):  # (an odd place in the row: no 16-byte rows)
+        whole = torch.full((b, m + 2, n + 16), 7.0, dtype=out_dtype, device="cuda")
+        api.matmul(a, w, whole[:, 1:m + 1, first:first + n])
+        got.append(whole[:, 1:m + 1, first:first + n].clone())
+        whole[:, 1:m + 1, first:first + n] = 7.0
+        assert bool((whole == 7.0).all())
+    assert torch.equal(got[0], got[1])
+    assert normwise(got[0].double().cpu().numpy(), (a.double() @ w.double()).cpu().numpy()) < (1e-5 if out_dtype == torch.float32 else H_TOL)
+    status_ok(L)

@@ -3,8 +3,8 @@
 //  * gemm_tc_kernel   : bf16 / fp16 inputs, fp32 accumulation in tensor memory. Persistent,
 //                       one CTA per SM, warp-specialised: warp 0 feeds a 4-stage shared-memory
 //                       ring with TMA, warp 1 issues tcgen05.mma (128 x BN x 16 per instruction),
-//                       warps 4-7 drain the accumulator (tcgen05.ld) and write C while the next
-//                       tile's MMAs run into the second accumulator stage.
+//                       warps 4-11 drain the accumulator (tcgen05.ld) and write C (TMA stores) while
+//                       the next tile's MMAs run into the second accumulator stage.
 //  * gemm_simt_kernel : any strides, any of {f32, bf16, f16}, FFMA with fp32 accumulation.
 //                       It is the fp32 path and the layout catch-all of the tensor-core path.
 //
@@ -22,7 +22,8 @@ namespace ytk {
 constexpr int TC_BM = 128;
 constexpr int TC_BK = 64;  // 64 x 16-bit = one 128-byte swizzle row
 constexpr int TC_STAGES = 4;
-constexpr int TC_THREADS = 256;
+constexpr int TC_EPI_WARPS = 8;  // two per quarter of the accumulator's lanes
+constexpr int TC_THREADS = 128 + 32 * TC_EPI_WARPS;
 
 struct GemmTcParams {
   int M, N, K;
@@ -48,7 +49,7 @@ struct GemmTcParams {
   const uint8_t* tile_live;
   // linear layers of the language models (LinearEpilogue, lm_ops.cuh)
   int epi;                 // EPI_NONE: the store rules above; otherwise tc_store_epilogue
-  int staged;              // linear layers with 16-byte aligned rows: stores go through tc_store_staged
+  int tma_out;             // C through TMA stores: 0 no, 1 yes, 2 added to what C holds (fp32)
   int act_cols;            // EPI_SILU
   float limit, alpha_gate, shift;  // EPI_CLAMP_PAIRS
   // grouped product: every 128-row block of A belongs to one group (expert) or to none (-1, passed over); group g
@@ -57,7 +58,7 @@ struct GemmTcParams {
   int group_rows;
 };
 
-constexpr int TC_OUT_BYTES = 32 * 128;  // staging area of an epilogue warp
+constexpr int TC_OUT_BYTES = 32 * 128;  // an epilogue warp's 32 rows of 128 bytes on their way to C
 template <int BN>
 struct TcSmem {
   static constexpr int A_BYTES = TC_BM * TC_BK * 2;
@@ -67,8 +68,8 @@ struct TcSmem {
   // full[STAGES], empty[STAGES], tmem_full[2], tmem_empty[2], tmem base word, abort word
   static constexpr int TOTAL = BAR_OFFSET + (2 * TC_STAGES + 4) * 8 + 16;
   static constexpr int DYN_BYTES = TOTAL + 1024;  // slack to align the ring to 1024 B
-  static constexpr int OUT_OFFSET = (TOTAL + 127) / 128 * 128;  // staged stores: the epilogue warps' areas
-  static constexpr int DYN_STAGED = OUT_OFFSET + 4 * TC_OUT_BYTES + 1024;
+  static constexpr int OUT_OFFSET = (TOTAL + 1023) / 1024 * 1024;  // TMA stores: the epilogue warps' areas
+  static constexpr int DYN_STAGED = OUT_OFFSET + TC_EPI_WARPS * TC_OUT_BYTES + 1024;
 };
 
 // Work item -> batch item of the operands, first and end k block; a product of planes counts its blocks pair by pair from 0
@@ -204,8 +205,11 @@ __device__ __forceinline__ void tc_activate(const GemmTcParams& p, const uint32_
   } else if (p.epi == EPI_SILU && gn0 + 32 <= p.act_cols) {
 #pragma unroll
     for (int j = 0; j < 16; ++j) w[j] = pack_bf16x2_rn(lm_silu_fast(at(2 * j)), lm_silu_fast(at(2 * j + 1)));
+  } else if (p.epi != EPI_SILU || gn0 >= p.act_cols) {
+#pragma unroll
+    for (int j = 0; j < 16; ++j) w[j] = pack_bf16x2_rn(at(2 * j), at(2 * j + 1));
   } else {
-    const int n = p.epi == EPI_SILU ? p.act_cols - gn0 : 0;  // (activated columns among these)
+    const int n = p.act_cols - gn0;  // (activated columns among these)
 #pragma unroll
     for (int j = 0; j < 16; ++j)
       w[j] = pack_bf16x2_rn(2 * j < n ? lm_silu_fast(at(2 * j)) : at(2 * j),
@@ -228,63 +232,78 @@ __device__ __forceinline__ void tc_store_epilogue(const GemmTcParams& p, const u
       dst[j] = static_cast<uint16_t>(w[j >> 1] >> ((j & 1) * 16));
 }
 
-// Store of a warp's 32 rows x 32 columns through its staging area, where a row's results gather until they fill 128 bytes;
-// then eight lanes write one row's 128 bytes (direct stores of 64 bytes per lane, a row apart, keep the epilogue behind the
-// products when k is short). buf: 32 rows of 128 bytes, 16-byte pieces exchanged by row against bank conflicts. base:
-// elements before the warp's first row, rows: how many of the 32 exist, tile_end: the tile's last column + 1.
-__device__ __forceinline__ void tc_store_staged(const GemmTcParams& p, const uint32_t (&r)[32], uint8_t* buf, int64_t base,
-                                                int rows, int gn0, int tile_end, int lane) {
-  const bool wide = p.epi == EPI_NONE, pairs = tc_pairs(p);  // (EPI_NONE: fp32 results)
-  const int esz = wide ? 4 : 2;
-  const int at = wide ? gn0 * 4 : pairs ? gn0 : gn0 * 2, bytes = wide ? 128 : pairs ? 32 : 64;  // within the output row
+// 32 columns of one row as ytcuda_gemm narrows them: 16 words of two 16-bit results.
+template <int OUT_DT>
+__device__ __forceinline__ void tc_narrow(const uint32_t (&r)[32], float alpha, uint32_t (&w)[16]) {
+#pragma unroll
+  for (int j = 0; j < 16; ++j) {
+    const float lo = alpha * __uint_as_float(r[2 * j]), hi = alpha * __uint_as_float(r[2 * j + 1]);
+    if constexpr (OUT_DT == YTC_BF16) w[j] = f32_to_bf16_bits_ref(lo) | (static_cast<uint32_t>(f32_to_bf16_bits_ref(hi)) << 16);
+    else w[j] = f32_to_f16_bits_ref(lo) | (static_cast<uint32_t>(f32_to_f16_bits_ref(hi)) << 16);
+  }
+}
+
+// A warp's share of an accumulator to C: every other group of columns that make 128 bytes of a row of C (32 fp32, 64 16-bit, 128
+// for gated pairs) is narrowed into the warp's 32 rows of 128 bytes, 16-byte pieces exchanged by row as the tensor map has them,
+// and leaves as one TMA store, which clips what lies outside C. Bound by the instructions of four schedulers: with one warp
+// on each, and 16-byte stores of its lanes, a 128 x 256 tile took 10.8 us (bf16; 6.2 with an activation that unrolled), more
+// than its MMAs for k below 2500; now 3.3. 4096 x 4096 x 1024 with nearest-even stores 53.6 -> 33.2 us, x 64 43.3 -> 13.2.
+// n0: C's column under the accumulator's first, m0: C's row under the warp's first, half: which of the groups.
+template <int BN>
+__device__ __forceinline__ void tc_drain(const GemmTcParams& p, const CUtensorMap* tmC, uint32_t t_row, uint8_t* buf, int n0, int m0,
+                                         int b, int half, int lane) {
+  if (m0 >= p.M) return;
+  const bool pairs = tc_pairs(p), wide = p.epi == EPI_NONE && p.out_dtype == YTC_F32;
+  const int cols = wide ? 32 : pairs ? 128 : 64;
   uint8_t* mine = buf + lane * 128;
-  const int piece0 = (at & 127) >> 4;
-  auto put = [&](int piece, uint32_t a, uint32_t b, uint32_t c, uint32_t d) {
-    *reinterpret_cast<uint4*>(mine + (((piece0 + piece) ^ (lane & 7)) << 4)) = make_uint4(a, b, c, d);
+  auto put = [&](int piece, uint32_t x, uint32_t y, uint32_t z, uint32_t w) {
+    *reinterpret_cast<uint4*>(mine + ((piece ^ (lane & 7)) << 4)) = make_uint4(x, y, z, w);
   };
-  if (wide) {
+#pragma unroll 1
+  for (int g = half * cols; g < BN && n0 + g < p.N; g += 2 * cols) {
+    if (lane == 0) tma_store_wait_read<0>();  // the rows of the store before this one have been read
+    __syncwarp();
+    int piece = 0;
+#pragma unroll 1
+    for (int c = 0; c < cols; c += 32) {
+      uint32_t r[32];
+      tmem_ld_32x32b_x32(t_row + g + c, r);
+      tmem_ld_wait();
+      if (wide) {
 #pragma unroll
-    for (int j = 0; j < 8; ++j) put(j, r[4 * j], r[4 * j + 1], r[4 * j + 2], r[4 * j + 3]);
-  } else {
-    uint32_t w[16];
-    tc_activate(p, r, gn0, w);
-    put(0, w[0], w[1], w[2], w[3]);
-    put(1, w[4], w[5], w[6], w[7]);
-    if (!pairs) {
-      put(2, w[8], w[9], w[10], w[11]);
-      put(3, w[12], w[13], w[14], w[15]);
+        for (int j = 0; j < 8; ++j)
+          put(j, __float_as_uint(p.alpha * __uint_as_float(r[4 * j])), __float_as_uint(p.alpha * __uint_as_float(r[4 * j + 1])),
+              __float_as_uint(p.alpha * __uint_as_float(r[4 * j + 2])), __float_as_uint(p.alpha * __uint_as_float(r[4 * j + 3])));
+        continue;
+      }
+      uint32_t w[16];
+      if (p.epi != EPI_NONE) tc_activate(p, r, n0 + g + c, w);
+      else if (p.out_dtype == YTC_BF16) tc_narrow<YTC_BF16>(r, p.alpha, w);
+      else tc_narrow<YTC_F16>(r, p.alpha, w);
+      put(piece, w[0], w[1], w[2], w[3]);
+      put(piece + 1, w[4], w[5], w[6], w[7]);
+      if (!pairs) {
+        put(piece + 2, w[8], w[9], w[10], w[11]);
+        put(piece + 3, w[12], w[13], w[14], w[15]);
+      }
+      piece += pairs ? 2 : 4;
+    }
+    fence_proxy_async_smem();
+    __syncwarp();
+    if (lane == 0) {
+      const int col = pairs ? (n0 + g) >> 1 : n0 + g;
+      if (p.tma_out == 2) tma_add_3d(tmC, buf, col, m0, b);
+      else tma_store_3d(tmC, buf, col, m0, b);
+      tma_store_commit();
     }
   }
-  if (((at + bytes) & 127) != 0 && gn0 + 32 < p.N && gn0 + 32 < tile_end) return;
-  __syncwarp();
-  const int seg = at & ~127, valid = at + bytes - seg;
-  const int row_bytes = (pairs ? p.N / 2 : p.N) * esz;
-  const int piece = lane & 7, to = seg + piece * 16;
-  char* out = static_cast<char*>(p.C) + base * esz + to;
-#pragma unroll
-  for (int i = 0; i < 8; ++i) {
-    const int row = i * 4 + (lane >> 3);
-    const uint4 v = *reinterpret_cast<const uint4*>(buf + row * 128 + ((piece ^ (row & 7)) << 4));
-    if (row >= rows || piece * 16 >= valid || to >= row_bytes) continue;
-    char* dst = out + static_cast<int64_t>(row) * p.rsc * esz;
-    if (to + 16 <= row_bytes) {
-      *reinterpret_cast<uint4*>(dst) = v;
-    } else {
-      const uint32_t words[4] = {v.x, v.y, v.z, v.w};
-#pragma unroll
-      for (int k = 0; k < 8; ++k)
-        if (to + 2 * k < row_bytes)
-          reinterpret_cast<uint16_t*>(dst)[k] = static_cast<uint16_t>(words[k >> 1] >> ((k & 1) * 16));
-    }
-  }
-  __syncwarp();
 }
 
 // PIECES: a product of planes, or k in pieces (the few instructions more cost an ordinary short product 0.2 us).
 template <int BN, bool PIECES>
 __global__ void __launch_bounds__(TC_THREADS, 1)
     gemm_tc_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ CUtensorMap tmB,
-                   const GemmTcParams p) {
+                   const __grid_constant__ CUtensorMap tmC, const GemmTcParams p) {
   using S = TcSmem<BN>;
   extern __shared__ uint8_t smem_raw[];
   // The 128-byte swizzle pattern is a function of the shared address: keep the ring 1024-byte aligned.
@@ -308,13 +327,14 @@ __global__ void __launch_bounds__(TC_THREADS, 1)
     }
     for (int s = 0; s < 2; ++s) {
       mbar_init(&tfull_bar[s], 1);
-      mbar_init(&tempty_bar[s], 4);
+      mbar_init(&tempty_bar[s], TC_EPI_WARPS);
     }
     *abort_word = 0;
     fence_mbar_init();
     fence_proxy_async_smem();
     tma_prefetch_desc(&tmA);
     tma_prefetch_desc(&tmB);
+    if (p.tma_out) tma_prefetch_desc(&tmC);
   }
   if (warp == 2) {
     tmem_alloc(tmem_slot, 2 * BN);
@@ -487,8 +507,9 @@ __global__ void __launch_bounds__(TC_THREADS, 1)
     }
   } else if (warp >= 4) {
     // ------------------------------------------------ epilogue (TMEM -> registers -> global)
-    const int q = warp & 3;  // a warp may only touch TMEM lanes 32q .. 32q+31
+    const int q = warp & 3, half = (warp - 4) >> 2;  // a warp may only touch TMEM lanes 32q .. 32q+31
     const int row = q * 32 + lane;
+    uint8_t* out_buf = smem + S::OUT_OFFSET + (warp - 4) * TC_OUT_BYTES;
     int acc = 0;
     uint32_t acc_phase = 0;
     const bool c_unit = (p.csc == 1);
@@ -509,20 +530,21 @@ __global__ void __launch_bounds__(TC_THREADS, 1)
           c_unit && (((reinterpret_cast<uint64_t>(p.C) + static_cast<uint64_t>(row_off) * esz) & 15u) == 0) &&
           ((static_cast<int64_t>(nb) * BN * esz & 15) == 0);
       const uint32_t t_row = tmem_base + static_cast<uint32_t>(acc * BN) + (static_cast<uint32_t>(q * 32) << 16);
+      if (p.tma_out) {
+        tc_drain<BN>(p, &tmC, t_row, out_buf, nb * BN, mb * TC_BM + q * 32, b, half, lane);
+      } else {
 #pragma unroll 1
-      for (int c0 = 0; c0 < BN; c0 += 32) {
-        uint32_t r[32];
-        tmem_ld_32x32b_x32(t_row + c0, r);
-        tmem_ld_wait();
-        const int gn0 = nb * BN + c0;
-        if (gn0 < p.N) {
-          if (p.staged)
-            tc_store_staged(p, r, smem + S::OUT_OFFSET + q * TC_OUT_BYTES, row_off - static_cast<int64_t>(lane) * p.rsc,
-                            p.M - (gm - lane), gn0, (nb + 1) * BN, lane);
-          else if (p.epi != EPI_NONE) tc_store_epilogue(p, r, row_off, gn0, row_ok);
-          else if (p.out_dtype == YTC_BF16) tc_store_chunk<BN, YTC_BF16>(p, r, row_off, gn0, row_ok, vec_ok);
-          else if (p.out_dtype == YTC_F32) tc_store_chunk<BN, YTC_F32>(p, r, row_off, gn0, row_ok, vec_ok);
-          else tc_store_chunk<BN, YTC_F16>(p, r, row_off, gn0, row_ok, vec_ok);
+        for (int c0 = half * (BN / 2); c0 < (half + 1) * (BN / 2); c0 += 32) {
+          uint32_t r[32];
+          tmem_ld_32x32b_x32(t_row + c0, r);
+          tmem_ld_wait();
+          const int gn0 = nb * BN + c0;
+          if (gn0 < p.N) {
+            if (p.epi != EPI_NONE) tc_store_epilogue(p, r, row_off, gn0, row_ok);
+            else if (p.out_dtype == YTC_BF16) tc_store_chunk<BN, YTC_BF16>(p, r, row_off, gn0, row_ok, vec_ok);
+            else if (p.out_dtype == YTC_F32) tc_store_chunk<BN, YTC_F32>(p, r, row_off, gn0, row_ok, vec_ok);
+            else tc_store_chunk<BN, YTC_F16>(p, r, row_off, gn0, row_ok, vec_ok);
+          }
         }
       }
       tc_fence_before();
@@ -531,6 +553,7 @@ __global__ void __launch_bounds__(TC_THREADS, 1)
       acc ^= 1;
       if (acc == 0) acc_phase ^= 1u;
     }
+    if (p.tma_out && lane == 0) tma_store_wait_all<0>();
   }
 
   tc_fence_before();
@@ -559,14 +582,14 @@ struct Tc2Smem {
   static constexpr int BAR_OFFSET = TC2_STAGES * STAGE_BYTES;
   static constexpr int TOTAL = BAR_OFFSET + (2 * TC2_STAGES + 4) * 8 + 16;
   static constexpr int DYN_BYTES = TOTAL + 1024;
-  static constexpr int OUT_OFFSET = (TOTAL + 127) / 128 * 128;
-  static constexpr int DYN_STAGED = OUT_OFFSET + 4 * TC_OUT_BYTES + 1024;
+  static constexpr int OUT_OFFSET = (TOTAL + 1023) / 1024 * 1024;
+  static constexpr int DYN_STAGED = OUT_OFFSET + TC_EPI_WARPS * TC_OUT_BYTES + 1024;
 };
 
 template <bool PIECES>
 __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(TC_THREADS, 1)
     gemm_tc2_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ CUtensorMap tmB,
-                    const GemmTcParams p) {
+                    const __grid_constant__ CUtensorMap tmC, const GemmTcParams p) {
   using S = Tc2Smem;
   extern __shared__ uint8_t smem_raw[];
   const uint32_t raw_addr = smem_u32(smem_raw);
@@ -589,13 +612,14 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(TC_THREADS, 1)
     }
     for (int s = 0; s < 2; ++s) {
       mbar_init(&tfull_bar[s], 1);
-      mbar_init(&tempty_bar[s], 8);  // 4 epilogue warps of each CTA
+      mbar_init(&tempty_bar[s], 2 * TC_EPI_WARPS);  // the epilogue warps of both CTAs
     }
     *abort_word = 0;
     fence_mbar_init();
     fence_proxy_async_smem();
     tma_prefetch_desc(&tmA);
     tma_prefetch_desc(&tmB);
+    if (p.tma_out) tma_prefetch_desc(&tmC);
   }
   if (warp == 2) {
     tmem_alloc_pair(tmem_slot, 512);
@@ -704,8 +728,9 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(TC_THREADS, 1)
     }
   } else if (warp >= 4) {
     // ------------------------------------------------ epilogue (both CTAs, own 128 rows x 256 columns)
-    const int q = warp & 3;
+    const int q = warp & 3, half = (warp - 4) >> 2;
     const int row = q * 32 + lane;
+    uint8_t* out_buf = smem + S::OUT_OFFSET + (warp - 4) * TC_OUT_BYTES;
     int acc = 0;
     uint32_t acc_phase = 0;
     const bool c_unit = (p.csc == 1);
@@ -723,20 +748,21 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(TC_THREADS, 1)
       const bool vec_ok =
           c_unit && (((reinterpret_cast<uint64_t>(p.C) + static_cast<uint64_t>(row_off) * esz) & 15u) == 0);
       const uint32_t t_row = tmem_base + static_cast<uint32_t>(acc * TC2_BN) + (static_cast<uint32_t>(q * 32) << 16);
+      if (p.tma_out) {
+        tc_drain<TC2_BN>(p, &tmC, t_row, out_buf, nb * TC2_BN, mb * 256 + static_cast<int>(cta) * TC_BM + q * 32, b, half, lane);
+      } else {
 #pragma unroll 1
-      for (int c0 = 0; c0 < TC2_BN; c0 += 32) {
-        uint32_t r[32];
-        tmem_ld_32x32b_x32(t_row + c0, r);
-        tmem_ld_wait();
-        const int gn0 = nb * TC2_BN + c0;
-        if (gn0 < p.N) {
-          if (p.staged)
-            tc_store_staged(p, r, smem + S::OUT_OFFSET + q * TC_OUT_BYTES, row_off - static_cast<int64_t>(lane) * p.rsc,
-                            p.M - (gm - lane), gn0, (nb + 1) * TC2_BN, lane);
-          else if (p.epi != EPI_NONE) tc_store_epilogue(p, r, row_off, gn0, row_ok);
-          else if (p.out_dtype == YTC_BF16) tc_store_chunk<TC2_BN, YTC_BF16>(p, r, row_off, gn0, row_ok, vec_ok);
-          else if (p.out_dtype == YTC_F32) tc_store_chunk<TC2_BN, YTC_F32>(p, r, row_off, gn0, row_ok, vec_ok);
-          else tc_store_chunk<TC2_BN, YTC_F16>(p, r, row_off, gn0, row_ok, vec_ok);
+        for (int c0 = half * (TC2_BN / 2); c0 < (half + 1) * (TC2_BN / 2); c0 += 32) {
+          uint32_t r[32];
+          tmem_ld_32x32b_x32(t_row + c0, r);
+          tmem_ld_wait();
+          const int gn0 = nb * TC2_BN + c0;
+          if (gn0 < p.N) {
+            if (p.epi != EPI_NONE) tc_store_epilogue(p, r, row_off, gn0, row_ok);
+            else if (p.out_dtype == YTC_BF16) tc_store_chunk<TC2_BN, YTC_BF16>(p, r, row_off, gn0, row_ok, vec_ok);
+            else if (p.out_dtype == YTC_F32) tc_store_chunk<TC2_BN, YTC_F32>(p, r, row_off, gn0, row_ok, vec_ok);
+            else tc_store_chunk<TC2_BN, YTC_F16>(p, r, row_off, gn0, row_ok, vec_ok);
+          }
         }
       }
       tc_fence_before();
@@ -745,6 +771,7 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(TC_THREADS, 1)
       acc ^= 1;
       if (acc == 0) acc_phase ^= 1u;
     }
+    if (p.tma_out && lane == 0) tma_store_wait_all<0>();
   }
 
   tc_fence_before();
@@ -1111,8 +1138,25 @@ static int launch_tc(int dtype_in, int dtype_out, const void* A, const void* B, 
   p.tile_live = nullptr;
   const LinearEpilogue none, *e = ex ? ex : &none;
   p.epi = e->epi;
-  p.staged = ex && csc == 1 && (reinterpret_cast<uint64_t>(C) & 15u) == 0 && (rsc * dtype_size(dtype_out)) % 16 == 0 &&
-             batch == 1 && (e->epi != EPI_NONE || dtype_out == YTC_F32);
+  // C through TMA stores: rows (and batch items, pieces of k) that start at 16 bytes. What C holds already is added there only
+  // where the caller leaves that to the memory's adders (which count numbers below 2^-126 as zero).
+  const int esz = dtype_size(dtype_out);
+  const int64_t items = batch * splits;
+  const bool rows16 = csc == 1 && rsc > 0 && (reinterpret_cast<uint64_t>(C) & 15u) == 0 && rsc * esz % 16 == 0 &&
+                      rsc * esz < (int64_t{1} << 40) && (items == 1 || (bsc > 0 && bsc * esz % 16 == 0 && bsc * esz < (int64_t{1} << 40)));
+  p.tma_out = !rows16 ? 0 : beta == 0.f ? 1 : e->add_in_memory && beta == 1.f && alpha == 1.f && dtype_out == YTC_F32 ? 2 : 0;
+  CUtensorMap tmC{};
+  if (p.tma_out) {
+    const uint64_t dims[3] = {static_cast<uint64_t>(epi_pairs(e->epi) ? n / 2 : n), static_cast<uint64_t>(m), static_cast<uint64_t>(items)};
+    const uint64_t strides[2] = {static_cast<uint64_t>(rsc * esz), items > 1 ? static_cast<uint64_t>(bsc * esz) : static_cast<uint64_t>(rsc * esz) * m};
+    const uint32_t box[3] = {static_cast<uint32_t>(128 / esz), 32, 1};
+    if (strides[1] >= (uint64_t{1} << 40)) p.tma_out = 0;
+    else {
+      const int s = encode_tensor_map(&tmC, esz == 4 ? CU_TENSOR_MAP_DATA_TYPE_FLOAT32 : CU_TENSOR_MAP_DATA_TYPE_UINT16, 3, C, dims, strides,
+                                      box, CU_TENSOR_MAP_SWIZZLE_128B);
+      if (s != YTC_OK) return s;
+    }
+  }
   p.act_cols = e->act_cols;
   p.limit = e->limit; p.alpha_gate = e->alpha; p.shift = e->shift;
   p.tile_group = grouped ? ex->tile_group : nullptr;
@@ -1127,14 +1171,14 @@ static int launch_tc(int dtype_in, int dtype_out, const void* A, const void* B, 
     p.tiles_m = (m + 255) / 256;
     p.tiles_n = (n + TC2_BN - 1) / TC2_BN;
     p.total_tiles = static_cast<int>(static_cast<int64_t>(p.tiles_m) * p.tiles_n * batch);
-    const int smem = p.staged ? Tc2Smem::DYN_STAGED : Tc2Smem::DYN_BYTES;
+    const int smem = p.tma_out ? Tc2Smem::DYN_STAGED : Tc2Smem::DYN_BYTES;
     int clusters = sm_count() / 2;
     if (clusters > p.total_tiles) clusters = p.total_tiles;
     {
       const int s = ensure_dynamic_smem(reinterpret_cast<const void*>(pieces ? gemm_tc2_kernel<true> : gemm_tc2_kernel<false>), smem);
       if (s != YTC_OK) return s;
     }
-    YTC_CUDA(launch_overlapped(pieces ? gemm_tc2_kernel<true> : gemm_tc2_kernel<false>, dim3(clusters * 2), dim3(TC_THREADS), smem, st, tmA, tmB, p));
+    YTC_CUDA(launch_overlapped(pieces ? gemm_tc2_kernel<true> : gemm_tc2_kernel<false>, dim3(clusters * 2), dim3(TC_THREADS), smem, st, tmA, tmB, tmC, p));
     count_launch();
     YTC_CUDA(cudaGetLastError());
     return YTC_OK;
@@ -1147,17 +1191,17 @@ static int launch_tc(int dtype_in, int dtype_out, const void* A, const void* B, 
     p.tile_live = live;
   }
   if (BN == 256) {
-    const int smem = p.staged ? TcSmem<256>::DYN_STAGED : TcSmem<256>::DYN_BYTES;
+    const int smem = p.tma_out ? TcSmem<256>::DYN_STAGED : TcSmem<256>::DYN_BYTES;
     auto* fn = pieces ? gemm_tc_kernel<256, true> : gemm_tc_kernel<256, false>;
     const int s = ensure_dynamic_smem(reinterpret_cast<const void*>(fn), smem);
     if (s != YTC_OK) return s;
-    YTC_CUDA(launch_overlapped(fn, dim3(grid), dim3(TC_THREADS), smem, st, tmA, tmB, p));
+    YTC_CUDA(launch_overlapped(fn, dim3(grid), dim3(TC_THREADS), smem, st, tmA, tmB, tmC, p));
   } else {
-    const int smem = p.staged ? TcSmem<128>::DYN_STAGED : TcSmem<128>::DYN_BYTES;
+    const int smem = p.tma_out ? TcSmem<128>::DYN_STAGED : TcSmem<128>::DYN_BYTES;
     auto* fn = pieces ? gemm_tc_kernel<128, true> : gemm_tc_kernel<128, false>;
     const int s = ensure_dynamic_smem(reinterpret_cast<const void*>(fn), smem);
     if (s != YTC_OK) return s;
-    YTC_CUDA(launch_overlapped(fn, dim3(grid), dim3(TC_THREADS), smem, st, tmA, tmB, p));
+    YTC_CUDA(launch_overlapped(fn, dim3(grid), dim3(TC_THREADS), smem, st, tmA, tmB, tmC, p));
   }
   count_launch();
   if (live) cudaFreeAsync(live, st);
@@ -1562,7 +1606,9 @@ int linear_two_planes(const void* planes, const void* w, float* y, int64_t ldy, 
     return s != YTC_OK ? s : ytcuda_gemm(YTC_BF16, YTC_F32, lo, w, y, m, n, k, 1.f, 1.f, k, 1, 1, k, ldy, 1, 1, 0, 0, 0, st);
   }
   const TcPlanes pl{2, 1, 2, 1u, 0u, static_cast<int64_t>(m) * k, static_cast<int64_t>(n) * k};
-  return launch_tc(YTC_BF16, YTC_F32, planes, w, y, m, n, k, 1.f, accumulate ? 1.f : 0.f, 0, k, 0, k, ldy, 1, 1, 0, 0, 0, st, nullptr, &pl);
+  LinearEpilogue ex;
+  ex.add_in_memory = true;
+  return launch_tc(YTC_BF16, YTC_F32, planes, w, y, m, n, k, 1.f, accumulate ? 1.f : 0.f, 0, k, 0, k, ldy, 1, 1, 0, 0, 0, st, &ex, &pl);
 }
 
 }  // namespace ytk
