@@ -1,7 +1,7 @@
 // GEMM for the YTensor device backend.
 //
 //  * gemm_tc_kernel   : bf16 / fp16 inputs, fp32 accumulation in tensor memory. Persistent,
-//                       one CTA per SM, warp-specialised: warp 0 feeds a 4-stage shared-memory
+//                       one CTA per SM, warp-specialised: warp 0 feeds a shared-memory
 //                       ring with TMA, warp 1 issues tcgen05.mma (128 x BN x 16 per instruction),
 //                       warps 4-11 drain the accumulator (tcgen05.ld) and write C (TMA stores) while
 //                       the next tile's MMAs run into the second accumulator stage.
@@ -21,7 +21,6 @@ namespace ytk {
 // ------------------------------------------------------------------ tcgen05 path
 constexpr int TC_BM = 128;
 constexpr int TC_BK = 64;  // 64 x 16-bit = one 128-byte swizzle row
-constexpr int TC_STAGES = 4;
 constexpr int TC_EPI_WARPS = 8;  // two per quarter of the accumulator's lanes
 constexpr int TC_THREADS = 128 + 32 * TC_EPI_WARPS;
 
@@ -61,12 +60,15 @@ struct GemmTcParams {
 constexpr int TC_OUT_BYTES = 32 * 128;  // an epilogue warp's 32 rows of 128 bytes on their way to C
 template <int BN>
 struct TcSmem {
+  // 192 KB of operands on their way: with four slots of 128 columns a block of k took 0.43 us on an idle chip, twice its MMAs
+  static constexpr int STAGES = BN == 128 ? 6 : 4;
+  static constexpr int FREED = BN == 128 ? 2 : 1;  // slots freed together
   static constexpr int A_BYTES = TC_BM * TC_BK * 2;
   static constexpr int B_BYTES = BN * TC_BK * 2;
   static constexpr int STAGE_BYTES = A_BYTES + B_BYTES;
-  static constexpr int BAR_OFFSET = TC_STAGES * STAGE_BYTES;
+  static constexpr int BAR_OFFSET = STAGES * STAGE_BYTES;
   // full[STAGES], empty[STAGES], tmem_full[2], tmem_empty[2], tmem base word, abort word
-  static constexpr int TOTAL = BAR_OFFSET + (2 * TC_STAGES + 4) * 8 + 16;
+  static constexpr int TOTAL = BAR_OFFSET + (2 * STAGES + 4) * 8 + 16;
   static constexpr int DYN_BYTES = TOTAL + 1024;  // slack to align the ring to 1024 B
   static constexpr int OUT_OFFSET = (TOTAL + 1023) / 1024 * 1024;  // TMA stores: the epilogue warps' areas
   static constexpr int DYN_STAGED = OUT_OFFSET + TC_EPI_WARPS * TC_OUT_BYTES + 1024;
@@ -305,6 +307,7 @@ __global__ void __launch_bounds__(TC_THREADS, 1)
     gemm_tc_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ CUtensorMap tmB,
                    const __grid_constant__ CUtensorMap tmC, const GemmTcParams p) {
   using S = TcSmem<BN>;
+  constexpr int TC_STAGES = S::STAGES;
   extern __shared__ uint8_t smem_raw[];
   // The 128-byte swizzle pattern is a function of the shared address: keep the ring 1024-byte aligned.
   const uint32_t raw_addr = smem_u32(smem_raw);
@@ -312,19 +315,17 @@ __global__ void __launch_bounds__(TC_THREADS, 1)
 
   uint64_t* full_bar = reinterpret_cast<uint64_t*>(smem + S::BAR_OFFSET);
   uint64_t* empty_bar = full_bar + TC_STAGES;
-  uint64_t* tfull_bar = empty_bar + TC_STAGES;
+  uint64_t* tfull_bar = empty_bar + TC_STAGES / S::FREED;
   uint64_t* tempty_bar = tfull_bar + 2;
   uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(tempty_bar + 2);
   volatile int* abort_word = reinterpret_cast<volatile int*>(tmem_slot + 1);
 
-  const int warp = threadIdx.x >> 5;
+  const int warp = __shfl_sync(0xffffffffu, threadIdx.x >> 5, 0);  // (known to be the same for the whole warp)
   const int lane = threadIdx.x & 31;
 
   if (threadIdx.x == 0) {
-    for (int s = 0; s < TC_STAGES; ++s) {
-      mbar_init(&full_bar[s], 1);
-      mbar_init(&empty_bar[s], 1);
-    }
+    for (int s = 0; s < TC_STAGES; ++s) mbar_init(&full_bar[s], 1);
+    for (int s = 0; s < TC_STAGES / S::FREED; ++s) mbar_init(&empty_bar[s], 1);
     for (int s = 0; s < 2; ++s) {
       mbar_init(&tfull_bar[s], 1);
       mbar_init(&tempty_bar[s], TC_EPI_WARPS);
@@ -352,158 +353,150 @@ __global__ void __launch_bounds__(TC_THREADS, 1)
   const int tiles_per_batch = p.tiles_m * p.tiles_n;
 
   if (warp == 0) {
-    // ------------------------------------------------ TMA producer
-    if (lane == 0) {
-      int stage = 0;
-      uint32_t phase = 0;
-      int issued = 0;
-      bool ok = true;
-      // A is streamed from HBM once; an L2 prefetch a few k-blocks ahead of the shared-memory ring
-      // takes the DRAM latency off the ring (B is small and stays L2-resident by reuse).
-      auto prefetch_a = [&](int tile, int kb) {
-        if (tile >= p.total_tiles) return;
-        const int b = tile / tiles_per_batch;
-        const int rem = tile - b * tiles_per_batch;
-        const int mb = rem / p.tiles_n;
-        const int ba = p.a_bcast ? 0 : b;
-        if (!p.a_mn) {
-          tma_prefetch_l2_3d(&tmA, kb * TC_BK, mb * TC_BM, ba);
+    // ------------------------------------------------ TMA producer (converged, as the MMA issuer: a copy issued inside a
+    // branch of one lane costs some hundred instructions; block by block they took 700 clk)
+    const uint32_t lead = lane == 0 ? 1u : 0u;
+    const uint32_t ring_at = smem_u32(smem), full_at = smem_u32(full_bar);
+    int stage = 0;
+    uint32_t phase = 0;
+    int issued = 0;
+    bool ok = true;
+    // A is streamed from HBM once; an L2 prefetch a few k-blocks ahead of the shared-memory ring
+    // takes the DRAM latency off the ring (B is small and stays L2-resident by reuse).
+    auto prefetch_a = [&](int tile, int kb) {
+      if (tile >= p.total_tiles) return;
+      const int b = tile / tiles_per_batch;
+      const int rem = tile - b * tiles_per_batch;
+      const int mb = rem / p.tiles_n;
+      const int ba = p.a_bcast ? 0 : b;
+      if (!p.a_mn) {
+        tma_prefetch_l2_3d_lead(&tmA, kb * TC_BK, mb * TC_BM, ba, lead);
+      } else {
+#pragma unroll
+        for (int c = 0; c < TC_BM / 64; ++c) tma_prefetch_l2_3d_lead(&tmA, mb * TC_BM + c * 64, kb * TC_BK, ba, lead);
+      }
+    };
+    int pf_tile = blockIdx.x, pf_kb = 0;
+    auto prefetch_next = [&]() {
+      prefetch_a(pf_tile, pf_kb);
+      if (++pf_kb == p.k_blocks) {
+        pf_kb = 0;
+        pf_tile += gridDim.x;
+      }
+    };
+#pragma unroll 1
+    for (int i = 0; i < p.a_prefetch; ++i) prefetch_next();
+    for (int tile = blockIdx.x; ok && tile < p.total_tiles; tile += gridDim.x) {
+      const int bf = tile / tiles_per_batch;
+      const int rem = tile - bf * tiles_per_batch;
+      TcPiece piece{bf, 0, p.k_blocks, 0};
+      if (PIECES) piece = tc_piece(p, bf);
+      if (p.tile_live && !p.tile_live[rem]) continue;
+      const int mb = rem / p.tiles_n;
+      const int nb = rem - mb * p.tiles_n;
+      const int group = p.tile_group ? __shfl_sync(0xffffffffu, p.tile_group[mb], 0) : 0;
+      if (group < 0) continue;
+      const int n_row0 = group * p.group_rows + nb * BN;
+      const int ba = p.a_bcast ? 0 : piece.b;
+      const int bb = p.b_bcast ? 0 : piece.b;
+      TcBlock<PIECES> at(p, piece, ba, bb);
+#pragma unroll 1
+      for (int kb = piece.kb0; kb < piece.kb1; ++kb, at.next(p, piece, ba, bb)) {
+        if (stage % S::FREED == 0 && !__all_sync(0xffffffffu, mbar_wait(&empty_bar[stage / S::FREED], phase ^ 1u, abort_word))) {
+          ok = false;
+          break;
+        }
+        if (p.a_prefetch > 0) prefetch_next();
+        const uint32_t bar = full_at + 8 * stage, sa = ring_at + stage * S::STAGE_BYTES, sb = sa + S::A_BYTES;
+        mbar_expect_tx_lead(bar, S::STAGE_BYTES, lead);
+        if (!p.a_mn && !p.split_loads) {
+          tma_load_3d_lead(sa, &tmA, bar, at.kk * TC_BK, mb * TC_BM, at.za, lead);
         } else {
-#pragma unroll
-          for (int c = 0; c < TC_BM / 64; ++c) tma_prefetch_l2_3d(&tmA, mb * TC_BM + c * 64, kb * TC_BK, ba);
-        }
-      };
-      int pf_tile = blockIdx.x, pf_kb = 0;
-      if (p.a_prefetch > 0) {
-        for (int i = 0; i < p.a_prefetch; ++i) {
-          prefetch_a(pf_tile, pf_kb);
-          if (++pf_kb == p.k_blocks) {
-            pf_kb = 0;
-            pf_tile += gridDim.x;
+#pragma unroll 1
+          for (int c = 0; c < TC_BM / 64; ++c) {
+            const int mn = mb * TC_BM + c * 64, kk = at.kk * TC_BK;
+            tma_load_3d_lead(sa + c * 8192, &tmA, bar, p.a_mn ? mn : kk, p.a_mn ? kk : mn, at.za, lead);
           }
         }
-      }
-      for (int tile = blockIdx.x; ok && tile < p.total_tiles; tile += gridDim.x) {
-        const int bf = tile / tiles_per_batch;
-        const int rem = tile - bf * tiles_per_batch;
-        TcPiece piece{bf, 0, p.k_blocks, 0};
-        if (PIECES) piece = tc_piece(p, bf);
-        if (p.tile_live && !p.tile_live[rem]) continue;
-        const int mb = rem / p.tiles_n;
-        const int nb = rem - mb * p.tiles_n;
-        const int group = p.tile_group ? p.tile_group[mb] : 0;
-        if (group < 0) continue;
-        const int n_row0 = group * p.group_rows + nb * BN;
-        const int ba = p.a_bcast ? 0 : piece.b;
-        const int bb = p.b_bcast ? 0 : piece.b;
-        TcBlock<PIECES> at(p, piece, ba, bb);
-        for (int kb = piece.kb0; kb < piece.kb1; ++kb, at.next(p, piece, ba, bb)) {
-          if (!mbar_wait(&empty_bar[stage], phase ^ 1u, abort_word)) {
-            ok = false;
-            break;
-          }
-          if (p.a_prefetch > 0) {
-            prefetch_a(pf_tile, pf_kb);
-            if (++pf_kb == p.k_blocks) {
-              pf_kb = 0;
-              pf_tile += gridDim.x;
-            }
-          }
-          mbar_expect_tx(&full_bar[stage], S::STAGE_BYTES);
-          uint8_t* sa = smem + stage * S::STAGE_BYTES;
-          uint8_t* sb = sa + S::A_BYTES;
-          if (!p.a_mn) {
-            if (p.split_loads) {
-#pragma unroll
-              for (int c = 0; c < TC_BM / 64; ++c)
-                tma_load_3d(sa + c * 8192, &tmA, &full_bar[stage], at.kk * TC_BK, mb * TC_BM + c * 64, at.za);
-            } else {
-              tma_load_3d(sa, &tmA, &full_bar[stage], at.kk * TC_BK, mb * TC_BM, at.za);
-            }
-          } else {
-#pragma unroll
-            for (int c = 0; c < TC_BM / 64; ++c)
-              tma_load_3d(sa + c * 8192, &tmA, &full_bar[stage], mb * TC_BM + c * 64, at.kk * TC_BK, at.za);
-          }
-          if (!p.b_mn) {
-            if (p.split_loads) {
-#pragma unroll
-              for (int c = 0; c < BN / 64; ++c)
-                tma_load_3d(sb + c * 8192, &tmB, &full_bar[stage], at.kk * TC_BK, n_row0 + c * 64, at.zb);
-            } else {
-              tma_load_3d(sb, &tmB, &full_bar[stage], at.kk * TC_BK, n_row0, at.zb);
-            }
-          } else {
-#pragma unroll
-            for (int c = 0; c < BN / 64; ++c)
-              tma_load_3d(sb + c * 8192, &tmB, &full_bar[stage], n_row0 + c * 64, at.kk * TC_BK, at.zb);
-          }
-          ++issued;
-          if (++stage == TC_STAGES) {
-            stage = 0;
-            phase ^= 1u;
+        if (!p.b_mn && !p.split_loads) {
+          tma_load_3d_lead(sb, &tmB, bar, at.kk * TC_BK, n_row0, at.zb, lead);
+        } else {
+#pragma unroll 1
+          for (int c = 0; c < BN / 64; ++c) {
+            const int mn = n_row0 + c * 64, kk = at.kk * TC_BK;
+            tma_load_3d_lead(sb + c * 8192, &tmB, bar, p.b_mn ? mn : kk, p.b_mn ? kk : mn, at.zb, lead);
           }
         }
-      }
-      if (!ok) {
-        // Give the copies already in flight a bounded time to land before the CTA goes away.
-        const int pending = issued < TC_STAGES ? issued : TC_STAGES;
-        int s = stage;
-        uint32_t ph = phase;
-        for (int i = 0; i < pending; ++i) {
-          if (--s < 0) {
-            s = TC_STAGES - 1;
-            ph ^= 1u;
-          }
-          const long long t0 = clock64();
-          while (!mbar_try_wait(&full_bar[s], ph) && clock64() - t0 < 20000000ll) {
-          }
+        ++issued;
+        if (++stage == TC_STAGES) {
+          stage = 0;
+          phase ^= 1u;
         }
       }
     }
+    if (!ok) {
+      // Give the copies already in flight a bounded time to land before the CTA goes away.
+      const int pending = issued < TC_STAGES ? issued : TC_STAGES;
+      int s = stage;
+      uint32_t ph = phase;
+      for (int i = 0; i < pending; ++i) {
+        if (--s < 0) {
+          s = TC_STAGES - 1;
+          ph ^= 1u;
+        }
+        const long long t0 = clock64();
+        while (!mbar_try_wait(&full_bar[s], ph) && clock64() - t0 < 20000000ll) {
+        }
+      }
+    }
+    __syncwarp();
   } else if (warp == 1) {
     // ------------------------------------------------ MMA issuer
-    if (lane == 0) {
-      int stage = 0;
-      uint32_t phase = 0;
-      int acc = 0;
-      uint32_t acc_phase = 0;
-      bool ok = true;
-      for (int tile = blockIdx.x; ok && tile < p.total_tiles; tile += gridDim.x) {
-        if (p.tile_live && !p.tile_live[tile % tiles_per_batch]) continue;
-        if (p.tile_group && p.tile_group[(tile % tiles_per_batch) / p.tiles_n] < 0) continue;
-        if (!mbar_wait(&tempty_bar[acc], acc_phase ^ 1u, abort_word)) break;
-        tc_fence_after();
-        const uint32_t d_tmem = tmem_base + static_cast<uint32_t>(acc * BN);
-        TcPiece piece{0, 0, p.k_blocks, 0};
-        if (PIECES) piece = tc_piece(p, tile / tiles_per_batch);
-        for (int kb = piece.kb0; kb < piece.kb1; ++kb) {
-          if (!mbar_wait(&full_bar[stage], phase, abort_word)) {
-            ok = false;
-            break;
-          }
-          tc_fence_after();
-          const uint32_t a_base = smem_u32(smem + stage * S::STAGE_BYTES);
-          const uint32_t b_base = a_base + S::A_BYTES;
-#pragma unroll
-          for (int k = 0; k < TC_BK / 16; ++k) {
-            const uint64_t adesc = p.a_mn ? umma_smem_desc_sw128(a_base + k * 2048, 8192, 1024)
-                                          : umma_smem_desc_sw128(a_base + k * 32, 16, 1024);
-            const uint64_t bdesc = p.b_mn ? umma_smem_desc_sw128(b_base + k * 2048, 8192, 1024)
-                                          : umma_smem_desc_sw128(b_base + k * 32, 16, 1024);
-            tc_mma_f16(d_tmem, adesc, bdesc, p.idesc, kb != piece.kb0 || k != 0 ? 1u : 0u);
-          }
-          tc_commit(&empty_bar[stage]);  // frees the stage once these MMAs have read it
-          if (++stage == TC_STAGES) {
-            stage = 0;
-            phase ^= 1u;
-          }
+    // The tensor pipe takes the next instruction only when it can start it, so whatever else the issuing warp does is time in
+    // which no MMA runs. The warp stays converged (operands in uniform registers), looks at the next slot before it issues this
+    // one's MMAs, and frees two slots with one commit: a block of k of 128 x 128 takes 290 clk to issue, of which 256 are MMAs;
+    // with one lane that waits, issues and commits block by block it took 576. With the producer's copies (below): 500 x 1024 x
+    // 4608 32.8 -> 22.9 us, 4096^3 105 -> 94, 8 x 2048 x 4096 x 4096 449 -> 409.
+    const uint32_t lead = lane == 0 ? 1u : 0u;
+    const uint32_t free_at = smem_u32(empty_bar), tfull_at = smem_u32(tfull_bar);
+    const uint64_t a_desc = p.a_mn ? umma_smem_desc_sw128(smem_u32(smem), 8192, 1024) : umma_smem_desc_sw128(smem_u32(smem), 16, 1024);
+    const uint64_t b_desc = (p.b_mn ? umma_smem_desc_sw128(smem_u32(smem), 8192, 1024) : umma_smem_desc_sw128(smem_u32(smem), 16, 1024)) + (S::A_BYTES >> 4);
+    const uint32_t a_step = p.a_mn ? 2048 >> 4 : 32 >> 4, b_step = p.b_mn ? 2048 >> 4 : 32 >> 4;
+    int stage = 0;
+    uint32_t phase = 0;
+    int acc = 0;
+    uint32_t acc_phase = 0;
+    bool ok = true, ready = false;
+    for (int tile = blockIdx.x; ok && tile < p.total_tiles; tile += gridDim.x) {
+      if (p.tile_live && !p.tile_live[tile % tiles_per_batch]) continue;
+      if (p.tile_group && p.tile_group[(tile % tiles_per_batch) / p.tiles_n] < 0) continue;
+      if (!__all_sync(0xffffffffu, mbar_wait(&tempty_bar[acc], acc_phase ^ 1u, abort_word))) break;
+      tc_fence_after();
+      const uint32_t d_tmem = tmem_base + static_cast<uint32_t>(acc * BN);
+      TcPiece piece{0, 0, p.k_blocks, 0};
+      if (PIECES) piece = tc_piece(p, tile / tiles_per_batch);
+#pragma unroll 1
+      for (int kb = piece.kb0; kb < piece.kb1; ++kb) {
+        if (!ready && !__all_sync(0xffffffffu, mbar_wait(&full_bar[stage], phase, abort_word))) {
+          ok = false;
+          break;
         }
-        if (!ok) break;
-        tc_commit(&tfull_bar[acc]);  // accumulator complete
-        acc ^= 1;
-        if (acc == 0) acc_phase ^= 1u;
+        const int next = stage + 1 == TC_STAGES ? 0 : stage + 1;
+        ready = __all_sync(0xffffffffu, mbar_test_wait(&full_bar[next], next ? phase : phase ^ 1u)) != 0;
+        tc_fence_after();
+        const uint64_t ad = a_desc + (stage * S::STAGE_BYTES >> 4), bd = b_desc + (stage * S::STAGE_BYTES >> 4);
+#pragma unroll
+        for (int k = 0; k < TC_BK / 16; ++k)
+          tc_mma_f16_lead(d_tmem, ad + k * a_step, bd + k * b_step, p.idesc, kb != piece.kb0 || k != 0 ? 1u : 0u, lead);
+        // frees the slots once their MMAs have read them
+        if (stage % S::FREED == S::FREED - 1) tc_commit_lead(free_at + 8 * (stage / S::FREED), lead);
+        stage = next;
+        if (next == 0) phase ^= 1u;
       }
+      if (!ok) break;
+      tc_commit_lead(tfull_at + 8 * acc, lead);  // accumulator complete
+      acc ^= 1;
+      if (acc == 0) acc_phase ^= 1u;
     }
   } else if (warp >= 4) {
     // ------------------------------------------------ epilogue (TMEM -> registers -> global)
@@ -596,20 +589,18 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(TC_THREADS, 1)
   uint8_t* smem = smem_raw + ((1024u - (raw_addr & 1023u)) & 1023u);
   uint64_t* full_bar = reinterpret_cast<uint64_t*>(smem + S::BAR_OFFSET);
   uint64_t* empty_bar = full_bar + TC2_STAGES;
-  uint64_t* tfull_bar = empty_bar + TC2_STAGES;
+  uint64_t* tfull_bar = empty_bar + TC2_STAGES / 2;  // (two slots are freed together)
   uint64_t* tempty_bar = tfull_bar + 2;
   uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(tempty_bar + 2);
   volatile int* abort_word = reinterpret_cast<volatile int*>(tmem_slot + 1);
 
-  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-  const uint32_t cta = cluster_ctarank();  // 0 = leader
+  const int warp = __shfl_sync(0xffffffffu, threadIdx.x >> 5, 0), lane = threadIdx.x & 31;
+  const uint32_t cta = blockIdx.x & 1;  // rank in the cluster, 0 = leader
   const bool leader = cta == 0;
 
   if (threadIdx.x == 0) {
-    for (int s = 0; s < TC2_STAGES; ++s) {
-      mbar_init(&full_bar[s], 1);
-      mbar_init(&empty_bar[s], 1);
-    }
+    for (int s = 0; s < TC2_STAGES; ++s) mbar_init(&full_bar[s], 1);
+    for (int s = 0; s < TC2_STAGES / 2; ++s) mbar_init(&empty_bar[s], 1);
     for (int s = 0; s < 2; ++s) {
       mbar_init(&tfull_bar[s], 1);
       mbar_init(&tempty_bar[s], 2 * TC_EPI_WARPS);  // the epilogue warps of both CTAs
@@ -640,88 +631,87 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(TC_THREADS, 1)
 
   if (warp == 0) {
     // ------------------------------------------------ TMA producer (both CTAs)
-    if (lane == 0) {
-      int stage = 0;
-      uint32_t phase = 0;
-      bool ok = true;
-      for (int tile = cluster_id; ok && tile < p.total_tiles; tile += n_clusters) {
-        const int b = tile / tiles_per_batch;
-        const int rem = tile - b * tiles_per_batch;
-        const int mb = rem / p.tiles_n;
-        const int nb = rem - mb * p.tiles_n;
-        const int ba = p.a_bcast ? 0 : b;
-        const int bb = p.b_bcast ? 0 : b;
-        const int m0 = mb * 256 + static_cast<int>(cta) * TC_BM;
-        const int n0 = nb * TC2_BN + static_cast<int>(cta) * (TC2_BN / 2);
-        const TcPiece piece{b, 0, p.k_blocks, 0};
-        TcBlock<PIECES> at(p, piece, ba, bb);
-        for (int kb = 0; kb < p.k_blocks; ++kb, at.next(p, piece, ba, bb)) {
-          if (!mbar_wait(&empty_bar[stage], phase ^ 1u, abort_word)) {
-            ok = false;
-            break;
-          }
-          const uint32_t full_leader = map_to_cta(smem_u32(&full_bar[stage]), 0);
-          if (leader) mbar_expect_tx(&full_bar[stage], 2 * S::STAGE_BYTES);
-          uint8_t* sa = smem + stage * S::STAGE_BYTES;
-          uint8_t* sb = sa + S::A_BYTES;
-          if (!p.a_mn) {
-            tma_load_3d_pair(sa, &tmA, full_leader, at.kk * TC_BK, m0, at.za);
-          } else {
-#pragma unroll
-            for (int c = 0; c < TC_BM / 64; ++c) tma_load_3d_pair(sa + c * 8192, &tmA, full_leader, m0 + c * 64, at.kk * TC_BK, at.za);
-          }
-          if (!p.b_mn) {
-            tma_load_3d_pair(sb, &tmB, full_leader, at.kk * TC_BK, n0, at.zb);
-          } else {
-#pragma unroll
-            for (int c = 0; c < TC2_BN / 128; ++c) tma_load_3d_pair(sb + c * 8192, &tmB, full_leader, n0 + c * 64, at.kk * TC_BK, at.zb);
-          }
-          if (++stage == TC2_STAGES) {
-            stage = 0;
-            phase ^= 1u;
-          }
+    const uint32_t lead = lane == 0 ? 1u : 0u, first_cta = leader ? lead : 0u;
+    const uint32_t ring_at = smem_u32(smem), full_at = smem_u32(full_bar), full_leader = map_to_cta(full_at, 0);
+    int stage = 0;
+    uint32_t phase = 0;
+    bool ok = true;
+    for (int tile = cluster_id; ok && tile < p.total_tiles; tile += n_clusters) {
+      const int b = tile / tiles_per_batch;
+      const int rem = tile - b * tiles_per_batch;
+      const int mb = rem / p.tiles_n;
+      const int nb = rem - mb * p.tiles_n;
+      const int ba = p.a_bcast ? 0 : b;
+      const int bb = p.b_bcast ? 0 : b;
+      const int m0 = mb * 256 + static_cast<int>(cta) * TC_BM;
+      const int n0 = nb * TC2_BN + static_cast<int>(cta) * (TC2_BN / 2);
+      const TcPiece piece{b, 0, p.k_blocks, 0};
+      TcBlock<PIECES> at(p, piece, ba, bb);
+#pragma unroll 1
+      for (int kb = 0; kb < p.k_blocks; ++kb, at.next(p, piece, ba, bb)) {
+        if ((stage & 1) == 0 && !__all_sync(0xffffffffu, mbar_wait(&empty_bar[stage >> 1], phase ^ 1u, abort_word))) {
+          ok = false;
+          break;
+        }
+        const uint32_t bar = full_leader + 8 * stage, sa = ring_at + stage * S::STAGE_BYTES, sb = sa + S::A_BYTES;
+        mbar_expect_tx_lead(full_at + 8 * stage, 2 * S::STAGE_BYTES, first_cta);
+        const int kk = at.kk * TC_BK;
+        if (!p.a_mn) {
+          tma_load_3d_pair_lead(sa, &tmA, bar, kk, m0, at.za, lead);
+        } else {
+#pragma unroll 1
+          for (int c = 0; c < TC_BM / 64; ++c) tma_load_3d_pair_lead(sa + c * 8192, &tmA, bar, m0 + c * 64, kk, at.za, lead);
+        }
+        if (!p.b_mn) {
+          tma_load_3d_pair_lead(sb, &tmB, bar, kk, n0, at.zb, lead);
+        } else {
+#pragma unroll 1
+          for (int c = 0; c < TC2_BN / 128; ++c) tma_load_3d_pair_lead(sb + c * 8192, &tmB, bar, n0 + c * 64, kk, at.zb, lead);
+        }
+        if (++stage == TC2_STAGES) {
+          stage = 0;
+          phase ^= 1u;
         }
       }
     }
+    __syncwarp();
   } else if (warp == 1) {
-    // ------------------------------------------------ MMA issuer (leader CTA only)
-    if (lane == 0 && leader) {
+    // ------------------------------------------------ MMA issuer (leader CTA only; see gemm_tc_kernel)
+    if (leader) {
+      const uint32_t lead = lane == 0 ? 1u : 0u;
+      const uint32_t free_at = smem_u32(empty_bar), tfull_at = smem_u32(tfull_bar);
+      const uint64_t a_desc = p.a_mn ? umma_smem_desc_sw128(smem_u32(smem), 8192, 1024) : umma_smem_desc_sw128(smem_u32(smem), 16, 1024);
+      const uint64_t b_desc = (p.b_mn ? umma_smem_desc_sw128(smem_u32(smem), 8192, 1024) : umma_smem_desc_sw128(smem_u32(smem), 16, 1024)) + (S::A_BYTES >> 4);
+      const uint32_t a_step = p.a_mn ? 2048 >> 4 : 32 >> 4, b_step = p.b_mn ? 2048 >> 4 : 32 >> 4;
       int stage = 0;
       uint32_t phase = 0;
       int acc = 0;
       uint32_t acc_phase = 0;
-      bool ok = true;
+      bool ok = true, ready = false;
       for (int tile = cluster_id; ok && tile < p.total_tiles; tile += n_clusters) {
-        if (!mbar_wait(&tempty_bar[acc], acc_phase ^ 1u, abort_word)) break;
+        if (!__all_sync(0xffffffffu, mbar_wait(&tempty_bar[acc], acc_phase ^ 1u, abort_word))) break;
         tc_fence_after();
         const uint32_t d_tmem = tmem_base + static_cast<uint32_t>(acc * TC2_BN);
+#pragma unroll 1
         for (int kb = 0; kb < p.k_blocks; ++kb) {
-          if (!mbar_wait(&full_bar[stage], phase, abort_word)) {
+          if (!ready && !__all_sync(0xffffffffu, mbar_wait(&full_bar[stage], phase, abort_word))) {
             ok = false;
             break;
           }
+          const int next = stage + 1 == TC2_STAGES ? 0 : stage + 1;
+          ready = __all_sync(0xffffffffu, mbar_test_wait(&full_bar[next], next ? phase : phase ^ 1u)) != 0;
           tc_fence_after();
-          const uint32_t a_base = smem_u32(smem + stage * S::STAGE_BYTES);
-          const uint32_t b_base = a_base + S::A_BYTES;
+          const uint64_t ad = a_desc + (stage * S::STAGE_BYTES >> 4), bd = b_desc + (stage * S::STAGE_BYTES >> 4);
 #pragma unroll
-          for (int k = 0; k < TC_BK / 16; ++k) {
-            const uint64_t adesc = p.a_mn ? umma_smem_desc_sw128(a_base + k * 2048, 8192, 1024)
-                                          : umma_smem_desc_sw128(a_base + k * 32, 16, 1024);
-            const uint64_t bdesc = p.b_mn ? umma_smem_desc_sw128(b_base + k * 2048, 8192, 1024)
-                                          : umma_smem_desc_sw128(b_base + k * 32, 16, 1024);
-            tc_mma_f16_pair(d_tmem, adesc, bdesc, p.idesc, (kb | k) != 0 ? 1u : 0u);
-          }
-          // the stage is free in both CTAs once these MMAs have read it
-          tc_commit_pair(smem_u32(&empty_bar[stage]));
-          tc_commit_pair(map_to_cta(smem_u32(&empty_bar[stage]), 1));
-          if (++stage == TC2_STAGES) {
-            stage = 0;
-            phase ^= 1u;
-          }
+          for (int k = 0; k < TC_BK / 16; ++k)
+            tc_mma_f16_pair_lead(d_tmem, ad + k * a_step, bd + k * b_step, p.idesc, (kb | k) != 0 ? 1u : 0u, lead);
+          // the slots are free in both CTAs once these MMAs have read them
+          if (stage & 1) tc_commit_pair_lead(free_at + 8 * (stage >> 1), 3, lead);
+          stage = next;
+          if (next == 0) phase ^= 1u;
         }
         if (!ok) break;
-        tc_commit_pair(smem_u32(&tfull_bar[acc]));
-        tc_commit_pair(map_to_cta(smem_u32(&tfull_bar[acc]), 1));
+        tc_commit_pair_lead(tfull_at + 8 * acc, 3, lead);
         acc ^= 1;
         if (acc == 0) acc_phase ^= 1u;
       }
