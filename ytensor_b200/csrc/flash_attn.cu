@@ -229,9 +229,9 @@ struct FaSmem {
 // Loads one [128 x D] tile as D/64 boxes of [128 rows x 128 bytes] (128-byte swizzle).
 template <int D>
 __device__ __forceinline__ void fa_load_tile(uint8_t* dst, const CUtensorMap* m, uint64_t* bar, int row, int head,
-                                             int batch) {
+                                             int batch, uint32_t lead) {
 #pragma unroll
-  for (int c = 0; c < D / 64; ++c) tma_load_4d(dst + c * (FA_BM * 128), m, bar, c * 64, row, head, batch);
+  for (int c = 0; c < D / 64; ++c) tma_load_4d_lead(smem_u32(dst) + c * (FA_BM * 128), m, smem_u32(bar), c * 64, row, head, batch, lead);
 }
 
 // Work item = one pair of query tiles (see the file header). The CTAs are persistent: CTA c handles items c,
@@ -308,7 +308,7 @@ __global__ void __launch_bounds__(FA_THREADS, 1)
   uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(p_half + 2);
   volatile int* abort_word = reinterpret_cast<volatile int*>(tmem_slot + 1);
 
-  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  const int warp = __shfl_sync(0xffffffffu, threadIdx.x >> 5, 0), lane = threadIdx.x & 31;  // (known to be the same for the warp)
 
   if (threadIdx.x == 0) {
     mbar_init(q_full, 1);
@@ -339,7 +339,7 @@ __global__ void __launch_bounds__(FA_THREADS, 1)
   tc_fence_before();
   __syncthreads();
   tc_fence_after();
-  const uint32_t tmem_base = *tmem_slot;
+  const uint32_t tmem_base = __shfl_sync(0xffffffffu, *tmem_slot, 0);
   // tensor-memory columns: S0/P0 at 0, S1/P1 at 128, O0 at 256, O1 at 384
   const uint32_t t_s[2] = {tmem_base, tmem_base + 128u};
   const uint32_t t_o[2] = {tmem_base + 256u, tmem_base + 384u};
@@ -348,7 +348,10 @@ __global__ void __launch_bounds__(FA_THREADS, 1)
 
   if (warp == 0) {
     // ------------------------------------------------------------ TMA producer
-    if (lane == 0) {
+    // (this role and the next run converged: copies and MMAs issued inside a branch of one lane cost some hundred instructions,
+    // and the tensor pipe stands still for every cycle the issuer spends on something else)
+    const uint32_t lead = lane == 0 ? 1u : 0u;
+    {
       int kv_cnt = 0;  // K/V tiles loaded so far: stage kv_cnt % 2, fill number kv_cnt / 2
       bool ok = true;
       int n_item = 0;
@@ -356,26 +359,26 @@ __global__ void __launch_bounds__(FA_THREADS, 1)
         const FaItem it = fa_decode_item<MODE>(p, w);
         if (it.n_max <= it.j0) continue;  // nothing visible: the softmax warpgroups write zeros on their own
         // (n_item counts only items with work; items without work touch no barrier in any role)
-        if (n_item > 0 && !mbar_wait(q_free, static_cast<uint32_t>((n_item - 1) & 1), abort_word)) break;
+        if (n_item > 0 && !mbar_wait_warp(q_free, static_cast<uint32_t>((n_item - 1) & 1), abort_word)) break;
         int n_q = 0;
         for (int t = 0; t < 2; ++t) n_q += it.tile_on[t] ? 1 : 0;
-        mbar_expect_tx(q_full, static_cast<uint32_t>(n_q) * S::TILE_BYTES);
+        mbar_expect_tx_lead(smem_u32(q_full), static_cast<uint32_t>(n_q) * S::TILE_BYTES, lead);
         for (int t = 0; t < 2; ++t)
           if (it.tile_on[t])
-            fa_load_tile<D>(smem + S::Q_OFF + t * S::TILE_BYTES, &tmQ, q_full, it.q_row0[t], it.q_head[t], it.b);
+            fa_load_tile<D>(smem + S::Q_OFF + t * S::TILE_BYTES, &tmQ, q_full, it.q_row0[t], it.q_head[t], it.b, lead);
         for (int j = it.j0; j < it.n_max; ++j, ++kv_cnt) {
           const int s = kv_cnt % FA_STAGES;
-          if (!mbar_wait(&kv_empty[s], static_cast<uint32_t>(((kv_cnt / FA_STAGES) & 1) ^ 1), abort_word)) {
+          if (!mbar_wait_warp(&kv_empty[s], static_cast<uint32_t>(((kv_cnt / FA_STAGES) & 1) ^ 1), abort_word)) {
             ok = false;
             break;
           }
           uint8_t* ks = smem + S::KV_OFF + s * 2 * S::TILE_BYTES;
           uint8_t* vs = ks + S::TILE_BYTES;
-          mbar_expect_tx(&k_full[s], S::TILE_BYTES);
+          mbar_expect_tx_lead(smem_u32(&k_full[s]), S::TILE_BYTES, lead);
           const int key_row = (MODE == FA_PLAIN ? j : (p.key_tile0 + j) % p.ring_tiles) * FA_BN;
-          fa_load_tile<D>(ks, &tmK, &k_full[s], key_row, it.kv_head, it.b);
-          mbar_expect_tx(&v_full[s], S::TILE_BYTES);
-          fa_load_tile<D>(vs, &tmV, &v_full[s], key_row, it.kv_head, it.b);
+          fa_load_tile<D>(ks, &tmK, &k_full[s], key_row, it.kv_head, it.b, lead);
+          mbar_expect_tx_lead(smem_u32(&v_full[s]), S::TILE_BYTES, lead);
+          fa_load_tile<D>(vs, &tmV, &v_full[s], key_row, it.kv_head, it.b, lead);
         }
         ++n_item;
       }
@@ -386,10 +389,12 @@ __global__ void __launch_bounds__(FA_THREADS, 1)
           while (!mbar_try_wait(&v_full[s], 0) && !mbar_try_wait(&v_full[s], 1) && clock64() - t0 < 20000000ll) {
           }
       }
+      __syncwarp();
     }
   } else if (warp == 1) {
     // ------------------------------------------------------------ MMA issuer
-    if (lane == 0) {
+    const uint32_t lead = lane == 0 ? 1u : 0u;
+    {
       const uint32_t q_base = smem_u32(smem + S::Q_OFF);
       int kv_cnt = 0;
       int p_cnt[2] = {0, 0};    // P tiles consumed so far per query tile (phase of p_full)
@@ -401,10 +406,10 @@ __global__ void __launch_bounds__(FA_THREADS, 1)
 #pragma unroll
         for (int kk = 0; kk < D / 16; ++kk) {
           const uint32_t off = (kk >> 2) * (FA_BM * 128) + (kk & 3) * 32;
-          tc_mma_f16(t_s[t], umma_smem_desc_sw128(qa + off, 16, 1024), umma_smem_desc_sw128(ka + off, 16, 1024),
-                     p.idesc_s, kk != 0 ? 1u : 0u);
+          tc_mma_f16_lead(t_s[t], umma_smem_desc_sw128(qa + off, 16, 1024), umma_smem_desc_sw128(ka + off, 16, 1024),
+                          p.idesc_s, kk != 0 ? 1u : 0u, lead);
         }
-        tc_commit(&s_full[t]);
+        tc_commit_lead(smem_u32(&s_full[t]), lead);
       };
       // O_t (+)= P_t . V : A = P from tensor memory (16-bit pairs, 8 columns per 16 keys),
       // B = V, unit stride along the value dim (MN-major): 16 keys = 2048 bytes, 64-wide chunks 16 KiB apart
@@ -414,45 +419,45 @@ __global__ void __launch_bounds__(FA_THREADS, 1)
         const uint32_t va = smem_u32(smem + S::KV_OFF + stage * 2 * S::TILE_BYTES + S::TILE_BYTES);
 #pragma unroll
         for (int kk = half * (FA_BN / 32); kk < (half + 1) * (FA_BN / 32); ++kk)
-          tc_mma_f16_ts(t_o[t], t_s[t] + kk * 8, umma_smem_desc_sw128(va + kk * 2048, FA_BM * 128, 1024), p.idesc_pv,
-                        (accumulate || kk != 0) ? 1u : 0u);
-        if (half == 1) tc_commit(&o_ready[t]);
+          tc_mma_f16_ts_lead(t_o[t], t_s[t] + kk * 8, umma_smem_desc_sw128(va + kk * 2048, FA_BM * 128, 1024), p.idesc_pv,
+                             (accumulate || kk != 0) ? 1u : 0u, lead);
+        if (half == 1) tc_commit_lead(smem_u32(&o_ready[t]), lead);
       };
       bool ok = true;
       int n_item = 0;
       for (int w = blockIdx.x; ok && w < p.n_items; w += gridDim.x) {
         const FaItem it = fa_decode_item<MODE>(p, w);
         if (it.n_max <= it.j0) continue;
-        if (!mbar_wait(q_full, static_cast<uint32_t>(n_item & 1), abort_word)) break;
-        if (!mbar_wait(&k_full[kv_cnt % FA_STAGES], static_cast<uint32_t>((kv_cnt / FA_STAGES) & 1), abort_word)) break;
+        if (!mbar_wait_warp(q_full, static_cast<uint32_t>(n_item & 1), abort_word)) break;
+        if (!mbar_wait_warp(&k_full[kv_cnt % FA_STAGES], static_cast<uint32_t>((kv_cnt / FA_STAGES) & 1), abort_word)) break;
         tc_fence_after();
         if (it.n_tiles[0] > it.j0) issue_s(0, kv_cnt % FA_STAGES);
         if (it.n_tiles[1] > it.j0) issue_s(1, kv_cnt % FA_STAGES);
-        if (it.n_max == it.j0 + 1) tc_commit(q_free);
+        if (it.n_max == it.j0 + 1) tc_commit_lead(smem_u32(q_free), lead);
         for (int j = it.j0; j < it.n_max && ok; ++j, ++kv_cnt) {
           const int s = kv_cnt % FA_STAGES;
           const int sn = (kv_cnt + 1) % FA_STAGES;
           const uint32_t ph = static_cast<uint32_t>((kv_cnt / FA_STAGES) & 1);
           const uint32_t ph_next = static_cast<uint32_t>(((kv_cnt + 1) / FA_STAGES) & 1);
-          if (!mbar_wait(&v_full[s], ph, abort_word)) {
+          if (!mbar_wait_warp(&v_full[s], ph, abort_word)) {
             ok = false;
             break;
           }
 #pragma unroll
           for (int t = 0; t < 2; ++t) {
             if (j < it.n_tiles[t]) {
-              if (!mbar_wait(&p_half[t], static_cast<uint32_t>(p_cnt[t] & 1), abort_word)) {
+              if (!mbar_wait_warp(&p_half[t], static_cast<uint32_t>(p_cnt[t] & 1), abort_word)) {
                 ok = false;
                 break;
               }
               if (j == it.j0 && e_cnt[t] > 0 &&
-                  !mbar_wait(&o_free[t], static_cast<uint32_t>((e_cnt[t] - 1) & 1), abort_word)) {
+                  !mbar_wait_warp(&o_free[t], static_cast<uint32_t>((e_cnt[t] - 1) & 1), abort_word)) {
                 ok = false;  // the first P.V of an item overwrites O_t: the previous epilogue must have read it
                 break;
               }
               tc_fence_after();
               issue_pv(t, s, j > it.j0, 0);
-              if (!mbar_wait(&p_full[t], static_cast<uint32_t>(p_cnt[t] & 1), abort_word)) {
+              if (!mbar_wait_warp(&p_full[t], static_cast<uint32_t>(p_cnt[t] & 1), abort_word)) {
                 ok = false;
                 break;
               }
@@ -461,7 +466,7 @@ __global__ void __launch_bounds__(FA_THREADS, 1)
               issue_pv(t, s, j > it.j0, 1);
             }
             if (j + 1 < it.n_tiles[t]) {
-              if (!mbar_wait(&k_full[sn], ph_next, abort_word)) {
+              if (!mbar_wait_warp(&k_full[sn], ph_next, abort_word)) {
                 ok = false;
                 break;
               }
@@ -470,8 +475,8 @@ __global__ void __launch_bounds__(FA_THREADS, 1)
             }
           }
           if (!ok) break;
-          if (j + 2 == it.n_max) tc_commit(q_free);  // the last S MMAs of this item have been issued
-          tc_commit(&kv_empty[s]);  // every MMA that read stage s has been issued before this point
+          if (j + 2 == it.n_max) tc_commit_lead(smem_u32(q_free), lead);  // the last S MMAs of this item have been issued
+          tc_commit_lead(smem_u32(&kv_empty[s]), lead);  // every MMA that read stage s has been issued before this point
         }
         for (int t = 0; t < 2; ++t)
           if (it.n_tiles[t] > it.j0) ++e_cnt[t];

@@ -96,6 +96,11 @@ __device__ __forceinline__ bool mbar_wait(uint64_t* bar, uint32_t parity, volati
   return mbar_wait_limit(bar, parity, abort_word, YTK_WAIT_CYCLES);
 }
 
+// The same for a whole converged warp: one answer.
+__device__ __forceinline__ bool mbar_wait_warp(uint64_t* bar, uint32_t parity, volatile int* abort_word) {
+  return __all_sync(0xffffffffu, mbar_wait(bar, parity, abort_word)) != 0;
+}
+
 // ---------------------------------------------------------------- TMA
 __device__ __forceinline__ void tma_prefetch_desc(const CUtensorMap* m) {
   asm volatile("prefetch.tensormap [%0];" ::"l"(reinterpret_cast<uint64_t>(m)) : "memory");
@@ -394,6 +399,13 @@ __device__ __forceinline__ void tma_load_3d_lead(uint32_t dst, const CUtensorMap
       "{\n\t.reg .pred q;\n\tsetp.ne.b32 q, %6, 0;\n\t"
       "@q cp.async.bulk.tensor.3d.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1, {%2, %3, %4}], [%5];\n\t}" ::"r"(dst),
       "l"(reinterpret_cast<uint64_t>(m)), "r"(c0), "r"(c1), "r"(c2), "r"(bar), "r"(lead)
+      : "memory");
+}
+__device__ __forceinline__ void tma_load_4d_lead(uint32_t dst, const CUtensorMap* m, uint32_t bar, int c0, int c1, int c2, int c3, uint32_t lead) {
+  asm volatile(
+      "{\n\t.reg .pred q;\n\tsetp.ne.b32 q, %7, 0;\n\t"
+      "@q cp.async.bulk.tensor.4d.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1, {%2, %3, %4, %5}], [%6];\n\t}" ::"r"(dst),
+      "l"(reinterpret_cast<uint64_t>(m)), "r"(c0), "r"(c1), "r"(c2), "r"(c3), "r"(bar), "r"(lead)
       : "memory");
 }
 __device__ __forceinline__ void tma_load_3d_pair_lead(uint32_t dst, const CUtensorMap* m, uint32_t bar_cluster_addr, int c0, int c1, int c2,
