@@ -291,6 +291,11 @@ __global__ void __launch_bounds__(FA_THREADS, 1)
     flash_tc_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__ CUtensorMap tmK,
                     const __grid_constant__ CUtensorMap tmV, const FlashParams p) {
   using S = FaSmem<D>;
+  // 64-wide heads, plain: the softmax is what an iteration waits for (their MMAs take three quarters of the time). The maximum
+  // loads scores 32 columns ahead and leaves the upper half of a row in registers, P begins with that half, kept over its own
+  // scores (columns 64 .. 95), and P.V is issued when all of P is there: 8 x 4 heads, 4096 keys 165 -> 160 us. 128-wide heads lose
+  // by it (312 -> 325 us at 2 x 32 heads): they read S twice and hand P over in halves.
+  constexpr bool KEEP = MODE == FA_PLAIN && D == 64;
   extern __shared__ uint8_t smem_raw[];
   const uint32_t raw_addr = smem_u32(smem_raw);
   uint8_t* smem = smem_raw + ((1024u - (raw_addr & 1023u)) & 1023u);
@@ -415,13 +420,16 @@ __global__ void __launch_bounds__(FA_THREADS, 1)
       // B = V, unit stride along the value dim (MN-major): 16 keys = 2048 bytes, 64-wide chunks 16 KiB apart
       // O_t (+)= P_t V in two halves of 64 keys: the first is issued as soon as the softmax warps have published the
       // first half of P, while they still compute the second.
+      constexpr bool HALVES = !KEEP;
+      constexpr int FIRST = KEEP ? 1 : 0;
       auto issue_pv = [&](int t, int stage, bool accumulate, int half) {
+        const uint32_t pa = t_s[t] + (KEEP && half == 1 ? 32 : 0);
         const uint32_t va = smem_u32(smem + S::KV_OFF + stage * 2 * S::TILE_BYTES + S::TILE_BYTES);
 #pragma unroll
         for (int kk = half * (FA_BN / 32); kk < (half + 1) * (FA_BN / 32); ++kk)
-          tc_mma_f16_ts_lead(t_o[t], t_s[t] + kk * 8, umma_smem_desc_sw128(va + kk * 2048, FA_BM * 128, 1024), p.idesc_pv,
-                             (accumulate || kk != 0) ? 1u : 0u, lead);
-        if (half == 1) tc_commit_lead(smem_u32(&o_ready[t]), lead);
+          tc_mma_f16_ts_lead(t_o[t], pa + kk * 8, umma_smem_desc_sw128(va + kk * 2048, FA_BM * 128, 1024), p.idesc_pv,
+                             (accumulate || half != FIRST || kk != half * (FA_BN / 32)) ? 1u : 0u, lead);
+        if (half != FIRST) tc_commit_lead(smem_u32(&o_ready[t]), lead);
       };
       bool ok = true;
       int n_item = 0;
@@ -446,7 +454,7 @@ __global__ void __launch_bounds__(FA_THREADS, 1)
 #pragma unroll
           for (int t = 0; t < 2; ++t) {
             if (j < it.n_tiles[t]) {
-              if (!mbar_wait_warp(&p_half[t], static_cast<uint32_t>(p_cnt[t] & 1), abort_word)) {
+              if (HALVES && !mbar_wait_warp(&p_half[t], static_cast<uint32_t>(p_cnt[t] & 1), abort_word)) {
                 ok = false;
                 break;
               }
@@ -455,18 +463,21 @@ __global__ void __launch_bounds__(FA_THREADS, 1)
                 ok = false;  // the first P.V of an item overwrites O_t: the previous epilogue must have read it
                 break;
               }
-              tc_fence_after();
-              issue_pv(t, s, j > it.j0, 0);
+              if (HALVES) {
+                tc_fence_after();
+                issue_pv(t, s, j > it.j0, FIRST);
+              }
               if (!mbar_wait_warp(&p_full[t], static_cast<uint32_t>(p_cnt[t] & 1), abort_word)) {
                 ok = false;
                 break;
               }
               ++p_cnt[t];
               tc_fence_after();
-              issue_pv(t, s, j > it.j0, 1);
+              if (!HALVES) issue_pv(t, s, j > it.j0, FIRST);
+              issue_pv(t, s, j > it.j0, 1 - FIRST);
             }
             if (j + 1 < it.n_tiles[t]) {
-              if (!mbar_wait_warp(&k_full[sn], ph_next, abort_word)) {
+              if ((t == 0 || j + 1 >= it.n_tiles[0]) && !mbar_wait_warp(&k_full[sn], ph_next, abort_word)) {
                 ok = false;
                 break;
               }
@@ -664,10 +675,37 @@ __global__ void __launch_bounds__(FA_THREADS, 1)
         // pass 1: row maximum. Without mask / bias the maximum is taken over the raw scores (one instruction per
         // element, two with the per-row limit) and scaled afterwards; a negative scale flips max into min.
         float mx = -CUDART_INF_F;
+        uint32_t ra[32], rb[32];  // scores in hand
+        const bool kept = KEEP && full && p.scale_log2 >= 0.f;  // ra, rb: columns 64 .. 127 after the maximum
         if (!elementwise_mask) {
           const bool pos = p.scale_log2 >= 0.f;
           const float ident = pos ? -CUDART_INF_F : CUDART_INF_F;
           float a0 = ident, a1 = ident, a2 = ident, a3 = ident;
+          if (kept) {
+            // the common tile: one three-input max per two elements, four independent chains; a load is on its way while the
+            // one before it is looked at, and the last two stay in registers
+            auto look = [&](const uint32_t (&r)[32]) {
+#pragma unroll
+              for (int e = 0; e < 32; e += 8) {
+                a0 = fmax3(a0, __uint_as_float(r[e]), __uint_as_float(r[e + 1]));
+                a1 = fmax3(a1, __uint_as_float(r[e + 2]), __uint_as_float(r[e + 3]));
+                a2 = fmax3(a2, __uint_as_float(r[e + 4]), __uint_as_float(r[e + 5]));
+                a3 = fmax3(a3, __uint_as_float(r[e + 6]), __uint_as_float(r[e + 7]));
+              }
+            };
+            tmem_ld_32x32b_x32(ts, ra);
+            tmem_ld_wait_for(ra);
+            tmem_ld_32x32b_x32(ts + 32, rb);
+            look(ra);
+            tmem_ld_wait_for(rb);
+            tmem_ld_32x32b_x32(ts + 64, ra);
+            look(rb);
+            tmem_ld_wait_for(ra);
+            tmem_ld_32x32b_x32(ts + 96, rb);
+            look(ra);
+            tmem_ld_wait_for(rb);
+            look(rb);
+          } else {
 #pragma unroll 1
           for (int c0 = 0; c0 < FA_BN; c0 += 64) {
             if (!full && __all_sync(0xffffffffu, cl < c0)) continue;  // no row of this warp sees these columns
@@ -706,6 +744,7 @@ __global__ void __launch_bounds__(FA_THREADS, 1)
                 }
               }
             }
+          }
           }
           const float ext = pos ? fmaxf(fmaxf(a0, a1), fmaxf(a2, a3)) : fminf(fminf(a0, a1), fminf(a2, a3));
           mx = (ext == ident) ? -CUDART_INF_F : ext * p.scale_log2;
@@ -764,13 +803,14 @@ __global__ void __launch_bounds__(FA_THREADS, 1)
           const __half2 h = __floats2half2_rn(p0, p1);
           return *reinterpret_cast<const uint32_t*>(&h);
         };
-        auto publish_half = [&]() {  // columns of P for keys 0..63 are stored: the MMA warp may start P.V on them
+        auto publish_half = [&]() {  // half of P's columns are stored: the MMA warp may start P.V on them
           tmem_st_wait();
           tc_fence_before();
           __syncwarp();
           if (lane == 0) mbar_arrive(&p_half[t]);
         };
-        if (!elementwise_mask) {
+        auto p_at = [&](int c0) { return ts + (KEEP && c0 >= 64 ? 32 : 0) + (c0 >> 1); };  // (see issue_pv)
+        if (!elementwise_mask && !KEEP) {
 #pragma unroll 1
           for (int c0 = 0; c0 < FA_BN; c0 += 64) {
             uint32_t pk[32];
@@ -833,9 +873,81 @@ __global__ void __launch_bounds__(FA_THREADS, 1)
             tmem_st_32x32b_x32(ts + (c0 >> 1), pk);
             if (c0 == 0) publish_half();
           }
+        } else if (!elementwise_mask) {
+          const uint64_t sc2 = f2_pack(p.scale_log2, p.scale_log2), nm2 = f2_pack(neg_m, neg_m);
+          uint64_t lacc = f2_pack(0.f, 0.f), lacc2 = f2_pack(0.f, 0.f);
+          auto body = [&](const uint32_t (&r)[32], int c0, int cc, auto is_bf, auto is_limited) {  // limited: columns 0..cc count
+            uint32_t pk[16];
+#pragma unroll
+            for (int e = 0; e < 32; e += 2) {
+              const uint64_t x2 = f2_fma(f2_pack(__uint_as_float(r[e]), __uint_as_float(r[e + 1])), sc2, nm2);
+              float p0, p1;
+              const bool emu = FA_EMU_EVERY > 0 && ((e >> 1) % (FA_EMU_EVERY > 0 ? FA_EMU_EVERY : 1)) == FA_EMU_EVERY - 1;
+              if (emu) {
+                exp2_emu2(x2, p0, p1);
+              } else {
+                float t0, t1;
+                f2_unpack(x2, t0, t1);
+                p0 = fast_exp2(t0);
+                p1 = fast_exp2(t1);
+              }
+              if (decltype(is_limited)::value) {  // a hidden score may be anything, its P is exactly zero
+                p0 = (e <= cc) ? p0 : 0.f;
+                p1 = (e + 1 <= cc) ? p1 : 0.f;
+              }
+              if (emu) lacc2 = f2_add(lacc2, f2_pack(p0, p1));
+              else lacc = f2_add(lacc, f2_pack(p0, p1));
+              if (decltype(is_bf)::value) {
+                const __nv_bfloat162 h = __floats2bfloat162_rn(p0, p1);
+                pk[e >> 1] = *reinterpret_cast<const uint32_t*>(&h);
+              } else {
+                const __half2 h = __floats2half2_rn(p0, p1);
+                pk[e >> 1] = *reinterpret_cast<const uint32_t*>(&h);
+              }
+            }
+            tmem_st_32x32b_x16(p_at(c0), pk);
+          };
+          auto both = [&](auto is_bf) {
+            if (kept) {  // the upper half is in hand; the lower one comes back while it is worked on
+              body(ra, 64, 32, is_bf, std::false_type{});
+              tmem_ld_32x32b_x32(ts, ra);
+              body(rb, 96, 32, is_bf, std::false_type{});
+              publish_half();
+              tmem_ld_wait_for(ra);
+              tmem_ld_32x32b_x32(ts + 32, rb);
+              body(ra, 0, 32, is_bf, std::false_type{});
+              tmem_ld_wait_for(rb);
+              body(rb, 32, 32, is_bf, std::false_type{});
+            } else {
+#pragma unroll 1
+              for (int i = 0; i < 4; ++i) {
+                const int c0 = ((i + 2) & 3) * 32;
+                // limited tiles: 32 columns that no row of this warp sees (right of the causal diagonal, past
+                // the last key) are written as zeros without reading S or computing exponentials
+                if (!full && __all_sync(0xffffffffu, cl < c0)) {
+                  uint32_t zero[16];
+#pragma unroll
+                  for (int e = 0; e < 16; ++e) zero[e] = 0u;
+                  tmem_st_32x32b_x16(p_at(c0), zero);
+                } else {
+                  tmem_ld_32x32b_x32(ts + c0, ra);
+                  tmem_ld_wait_for(ra);
+                  body(ra, c0, full ? 32 : cl - c0, is_bf, std::true_type{});
+                }
+                if (i == 1) publish_half();
+              }
+            }
+          };
+          if (p.is_bf16) both(std::true_type{});
+          else both(std::false_type{});
+          float la, lb;
+          f2_unpack(f2_add(lacc, lacc2), la, lb);
+          l0 += la;
+          l1 += lb;
         } else {
 #pragma unroll 1
-          for (int c0 = 0; c0 < FA_BN; c0 += 32) {
+          for (int i = 0; i < 4; ++i) {
+            const int c0 = KEEP ? ((i + 2) & 3) * 32 : i * 32;
             uint32_t r[32];
             tmem_ld_32x32b_x32(ts + c0, r);
             tmem_ld_wait();
@@ -848,8 +960,8 @@ __global__ void __launch_bounds__(FA_THREADS, 1)
               l1 += p1;
               pk[e >> 1] = pack2(p0, p1);
             }
-            tmem_st_32x32b_x16(ts + (c0 >> 1), pk);
-            if (c0 == 32) publish_half();
+            tmem_st_32x32b_x16(p_at(c0), pk);
+            if (i == 1) publish_half();
           }
         }
         l_run += l0 + l1;

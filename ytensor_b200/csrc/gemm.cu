@@ -402,7 +402,7 @@ __global__ void __launch_bounds__(TC_THREADS, 1)
       TcBlock<PIECES> at(p, piece, ba, bb);
 #pragma unroll 1
       for (int kb = piece.kb0; kb < piece.kb1; ++kb, at.next(p, piece, ba, bb)) {
-        if (stage % S::FREED == 0 && !__all_sync(0xffffffffu, mbar_wait(&empty_bar[stage / S::FREED], phase ^ 1u, abort_word))) {
+        if (stage % S::FREED == 0 && !mbar_wait_warp(&empty_bar[stage / S::FREED], phase ^ 1u, abort_word)) {
           ok = false;
           break;
         }
@@ -470,14 +470,14 @@ __global__ void __launch_bounds__(TC_THREADS, 1)
     for (int tile = blockIdx.x; ok && tile < p.total_tiles; tile += gridDim.x) {
       if (p.tile_live && !p.tile_live[tile % tiles_per_batch]) continue;
       if (p.tile_group && p.tile_group[(tile % tiles_per_batch) / p.tiles_n] < 0) continue;
-      if (!__all_sync(0xffffffffu, mbar_wait(&tempty_bar[acc], acc_phase ^ 1u, abort_word))) break;
+      if (!mbar_wait_warp(&tempty_bar[acc], acc_phase ^ 1u, abort_word)) break;
       tc_fence_after();
       const uint32_t d_tmem = tmem_base + static_cast<uint32_t>(acc * BN);
       TcPiece piece{0, 0, p.k_blocks, 0};
       if (PIECES) piece = tc_piece(p, tile / tiles_per_batch);
 #pragma unroll 1
       for (int kb = piece.kb0; kb < piece.kb1; ++kb) {
-        if (!ready && !__all_sync(0xffffffffu, mbar_wait(&full_bar[stage], phase, abort_word))) {
+        if (!ready && !mbar_wait_warp(&full_bar[stage], phase, abort_word)) {
           ok = false;
           break;
         }
@@ -649,7 +649,7 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(TC_THREADS, 1)
       TcBlock<PIECES> at(p, piece, ba, bb);
 #pragma unroll 1
       for (int kb = 0; kb < p.k_blocks; ++kb, at.next(p, piece, ba, bb)) {
-        if ((stage & 1) == 0 && !__all_sync(0xffffffffu, mbar_wait(&empty_bar[stage >> 1], phase ^ 1u, abort_word))) {
+        if ((stage & 1) == 0 && !mbar_wait_warp(&empty_bar[stage >> 1], phase ^ 1u, abort_word)) {
           ok = false;
           break;
         }
@@ -689,12 +689,12 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(TC_THREADS, 1)
       uint32_t acc_phase = 0;
       bool ok = true, ready = false;
       for (int tile = cluster_id; ok && tile < p.total_tiles; tile += n_clusters) {
-        if (!__all_sync(0xffffffffu, mbar_wait(&tempty_bar[acc], acc_phase ^ 1u, abort_word))) break;
+        if (!mbar_wait_warp(&tempty_bar[acc], acc_phase ^ 1u, abort_word)) break;
         tc_fence_after();
         const uint32_t d_tmem = tmem_base + static_cast<uint32_t>(acc * TC2_BN);
 #pragma unroll 1
         for (int kb = 0; kb < p.k_blocks; ++kb) {
-          if (!ready && !__all_sync(0xffffffffu, mbar_wait(&full_bar[stage], phase, abort_word))) {
+          if (!ready && !mbar_wait_warp(&full_bar[stage], phase, abort_word)) {
             ok = false;
             break;
           }
