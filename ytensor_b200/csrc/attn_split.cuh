@@ -146,7 +146,7 @@ __global__ void __launch_bounds__(SA_THREADS, 1)
   uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(bars + SA_NBAR);
   volatile int* abort_word = reinterpret_cast<volatile int*>(tmem_slot + 1);
   int* unfit_word = reinterpret_cast<int*>(tmem_slot + 2);
-  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  const int warp = __shfl_sync(0xffffffffu, threadIdx.x >> 5, 0), lane = threadIdx.x & 31;  // (known to be the same for the warp)
   const int bkv = p.a.batch * p.a.kv_heads;
 
   if (threadIdx.x == 0) {
@@ -189,53 +189,52 @@ __global__ void __launch_bounds__(SA_THREADS, 1)
     asm volatile("setmaxnreg.dec.sync.aligned.u32 72;");
     if (warp == 0) {
       // ------------------------------------------------------------ TMA producer
-      if (lane == 0) {
-        const int kblocks = (p.a.d + 63) / 64, vblocks = (p.a.dv + 63) / 64;
-        int n_pl = 0;
-        auto load = [&](const CUtensorMap* tm, int blocks, int tile, int bh) {
+      // (converged like the issuer: inside a branch of one lane the twelve copies of a tile took as long as its MMAs)
+      const uint32_t lead = lane == 0 ? 1u : 0u;
+      const uint32_t ring_at = smem_u32(smem + SA_RING_OFF), full_at = smem_u32(full);
+      const int kblocks = (p.a.d + 63) / 64, vblocks = (p.a.dv + 63) / 64;
+      int n_pl = 0;
+      auto load = [&](const CUtensorMap* tm, int blocks, int tile, int bh) {
 #pragma unroll 1
-          for (int i = p.planes - 1; i >= 0; --i, ++n_pl) {
-            const int s = n_pl % SA_SLOTS;
-            if (!mbar_wait(&empty[s], ((n_pl / SA_SLOTS) & 1) ^ 1, abort_word)) return false;
-            mbar_expect_tx(&full[s], static_cast<uint32_t>(blocks * SA_BLOCK));
+        for (int i = p.planes - 1; i >= 0; --i, ++n_pl) {
+          const int s = n_pl % SA_SLOTS;
+          if (!mbar_wait_warp(&empty[s], ((n_pl / SA_SLOTS) & 1) ^ 1, abort_word)) return false;
+          mbar_expect_tx_lead(full_at + 8 * s, static_cast<uint32_t>(blocks * SA_BLOCK), lead);
 #pragma unroll 1
-            for (int c = 0; c < blocks; ++c)
-              tma_load_3d(smem + SA_RING_OFF + s * SA_PLANE + c * SA_BLOCK, tm, &full[s], c * 64, tile * SA_BN, i * bkv + bh);
-          }
-          return true;
-        };
-        bool ok = true;
-        for (int w = blockIdx.x; ok && w < p.n_items; w += gridDim.x) {
-          const SplitItem it = split_item(p, w);
-          const int bh = p.flat ? it.unit : it.unit / p.a.groups;
-          for (int j = 0; ok && j < 2 && j < it.n; ++j) ok = load(&tmK, kblocks, j, bh);
-          for (int j = 0; ok && j < it.n; ++j) {
-            ok = load(&tmV, vblocks, j, bh);
-            if (ok && j + 2 < it.n) ok = load(&tmK, kblocks, j + 2, bh);
-          }
+          for (int c = 0; c < blocks; ++c)
+            tma_load_3d_lead(ring_at + s * SA_PLANE + c * SA_BLOCK, tm, full_at + 8 * s, c * 64, tile * SA_BN, i * bkv + bh, lead);
         }
-        // a give-up elsewhere: bounded drain of the last copies
-        const long long t0 = clock64();
-        for (int k = n_pl - SA_SLOTS > 0 ? n_pl - SA_SLOTS : 0; k < n_pl; ++k)
-          while (!mbar_try_wait(&full[k % SA_SLOTS], (k / SA_SLOTS) & 1) && clock64() - t0 < 20000000ll) {
-          }
+        return true;
+      };
+      bool ok = true;
+      for (int w = blockIdx.x; ok && w < p.n_items; w += gridDim.x) {
+        const SplitItem it = split_item(p, w);
+        const int bh = p.flat ? it.unit : it.unit / p.a.groups;
+        for (int j = 0; ok && j < 2 && j < it.n; ++j) ok = load(&tmK, kblocks, j, bh);
+        for (int j = 0; ok && j < it.n; ++j) {
+          ok = load(&tmV, vblocks, j, bh);
+          if (ok && j + 2 < it.n) ok = load(&tmK, kblocks, j + 2, bh);
+        }
       }
+      // a give-up elsewhere: bounded drain of the last copies
+      const long long t0 = clock64();
+      for (int k = n_pl - SA_SLOTS > 0 ? n_pl - SA_SLOTS : 0; k < n_pl; ++k)
+        while (!mbar_try_wait(&full[k % SA_SLOTS], (k / SA_SLOTS) & 1) && clock64() - t0 < 20000000ll) {
+        }
+      __syncwarp();
     } else if (warp == 1) {
       // ------------------------------------------------------------ MMA issuer
       // The whole warp runs this code and lane 0 issues: straight code, constant offsets, operands in uniform registers
       // (a loop that forms descriptors in a one-lane branch costs 190 clocks per MMA, the tensor pipe needs 64).
-      const uint32_t lead = lane == 0;
+      const uint32_t lead = lane == 0 ? 1u : 0u;
       const uint64_t qd = umma_smem_desc_sw128(smem_u32(smem + SA_Q_OFF), 16, 1024);
       const uint64_t kd = umma_smem_desc_sw128(smem_u32(smem + SA_RING_OFF), 16, 1024);
       const uint64_t vd = umma_smem_desc_sw128(smem_u32(smem + SA_RING_OFF), SA_BLOCK, 1024);
       constexpr uint32_t PLANE = SA_PLANE / 16, BLOCK = SA_BLOCK / 16;  // (descriptors count 16 bytes)
       const int ksteps = (p.a.d + 15) / 16;
       // (every lane waits: a give-up is agreed on before the next step)
-      auto wait = [&](uint64_t* bar, uint32_t ph) { return __all_sync(0xffffffffu, mbar_wait(bar, ph, abort_word)) != 0; };
-      auto commit = [&](uint64_t* bar) {
-        if (lead) tc_commit(bar);
-        __syncwarp();
-      };
+      auto wait = [&](uint64_t* bar, uint32_t ph) { return mbar_wait_warp(bar, ph, abort_word); };
+      auto commit = [&](uint64_t* bar) { tc_commit_lead(smem_u32(bar), lead); };
       int n_pl = 0;
       // The products of plane J of K (or V) with planes I of Q (or P), I + J <= 2, the smallest first
       auto k_plane = [&](auto plane, uint32_t ds, uint32_t idesc) {
