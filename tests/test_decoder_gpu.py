@@ -322,6 +322,22 @@ def test_long_prompts_of_wide_models(Q):
     m.close()
 
 
+@pytest.mark.parametrize("inter,rows", [(2816, 1100), (2824, 1025), (4104, 600)])
+def test_activation_in_the_products_epilogue(Q, inter, rows):
+    """Prompts long enough for CTA pairs: swish(gate) * up and its planes come from the gate / up product itself, at FFN widths that
+    end inside a tile of 128 outputs and rows that end inside one of 256. The same prompt in parts of 100 rows takes the other
+    kernels; both keep two planes and fp32 sums."""
+    cfg = Q.Qwen3Config(**{**SMALL, "hidden_size": 256, "intermediate_size": inter, "max_position_embeddings": 1200})
+    m = Q.Qwen3ForCausalLM(cfg)
+    m.load_weights(Q.random_weights(cfg, seed=3, std=0.05))
+    ids = np.random.default_rng(1).integers(0, 512, (1, rows))
+    for i in range(0, rows, 100):
+        want = m.forward(dev_ids(ids[:, i:i + 100])).cpu().numpy()
+    m.reset_kv_cache()
+    assert normwise(m.forward(dev_ids(ids)).cpu().numpy(), want) < 2e-5
+    m.close()
+
+
 def test_long_prompts_of_an_odd_share_of_the_ffn(Q):
     """A rank whose share of the FFN has rows that do not start at 16 bytes (40 / 2 columns) computes what one GPU does with
     the same weights and columns of zeros behind them. The sums over the ranks are left out."""

@@ -385,72 +385,91 @@ __global__ void __launch_bounds__(256) swiglu_split_kernel(const float* gu, uint
 }
 
 // ------------------------------------------------------------------ per-head RMSNorm + RoPE + KV append
-// qkv [B, L, (H + 2*KVH) * D] fp32 (the fused projection output). One warp per (b, t, head) vector, D == 128:
+// qkv [B, L, (H + 2*KVH) * D] fp32 (the fused projection output). One warp per (b, t) and four heads, D == 128, four neighbouring
+// dims of each a lane:
 //   q heads: rmsNorm over D with q_norm, rotate-half RoPE at position pos0 + t -> q_out [B, H, L, D]
 //   k heads: rmsNorm with k_norm, RoPE -> k_cache [B, KVH, max_len, D] at slot (slot0 + t) % max_len (the cache is a
 //            ring buffer: KVCache::append, qwen3.cpp:70-88)
 //   v heads: copy -> v_cache at the same slot
 // (reference qwen3.cpp:237-247: slice/reshape/permute, HeadRMSNorm, ops::rope, KVCache::append; rope math :522-559).
+// Bound by memory: 4 bytes read and written a value. A warp has its four vectors on their way at once (eight: 20.1 us, fewer warps fit):
+// 2000 rows of 32 heads 23.0 -> 18.6 us (one vector after another).
+// One head a warp where four would leave SMs without work.
+template <int QP_HEADS>
 __global__ void __launch_bounds__(128) qkv_post_kernel(const float* qkv, float* q_out, float* k_cache, float* v_cache,
                                                        const float* q_norm, const float* k_norm, const float* cos_t,
                                                        const float* sin_t, int B, int L, int H, int KVH, int max_len,
-                                                       int pos0, int slot0, float eps, int n_part, int64_t mn) {
+                                                       int pos0, int slot0, float eps, int n_part, int64_t mn, int wide) {
   dependent_wait();
   dependent_trigger();
   constexpr int D = 128;
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   const int heads_all = H + 2 * KVH;
-  const int64_t vecs = static_cast<int64_t>(B) * L * heads_all;
-  for (int64_t v = static_cast<int64_t>(blockIdx.x) * 4 + warp; v < vecs; v += static_cast<int64_t>(gridDim.x) * 4) {
-    const int hh = static_cast<int>(v % heads_all);
-    const int t = static_cast<int>((v / heads_all) % L);
-    const int b = static_cast<int>(v / (static_cast<int64_t>(heads_all) * L));
-    const float* src = qkv + (static_cast<int64_t>(b) * L + t) * heads_all * D + static_cast<int64_t>(hh) * D;
-    float x[4];
-    if (n_part > 0) {  // `qkv` holds the k-split partial products [pieces][2][B * L][heads_all * D]: add them here
-#pragma unroll
-      for (int i = 0; i < 4; ++i) x[i] = 0.f;
-#pragma unroll 8
-      for (int p = 0; p < n_part; ++p) {
-#pragma unroll
-        for (int i = 0; i < 4; ++i) x[i] += src[2 * p * mn + lane + 32 * i] + src[(2 * p + 1) * mn + lane + 32 * i];
-      }
+  auto get = [&](const float* p) {  // (wide: every tensor starts at 16 bytes)
+    return wide ? *reinterpret_cast<const float4*>(p) : make_float4(p[0], p[1], p[2], p[3]);
+  };
+  auto put = [&](float* p, const float4& x) {
+    if (wide) {
+      *reinterpret_cast<float4*>(p) = x;
     } else {
-#pragma unroll
-      for (int i = 0; i < 4; ++i) x[i] = src[lane + 32 * i];
+      p[0] = x.x; p[1] = x.y; p[2] = x.z; p[3] = x.w;
     }
-    if (hh >= H + KVH) {  // value head
-      float* dst = v_cache + ((static_cast<int64_t>(b) * KVH + (hh - H - KVH)) * max_len + (slot0 + t) % max_len) * D;
-#pragma unroll
-      for (int i = 0; i < 4; ++i) dst[lane + 32 * i] = x[i];
-      continue;
+  };
+  const float4 gq = get(q_norm + 4 * lane), gk = get(k_norm + 4 * lane);
+  auto load = [&](int64_t v) {
+    const float* src = qkv + v * D + 4 * lane;
+    float4 x = make_float4(0.f, 0.f, 0.f, 0.f);
+    if (n_part == 0) return get(src);
+#pragma unroll 4
+    for (int p = 0; p < n_part; ++p) {  // the k-split partial products [pieces][2][B * L][heads_all * D]: added here
+      const float4 a = *reinterpret_cast<const float4*>(src + 2 * p * mn), b = *reinterpret_cast<const float4*>(src + (2 * p + 1) * mn);
+      x.x += a.x + b.x; x.y += a.y + b.y; x.z += a.z + b.z; x.w += a.w + b.w;
     }
-    const bool is_q = hh < H;
-    float ss = x[0] * x[0];
-    ss = fmaf(x[1], x[1], ss);
-    ss = fmaf(x[2], x[2], ss);
-    ss = fmaf(x[3], x[3], ss);
+    return x;
+  };
+  const int groups = (heads_all + QP_HEADS - 1) / QP_HEADS;
+  const int64_t tasks = static_cast<int64_t>(B) * L * groups;
+  for (int64_t task = static_cast<int64_t>(blockIdx.x) * 4 + warp; task < tasks; task += static_cast<int64_t>(gridDim.x) * 4) {
+    const int64_t row = tasks <= 0xffffffffll ? static_cast<uint32_t>(task) / static_cast<uint32_t>(groups) : task / groups;
+    const int h0 = static_cast<int>(task - row * groups) * QP_HEADS;
+    const int b = static_cast<int>(row <= 0xffffffffll ? static_cast<uint32_t>(row) / static_cast<uint32_t>(L) : row / L);
+    const int t = static_cast<int>(row - static_cast<int64_t>(b) * L);
+    int slot = slot0 + t;  // (len <= max_len)
+    if (slot >= max_len) slot -= max_len;
+    float4 x[QP_HEADS];
 #pragma unroll
-    for (int o = 16; o > 0; o >>= 1) ss += __shfl_xor_sync(0xffffffffu, ss, o);
-    const float denom = sqrtf(ss * (1.0f / D) + eps);
-    const float* wn = is_q ? q_norm : k_norm;
+    for (int i = 0; i < QP_HEADS; ++i)
+      if (h0 + i < heads_all) x[i] = load(row * heads_all + h0 + i);
+    // rotate-half pairs (i, i + 64): the other one is 16 lanes away; both halves of a row of the tables hold the same values
+    const float4 c4 = get(cos_t + static_cast<int64_t>(pos0 + t) * D + 4 * lane);
+    float4 s4 = get(sin_t + static_cast<int64_t>(pos0 + t) * D + 4 * lane);
+    if (lane < 16) s4 = make_float4(-s4.x, -s4.y, -s4.z, -s4.w);
 #pragma unroll
-    for (int i = 0; i < 4; ++i) x[i] = (x[i] / denom) * wn[lane + 32 * i];
-    // rotate-half pairs (i, i + 64): elements {lane, lane+64} and {lane+32, lane+96} sit in this lane
-    const float* cr = cos_t + static_cast<int64_t>(pos0 + t) * D;
-    const float* sr = sin_t + static_cast<int64_t>(pos0 + t) * D;
-    float y[4];
+    for (int i = 0; i < QP_HEADS; ++i) {
+      const int hh = h0 + i;
+      if (hh >= heads_all) break;
+      if (hh >= H + KVH) {  // value head
+        put(v_cache + ((static_cast<int64_t>(b) * KVH + (hh - H - KVH)) * max_len + slot) * D + 4 * lane, x[i]);
+        continue;
+      }
+      const bool is_q = hh < H;
+      float ss = x[i].x * x[i].x;
+      ss = fmaf(x[i].y, x[i].y, ss);
+      ss = fmaf(x[i].z, x[i].z, ss);
+      ss = fmaf(x[i].w, x[i].w, ss);
 #pragma unroll
-    for (int i = 0; i < 2; ++i) {
-      const float c = cr[lane + 32 * i], s = sr[lane + 32 * i];
-      const float re = x[i], im = x[i + 2];
-      y[i] = re * c - im * s;
-      y[i + 2] = im * c + re * s;
+      for (int o = 16; o > 0; o >>= 1) ss += __shfl_xor_sync(0xffffffffu, ss, o);
+      const float inv = 1.0f / sqrtf(ss * (1.0f / D) + eps);
+      const float4 g = is_q ? gq : gk;
+      const float4 n = make_float4(x[i].x * inv * g.x, x[i].y * inv * g.y, x[i].z * inv * g.z, x[i].w * inv * g.w);
+      float4 y;
+      y.x = n.x * c4.x + __shfl_xor_sync(0xffffffffu, n.x, 16) * s4.x;
+      y.y = n.y * c4.y + __shfl_xor_sync(0xffffffffu, n.y, 16) * s4.y;
+      y.z = n.z * c4.z + __shfl_xor_sync(0xffffffffu, n.z, 16) * s4.z;
+      y.w = n.w * c4.w + __shfl_xor_sync(0xffffffffu, n.w, 16) * s4.w;
+      put((is_q ? q_out + ((static_cast<int64_t>(b) * H + hh) * L + t) * D
+                : k_cache + ((static_cast<int64_t>(b) * KVH + (hh - H)) * max_len + slot) * D) + 4 * lane, y);
     }
-    float* dst = is_q ? q_out + ((static_cast<int64_t>(b) * H + hh) * L + t) * D
-                      : k_cache + ((static_cast<int64_t>(b) * KVH + (hh - H)) * max_len + (slot0 + t) % max_len) * D;
-#pragma unroll
-    for (int i = 0; i < 4; ++i) dst[lane + 32 * i] = y[i];
   }
 }
 
@@ -716,12 +735,17 @@ static int qkv_post_launch(const float* qkv, int n_part, int64_t mn, float* q_ou
               "ytcuda_qwen3_qkv_post: %d new tokens at slot %d do not fit a ring of %d slots", len, slot0, max_len);
   YTC_REQUIRE(pos0 >= 0 && pos0 + len <= max_len, "ytcuda_qwen3_qkv_post: rotary positions %d .. %d outside the table of %d",
               pos0, pos0 + len - 1, max_len);
-  const int64_t vecs = static_cast<int64_t>(batch) * len * (heads + 2 * kv_heads);
-  const int64_t blocks = (vecs + 3) / 4;
-  const int64_t cap = static_cast<int64_t>(sm_count()) * 16;
-  YTC_CUDA(launch_overlapped(qkv_post_kernel, dim3(static_cast<unsigned>(blocks < cap ? blocks : cap)), dim3(128), 0,
+  uint64_t places = 0;
+  for (const void* x : {static_cast<const void*>(qkv), static_cast<const void*>(q_out), static_cast<const void*>(k_cache), static_cast<const void*>(v_cache),
+                        static_cast<const void*>(q_norm), static_cast<const void*>(k_norm), static_cast<const void*>(cos_table), static_cast<const void*>(sin_table)})
+    places |= reinterpret_cast<uint64_t>(x);
+  const int wide = (places & 15) == 0 ? 1 : 0;
+  const int64_t rows = static_cast<int64_t>(batch) * len, cap = static_cast<int64_t>(sm_count()) * 16;
+  const bool four = rows * ((heads + 2 * kv_heads + 3) / 4) >= cap;
+  const int64_t blocks = (rows * (four ? (heads + 2 * kv_heads + 3) / 4 : heads + 2 * kv_heads) + 3) / 4;
+  YTC_CUDA(launch_overlapped(four ? qkv_post_kernel<4> : qkv_post_kernel<1>, dim3(static_cast<unsigned>(blocks < cap ? blocks : cap)), dim3(128), 0,
                              static_cast<cudaStream_t>(stream), qkv, q_out, k_cache, v_cache, q_norm, k_norm, cos_table,
-                             sin_table, batch, len, heads, kv_heads, max_len, pos0, slot0, eps, n_part, mn));
+                             sin_table, batch, len, heads, kv_heads, max_len, pos0, slot0, eps, n_part, mn, wide));
   count_launch();
   YTC_CUDA(cudaGetLastError());
   return YTC_OK;
@@ -1388,13 +1412,21 @@ int ytcuda_qwen3_forward(void* handle, const int32_t* ids, int len, float* logit
     float* mlp = m->tp_world == 1 ? m->x : m->proj;  // (x2 += mlp, or this rank's share of it)
     if (planes) {
       if ((s = rmsnorm_planes(m->x, W.norm2, m->hi, rows, Hd, m->eps, st)) != YTC_OK) return s;
-      if ((s = linear_two_planes(m->hi, W.gate_up, m->gu, 2 * m->l_inter, static_cast<int>(rows), 2 * m->l_inter, Hd, false, st)) != YTC_OK)
+      // (the planes of the activation lie in m->act, 4 bytes a value: the product still reads those in m->hi)
+      uint16_t* act = reinterpret_cast<uint16_t*>(m->act);
+      s = swiglu_two_planes(m->hi, W.gate_up, act, static_cast<int>(rows), m->l_inter, Hd, st);
+      if (s == YTC_UNSUPPORTED) {
+        act = m->hi;
+        if ((s = linear_two_planes(m->hi, W.gate_up, m->gu, 2 * m->l_inter, static_cast<int>(rows), 2 * m->l_inter, Hd, false, st)) != YTC_OK)
+          return s;
+        const int64_t blocks = (rows * (m->l_inter / 4) + 255) / 256;
+        YTC_CUDA(launch_overlapped(swiglu_split_kernel, dim3(static_cast<unsigned>(blocks < glue_cap ? blocks : glue_cap)), dim3(256), 0,
+                                   st, m->gu, m->hi, m->hi + rows * m->l_inter, rows, m->l_inter));
+        count_launch();
+      } else if (s != YTC_OK) {
         return s;
-      const int64_t blocks = (rows * (m->l_inter / 4) + 255) / 256;
-      YTC_CUDA(launch_overlapped(swiglu_split_kernel, dim3(static_cast<unsigned>(blocks < glue_cap ? blocks : glue_cap)), dim3(256), 0,
-                                 st, m->gu, m->hi, m->hi + rows * m->l_inter, rows, m->l_inter));
-      count_launch();
-      if ((s = linear_two_planes(m->hi, W.down, mlp, Hd, static_cast<int>(rows), Hd, m->l_inter, m->tp_world == 1, st)) != YTC_OK)
+      }
+      if ((s = linear_two_planes(act, W.down, mlp, Hd, static_cast<int>(rows), Hd, m->l_inter, m->tp_world == 1, st)) != YTC_OK)
         return s;
     } else {
       if ((s = rmsnorm_rows(m->x, W.norm2, m->h, rows, Hd, m->eps, st)) != YTC_OK) return s;

@@ -76,7 +76,8 @@ struct Vec8<uint16_t> {
 // columns, the others as they are; EPI_CLAMP_PAIRS: gate and up rows as in EPI_SWIGLU_PAIRS, g = min(gate, limit),
 // u = up bounded to [-limit, limit], g sigmoid(alpha g) (u + shift). All but EPI_NONE store bf16 (linear_tc) or fp32
 // (linear_f32).
-enum { EPI_NONE = 0, EPI_BF16 = 1, EPI_GELU_ERF = 2, EPI_SWIGLU_PAIRS = 3, EPI_RELU2 = 4, EPI_SILU = 5, EPI_CLAMP_PAIRS = 6 };
+enum { EPI_NONE = 0, EPI_BF16 = 1, EPI_GELU_ERF = 2, EPI_SWIGLU_PAIRS = 3, EPI_RELU2 = 4, EPI_SILU = 5, EPI_CLAMP_PAIRS = 6,
+       EPI_SWIGLU_PLANES = 7 };  // (swiglu_two_planes)
 inline bool epi_pairs(int epi) { return epi == EPI_SWIGLU_PAIRS || epi == EPI_CLAMP_PAIRS; }
 struct LinearEpilogue {
   int epi = EPI_NONE;

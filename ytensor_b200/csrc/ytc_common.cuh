@@ -280,6 +280,9 @@ int gemm_into_workspace(int dtype_in, int dtype_out, const void* A, const void* 
                         int64_t bsa, int64_t bsb, int64_t bsc, cudaStream_t st);
 // y[m, n] (+)= (hi + lo)[m, k] . W[n, k]^T, planes = hi [m][k], then lo, bf16 (gemm.cu).
 int linear_two_planes(const void* planes, const void* w, float* y, int64_t ldy, int m, int n, int k, bool accumulate, cudaStream_t st);
+// out = planes (hi [m][inter], then lo, bf16) of swish(gate) * up with [gate; up] = (hi + lo)[m, k] . W[2 inter, k]^T (gemm.cu);
+// YTC_UNSUPPORTED (nothing queued) for products that CTA pairs do not take.
+int swiglu_two_planes(const void* planes, const void* w, void* out, int m, int inter, int k, cudaStream_t st);
 // rmsNorm of contiguous fp32 rows into two bf16 planes, hi [rows][hidden], then lo (rowops.cu); hidden % 4 == 0, at most:
 constexpr int RMS_PLANES_MAX = 16384;
 int rmsnorm_planes(const float* x, const float* w, uint16_t* planes, int64_t rows, int hidden, float eps, cudaStream_t st);
