@@ -256,3 +256,22 @@ def test_channel_norms_of_many_short_lines(api):
     for got, axes in ((api.instanceNorm(x, w, b), (2,)), (api.batchNorm(x, w, b), (0, 2))):
         want = _sixty_four(x, axes, "layerNorm", w.double()[:, None], b.double()[:, None])
         assert (got.double() - want).abs().max() <= 1e-5 * want.abs().max()  # (variances near zero: eps of 1e-5 under the root)
+
+
+@pytest.mark.parametrize("n,c,h,w", [(1, 3, 16, 32), (3, 5, 8, 64), (2, 7, 37, 44), (16, 96, 28, 28), (1, 2, 300, 260), (5, 300, 12, 12)])
+def test_channel_norm_by_bulk_copies(n, c, h, w):
+    """fp32 channel norms whose runs (h * w elements, a multiple of four, from 128 on) come and go as bulk copies: one and several
+    shares per channel, shares that end inside a run and are empty, in place, gamma and bias per channel or none. 64-bit oracle;
+    fp32 statistics of R values are off by a few 2^-24, tolerance 2e-6."""
+    from ytensor_b200 import api
+    g = torch.Generator(device="cuda").manual_seed(n * c + h)
+    x = torch.randn(n, c, h, w, generator=g, device="cuda") * 1.5 + 0.3
+    ga, be = (torch.randn(c, generator=g, device="cuda") for _ in range(2))
+    d = x.double()
+    want = (d - d.mean((0, 2, 3), keepdim=True)) / torch.sqrt(d.var((0, 2, 3), unbiased=False, keepdim=True) + 1e-5)
+    affine = want * ga.double()[:, None, None] + be.double()[:, None, None]
+    for got, ref in ((api.batchNorm(x), want), (api.batchNorm(x, ga, be), affine), (api.batchNorm_(x.clone(), ga, be), affine)):
+        assert float((got.double() - ref).abs().max() / ref.abs().max()) < 2e-6
+    plane = api.layerNorm(x, torch.ones(h, w, device="cuda") * 2, torch.ones(h, w, device="cuda"), (2, 3))  # runs without a channel
+    ref = (d - d.mean((2, 3), keepdim=True)) / torch.sqrt(d.var((2, 3), unbiased=False, keepdim=True) + 1e-5) * 2 + 1
+    assert float((plane.double() - ref).abs().max() / ref.abs().max()) < 2e-6

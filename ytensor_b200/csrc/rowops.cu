@@ -585,8 +585,9 @@ __global__ void __launch_bounds__(128) line_kernel(const LineParams p) {
 // a share per CTA of a cluster, and pass the partial results through distributed shared memory in the order of the ranks:
 // one read and one write of HBM per element and one launch, where line_kernel walks an odometer with a 64-bit division per
 // element and pass, on one CTA (or thread) per line. Shares above CACHE_FLOATS are read again instead.
-// What bounds them: span_kernel the loads in flight while a share comes in and goes out (16 x 96 x 56 x 56 fp32 over all axes but
-// the channel, gamma and bias included: 965 us with line_kernel and two elementwise passes, 25 here, 6 at the copy rate);
+// What bounds them: span_kernel the two trips to memory with the sums between them: fp32 shares come in and leave as bulk copies
+// of whole runs (16 x 96 x 56 x 56 fp32 over all axes but the channel, gamma and bias included: 965 us with line_kernel and two
+// elementwise passes, 22.6 with four 16-byte loads a thread in flight and a division a load, 15.8 here, 6 at the copy rate);
 // column_kernel the latency of its 32-column rows (softmax of fp32 2048 x 4096 along the first axis: 2891 / 60 us).
 constexpr int SHARE_UNROLL = 4, MAX_SHARES = 8;
 constexpr uint32_t CACHE_FLOATS = 50u * 1024;
@@ -606,6 +607,8 @@ struct ShareParams {
   uint32_t share;          // elements per CTA
   int shares;
   int cached;
+  int bulk_in, bulk_out;   // span_kernel: whole runs come into the cache, results leave it, as bulk copies (fp32)
+  int* status;
   float eps, lp;
   int dt_in, dt_out, dt_w;
 };
@@ -690,6 +693,15 @@ __device__ __forceinline__ void line_passes(const ShareParams& p, Sweep&& sweep,
   }
 }
 
+__device__ __forceinline__ void share_copy_in(void* dst, const void* src, uint32_t bytes, uint64_t* bar) {
+  asm volatile("cp.async.bulk.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1], %2, [%3];" ::"r"(smem_u32(dst)), "l"(src),
+               "r"(bytes), "r"(smem_u32(bar))
+               : "memory");
+}
+__device__ __forceinline__ void share_copy_out(void* dst, const void* src, uint32_t bytes) {
+  asm volatile("cp.async.bulk.global.shared::cta.bulk_group [%0], [%1], %2;" ::"l"(dst), "r"(smem_u32(src)), "r"(bytes) : "memory");
+}
+
 template <int OP, int VEC, int THREADS>
 __global__ void __launch_bounds__(THREADS) span_kernel(const ShareParams p) {
   extern __shared__ __align__(16) float cache[];
@@ -707,6 +719,30 @@ __global__ void __launch_bounds__(THREADS) span_kernel(const ShareParams p) {
     wb += c * p.kws[d];
   }
   const uint32_t begin = rank * p.share, end = min(begin + p.share, p.R);
+  // f(element of the share, its run, its place in the run, elements) for the parts of runs that the share holds, by one warp
+  auto parts = [&](auto f) {
+    const uint32_t first = begin < end ? begin / p.R2 : 0, n = begin < end ? (end - 1) / p.R2 - first + 1 : 0;
+    for (uint32_t k = tid; k < n && tid < 32; k += 32) {
+      const uint32_t run = first + k, lo = max(begin, run * p.R2), hi = min(end, (run + 1) * p.R2);
+      f(lo - begin, run, lo - run * p.R2, hi - lo);
+    }
+  };
+  const bool bulk_in = VEC == 4 && p.bulk_in;
+  if (bulk_in) {
+    __shared__ __align__(8) uint64_t arrived;
+    __shared__ int abort_word;
+    if (tid == 0) {
+      abort_word = 0;
+      mbar_init(&arrived, 1);
+      fence_mbar_init();
+      mbar_expect_tx(&arrived, (begin < end ? end - begin : 0) * 4);
+    }
+    __syncthreads();
+    parts([&](uint32_t at, uint32_t run, uint32_t off, uint32_t n) {
+      share_copy_in(cache + at, static_cast<const float*>(p.x) + xb + run * p.xs1 + off, n * 4, &arrived);
+    });
+    if (!mbar_wait(&arrived, 0, &abort_word)) atomicExch(p.status, YTC_TIMEOUT);
+  }
   auto load = [&](uint32_t r) {
     const uint32_t r1 = p.R2 == p.R ? 0u : r / p.R2;
     const int64_t o = xb + r1 * p.xs1 + (r - r1 * p.R2);
@@ -735,12 +771,12 @@ __global__ void __launch_bounds__(THREADS) span_kernel(const ShareParams p) {
       F4 x[SHARE_UNROLL];
 #pragma unroll
       for (int u = 0; u < SHARE_UNROLL; ++u)
-        if (r0 + u * STEP < end) x[u] = first ? load(r0 + u * STEP) : cached(r0 + u * STEP);
+        if (r0 + u * STEP < end) x[u] = first && !bulk_in ? load(r0 + u * STEP) : cached(r0 + u * STEP);
 #pragma unroll
       for (int u = 0; u < SHARE_UNROLL; ++u) {
         const uint32_t r = r0 + u * STEP;
         if (r >= end) break;
-        if (first && p.cached && OP != OP_SUM && OP != OP_MEAN && OP != OP_MAX) {
+        if (first && !bulk_in && p.cached && OP != OP_SUM && OP != OP_MEAN && OP != OP_MAX) {
           if constexpr (VEC == 4) *reinterpret_cast<float4*>(cache + (r - begin)) = make_float4(x[u].v[0], x[u].v[1], x[u].v[2], x[u].v[3]);
           else cache[r - begin] = x[u].v[0];
         }
@@ -755,8 +791,38 @@ __global__ void __launch_bounds__(THREADS) span_kernel(const ShareParams p) {
       [&](float v, int k) { return over_shares(group_max<THREADS>(v, red, 0, tid), &slot[k], tid == 0, p.shares, ShareMax{}); },
       [&](MaxIdx m) { return over_shares(group_maxidx<THREADS>(m, red, redi, 0, tid), &slot[0], &islot, tid == 0, p.shares); },
       [&](auto g) {
-        // (gamma and beta of several trips are asked for before the first result is stored: one trip to the L2 for all)
         constexpr uint32_t STEP = THREADS * VEC;
+        if (VEC == 4 && p.bulk_out) {  // results over the cache, then out
+          const bool one_w = p.ws1 == 0 && p.ws2 == 0;  // gamma and beta belong to the line
+          const float w0 = p.w && one_w ? load_as_f32(p.w, wb, p.dt_w) : 1.f, b0 = p.b && one_w ? load_as_f32(p.b, wb, p.dt_w) : 0.f;
+#pragma unroll 2
+          for (uint32_t r = begin + tid * VEC; r < end; r += STEP) {
+            F4 v = cached(r), wv, bv;
+            if (!one_w) {
+              const uint32_t r1 = p.R2 == p.R ? 0u : r / p.R2;
+              const int64_t wo = wb + r1 * p.ws1 + (r - r1 * p.R2) * p.ws2;
+              if (p.w) wv = weights(p.w, wo);
+              if (p.b) bv = weights(p.b, wo);
+            }
+#pragma unroll
+            for (int e = 0; e < VEC; ++e) {
+              const float x = g(v.v[e]), a = one_w ? w0 : wv.v[e], c = one_w ? b0 : bv.v[e];
+              v.v[e] = p.w && p.b ? fmaf(x, a, c) : p.w ? x * a : p.b ? x + c : x;
+            }
+            *reinterpret_cast<float4*>(cache + (r - begin)) = make_float4(v.v[0], v.v[VEC > 1 ? 1 : 0], v.v[VEC > 1 ? 2 : 0], v.v[VEC > 1 ? 3 : 0]);
+          }
+          fence_proxy_async_smem();
+          __syncthreads();
+          parts([&](uint32_t at, uint32_t run, uint32_t off, uint32_t n) {
+            share_copy_out(static_cast<float*>(p.y) + yb + run * p.ys1 + off, cache + at, n * 4);
+          });
+          if (tid < 32) {
+            tma_store_commit();
+            tma_store_wait_all<0>();
+          }
+          return;
+        }
+        // (gamma and beta of several trips are asked for before the first result is stored: one trip to the L2 for all)
         for (uint32_t r0 = begin + tid * VEC; r0 < end; r0 += STEP * SHARE_UNROLL) {
           F4 v[SHARE_UNROLL], wv[SHARE_UNROLL], bv[SHARE_UNROLL];
 #pragma unroll
@@ -1201,6 +1267,12 @@ static int launch_shared_line(int op, const LineParams& lp, const NdArgs& a, con
   p.share = share_of(shares);
   p.cached = keeps && static_cast<uint64_t>(p.share) * floats <= CACHE_FLOATS;
   const size_t smem = p.cached ? static_cast<size_t>(p.share) * floats * 4 : 0;
+  // Runs of 512 bytes and more, fp32: copied whole, all of a share at once, instead of 64 bytes a thread and trip.
+  const bool runs = kind == 4 && p.cached && (p.R2 == p.R || p.R2 >= 128);
+  p.bulk_in = runs && lp.dt_in == YTC_F32;
+  p.bulk_out = p.bulk_in && lp.dt_out == YTC_F32;
+  p.status = device_status_word();
+  if (!p.status) p.bulk_in = p.bulk_out = 0;
   // A share of which only one fits an SM needs more threads to keep enough loads in flight (batchNorm, bf16, 32 x 256 x 112 x
   // 112: 1617 us with 256 threads, 605 with 1024); where more fit, 256 are faster (16 x 96 x 56 x 56 fp32: 25 us, 37).
   const bool many = smem > 110 * 1024;
