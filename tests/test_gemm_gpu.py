@@ -582,3 +582,28 @@ def test_results_through_tma_stores(L, api, out_dtype, b, m, n, k):
     assert torch.equal(got[0], got[1])
     assert normwise(got[0].double().cpu().numpy(), (a.double() @ w.double()).cpu().numpy()) < (1e-5 if out_dtype == torch.float32 else H_TOL)
     status_ok(L)
+
+
+@pytest.mark.parametrize("b,m,n,k,dt", [(1, 500, 1024, 2304, "bf16"), (1, 1, 136, 4096, "f16"), (3, 130, 264, 2056, "bf16"), (2, 300, 700, 1088, "f16"),
+                                        (1, 1024, 1032, 1032, "bf16"), (1, 1024, 1024, 520, "f32"),
+                                        (1, 700, 264, 512, "f32"), (1, 1000, 2000, 256, "f32")])
+def test_k_shared_by_a_cluster(L, api, b, m, n, k, dt):
+    """Few tiles and a long k: the CTAs of a cluster take a piece of k each. Two and four pieces, planes of fp32
+    operands, ragged m, n and k, operands of either order, aligned and other C, alpha and beta. 64-bit reference: fp32 sums of k
+    products are off by less than the file's tolerances."""
+    t = {"bf16": torch.bfloat16, "f16": torch.float16, "f32": torch.float32}[dt]
+    g = torch.Generator(device="cuda").manual_seed(m + k)
+    a, w = (torch.randn(s, generator=g, device="cuda").to(t) for s in ((b, m, k), (k, n)))
+    want = (a.double() @ w.double()).cpu().numpy()
+    tol = F32_TOL if dt == "f32" else H_TOL
+    for x in (a, a.transpose(1, 2).contiguous().transpose(1, 2)):
+        for y in (w, w.t().contiguous().t()):
+            assert normwise(api.matmul(x, y).double().cpu().numpy(), want) < tol
+    if dt != "f32":
+        wide = api.matmul(a, w, out_dtype=torch.float32)
+        assert normwise(wide.double().cpu().numpy(), want) < 1e-5
+        assert torch.equal(wide, api.matmul(a, w, out_dtype=torch.float32))
+    out = torch.ones(b, m, n + 1, dtype=t, device="cuda")[:, :, 1:]
+    api.matmul(a, w, out, alpha=0.5, beta=2.0)
+    assert normwise(out.double().cpu().numpy(), 0.5 * want + 2.0) < tol
+    status_ok(L)

@@ -48,6 +48,7 @@ struct GemmTcParams {
   const uint8_t* tile_live;
   // linear layers of the language models (LinearEpilogue, lm_ops.cuh)
   int epi;                 // EPI_NONE: the store rules above; otherwise tc_store_epilogue
+  int cluster;             // pieces of k that the CTAs of a cluster share (gemm_split_kernel)
   int n_step, n_cta;       // CTA pairs: columns from one tile to the next, from the one CTA's share of B to the other's
   int tma_out;             // C through TMA stores: 0 no, 1 yes, 2 added to what C holds (fp32)
   int act_cols;            // EPI_SILU
@@ -252,9 +253,13 @@ __device__ __forceinline__ void tc_narrow(const uint32_t (&r)[32], float alpha, 
 // on each, and 16-byte stores of its lanes, a 128 x 256 tile took 10.8 us (bf16; 6.2 with an activation that unrolled), more
 // than its MMAs for k below 2500; now 3.3. 4096 x 4096 x 1024 with nearest-even stores 53.6 -> 33.2 us, x 64 43.3 -> 13.2.
 // n0: C's column under the accumulator's first, m0: C's row under the warp's first, half: which of the groups.
-template <int BN>
+struct TcNothing {
+  __device__ __forceinline__ void operator()(uint32_t (&)[32], int) const {}
+};
+// more(r, c): what is added to columns c .. c + 31 of the accumulator first.
+template <int BN, class More = TcNothing>
 __device__ __forceinline__ void tc_drain(const GemmTcParams& p, const CUtensorMap* tmC, uint32_t t_row, uint8_t* buf, int n0, int m0,
-                                         int b, int half, int lane) {
+                                         int b, int half, int lane, More more = More{}) {
   if (m0 >= p.M) return;
   const bool pairs = tc_pairs(p), wide = p.epi == EPI_NONE && p.out_dtype == YTC_F32;
   const int cols = wide ? 32 : pairs ? 128 : 64;
@@ -272,6 +277,7 @@ __device__ __forceinline__ void tc_drain(const GemmTcParams& p, const CUtensorMa
       uint32_t r[32];
       tmem_ld_32x32b_x32(t_row + g + c, r);
       tmem_ld_wait();
+      more(r, g + c);
       if (wide) {
 #pragma unroll
         for (int j = 0; j < 8; ++j)
@@ -825,6 +831,218 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(TC_THREADS, 1)
   if (threadIdx.x == 0 && *abort_word) atomicExch(p.status, YTC_TIMEOUT);
 }
 
+// ------------------------------------------------------------------ tcgen05 path, k shared by a cluster
+// Products of less than half as many 128 x 128 tiles as the chip has SMs: the two or four CTAs of a cluster take a piece of k of one
+// tile each (of every pair of planes), and the accumulators meet in the cluster: CTA j finishes the j-th share of the tile's rows,
+// whose partial sums the others push into its shared memory, where its operands were (it says so first), and adds them to its
+// own in a fixed order. No partial sums in memory, no second launch, and every store rule of the other kernels (tc_drain).
+// What bounds it is the issue of one tile's blocks, now a half or a quarter of them, and 2 us for the exchange. Before / here: bf16
+// 500 x 1024 x 4608 22.9 / 15.2 us, two planes 43.7 / 25.4; fp32 1024^3 (six products, two launches) 31.7 / 23.8.
+__device__ __forceinline__ void tc_push4(uint32_t dst, uint32_t bar, uint32_t a, uint32_t b, uint32_t c, uint32_t d) {
+  asm volatile("st.async.shared::cluster.mbarrier::complete_tx::bytes.v4.b32 [%0], {%1, %2, %3, %4}, [%5];" ::"r"(dst), "r"(a),
+               "r"(b), "r"(c), "r"(d), "r"(bar)
+               : "memory");
+}
+__global__ void __launch_bounds__(TC_THREADS, 1)
+    gemm_split_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ CUtensorMap tmB,
+                      const __grid_constant__ CUtensorMap tmC, const GemmTcParams p) {
+  using S = TcSmem<128>;
+  constexpr int BN = 128, STAGES = S::STAGES;
+  extern __shared__ uint8_t smem_raw[];
+  uint8_t* smem = smem_raw + ((1024u - (smem_u32(smem_raw) & 1023u)) & 1023u);
+  uint64_t* full_bar = reinterpret_cast<uint64_t*>(smem + S::BAR_OFFSET);
+  uint64_t* empty_bar = full_bar + STAGES;
+  uint64_t *tfull_bar = empty_bar + STAGES / 2, *ready_bar = tfull_bar + 1, *recv_bar = tfull_bar + 2;
+  uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(tfull_bar + 4);
+  volatile int* abort_word = reinterpret_cast<volatile int*>(tmem_slot + 1);
+  static_assert(S::FREED == 2 && STAGES % 2 == 0 && (STAGES + STAGES / 2 + 4) * 8 + 8 <= (2 * STAGES + 4) * 8 + 16, "barriers");
+  const int warp = __shfl_sync(0xffffffffu, threadIdx.x >> 5, 0), lane = threadIdx.x & 31;
+  const int pieces = p.cluster, piece = blockIdx.x % pieces, tile = blockIdx.x / pieces;
+  const int tiles_per_batch = p.tiles_m * p.tiles_n;
+  const int b = tile / tiles_per_batch, rem = tile - b * tiles_per_batch, mb = rem / p.tiles_n, nb = rem - mb * p.tiles_n;
+  // blocks [f0, f1) of k of each pair of planes (an ordinary product is one pair)
+  const int fold = p.fold > 0 ? p.fold : p.k_blocks, pairs = p.k_blocks / fold;
+  const int f0 = fold * piece / pieces, f1 = fold * (piece + 1) / pieces;
+  const int quads = 4 / pieces;  // quarters of the accumulator's lanes that a CTA finishes
+
+  if (threadIdx.x == 0) {
+    for (int s = 0; s < STAGES; ++s) mbar_init(&full_bar[s], 1);
+    for (int s = 0; s < STAGES / 2; ++s) mbar_init(&empty_bar[s], 1);
+    mbar_init(tfull_bar, 1);
+    mbar_init(ready_bar, pieces - 1);
+    mbar_init(recv_bar, 1);
+    *abort_word = 0;
+    fence_mbar_init();
+    fence_proxy_async_smem();
+    mbar_expect_tx(recv_bar, (pieces - 1) * quads * (BN / 4) * 512);
+    tma_prefetch_desc(&tmA);
+    tma_prefetch_desc(&tmB);
+    if (p.tma_out) tma_prefetch_desc(&tmC);
+  }
+  if (warp == 2) {
+    tmem_alloc(tmem_slot, BN);
+    tmem_relinquish();
+  }
+  tc_fence_before();
+  __syncthreads();
+  cluster_sync_all();  // everyone's barriers are there
+  tc_fence_after();
+  const uint32_t tmem = __shfl_sync(0xffffffffu, *tmem_slot, 0);
+  dependent_wait();
+  dependent_trigger();
+
+  if (warp == 0) {
+    // ------------------------------------------------ TMA producer
+    const uint32_t lead = lane == 0 ? 1u : 0u;
+    const uint32_t ring_at = smem_u32(smem), full_at = smem_u32(full_bar);
+    const int ba = p.a_bcast ? 0 : b, bb = p.b_bcast ? 0 : b;
+    const int m0 = mb * TC_BM, n0 = nb * BN;
+    int stage = 0, issued = 0;
+    uint32_t phase = 0;
+    bool ok = true;
+#pragma unroll 1
+    for (int i = 0; i < pairs && ok; ++i) {
+      const int za = p.fold > 0 ? ba * p.planes_a + static_cast<int>((p.pa >> (2 * i)) & 3) : ba;
+      const int zb = p.fold > 0 ? bb * p.planes_b + static_cast<int>((p.pb >> (2 * i)) & 3) : bb;
+#pragma unroll 1
+      for (int f = f0; f < f1; ++f) {
+        if ((stage & 1) == 0 && !mbar_wait_warp(&empty_bar[stage >> 1], phase ^ 1u, abort_word)) {
+          ok = false;
+          break;
+        }
+        const uint32_t bar = full_at + 8 * stage, sa = ring_at + stage * S::STAGE_BYTES, sb = sa + S::A_BYTES;
+        mbar_expect_tx_lead(bar, S::STAGE_BYTES, lead);
+        const int kk = f * TC_BK;
+#pragma unroll 1
+        for (int c = 0; c < (p.a_mn ? 2 : 1); ++c)
+          tma_load_3d_lead(sa + c * 8192, &tmA, bar, p.a_mn ? m0 + c * 64 : kk, p.a_mn ? kk : m0, za, lead);
+#pragma unroll 1
+        for (int c = 0; c < (p.b_mn ? 2 : 1); ++c)
+          tma_load_3d_lead(sb + c * 8192, &tmB, bar, p.b_mn ? n0 + c * 64 : kk, p.b_mn ? kk : n0, zb, lead);
+        ++issued;
+        if (++stage == STAGES) {
+          stage = 0;
+          phase ^= 1u;
+        }
+      }
+    }
+    if (!ok) {  // copies in flight land before the CTA goes away
+      const long long t0 = clock64();
+      for (int i = issued > STAGES ? issued - STAGES : 0; i < issued; ++i)
+        while (!mbar_try_wait(&full_bar[i % STAGES], (i / STAGES) & 1) && clock64() - t0 < 20000000ll) {
+        }
+    }
+    __syncwarp();
+  } else if (warp == 1) {
+    // ------------------------------------------------ MMA issuer (see gemm_tc_kernel)
+    const uint32_t lead = lane == 0 ? 1u : 0u;
+    const uint32_t free_at = smem_u32(empty_bar);
+    const uint64_t a_desc = p.a_mn ? umma_smem_desc_sw128(smem_u32(smem), 8192, 1024) : umma_smem_desc_sw128(smem_u32(smem), 16, 1024);
+    const uint64_t b_desc = (p.b_mn ? umma_smem_desc_sw128(smem_u32(smem), 8192, 1024) : umma_smem_desc_sw128(smem_u32(smem), 16, 1024)) + (S::A_BYTES >> 4);
+    const uint32_t a_step = p.a_mn ? 2048 >> 4 : 32 >> 4, b_step = p.b_mn ? 2048 >> 4 : 32 >> 4;
+    const int blocks = pairs * (f1 - f0);
+    int stage = 0;
+    uint32_t phase = 0;
+    bool ok = true, ready = false;
+#pragma unroll 1
+    for (int i = 0; i < blocks; ++i) {
+      if (!ready && !mbar_wait_warp(&full_bar[stage], phase, abort_word)) {
+        ok = false;
+        break;
+      }
+      const int next = stage + 1 == STAGES ? 0 : stage + 1;
+      ready = __all_sync(0xffffffffu, mbar_test_wait(&full_bar[next], next ? phase : phase ^ 1u)) != 0;
+      tc_fence_after();
+      const uint64_t ad = a_desc + (stage * S::STAGE_BYTES >> 4), bd = b_desc + (stage * S::STAGE_BYTES >> 4);
+#pragma unroll
+      for (int k = 0; k < TC_BK / 16; ++k)
+        tc_mma_f16_lead(tmem, ad + k * a_step, bd + k * b_step, p.idesc, (i | k) != 0 ? 1u : 0u, lead);
+      if (stage & 1) tc_commit_lead(free_at + 8 * (stage >> 1), lead);
+      stage = next;
+      if (next == 0) phase ^= 1u;
+    }
+    if (ok) tc_commit_lead(smem_u32(tfull_bar), lead);
+    __syncwarp();
+  } else if (warp >= 4) {
+    // ------------------------------------------------ exchange, then the epilogue of this CTA's share of the rows
+    const int q = warp & 3, half = (warp - 4) >> 2;
+    const int dest = q / quads, ql = q - dest * quads;
+    uint8_t* out_buf = smem + S::OUT_OFFSET + (warp - 4) * TC_OUT_BYTES;
+    const uint32_t t_row = tmem + (static_cast<uint32_t>(q * 32) << 16);
+    bool ok = mbar_wait_warp(tfull_bar, 0, abort_word);  // (the operands have been read: their place is free)
+    tc_fence_after();
+    if (ok && warp == 4 && lane < pieces && lane != piece) mbar_arrive_cluster(map_to_cta(smem_u32(ready_bar), lane));
+    __syncwarp();
+    if (ok && dest != piece) {
+      ok = mbar_wait_warp(ready_bar, 0, abort_word);
+      const uint32_t bar = map_to_cta(smem_u32(recv_bar), dest);
+      const int slot = piece < dest ? piece : piece - 1;  // among the pieces other than dest
+      const uint32_t dst = map_to_cta(smem_u32(smem), dest) + (slot * quads + ql) * (BN / 4) * 512 + lane * 16;
+#pragma unroll 1
+      for (int c = half * (BN / 2); ok && c < (half + 1) * (BN / 2); c += 32) {
+        uint32_t r[32];
+        tmem_ld_32x32b_x32(t_row + c, r);
+        tmem_ld_wait();
+#pragma unroll
+        for (int j = 0; j < 8; ++j) tc_push4(dst + (c / 4 + j) * 512, bar, r[4 * j], r[4 * j + 1], r[4 * j + 2], r[4 * j + 3]);
+      }
+    } else if (ok && mbar_wait_warp(recv_bar, 0, abort_word)) {
+      auto more = [&](uint32_t (&r)[32], int c) {  // the others' parts, in the order of the pieces
+#pragma unroll 1
+        for (int i = 0; i < pieces - 1; ++i) {
+          const uint8_t* from = smem + ((i * quads + ql) * (BN / 4) + c / 4) * 512 + lane * 16;
+#pragma unroll
+          for (int j = 0; j < 8; ++j) {
+            const float4 v = *reinterpret_cast<const float4*>(from + j * 512);
+            r[4 * j] = __float_as_uint(__uint_as_float(r[4 * j]) + v.x);
+            r[4 * j + 1] = __float_as_uint(__uint_as_float(r[4 * j + 1]) + v.y);
+            r[4 * j + 2] = __float_as_uint(__uint_as_float(r[4 * j + 2]) + v.z);
+            r[4 * j + 3] = __float_as_uint(__uint_as_float(r[4 * j + 3]) + v.w);
+          }
+        }
+      };
+      const int m_first = mb * TC_BM + q * 32;
+      if (p.tma_out) {
+        tc_drain<BN>(p, &tmC, t_row, out_buf, nb * BN, m_first, b, half, lane, more);
+        if (lane == 0) tma_store_wait_all<0>();
+      } else {
+        const int gm = m_first + lane;
+        const bool row_ok = gm < p.M;
+        const int esz = p.out_dtype == YTC_F32 ? 4 : 2;
+        const int64_t row_off = static_cast<int64_t>(b) * p.bsc + static_cast<int64_t>(gm) * p.rsc;
+        const bool vec_ok = p.csc == 1 && (((reinterpret_cast<uint64_t>(p.C) + static_cast<uint64_t>(row_off) * esz) & 15u) == 0);
+#pragma unroll 1
+        for (int c0 = half * (BN / 2); c0 < (half + 1) * (BN / 2); c0 += 32) {
+          uint32_t r[32];
+          tmem_ld_32x32b_x32(t_row + c0, r);
+          tmem_ld_wait();
+          more(r, c0);
+          const int gn0 = nb * BN + c0;
+          if (gn0 >= p.N) continue;
+          if (p.epi != EPI_NONE) tc_store_epilogue(p, r, row_off, gn0, row_ok);
+          else if (p.out_dtype == YTC_BF16) tc_store_chunk<BN, YTC_BF16>(p, r, row_off, gn0, row_ok, vec_ok);
+          else if (p.out_dtype == YTC_F32) tc_store_chunk<BN, YTC_F32>(p, r, row_off, gn0, row_ok, vec_ok);
+          else tc_store_chunk<BN, YTC_F16>(p, r, row_off, gn0, row_ok, vec_ok);
+        }
+      }
+    }
+    tc_fence_before();
+  }
+  __syncthreads();
+  if (*abort_word && threadIdx.x < 32) {  // a give-up: what is on its way into this CTA's memory lands first
+    const long long t0 = clock64();
+    while (clock64() - t0 < 4000000ll) {
+    }
+  }
+  __syncwarp();
+  cluster_sync_all();  // nobody leaves while others may still write here
+  if (warp == 2) {
+    tc_fence_after();
+    tmem_dealloc(tmem, BN);
+  }
+  if (threadIdx.x == 0 && *abort_word) atomicExch(p.status, YTC_TIMEOUT);
+}
+
 // ------------------------------------------------------------------ FFMA path
 constexpr int SM_BM = 128, SM_BN = 128, SM_BK = 16, SM_THREADS = 256, SM_PAD = 4;
 
@@ -1079,6 +1297,16 @@ static bool tc_takes_pairs(int m, int n, int64_t k, int64_t batch) {
 static int tc_tile_n(int m, int n, int64_t batch) {
   return (n <= 128 || static_cast<int64_t>((m + 127) / 128) * ((n + 255) / 256) * batch < sm_count() / 2) ? 128 : 256;
 }
+// Pieces of k for gemm_split_kernel (0: not its product): as many as keep every CTA resident (66 clusters of two fit any B200
+// seen, 33 of four) and leave a piece eight blocks of k, the exchange costing about as much as seven (2 us). (256 x 256 tiles of two
+// pairs of CTAs for products of 72 to 132 tiles of 128, half the operand bytes per result, lost: 2000 x 1024 x 2048 14.4 -> 17.4 us.)
+static int tc_cluster(int m, int n, int64_t fold, int64_t pairs, int64_t batch) {
+  if (g_mask.kind != 0 || g_tc_pair != 0 || g_tc_split_loads) return 0;
+  const int64_t tiles = static_cast<int64_t>((m + 127) / 128) * ((n + 127) / 128) * batch, blocks = fold * pairs;
+  if (tiles <= 33 && blocks >= 32 && fold >= 4) return 4;
+  if (tiles <= 66 && blocks >= 16 && fold >= 2) return 2;
+  return 0;
+}
 // Pieces of k that fill the SMs when the tiles alone leave more than half of them idle; a piece keeps 512 / pairs of k. Not for
 // products of less than 6144 / pairs of k: their time is the caller's (30 us for a call of api.matmul, 0.35 us per block of 64 here),
 // and the launch that adds the pieces 2 to 4 us of it. Measured, bf16 16 x 4096 x k, one piece / pieces, calls one after the other:
@@ -1095,6 +1323,8 @@ static int tc_splits(int m, int n, int k, int pairs, int64_t batch) {
   int64_t want = sm_count() / tiles < most ? sm_count() / tiles : most;
   if (want > k_blocks) want = k_blocks;
   if (want < 2) return 1;
+  // (a cluster's pieces need no scratch and no second launch; more than four only where they are many more)
+  if (want <= 6 && tc_cluster(m, n, k_blocks, pairs, batch)) return 1;
   const int64_t per = (k_blocks + want - 1) / want;
   return static_cast<int>((k_blocks + per - 1) / per);
 }
@@ -1113,6 +1343,7 @@ static int launch_tc(int dtype_in, int dtype_out, const void* A, const void* B, 
   const bool grouped = ex && ex->tile_group;
   // (k pieces are work items of the one-CTA kernel; gemm_tc2_kernel knows whole products only)
   const bool pair = !grouped && splits == 1 && tc_takes_pairs(m, n, pl ? static_cast<int64_t>(k) * pl->pairs : k, batch);
+  const int cluster = grouped || pair || splits > 1 ? 0 : tc_cluster(m, n, (k + TC_BK - 1) / TC_BK, pl ? pl->pairs : 1, batch);
   if (splits > 1 && (ex || g_mask.kind != 0 || splits > (k + TC_BK - 1) / TC_BK)) {
     set_last_error("ytcuda_gemm: %d pieces of k = %d do not go with an epilogue or a mask", splits, k);
     return YTC_UNSUPPORTED;
@@ -1136,7 +1367,7 @@ static int launch_tc(int dtype_in, int dtype_out, const void* A, const void* B, 
     uint64_t dims[3], strides[2];
     uint32_t box[3];
     const uint64_t b_rows = grouped ? static_cast<uint64_t>(n) * ex->groups : static_cast<uint64_t>(n);
-    if (!b_mn) { dims[0] = k; dims[1] = b_rows; box[0] = TC_BK; box[1] = pair ? 128u : (g_tc_split_loads ? 64u : static_cast<uint32_t>(BN)); }
+    if (!b_mn) { dims[0] = k; dims[1] = b_rows; box[0] = TC_BK; box[1] = pair || cluster ? 128u : (g_tc_split_loads ? 64u : static_cast<uint32_t>(BN)); }
     else       { dims[0] = n; dims[1] = k; box[0] = 64;    box[1] = TC_BK; }
     dims[2] = nb * (pl ? pl->planes_b : 1);
     box[2] = 1;
@@ -1210,6 +1441,31 @@ static int launch_tc(int dtype_in, int dtype_out, const void* A, const void* B, 
   if (!p.status) {
     set_last_error("ytcuda_gemm: no device status word");
     return YTC_CUDA_ERROR;
+  }
+  if (cluster) {
+    p.cluster = cluster;
+    p.idesc = umma_idesc(dtype_in == YTC_BF16 ? 1u : 0u, a_mn, b_mn, TC_BM, 128);
+    p.tiles_n = (n + 127) / 128;
+    p.total_tiles = static_cast<int>(static_cast<int64_t>(p.tiles_m) * p.tiles_n * batch);
+    const int s = ensure_dynamic_smem(reinterpret_cast<const void*>(gemm_split_kernel), TcSmem<128>::DYN_STAGED);
+    if (s != YTC_OK) return s;
+    cudaLaunchConfig_t cfg{};
+    cfg.gridDim = dim3(static_cast<unsigned>(p.total_tiles * cluster));
+    cfg.blockDim = dim3(TC_THREADS);
+    cfg.dynamicSmemBytes = TcSmem<128>::DYN_STAGED;
+    cfg.stream = st;
+    cudaLaunchAttribute attr[2];
+    attr[0].id = cudaLaunchAttributeClusterDimension;
+    attr[0].val.clusterDim.x = cluster;
+    attr[0].val.clusterDim.y = attr[0].val.clusterDim.z = 1;
+    attr[1].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+    attr[1].val.programmaticStreamSerializationAllowed = 1;
+    cfg.attrs = attr;
+    cfg.numAttrs = overlap_scope() ? 2 : 1;
+    YTC_CUDA(cudaLaunchKernelEx(&cfg, gemm_split_kernel, tmA, tmB, tmC, p));
+    count_launch();
+    YTC_CUDA(cudaGetLastError());
+    return YTC_OK;
   }
   if (pair) {
     p.idesc = umma_idesc(dtype_in == YTC_BF16 ? 1u : 0u, a_mn, b_mn, 256, TC2_BN);
