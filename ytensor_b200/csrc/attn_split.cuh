@@ -14,7 +14,8 @@
 //
 // What bounds it: the tensor pipe and the shared memory that feeds it (Q K^T reads 8 KB per MMA of 64 clocks, the copies add a
 // quarter): 6 products of 128 x 128 x 128 for S and for P V, 96 MMAs a tile. Measured on a B200, causal, fp32, 16 query and 8
-// key heads of 128, planes and check included, FFMA kernel / here: 1000 queries and keys 256 / 70 us, 2000: 761 / 159; bf16,
+// key heads of 128, planes and check included, FFMA kernel / here: 1000 queries and keys 256 / 64 us, 2000: 761 / 146 (68 and 158
+// while one lane of the service warps issued copies, MMAs and commits inside a branch); bf16,
 // 8 heads of 80, 1024: 1345 / 58. (Q in tensor memory and tiles of 64 keys: 78, 185 and 59 us; an MMA of 64 columns takes as
 // long there as one of 128.) Error against 64 bits (2-norm) at 1000 keys: 3.9e-7 / 2.1e-7.
 #pragma once
