@@ -879,7 +879,7 @@ size_t plane_bytes(const WdPlan& p, int k) { return static_cast<size_t>(k) * 2 *
 bool wide_step_supported(const WdShape& s) {
   // One attention unit per CTA: the form of two or more in a row faulted on 32 sequences behind 513 keys, its cause is open;
   // one per CTA ran to 3500 keys. What does not fit takes one launch per operator.
-  if (s.batch * s.kv_heads > WD_CTAS) return false;
+  if (s.B * s.kv_heads > WD_CTAS) return false;
   WdPlan p;
   if (!wide_plan(s, &p)) return false;
   // All clusters have to be resident at once. How many fit depends on the GPU's layout of SMs: asked once per device and kernel.
