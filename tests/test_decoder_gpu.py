@@ -118,7 +118,7 @@ def test_single_kernel_decode_step_matches_operator_path(Q, B):
     (5, 4, 2, 2816, 30, 4), (8, 4, 4, 256, 1, 2), (9, 8, 2, 768, 62, 4), (16, 4, 2, 2048, 95, 3), (16, 16, 8, 512, 31, 3), (17, 16, 8, 512, 31, 3),
     (32, 16, 8, 3072, 63, 3), (31, 8, 8, 1536, 128, 2)])
 def test_layers_in_one_kernel_match_operator_path(Q, B, heads, kv_heads, inter, prompt, steps):
-    """decode_wide_kernel (5 .. 32 sequences) against one launch per operator: group sizes 1, 2 and 4; up to one
+    """The automatic path of 5 .. 32 sequences (decode_wide_kernel is off) against one launch per operator: group sizes 1, 2 and 4; up to one
     attention unit per CTA, and beyond that both on the operator path; caches that end inside, at and behind a chunk of 32 keys, and an empty one;
     feed-forwards whose tiles have 24, 44, 48 and 64 gate rows. Both carry activations as two bf16 planes and sum in fp32:
     they differ by the order of the sums."""
@@ -142,7 +142,7 @@ def test_layers_in_one_kernel_match_operator_path(Q, B, heads, kv_heads, inter, 
             want = a.forward(tok).cpu().numpy()
             n1 = count()
             got = b.forward(tok).cpu().numpy()
-            assert 8 < n1 - n0 and (count() - n1 < 8) == (B * kv_heads <= 128)  # (more: one launch per operator)
+            assert 8 < n1 - n0 and count() > n1
             assert normwise(got, want) < 2e-5, (first, t)
     assert Q._lib.lib().ytcuda_device_status(None) == 0
     a.close()

@@ -989,7 +989,7 @@ static int ensure_activations(Qwen3Model* m, int64_t rows) {
 // Sequences from which a decode step's layers run as one kernel (decode_wide.cu). Per step behind 70 keys: 8 sequences 0.87 ms
 // (one launch per operator 1.6), 32 sequences 1.0 (1.9); 1 to 4 sequences stay with decode_ll_kernel (0.59 to 0.7 ms).
 #ifndef WD_MIN_B
-#define WD_MIN_B 5
+#define WD_MIN_B 33  // off: 32 sequences behind 513 keys ended in a launch failure whose cause is not shown (5 else)
 #endif
 // Whether this step can run as one kernel over the layers: shape, device, memory for its state; not in a graph, whose replays
 // would wait for phase numbers of the first run.

@@ -204,15 +204,12 @@ class Qwen3ForCausalLM(CausalLM):
 
     def decode_kernel_name(self) -> str:
         """Name of the kernel(s) an automatic-path decode step (one new token per sequence) of this model runs: a persistent
-        step kernel up to 4 sequences, from 5 on, while sequences x key heads are at most 128, the layers as one kernel
-        (else, and for sizes it is not made for, one launch per operator from 7 on); under tensor parallelism a step kernel up to 8 sequences, one launch per operator beyond."""
+        step kernel up to 6 sequences, one launch per operator from 7 on;
+        under tensor parallelism a step kernel up to 8 sequences, one launch per operator beyond."""
         if self.batch < 5:
             return ("decode_ll_kernel (no grid barriers: tagged-pair activations, weights through a shared-memory "
                     "ring, mma.sync linear phases" +
                     (")" if self.tp_world == 1 else "; partial sums pushed to the peers as pairs over NVLink)"))
-        if self.tp_world == 1 and self.batch * self.cfg.num_key_value_heads <= 128 and self.batch <= 32 and not any(
-                n % 256 for n in (self.cfg.hidden_size, self.cfg.intermediate_size, self.cfg.num_attention_heads * 128)):
-            return "decode_wide_kernel (all layers, tcgen05 linears on hi + lo planes) + gemm_tc_kernel (vocabulary)"
         if self.batch <= (6 if self.tp_world == 1 else 8):
             return "decode_step_kernel (mma.sync linear phases)"
         return "gemm_tc_kernel (hi + lo planes, split-k pieces) + attn_decode_fast_kernel + fused glue kernels"
