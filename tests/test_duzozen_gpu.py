@@ -188,6 +188,22 @@ def test_linear_with_activation(D, dtype, m, n, k):
         assert normwise(y.float().cpu().numpy(), want) < (2e-6 if dtype == "float32" else 5e-3)
 
 
+@pytest.mark.parametrize("n,k", [(1024, 4608), (1024, 1024), (512, 2048)])
+def test_rows_of_a_bf16_layer_do_not_depend_on_the_prompts_length(D, n, k):
+    """The same bits for a token whether 3, 500 or 4096 rows go through the layer: one accumulator takes k in its order."""
+    from ytensor_b200 import _lib
+    rng = np.random.default_rng(k)
+    x, w = dev(rng.standard_normal((4096, k)), torch.bfloat16), dev(rng.standard_normal((n, k)) / np.sqrt(k), torch.bfloat16)
+    ys = []
+    for m in (4096, 500, 129, 3):
+        y = torch.empty(m, n, dtype=torch.bfloat16, device="cuda")
+        _lib.check(_lib.lib().ytcuda_linear_act(_lib.BF16, 0, x.data_ptr(), k, w.data_ptr(), y.data_ptr(), n, m, n, k, 0, 0.0,
+                                                None, 1, torch.cuda.current_stream().cuda_stream))
+        ys.append(y)
+    for y in ys[1:]:
+        assert torch.equal(y, ys[0][:len(y)])
+
+
 @pytest.mark.parametrize("dtype", ["float32", "bfloat16"])
 def test_grouped_linear(D, dtype):
     from ytensor_b200 import _lib
