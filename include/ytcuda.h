@@ -347,9 +347,8 @@ int ytcuda_qwen3_set_allreduce(void* handle, int (*fn)(void* buf, int64_t count,
 int ytcuda_qwen3_reset(void* handle);
 int ytcuda_qwen3_cache_len(void* handle);
 /* How a forward of ONE new token per sequence runs: 0 = automatic (one persistent cooperative kernel for the whole
- * step for batch <= 4, one for all layers for 5 to 32 sequences (sizes that are multiples of 256, no stream capture, a ring that
- * has not wrapped; else batch <= 6 as for 4, one launch per operator beyond); under tensor parallelism the step kernel for
- * batch <= 8, which needs connected exchange buffers, see ytcuda_qwen3_tp_export),
+ * step for batch <= 6, or <= 8 under tensor parallelism, where it needs connected exchange buffers, see
+ * ytcuda_qwen3_tp_export; one launch per operator beyond),
  * 1 = one launch per operator as for longer inputs, 2 = the persistent kernel (batch <= 32) or YTC_UNSUPPORTED.
  * 3 = as 2, with the FFMA form of the kernel's linear phases even where the tensor-core form (five or more
  * sequences, hidden <= 1024) applies. Up to four sequences the kernel streams its weights through a ring of

@@ -25,7 +25,6 @@
 #include "decode_step.cuh"
 #include "decode_stream.cuh"
 #include "decode_ll.cuh"
-#include "decode_wide.cuh"
 #include "ytc_common.cuh"
 
 namespace ytk {
@@ -516,7 +515,6 @@ struct Qwen3Model {
   int trace_cap = 0;
   DsLayer* ds_lw = nullptr;         // device copy of the per-layer weight pointers
   bool ds_lw_stale = true;
-  WdState wide;                     // decode steps of several sequences as one kernel (decode_wide.cu)
   float* ds_part = nullptr;         // attention partials
   unsigned int* ds_sync = nullptr;  // barrier counter + per (sequence, kv head) chunk counters
   // exchange buffers of the tensor-parallel step kernel: this rank's (mailbox, flag words, release word) and the
@@ -864,7 +862,7 @@ int ytcuda_qwen3_set_weight(void* handle, const char* name, int layer, const voi
   YTC_REQUIRE(m && name && dptr, "ytcuda_qwen3_set_weight: null argument");
   YTC_REQUIRE((reinterpret_cast<uint64_t>(dptr) & 15) == 0, "ytcuda_qwen3_set_weight: weights must be 16-byte aligned");
   const std::string n(name);
-  m->ds_lw_stale = m->wide.stale = true;
+  m->ds_lw_stale = true;
   if (n == "embed") { m->embed = static_cast<const uint16_t*>(dptr); return YTC_OK; }
   if (n == "lm_head") { m->lm_head = static_cast<const uint16_t*>(dptr); return YTC_OK; }
   if (n == "norm") { m->final_norm = static_cast<const float*>(dptr); return YTC_OK; }
@@ -984,27 +982,6 @@ static int ensure_activations(Qwen3Model* m, int64_t rows) {
     return s;
   m->act_rows = rows;
   return YTC_OK;
-}
-
-// Sequences from which a decode step's layers run as one kernel (decode_wide.cu). Per step behind 70 keys: 8 sequences 0.87 ms
-// (one launch per operator 1.6), 32 sequences 1.0 (1.9); 1 to 4 sequences stay with decode_ll_kernel (0.59 to 0.7 ms).
-#ifndef WD_MIN_B
-#define WD_MIN_B 33  // off: 32 sequences behind 513 keys ended in a launch failure whose cause is not shown (5 else)
-#endif
-// Whether this step can run as one kernel over the layers: shape, device, memory for its state; not in a graph, whose replays
-// would wait for phase numbers of the first run.
-static bool wide_step_ready(Qwen3Model* m, const WdShape& ws, cudaStream_t st) {
-  cudaStreamCaptureStatus cap = cudaStreamCaptureStatusNone;
-  if (cudaStreamIsCapturing(st, &cap) != cudaSuccess || cap != cudaStreamCaptureStatusNone || !wide_step_supported(ws)) return false;
-  if (!m->wide.dev) {
-    if (cudaMalloc(&m->wide.dev, wide_state_bytes(ws)) != cudaSuccess) {
-      (void)cudaGetLastError();
-      m->wide.dev = nullptr;
-      return false;
-    }
-    m->owned.push_back(m->wide.dev);
-  }
-  return true;
 }
 
 constexpr int DS_MAX_CHUNKS = 64;
@@ -1296,9 +1273,7 @@ int ytcuda_qwen3_forward(void* handle, const int32_t* ids, int len, float* logit
   // Automatic choice: the step kernel up to ds_auto_b() sequences. Beyond that its linear phases lose against the
   // tensor-core linears of the operator path (measured at 16 and 32 sequences), so it runs only when asked for.
   const bool want_step = m->decode_path >= 2 && m->decode_path <= 5;  // (6: operator path, sums over ranks by callback)
-  const WdShape ws{B, Hd, m->layers, m->l_heads, m->l_kv_heads, m->l_inter, m->vocab, m->max_pos};
-  const bool wide = len == 1 && m->decode_path == 0 && m->tp_world == 1 && !wrap_step && B >= WD_MIN_B && wide_step_ready(m, ws, st);
-  if (!wide && len == 1 && (want_step || (m->decode_path == 0 && m->batch <= ds_auto_b(m))) && decode_step_supported(m)) {
+  if (len == 1 && (want_step || (m->decode_path == 0 && m->batch <= ds_auto_b(m))) && decode_step_supported(m)) {
     if ((s = decode_step_launch(m, ids, logits, st)) != YTC_OK) return s;
     advance();
     return YTC_OK;
@@ -1313,20 +1288,13 @@ int ytcuda_qwen3_forward(void* handle, const int32_t* ids, int len, float* logit
   const float scale = 1.0f / std::sqrt(static_cast<float>(D));
   const size_t cache_layer = static_cast<size_t>(B) * m->l_kv_heads * m->max_pos * D;
 
-  // One new token of several sequences: the layers as one kernel.
-  if (wide) {
-    std::vector<WdLayer> wl;
-    if (m->wide.stale)
-      for (const LayerW& L : m->lw) wl.push_back(WdLayer{L.qkv, L.o, L.gate_up, L.down, L.q_norm, L.k_norm, L.norm1, L.norm2});
-    const WdStep step{pos0, m->eps, scale, ids, m->embed, m->cos_t, m->sin_t, m->k_cache, m->v_cache, m->x, m->qkv};
-    if ((s = wide_step_launch(ws, step, wl.data(), m->wide, st)) != YTC_OK) return s;
-  } else if ((s = ytcuda_embedding(m->embed, ids, m->x, rows, Hd, m->vocab, st)) != YTC_OK) return s;
+  if ((s = ytcuda_embedding(m->embed, ids, m->x, rows, Hd, m->vocab, st)) != YTC_OK) return s;
   // 5 .. 128 rows on one GPU: every projection runs as k pieces on the tensor cores, and the kernels between two
   // projections (sum of the pieces, residual, rmsNorm or SwiGLU or the per-head norm + RoPE, the split into bf16
   // planes) are one launch each: 11 launches per layer instead of 18.
   // Tensor parallel (exchange buffers connected, up to TP_PUSH_ROWS rows): the same launches; the kernel that adds the
   // pieces of the o or down projection to the residual stream also exchanges the ranks' shares (no collective call).
-  const bool fused_glue = !wide && (m->tp_world == 1 || (m->tp_ready && rows <= TP_PUSH_ROWS && m->decode_path != 6)) &&
+  const bool fused_glue = (m->tp_world == 1 || (m->tp_ready && rows <= TP_PUSH_ROWS && m->decode_path != 6)) &&
                           rows > SK_MAX_ROWS && split_k_ok(rows, Hd) && split_k_ok(rows, m->l_heads * D) &&
                           split_k_ok(rows, m->l_inter) && Hd <= 3072;
   if (fused_glue) {
@@ -1376,7 +1344,7 @@ int ytcuda_qwen3_forward(void* handle, const int32_t* ids, int len, float* logit
   // More rows: the norms and SwiGLU write the planes that the projection behind them reads (as far as their kernels go).
   const bool planes = rows > 128 && Hd <= RMS_PLANES_MAX && m->l_inter % 4 == 0;
   const int64_t glue_cap = static_cast<int64_t>(sm_count()) * 16;
-  for (int l = wide || fused_glue ? m->layers : 0; l < m->layers; ++l) {
+  for (int l = fused_glue ? m->layers : 0; l < m->layers; ++l) {
     const LayerW& W = m->lw[l];
     float* kc = m->k_cache + l * cache_layer;
     float* vc = m->v_cache + l * cache_layer;

@@ -55,7 +55,7 @@ MODELS = {
     "Duzozen": Model("Duzozen", ("bfloat16", "float32"), _NATIVE + ("duzozen",), _load_duzozen),
     "Derupel": Model("Derupel", ("bfloat16", "float32"), _NATIVE + ("latent_attn", "decayed_attn", "derupel"), _load_derupel),
     # (bf16 weights with fp32 activations: the one format it has)
-    "Qwen3ForCausalLM": Model("Qwen3ForCausalLM", ("bfloat16",), _CORE + ("elementwise", "decoder", "decode_wide"), _load_qwen3),
+    "Qwen3ForCausalLM": Model("Qwen3ForCausalLM", ("bfloat16",), _CORE + ("elementwise", "decoder"), _load_qwen3),
 }
 
 
