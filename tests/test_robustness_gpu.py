@@ -2,6 +2,10 @@
 under two streams, and the shared-memory attribute on every device of a process. No test here faults or hangs a GPU:
 the wait that runs out is a wait with a short cycle budget on a barrier nothing arrives on, after which the kernel
 returns by itself."""
+import subprocess
+import sys
+from pathlib import Path
+
 import numpy as np
 import pytest
 
@@ -69,6 +73,31 @@ def test_scratch_is_per_stream(L):
         torch.cuda.synchronize()
         for got, w in zip((g1, g2, g3, g4), want):
             assert torch.equal(got, w)
+
+
+CAPTURED_FIRST = """
+import torch
+from ytensor_b200 import api
+g = torch.Generator(device="cuda").manual_seed(1)
+x, w, b = (torch.randn(s, device="cuda", generator=g) for s in ((4, 16, 32, 32), (16,), (16,)))
+m = torch.randn(256, 64, device="cuda", dtype=torch.bfloat16, generator=g)
+calls = dict(batchNorm=lambda: api.batchNorm(x, w, b), sum=lambda: api.sum(x, (0, 2, 3)), matmul=lambda: api.matmul(m.T, m))
+torch.cuda.synchronize()
+graph = torch.cuda.CUDAGraph()
+with torch.cuda.graph(graph):
+    y = calls["{}"]()
+graph.replay()
+torch.cuda.synchronize()
+assert torch.equal(y, calls["{}"]())
+"""
+
+
+@pytest.mark.parametrize("call", ["batchNorm", "sum", "matmul"])
+def test_first_call_of_a_process_may_be_captured(L, call):
+    """Whatever the library makes once per device may be made inside a stream capture: nothing it does then ends the capture."""
+    r = subprocess.run([sys.executable, "-c", CAPTURED_FIRST.format(call, call)], cwd=Path(__file__).resolve().parents[1],
+                       capture_output=True, text=True, timeout=300)
+    assert r.returncode == 0, r.stderr[-2000:]
 
 
 def test_every_device_of_a_process_gets_its_shared_memory_limit(L):

@@ -1271,7 +1271,7 @@ static int launch_shared_line(int op, const LineParams& lp, const NdArgs& a, con
   const bool runs = kind == 4 && p.cached && (p.R2 == p.R || p.R2 >= 128);
   p.bulk_in = runs && lp.dt_in == YTC_F32;
   p.bulk_out = p.bulk_in && lp.dt_out == YTC_F32;
-  p.status = device_status_word();
+  p.status = runs ? device_status_word() : nullptr;
   if (!p.status) p.bulk_in = p.bulk_out = 0;
   // A share of which only one fits an SM needs more threads to keep enough loads in flight (batchNorm, bf16, 32 x 256 x 112 x
   // 112: 1617 us with 256 threads, 605 with 1024); where more fit, 256 are faster (16 x 96 x 56 x 56 fp32: 25 us, 37).

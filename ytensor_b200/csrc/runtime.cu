@@ -57,10 +57,19 @@ int* device_status_word() {
   if (cudaGetDevice(&dev) != cudaSuccess || dev < 0 || dev >= kMaxDev) return nullptr;
   std::lock_guard<std::mutex> lk(g_mu);
   if (!g_status[dev]) {
+    // The first call of a process may be one that a stream capture records (here or in another thread): a plain cudaMalloc or a
+    // memset on the legacy stream would end that capture.
+    cudaStreamCaptureMode mode = cudaStreamCaptureModeRelaxed;
+    if (cudaThreadExchangeStreamCaptureMode(&mode) != cudaSuccess) return nullptr;
     int* p = nullptr;
-    if (cudaMalloc(&p, 256) != cudaSuccess) return nullptr;
-    if (cudaMemset(p, 0, 256) != cudaSuccess) return nullptr;
-    g_status[dev] = p;
+    cudaStream_t own = nullptr;
+    const bool ok = cudaMalloc(&p, 256) == cudaSuccess && cudaStreamCreateWithFlags(&own, cudaStreamNonBlocking) == cudaSuccess &&
+                    cudaMemsetAsync(p, 0, 256, own) == cudaSuccess && cudaStreamSynchronize(own) == cudaSuccess;
+    if (!ok) (void)cudaGetLastError();
+    if (own) cudaStreamDestroy(own);
+    if (ok) g_status[dev] = p;
+    else if (p) cudaFree(p);
+    (void)cudaThreadExchangeStreamCaptureMode(&mode);
   }
   return g_status[dev];
 }
