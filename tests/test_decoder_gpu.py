@@ -271,6 +271,47 @@ def test_full_model_greedy_tokens_match_reference(Q, qwen3_golden):
     m2.close()
 
 
+def qkv_post(Q, qkv, qn, kn, cos, sin, B, T, H, G, max_len, pos0, slot0, eps, off):
+    """ytcuda_qwen3_qkv_post on numpy arrays, every tensor `off` floats behind a 16-byte boundary -> q, k_cache, v_cache (7 where
+    nothing was written)."""
+    from ytensor_b200 import _lib
+
+    def place(shape, a=None):
+        t = torch.full((off + int(np.prod(shape)),), 7.0, device="cuda")[off:].reshape(shape)
+        return t if a is None else t.copy_(torch.from_numpy(np.ascontiguousarray(a, np.float32)))
+
+    q, kc, vc = place((B, H, T, 128)), place((B, G, max_len, 128)), place((B, G, max_len, 128))
+    ins = [place(a.shape, a) for a in (qkv, qn, kn, cos, sin)]
+    _lib.check(_lib.lib().ytcuda_qwen3_qkv_post(ins[0].data_ptr(), q.data_ptr(), kc.data_ptr(), vc.data_ptr(),
+                                                *(t.data_ptr() for t in ins[1:]), B, T, H, G, 128, max_len, pos0, slot0, eps,
+                                                torch.cuda.current_stream().cuda_stream))
+    return [t.cpu().numpy() for t in (q, kc, vc)]
+
+
+# up to 2367 groups of four heads a warp takes one head, from 2368 on (16 warps an SM) four; heads that four does not divide
+QKV_POST = [(1, 3, 4, 2, 0), (2, 5, 3, 1, 1), (1, 1183, 5, 1, 0), (1, 1184, 5, 1, 0), (2, 700, 3, 1, 0), (1, 1300, 5, 1, 3), (3, 200, 14, 2, 0)]
+
+
+@pytest.mark.parametrize("B,T,H,G,off", QKV_POST)
+def test_norms_behind_the_qkv_projection_round_as_fp32_does(Q, B, T, H, G, off):
+    """Small whole numbers make the sums of squares exact, and cos = 1, sin = 0 leave the norm alone: (x / rms) * w in fp32, to the bit.
+    The ring ends inside the new tokens."""
+    rng = np.random.default_rng(T)
+    qkv = rng.integers(-8, 9, (B, T, H + 2 * G, 128)).astype(np.float32)
+    qn, kn = (rng.uniform(0.5, 1.5, 128).astype(np.float32) for _ in range(2))
+    max_len, pos0, slot0, eps = T + 9, 4, T + 7, np.float32(1e-6)
+    cos, sin = np.ones((max_len, 128), np.float32), np.zeros((max_len, 128), np.float32)
+    q, kc, vc = qkv_post(Q, qkv, qn, kn, cos, sin, B, T, H, G, max_len, pos0, slot0, eps, off)
+    rms = np.sqrt((qkv * qkv).sum(-1, keepdims=True) / np.float32(128) + eps)
+    x = (qkv / rms).transpose(0, 2, 1, 3)
+    slots = (slot0 + np.arange(T)) % max_len
+    assert np.array_equal(q, x[:, :H] * qn)
+    assert np.array_equal(kc[:, :, slots], x[:, H:H + G] * kn)
+    assert np.array_equal(vc[:, :, slots], qkv.transpose(0, 2, 1, 3)[:, H + G:])
+    rest = np.setdiff1d(np.arange(max_len), slots)
+    assert (kc[:, :, rest] == 7).all() and (vc[:, :, rest] == 7).all()
+
+
 def test_full_model_32_sequences_match_reference(Q):
     """benchmark configuration 5 at batch 32: the operator path that 32 sequences take (tcgen05 linears on hi + lo bf16 planes
     with split-k pieces, attn_decode_fast_kernel, fused glue) against the reference run with 32 distinct prompts.

@@ -458,9 +458,9 @@ __global__ void __launch_bounds__(128) qkv_post_kernel(const float* qkv, float* 
       ss = fmaf(x[i].w, x[i].w, ss);
 #pragma unroll
       for (int o = 16; o > 0; o >>= 1) ss += __shfl_xor_sync(0xffffffffu, ss, o);
-      const float inv = 1.0f / sqrtf(ss * (1.0f / D) + eps);
+      const float rms = sqrtf(ss * (1.0f / D) + eps);
       const float4 g = is_q ? gq : gk;
-      const float4 n = make_float4(x[i].x * inv * g.x, x[i].y * inv * g.y, x[i].z * inv * g.z, x[i].w * inv * g.w);
+      const float4 n = make_float4(x[i].x / rms * g.x, x[i].y / rms * g.y, x[i].z / rms * g.z, x[i].w / rms * g.w);
       float4 y;
       y.x = n.x * c4.x + __shfl_xor_sync(0xffffffffu, n.x, 16) * s4.x;
       y.y = n.y * c4.y + __shfl_xor_sync(0xffffffffu, n.y, 16) * s4.y;
