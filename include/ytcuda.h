@@ -323,8 +323,8 @@ int ytcuda_topk_sample(const float* logits, int64_t row_stride, int rows, int vo
 
 /* Fused per-head RMSNorm (q, k) + rotate-half RoPE + KV-cache append on the fused projection output
  * qkv [batch, len, (heads + 2 kv_heads) * 128] -> q_out [batch, heads, len, 128], k_cache / v_cache
- * [batch, kv_heads, max_len, 128] at slots slot0 .. slot0 + len - 1, RoPE positions pos0 .. (qwen3.cpp:237-247,
- * 70-88, 522-559). */
+ * [batch, kv_heads, max_len, 128] at slots slot0 .. slot0 + len - 1 (modulo max_len), RoPE positions pos0 ..
+ * (qwen3.cpp:237-247, 70-88, 522-559). cos_table / sin_table [max_len, 128], of which the first 64 of a row are read. */
 int ytcuda_qwen3_qkv_post(const float* qkv, float* q_out, float* k_cache, float* v_cache, const float* q_norm,
                           const float* k_norm, const float* cos_table, const float* sin_table, int batch, int len,
                           int heads, int kv_heads, int head_dim, int max_len, int pos0, int slot0, float eps,

@@ -312,6 +312,25 @@ def test_norms_behind_the_qkv_projection_round_as_fp32_does(Q, B, T, H, G, off):
     assert (kc[:, :, rest] == 7).all() and (vc[:, :, rest] == 7).all()
 
 
+@pytest.mark.parametrize("B,T,H,G,off", QKV_POST)
+def test_rotation_reads_the_first_half_of_the_tables(Q, B, T, H, G, off):
+    """Rotate-half RoPE against float64: 1e-6 normwise (fp32 products, one rounding each of x / rms, times w and two of the rotation).
+    Values 64 .. 127 of a row of the tables are not read: NaN there changes nothing."""
+    rng = np.random.default_rng(T + 1)
+    qkv = rng.standard_normal((B, T, H + 2 * G, 128)).astype(np.float32)
+    qn, kn = (rng.uniform(0.5, 1.5, 128).astype(np.float32) for _ in range(2))
+    max_len, pos0, slot0 = T + 9, 4, 2
+    angle = rng.uniform(0, 6, (max_len, 64))
+    cos, sin = (np.concatenate([f(angle), np.full_like(angle, np.nan)], 1).astype(np.float32) for f in (np.cos, np.sin))
+    q, kc, _ = qkv_post(Q, qkv, qn, kn, cos, sin, B, T, H, G, max_len, pos0, slot0, 1e-6, off)
+    x = qkv.astype(np.float64).transpose(0, 2, 1, 3)
+    x = x / np.sqrt((x * x).mean(-1, keepdims=True) + 1e-6)
+    c, s = (t[pos0:pos0 + T, :64].astype(np.float64) for t in (cos, sin))
+    turned = lambda v: np.concatenate([v[..., :64] * c - v[..., 64:] * s, v[..., 64:] * c + v[..., :64] * s], -1)  # noqa: E731
+    assert normwise(q, turned(x[:, :H] * qn)) < 1e-6
+    assert normwise(kc[:, :, slot0:slot0 + T], turned(x[:, H:H + G] * kn)) < 1e-6
+
+
 def test_full_model_32_sequences_match_reference(Q):
     """benchmark configuration 5 at batch 32: the operator path that 32 sequences take (tcgen05 linears on hi + lo bf16 planes
     with split-k pieces, attn_decode_fast_kernel, fused glue) against the reference run with 32 distinct prompts.

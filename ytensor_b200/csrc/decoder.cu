@@ -439,9 +439,9 @@ __global__ void __launch_bounds__(128) qkv_post_kernel(const float* qkv, float* 
 #pragma unroll
     for (int i = 0; i < QP_HEADS; ++i)
       if (h0 + i < heads_all) x[i] = load(row * heads_all + h0 + i);
-    // rotate-half pairs (i, i + 64): the other one is 16 lanes away; both halves of a row of the tables hold the same values
-    const float4 c4 = get(cos_t + static_cast<int64_t>(pos0 + t) * D + 4 * lane);
-    float4 s4 = get(sin_t + static_cast<int64_t>(pos0 + t) * D + 4 * lane);
+    // rotate-half pairs (i, i + 64): the other one is 16 lanes away, and the first half of a row of the tables serves both
+    const float4 c4 = get(cos_t + static_cast<int64_t>(pos0 + t) * D + 4 * (lane & 15));
+    float4 s4 = get(sin_t + static_cast<int64_t>(pos0 + t) * D + 4 * (lane & 15));
     if (lane < 16) s4 = make_float4(-s4.x, -s4.y, -s4.z, -s4.w);
 #pragma unroll
     for (int i = 0; i < QP_HEADS; ++i) {
