@@ -397,6 +397,28 @@ def test_activation_in_the_products_epilogue(Q, inter, rows):
     m.close()
 
 
+@pytest.mark.parametrize("hidden,rows", [(256, 300), (1024, 1100), (2048, 2400), (264, 131)])
+def test_residual_stream_of_a_long_prompt_keeps_every_fp32_number(Q, hidden, rows):
+    """Embeddings below 2^-126 through a layer whose o and down projections are zero: the stream stays what it was, whichever kernel adds
+    to it in memory (k shared by a cluster, one CTA a tile, CTA pairs, columns that end inside a tile). The final norm, whose root is
+    that of its eps, and an output matrix of its own show it: 2e-5, two bf16 planes."""
+    cfg = Q.Qwen3Config(**{**SMALL, "hidden_size": hidden, "num_hidden_layers": 1, "intermediate_size": 512, "max_position_embeddings": 2400})
+    w = Q.random_weights(cfg, seed=3, std=0.05)
+    rng = np.random.default_rng(rows)
+    w["lm_head"] = w["embed"]
+    w["embed"] = Q.f32_to_bf16_bits((rng.uniform(0.25, 1, w["embed"].shape) * rng.choice([-1, 1], w["embed"].shape) * 2.0 ** -127).astype(np.float32)).reshape(w["embed"].shape)
+    w["norm"] = np.full(hidden, 2.0 ** 100, np.float32)
+    for name in ("o", "down"):
+        w[(name, 0)] = np.zeros_like(w[(name, 0)])
+    m = Q.Qwen3ForCausalLM(cfg)
+    m.load_weights(w)
+    ids = rng.integers(0, 512, (1, rows))
+    got = m.forward(dev_ids(ids)).cpu().numpy()[0]
+    x = Q.bf16_bits_to_f32(w["embed"])[ids[0, -1]].astype(np.float64) / np.sqrt(cfg.rms_norm_eps) * 2.0 ** 100
+    assert normwise(got, Q.bf16_bits_to_f32(w["lm_head"]).astype(np.float64) @ x) < 2e-5
+    m.close()
+
+
 def test_long_prompts_of_an_odd_share_of_the_ffn(Q):
     """A rank whose share of the FFN has rows that do not start at 16 bytes (40 / 2 columns) computes what one GPU does with
     the same weights and columns of zeros behind them. The sums over the ranks are left out."""

@@ -87,7 +87,7 @@ struct LinearEpilogue {
   // matrices of n rows), blocks with tile_group[i] < 0 are passed over
   const int* tile_group = nullptr;
   int groups = 1;
-  bool add_in_memory = false;  // beta = 1: the memory's adders may add (numbers below 2^-126 count as zero there)
+  bool add_in_memory = false;  // beta = 1: the memory's adders may add
 };
 #ifdef __CUDACC__
 // The fp32 forms: column n of a plain epilogue, a (gate, up) pair of a gated one.
