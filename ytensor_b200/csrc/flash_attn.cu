@@ -309,7 +309,7 @@ __global__ void __launch_bounds__(FA_THREADS, 1)
   uint64_t* o_ready = p_full + 2;
   uint64_t* q_free = o_ready + 2;   // the MMAs no longer read the Q tiles of the current item
   uint64_t* o_free = q_free + 1;    // [2] the epilogue has read O_t
-  uint64_t* p_half = o_free + 2;    // [2] the first 64 keys' columns of P_t are in tensor memory
+  uint64_t* p_half = o_free + 2;    // [2] half of P_t's columns are in tensor memory (not KEEP: there the MMA warp waits for all of P_t)
   uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(p_half + 2);
   volatile int* abort_word = reinterpret_cast<volatile int*>(tmem_slot + 1);
 
@@ -803,7 +803,8 @@ __global__ void __launch_bounds__(FA_THREADS, 1)
           const __half2 h = __floats2half2_rn(p0, p1);
           return *reinterpret_cast<const uint32_t*>(&h);
         };
-        auto publish_half = [&]() {  // half of P's columns are stored: the MMA warp may start P.V on them
+        auto publish_half = [&]() {  // half of P's columns are stored: the MMA warp may start P.V on them (see HALVES)
+          if constexpr (KEEP) return;
           tmem_st_wait();
           tc_fence_before();
           __syncwarp();
