@@ -100,6 +100,26 @@ def test_first_call_of_a_process_may_be_captured(L, call):
     assert r.returncode == 0, r.stderr[-2000:]
 
 
+SMALL_THEN_LARGER = """
+import torch
+from ytensor_b200 import api
+for dtype in (torch.float32, torch.bfloat16):
+    for n, c, h, w in ((16, 16, 16, 16), (1, 300, 60, 64), (1, 300, 64, 127)):
+        x = torch.randn(n, c, h, w, device="cuda").to(dtype)
+        y, d = api.batchNorm(x).double(), x.double()
+        want = (d - d.mean((0, 2, 3), keepdim=True)) / torch.sqrt(d.var((0, 2, 3), unbiased=False, keepdim=True) + 1e-5)
+        assert (y - want).abs().max() < (1e-5 if dtype == torch.float32 else 0.05)
+"""
+
+
+def test_a_call_of_little_shared_memory_leaves_room_for_the_next(L):
+    """A kernel's limit is raised for the launches that need it and never lowered: 8 KB in a cluster, then 15 and 32 KB in plain launches
+    of the same kernel, in a process of its own (bf16: one of its steps from 4 sigma on is 0.031)."""
+    r = subprocess.run([sys.executable, "-c", SMALL_THEN_LARGER], cwd=Path(__file__).resolve().parents[1], capture_output=True,
+                       text=True, timeout=300)
+    assert r.returncode == 0, r.stderr[-2000:]
+
+
 def test_every_device_of_a_process_gets_its_shared_memory_limit(L):
     """The tcgen05 GEMM needs more dynamic shared memory than the default limit; a process that uses two GPUs must be
     able to launch it on both."""

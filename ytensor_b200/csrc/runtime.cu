@@ -170,6 +170,11 @@ int ensure_dynamic_smem(const void* fn, int bytes) {
   YTC_CUDA(cudaGetDevice(&dev));
   std::lock_guard<std::mutex> lk(g_mu);
   int& cur = g_smem_limit[FnKey{dev, fn}];
+  if (cur == 0) {  // the limit that plain launches rely on is never lowered
+    cudaFuncAttributes a;
+    YTC_CUDA(cudaFuncGetAttributes(&a, fn));
+    cur = a.maxDynamicSharedSizeBytes;
+  }
   if (cur < bytes) {
     YTC_CUDA(cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, bytes));
     cur = bytes;
