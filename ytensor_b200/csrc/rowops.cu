@@ -587,7 +587,7 @@ __global__ void __launch_bounds__(128) line_kernel(const LineParams p) {
 // element and pass, on one CTA (or thread) per line. Shares above CACHE_FLOATS are read again instead.
 // What bounds them: span_kernel the two trips to memory with the sums between them: fp32 shares come in and leave as bulk copies
 // of whole runs (16 x 96 x 56 x 56 fp32 over all axes but the channel, gamma and bias included: 965 us with line_kernel and two
-// elementwise passes, 22.6 with four 16-byte loads a thread in flight and a division a load, 15.8 here, 6 at the copy rate);
+// elementwise passes, 20.9 with four 16-byte loads a thread in flight and a division a load, 12.2 here, 6 at the copy rate);
 // column_kernel the latency of its 32-column rows (softmax of fp32 2048 x 4096 along the first axis: 2891 / 60 us).
 constexpr int SHARE_UNROLL = 4, MAX_SHARES = 8;
 constexpr uint32_t CACHE_FLOATS = 50u * 1024;
@@ -607,7 +607,7 @@ struct ShareParams {
   uint32_t share;          // elements per CTA
   int shares;
   int cached;
-  int bulk_in, bulk_out;   // span_kernel: whole runs come into the cache, results leave it, as bulk copies (fp32)
+  int bulk;                // span_kernel<.., BULK>
   int* status;
   float eps, lp;
   int dt_in, dt_out, dt_w;
@@ -702,8 +702,10 @@ __device__ __forceinline__ void share_copy_out(void* dst, const void* src, uint3
   asm volatile("cp.async.bulk.global.shared::cta.bulk_group [%0], [%1], %2;" ::"l"(dst), "r"(smem_u32(src)), "r"(bytes) : "memory");
 }
 
-template <int OP, int VEC, int THREADS>
+// BULK (fp32): whole runs come into the cache, and results leave it, as bulk copies.
+template <int OP, int VEC, int THREADS, bool BULK>
 __global__ void __launch_bounds__(THREADS) span_kernel(const ShareParams p) {
+  static_assert(!BULK || VEC == 4, "whole runs start at 16 bytes");
   extern __shared__ __align__(16) float cache[];
   __shared__ float red[32], slot[2];
   __shared__ int redi[32], islot;
@@ -727,8 +729,7 @@ __global__ void __launch_bounds__(THREADS) span_kernel(const ShareParams p) {
       f(lo - begin, run, lo - run * p.R2, hi - lo);
     }
   };
-  const bool bulk_in = VEC == 4 && p.bulk_in;
-  if (bulk_in) {
+  if constexpr (BULK) {
     __shared__ __align__(8) uint64_t arrived;
     __shared__ int abort_word;
     if (tid == 0) {
@@ -750,7 +751,7 @@ __global__ void __launch_bounds__(THREADS) span_kernel(const ShareParams p) {
     else return F4{{load_as_f32(p.x, o, p.dt_in), 0.f, 0.f, 0.f}};
   };
   auto cached = [&](uint32_t r) {
-    if (!p.cached) return load(r);
+    if (!BULK && !p.cached) return load(r);
     if constexpr (VEC == 4) {
       const float4 t = *reinterpret_cast<const float4*>(cache + (r - begin));
       return F4{{t.x, t.y, t.z, t.w}};
@@ -771,12 +772,12 @@ __global__ void __launch_bounds__(THREADS) span_kernel(const ShareParams p) {
       F4 x[SHARE_UNROLL];
 #pragma unroll
       for (int u = 0; u < SHARE_UNROLL; ++u)
-        if (r0 + u * STEP < end) x[u] = first && !bulk_in ? load(r0 + u * STEP) : cached(r0 + u * STEP);
+        if (r0 + u * STEP < end) x[u] = first && !BULK ? load(r0 + u * STEP) : cached(r0 + u * STEP);
 #pragma unroll
       for (int u = 0; u < SHARE_UNROLL; ++u) {
         const uint32_t r = r0 + u * STEP;
         if (r >= end) break;
-        if (first && !bulk_in && p.cached && OP != OP_SUM && OP != OP_MEAN && OP != OP_MAX) {
+        if (first && !BULK && p.cached && OP != OP_SUM && OP != OP_MEAN && OP != OP_MAX) {
           if constexpr (VEC == 4) *reinterpret_cast<float4*>(cache + (r - begin)) = make_float4(x[u].v[0], x[u].v[1], x[u].v[2], x[u].v[3]);
           else cache[r - begin] = x[u].v[0];
         }
@@ -792,24 +793,17 @@ __global__ void __launch_bounds__(THREADS) span_kernel(const ShareParams p) {
       [&](MaxIdx m) { return over_shares(group_maxidx<THREADS>(m, red, redi, 0, tid), &slot[0], &islot, tid == 0, p.shares); },
       [&](auto g) {
         constexpr uint32_t STEP = THREADS * VEC;
-        if (VEC == 4 && p.bulk_out) {  // results over the cache, then out
-          const bool one_w = p.ws1 == 0 && p.ws2 == 0;  // gamma and beta belong to the line
-          const float w0 = p.w && one_w ? load_as_f32(p.w, wb, p.dt_w) : 1.f, b0 = p.b && one_w ? load_as_f32(p.b, wb, p.dt_w) : 0.f;
+        if constexpr (BULK) {  // results over the cache, then out (gamma and beta belong to the line)
+          const float w = p.w ? load_as_f32(p.w, wb, p.dt_w) : 1.f, b = p.b ? load_as_f32(p.b, wb, p.dt_w) : 0.f;
 #pragma unroll 2
           for (uint32_t r = begin + tid * VEC; r < end; r += STEP) {
-            F4 v = cached(r), wv, bv;
-            if (!one_w) {
-              const uint32_t r1 = p.R2 == p.R ? 0u : r / p.R2;
-              const int64_t wo = wb + r1 * p.ws1 + (r - r1 * p.R2) * p.ws2;
-              if (p.w) wv = weights(p.w, wo);
-              if (p.b) bv = weights(p.b, wo);
-            }
+            F4 v = cached(r);
 #pragma unroll
             for (int e = 0; e < VEC; ++e) {
-              const float x = g(v.v[e]), a = one_w ? w0 : wv.v[e], c = one_w ? b0 : bv.v[e];
-              v.v[e] = p.w && p.b ? fmaf(x, a, c) : p.w ? x * a : p.b ? x + c : x;
+              const float x = g(v.v[e]);
+              v.v[e] = p.w && p.b ? fmaf(x, w, b) : p.w ? x * w : p.b ? x + b : x;
             }
-            *reinterpret_cast<float4*>(cache + (r - begin)) = make_float4(v.v[0], v.v[VEC > 1 ? 1 : 0], v.v[VEC > 1 ? 2 : 0], v.v[VEC > 1 ? 3 : 0]);
+            *reinterpret_cast<float4*>(cache + (r - begin)) = make_float4(v.v[0], v.v[1], v.v[2], v.v[3]);
           }
           fence_proxy_async_smem();
           __syncthreads();
@@ -1173,8 +1167,10 @@ static int launch_share(K kernel, const ShareParams& p, int64_t blocks, int thre
 template <int OP, int THREADS>
 static int launch_share_op(int kind, const ShareParams& p, int64_t blocks, size_t smem, cudaStream_t st) {
   if (kind == 0) return launch_share(column_kernel<OP, THREADS>, p, blocks, THREADS, smem, st);
-  return kind == 4 ? launch_share(span_kernel<OP, 4, THREADS>, p, blocks, THREADS, smem, st)
-                   : launch_share(span_kernel<OP, 1, THREADS>, p, blocks, THREADS, smem, st);
+  if constexpr (OP != OP_SUM && OP != OP_MEAN && OP != OP_MAX)
+    if (p.bulk) return launch_share(span_kernel<OP, 4, THREADS, true>, p, blocks, THREADS, smem, st);
+  return kind == 4 ? launch_share(span_kernel<OP, 4, THREADS, false>, p, blocks, THREADS, smem, st)
+                   : launch_share(span_kernel<OP, 1, THREADS, false>, p, blocks, THREADS, smem, st);
 }
 template <int OP>
 static int launch_share_threads(int kind, const ShareParams& p, int64_t blocks, size_t smem, bool many, cudaStream_t st) {
@@ -1267,12 +1263,14 @@ static int launch_shared_line(int op, const LineParams& lp, const NdArgs& a, con
   p.share = share_of(shares);
   p.cached = keeps && static_cast<uint64_t>(p.share) * floats <= CACHE_FLOATS;
   const size_t smem = p.cached ? static_cast<size_t>(p.share) * floats * 4 : 0;
-  // Runs of 512 bytes and more, fp32: copied whole, all of a share at once, instead of 64 bytes a thread and trip.
-  const bool runs = kind == 4 && p.cached && (p.R2 == p.R || p.R2 >= 128);
-  p.bulk_in = runs && lp.dt_in == YTC_F32;
-  p.bulk_out = p.bulk_in && lp.dt_out == YTC_F32;
-  p.status = runs ? device_status_word() : nullptr;
-  if (!p.status) p.bulk_in = p.bulk_out = 0;
+  // Runs of 512 bytes and more, fp32, with one gamma and beta a line or none: copied whole, all of a share at once, instead of 64
+  // bytes a thread and trip. Registers / copies, calls back to back: batchNorm of 16 x 96 x 56 x 56 20.9 / 12.2 us, 256 channels of 512
+  // values 4.3 / 3.8. With gamma and beta inside the line (groupNorm) a second pass asks for them per element and the copies only wait
+  // one for the other: 32 x 256 x 14 x 14 in 8 groups 16.8 / 20.3. 16-bit shares have no such form, and keep the code without it: the
+  // two in one kernel cost them 5 to 9 %.
+  p.bulk = kind == 4 && p.cached && (p.R2 == p.R || p.R2 >= 128) && lp.dt_in == YTC_F32 && lp.dt_out == YTC_F32 &&
+           (!(lp.w || lp.b) || (p.ws1 == 0 && p.ws2 == 0));
+  if (p.bulk && !(p.status = device_status_word())) p.bulk = 0;
   // A share of which only one fits an SM needs more threads to keep enough loads in flight (batchNorm, bf16, 32 x 256 x 112 x
   // 112: 1617 us with 256 threads, 605 with 1024); where more fit, 256 are faster (16 x 96 x 56 x 56 fp32: 25 us, 37).
   const bool many = smem > 110 * 1024;
