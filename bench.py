@@ -639,7 +639,7 @@ def gemm32_arm(args) -> dict | None:
         "vs_baseline": None, "dtype": "f32 (three bf16 planes per operand, fp32 accumulate)", "data": "synthetic",
         "config": {"workload": "configs[0]: fp32 GEMM 1024 x 1024 x 1024", "l2": "flushed between steps (192 MB write)"},
         "roofline": {"bound": "tensor", "achieved": val, "peak": peak, "unit": "TFLOP/s", "frac": val / peak,
-                     "traffic": None, "kernel": "gemm_planes_kernel (one launch for both operands) + gemm_tc_kernel over six pairs of planes, k in pieces + gemm_sum_kernel, queued as dependent launches",
+                     "traffic": None, "kernel": "gemm_planes_kernel (one launch for both operands) + gemm_split_kernel over six pairs of planes, k shared by a cluster's CTAs, queued as dependent launches",
                      "peak_source": f"{peaks['source']} (burst cuBLAS bf16 / 6 partial products)",
                      "algorithmic_flops_per_launch": flops},
         "ffma_kernel": {"ms_per_step": res["ffma"][0], "tflops": flops / (res["ffma"][0] * 1e-3) / 1e12},

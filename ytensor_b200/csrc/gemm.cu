@@ -1308,9 +1308,10 @@ static int tc_cluster(int m, int n, int64_t fold, int64_t pairs, int64_t batch) 
   return 0;
 }
 // Pieces of k that fill the SMs when the tiles alone leave more than half of them idle; a piece keeps 512 / pairs of k. Not for
-// products of less than 6144 / pairs of k: their time is the caller's (30 us for a call of api.matmul, 0.35 us per block of 64 here),
-// and the launch that adds the pieces 2 to 4 us of it. Measured, bf16 16 x 4096 x k, one piece / pieces, calls one after the other:
-// k = 2048 30.5 / 32.7 us, 4096 30.5 / 32.9, 6144 34.8 / 33.0, 8192 45.1 / 33.4.
+// products of less than 6144 / pairs of k: they take a cluster's pieces, if any, need no scratch and no second launch, and stay below
+// the 16 us that a call of api.matmul takes by itself. One call behind the other from C, bf16, without / with pieces: 16 x 1024 x k,
+// k = 2048 10.4 / 8.0 us, 4096 12.4 / 7.9, 6144 14.4 / 8.7, 8192 16.5 / 8.5, 16384 22.6 / 11.1; 300 x 512 x 4096 12.4 / 9.9, x 6144
+// 14.4 / 10.9; 128 x 4096 x 6144 16.1 / 16.9.
 constexpr int SPLIT_MIN_BLOCKS = 96;
 static int tc_splits(int m, int n, int k, int pairs, int64_t batch) {
   const int k_blocks = (k + TC_BK - 1) / TC_BK;
@@ -1718,11 +1719,14 @@ static std::atomic<int> g_gemm_path{0};
 // 2 = whenever the shapes allow.
 static std::atomic<int> g_f32_split{0};
 
-// The FFMA kernel takes 0.17 to 0.22 us (fp32; 16 bit 0.25 to 0.36) per element of k and wave of 128 x 128 tiles, the less where the
-// left operand has few rows to load. The planes cost 19 us of launches, 10 bytes of traffic a value, six products a sixth of the
-// tensor rate, and 8 bytes per result and 256 of k for its partial sums. Measured (FFMA / planes, us): fp32 1 x 512 x 120 27.8 / 32.4,
-// x 180 34.9 / 32.9, 60 x 1001 x 120 34.9 / 32.5, 16 x 4096 x 4096 709 / 82, 777 x 1001 x 1111 227 / 47, 2000 x 4001 x 64 82 / 142, 2000 x
-// 2001 x 257 107 / 74; bf16 1 x 513 x 101 27.1 / 30.3, x 131 32.8 / 30.1, 60 x 1002 x 75 32.8 / 30.0, 777 x 1001 x 1111 340 / 30.
+// What FFMA and the planes take, as estimates: FFMA 0.17 to 0.22 us (fp32; 16 bit 0.25 to 0.36) per element of k and wave of 128 x 128
+// tiles, the less where the left operand has few rows to load; the planes 19 us of launches, 10 bytes of traffic a value, six products a
+// sixth of the tensor rate, and 8 bytes per result and 256 of k for their partial sums. The callers ask for a ratio of 1.5, and the
+// estimate of the planes is high by up to 10 us for small operands since the products behind them became shorter, so the line lies on
+// FFMA's side: what is near it keeps FFMA's sums and needs no scratch. One call behind the other, FFMA / planes, us, * on FFMA's side:
+// fp32 1 x 512 x 60 14.5 / 13.1 *, x 120 26.7 / 14.4 *, x 180 37.0 / 16.5, 60 x 1001 x 60 24.6 / 21.8 *, x 120 36.9 / 22.8 *, x 180
+// 47.2 / 28.8, 16 x 4096 x 120 34.9 / 16.5 *, x 180 47.1 / 18.5, 2000 x 500 x 180 61.5 / 22.6 *, x 257 75.9 / 28.8, 777 x 1001 x 777
+// 168 / 38; bf16 1 x 513 x 101 26.7 / 8.2 *, x 131 32.9 / 8.2, 60 x 1002 x 75 32.8 / 13.9 *, x 101 41.0 / 14.1, 777 x 1001 x 501 172 / 28.
 static double simt_us(int m, int n, int k, int64_t batch, bool wide) {
   const int64_t tiles = static_cast<int64_t>((m + SM_BM - 1) / SM_BM) * ((n + SM_BN - 1) / SM_BN) * batch;
   const double each = wide ? (m < 16 ? 0.17 : 0.22) : (m < 16 ? 0.25 : 0.36);
