@@ -1348,7 +1348,14 @@ static int launch_tc(int dtype_in, int dtype_out, const void* A, const void* B, 
   // stored and the layers behind carry it on, so a token's logits would depend on how many tokens its prompt has. (500 tokens through
   // 12 Derupel layers: 0.11 ms more than with shared k, and the same bits in any company.)
   const bool one_sum = ex && !ex->add_in_memory;
-  const int cluster = grouped || pair || splits > 1 || one_sum ? 0 : tc_cluster(m, n, (k + TC_BK - 1) / TC_BK, pl ? pl->pairs : 1, batch);
+  const int esz = dtype_size(dtype_out);
+  const int64_t items = batch * splits;
+  const bool rows16 = csc == 1 && rsc > 0 && (reinterpret_cast<uint64_t>(C) & 15u) == 0 && rsc * esz % 16 == 0 &&
+                      rsc * esz < (int64_t{1} << 40) && (items == 1 || (bsc > 0 && bsc * esz % 16 == 0 && bsc * esz < (int64_t{1} << 40)));
+  // (and where C's rows don't start at 16 bytes the exchange leaves half of the warps to store element by element what all of them
+  // would have: fp32 60 x 1001 x 180, 18 blocks, 27.7 us without, 29.8 with it)
+  const int64_t k64 = (k + TC_BK - 1) / TC_BK, n_pairs = pl ? pl->pairs : 1;
+  const int cluster = grouped || pair || splits > 1 || one_sum || (!rows16 && k64 * n_pairs < 32) ? 0 : tc_cluster(m, n, k64, n_pairs, batch);
   if (splits > 1 && (ex || g_mask.kind != 0 || splits > (k + TC_BK - 1) / TC_BK)) {
     set_last_error("ytcuda_gemm: %d pieces of k = %d do not go with an epilogue or a mask", splits, k);
     return YTC_UNSUPPORTED;
@@ -1420,10 +1427,6 @@ static int launch_tc(int dtype_in, int dtype_out, const void* A, const void* B, 
   // C through TMA stores: rows (and batch items, pieces of k) that start at 16 bytes. What C holds already is added there only
   // where the caller leaves that to the memory's adders (IEEE sums like an epilogue's, subnormal numbers kept: 1024 sums of such
   // operands the same bits as the host's; the epilogue's own reads of C cost a prompt of 2000 tokens 1.6 %).
-  const int esz = dtype_size(dtype_out);
-  const int64_t items = batch * splits;
-  const bool rows16 = csc == 1 && rsc > 0 && (reinterpret_cast<uint64_t>(C) & 15u) == 0 && rsc * esz % 16 == 0 &&
-                      rsc * esz < (int64_t{1} << 40) && (items == 1 || (bsc > 0 && bsc * esz % 16 == 0 && bsc * esz < (int64_t{1} << 40)));
   p.tma_out = !rows16 ? 0 : beta == 0.f ? 1 : e->add_in_memory && beta == 1.f && alpha == 1.f && dtype_out == YTC_F32 ? 2 : 0;
   CUtensorMap tmC{};
   if (p.tma_out) {
