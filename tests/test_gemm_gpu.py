@@ -563,6 +563,25 @@ def test_threads_share_a_stream(api):
     assert not torch.stack(bad).any()
 
 
+@pytest.mark.parametrize("b,m,n,k", [(1, 60, 1001, 180), (1, 777, 1001, 200), (3, 130, 203, 255), (1, 1, 1999, 256), (1, 200, 1501, 181)])
+def test_odd_rows_of_one_piece_are_copied_into_place(L, api, b, m, n, k):
+    """fp32 products of at most 256 of k whose C has rows off 16 bytes go through partial sums of one piece: 64-bit reference, an infinity
+    and a NaN where FFMA answers, C inside a larger tensor, and nothing outside C. fp32 sums of 256 products: the file's tolerance."""
+    g = torch.Generator(device="cuda").manual_seed(m + k)
+    a, w = torch.randn(b, m, k, generator=g, device="cuda"), torch.randn(k, n, generator=g, device="cuda")
+    whole = torch.full((b, m, n + 3), 7.0, device="cuda")
+    api.matmul(a, w, whole[:, :, 1:n + 1])
+    assert normwise(whole[:, :, 1:n + 1].double().cpu().numpy(), (a.double() @ w.double()).cpu().numpy()) < F32_TOL
+    assert bool((whole[:, :, 0] == 7).all()) and bool((whole[:, :, n + 1:] == 7).all())
+    a[0, m // 2, 3] = float("inf") if m > 1 else 1.0
+    w[k - 1, n // 2] = float("nan")
+    got, want = api.matmul(a, w), a.double() @ w.double()
+    assert torch.equal(got.isnan(), want.isnan()) and torch.equal(got.isinf(), want.isinf())
+    fine = want.isfinite()
+    assert float((got.double() - want)[fine].abs().max()) < F32_TOL * float(want[fine].abs().max())
+    status_ok(L)
+
+
 @pytest.mark.parametrize("out_dtype", [torch.float32, torch.bfloat16, torch.float16])
 @pytest.mark.parametrize("b,m,n,k", [(1, 1, 8, 72), (1, 33, 24, 64), (3, 127, 136, 200), (1, 129, 264, 72), (2, 160, 520, 136),
                                      (1, 4097, 1032, 264), (2, 2304, 1288, 256)])

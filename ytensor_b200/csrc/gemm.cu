@@ -1348,14 +1348,7 @@ static int launch_tc(int dtype_in, int dtype_out, const void* A, const void* B, 
   // stored and the layers behind carry it on, so a token's logits would depend on how many tokens its prompt has. (500 tokens through
   // 12 Derupel layers: 0.11 ms more than with shared k, and the same bits in any company.)
   const bool one_sum = ex && !ex->add_in_memory;
-  const int esz = dtype_size(dtype_out);
-  const int64_t items = batch * splits;
-  const bool rows16 = csc == 1 && rsc > 0 && (reinterpret_cast<uint64_t>(C) & 15u) == 0 && rsc * esz % 16 == 0 &&
-                      rsc * esz < (int64_t{1} << 40) && (items == 1 || (bsc > 0 && bsc * esz % 16 == 0 && bsc * esz < (int64_t{1} << 40)));
-  // (and where C's rows don't start at 16 bytes the exchange leaves half of the warps to store element by element what all of them
-  // would have: fp32 60 x 1001 x 180, 18 blocks, 27.7 us without, 29.8 with it)
-  const int64_t k64 = (k + TC_BK - 1) / TC_BK, n_pairs = pl ? pl->pairs : 1;
-  const int cluster = grouped || pair || splits > 1 || one_sum || (!rows16 && k64 * n_pairs < 32) ? 0 : tc_cluster(m, n, k64, n_pairs, batch);
+  const int cluster = grouped || pair || splits > 1 || one_sum ? 0 : tc_cluster(m, n, (k + TC_BK - 1) / TC_BK, pl ? pl->pairs : 1, batch);
   if (splits > 1 && (ex || g_mask.kind != 0 || splits > (k + TC_BK - 1) / TC_BK)) {
     set_last_error("ytcuda_gemm: %d pieces of k = %d do not go with an epilogue or a mask", splits, k);
     return YTC_UNSUPPORTED;
@@ -1427,6 +1420,10 @@ static int launch_tc(int dtype_in, int dtype_out, const void* A, const void* B, 
   // C through TMA stores: rows (and batch items, pieces of k) that start at 16 bytes. What C holds already is added there only
   // where the caller leaves that to the memory's adders (IEEE sums like an epilogue's, subnormal numbers kept: 1024 sums of such
   // operands the same bits as the host's; the epilogue's own reads of C cost a prompt of 2000 tokens 1.6 %).
+  const int esz = dtype_size(dtype_out);
+  const int64_t items = batch * splits;
+  const bool rows16 = csc == 1 && rsc > 0 && (reinterpret_cast<uint64_t>(C) & 15u) == 0 && rsc * esz % 16 == 0 &&
+                      rsc * esz < (int64_t{1} << 40) && (items == 1 || (bsc > 0 && bsc * esz % 16 == 0 && bsc * esz < (int64_t{1} << 40)));
   p.tma_out = !rows16 ? 0 : beta == 0.f ? 1 : e->add_in_memory && beta == 1.f && alpha == 1.f && dtype_out == YTC_F32 ? 2 : 0;
   CUtensorMap tmC{};
   if (p.tma_out) {
@@ -1727,8 +1724,8 @@ static std::atomic<int> g_f32_split{0};
 // sixth of the tensor rate, and 8 bytes per result and 256 of k for their partial sums. The callers ask for a ratio of 1.5, and the
 // estimate of the planes is high by up to 10 us for small operands since the products behind them became shorter, so the line lies on
 // FFMA's side: what is near it keeps FFMA's sums and needs no scratch. One call behind the other, FFMA / planes, us, * on FFMA's side:
-// fp32 1 x 512 x 60 14.5 / 13.1 *, x 120 26.7 / 14.4 *, x 180 37.0 / 16.5, 60 x 1001 x 60 24.6 / 21.8 *, x 120 36.9 / 22.8 *, x 180
-// 47.2 / 28.8, 16 x 4096 x 120 34.9 / 16.5 *, x 180 47.1 / 18.5, 2000 x 500 x 180 61.5 / 22.6 *, x 257 75.9 / 28.8, 777 x 1001 x 777
+// fp32 1 x 512 x 60 14.5 / 13.1 *, x 120 26.7 / 14.4 *, x 180 37.0 / 16.5, 60 x 1001 x 180
+// 47.2 / 18.5, 16 x 4096 x 120 34.9 / 16.5 *, x 180 47.1 / 18.5, 2000 x 500 x 180 61.5 / 22.6 *, x 257 75.9 / 28.8, 777 x 1001 x 777
 // 168 / 38; bf16 1 x 513 x 101 26.7 / 8.2 *, x 131 32.9 / 8.2, 60 x 1002 x 75 32.8 / 13.9 *, x 101 41.0 / 14.1, 777 x 1001 x 501 172 / 28.
 static double simt_us(int m, int n, int k, int64_t batch, bool wide) {
   const int64_t tiles = static_cast<int64_t>((m + SM_BM - 1) / SM_BM) * ((n + SM_BN - 1) / SM_BN) * batch;
@@ -1827,9 +1824,10 @@ static int launch_planes(const void* A, const void* B, void* C, int dtype_out, i
     splits = side < 1 ? 1 : static_cast<int>(side);
     if (splits < pieces) window = splits * PIECE;
   }
-  // C itself takes the sums: of one window, and of several where its rows start at 16 bytes
+  // C itself takes the sums where its rows start at 16 bytes. Elsewhere its elements would be stored one by one (777 x 1001 x 200: 34.9 us,
+  // 22.7 through partial sums; 60 x 1001 x 180 29.8, 18.5), which is left to a C that is larger than the room for them, and to products without FFMA behind them.
   const bool rows16 = csc == 1 && rsc % 4 == 0 && (batch == 1 || bsc % 4 == 0) && (reinterpret_cast<uint64_t>(C) & 15) == 0;
-  const bool direct = splits == 1 && (rows16 || window == k);
+  const bool direct = splits == 1 && (rows16 || (window == k && !(check && chunk * mn * 4 <= PART_ROOM)));
   auto up = [](int64_t v) { return static_cast<size_t>((v + 255) / 256 * 256); };
   // CTAs (and words of the gate) of either operand: those of the first, largest rewriting
   const PlaneOp largest_a = a_op(0, a_shared ? 1 : chunk, 0, window), largest_b = b_op(0, b_shared ? 1 : chunk, 0, window);
